@@ -341,3 +341,82 @@ def tolerance(case):
         return {"rel": 2e-2, "max": 0.1}
     # 16-bit P and dS [bf16 2.6e-3, 5.3e-2; fp16 3e-4, 1.4e-3]; the score and the LSE are fp32 [2e-6]
     return {"rel": 1e-2, "max": 0.2} if dtype == "bf16" else {"rel": 1.2e-3, "max": 6e-3}
+
+
+# ------------------------------------------------------------------------------------------------------------------------
+# the same outputs in 64 bits
+# ------------------------------------------------------------------------------------------------------------------------
+def _exact_head(c, q, k, v, grad=None):
+    """One (batch, query head): O, LSE, the column sums of P and, with ``grad``, dQ, dK, dV."""
+    s = (q @ k.T) / math.sqrt(c["D"])
+    if c["causal"]:
+        Sq, Skv = s.shape
+        s.masked_fill_(torch.ones(Sq, Skv, dtype=torch.bool, device=s.device).triu_(Skv - Sq + 1), float("-inf"))
+    lse = torch.logsumexp(s, -1)
+    p = torch.exp(s - lse[:, None])
+    out = p @ v
+    r = dict(out=out, lse=lse, score=p.sum(0))
+    if grad is not None:
+        ds = p * (grad @ v.T - (grad * out).sum(-1, keepdim=True)) / math.sqrt(c["D"])
+        r.update(dq=ds @ k, dk=ds.T @ q, dv=p.T @ grad)
+    return r
+
+
+def _exact_attention(c, state):
+    b_h_s_d = (lambda t: t.transpose(1, 2)) if c.get("layout") == "bshd" else (lambda t: t)
+    q, k, v = (b_h_s_d(state[n]) for n in "qkv")
+    grad = b_h_s_d(state["grad"]) if "grad" in state else None
+    scales = state.get("scales", (1.0, 1.0, 1.0))
+    f64 = dict(dtype=torch.float64, device=q.device)
+    B, Hq, Hkv, group = c["B"], c["Hq"], c["Hkv"], c["Hq"] // c["Hkv"]
+    full = dict(out=torch.empty(q.shape, **f64), lse=torch.empty(q.shape[:3], **f64), score=torch.empty(B, Hq, c["Skv"], **f64))
+    if grad is not None:
+        full.update(dq=torch.empty(q.shape, **f64), dk=torch.zeros(k.shape, **f64), dv=torch.zeros(v.shape, **f64))
+    for b in range(B):
+        for h in range(Hkv):
+            kh, vh = k[b, h].double() * scales[1], v[b, h].double() * scales[2]
+            for g in range(h * group, (h + 1) * group):
+                r = _exact_head(c, q[b, g].double() * scales[0], kh, vh, None if grad is None else grad[b, g].double())
+                for name, t in r.items():
+                    if name in ("dk", "dv"):
+                        full[name][b, h] += t
+                    else:
+                        full[name][b, g] = t
+    out = {n: b_h_s_d(t) if t.dim() == 4 else t for n, t in full.items()}
+    if c["kind"] == "train":
+        return {n: out[n] for n in ("out", "lse", "dq", "dk", "dv")}
+    if c["kind"] == "h2o":
+        return out["out"], out["score"]
+    return (out["out"], out["lse"]) if c["lse"] else out["out"]
+
+
+def exact(case, seed):
+    c, state = case, prepare(case, seed)
+    if c["kind"] in ("attention", "train", "h2o"):
+        return _exact_attention(c, state)
+    if c["kind"] == "linear":
+        y = state["x"].double() @ state["w"].double().T
+        if c["row_scale"]:
+            y = y * state["row_scale_t"].double()[:, None]
+        if c["bias"]:
+            y = y + state["bias_t"].double()
+        if c["epilogue"] == "swiglu":
+            gate, up = y.chunk(2, -1)
+            y = torch.nn.functional.silu(gate) * up
+        elif c["epilogue"] == "silu":
+            y = torch.nn.functional.silu(y)
+        elif c["epilogue"] == "gelu_tanh":
+            y = torch.nn.functional.gelu(y, approximate="tanh")
+        return y + state["residual_t"].double() if c["residual"] else y
+    if c["kind"] == "bmm":
+        return torch.stack([a.double() @ b.double() for a, b in zip(state["a"], state["b"])])
+    if c["kind"] == "rowwise":
+        x = [t.double() for t in state["inputs"]]
+        if c["program"] == "softmax":
+            return torch.softmax(0.125 * x[0], -1)
+        if c["program"] == "silu_mul":
+            return torch.nn.functional.silu(x[0]) * x[1]
+        x = x[0] - x[0].mean(-1, keepdim=True)
+        return x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-5)
+    layer = state["layer"]._orig_mod.double()
+    return torch.cat([layer(x[None].double()) for x in state["x"]])
