@@ -142,7 +142,7 @@ ROWWISE_AUTO, ROWWISE_INTERPRET, ROWWISE_COMPILED = 0, 1, 2
 
 # every symbol include/heddle_b200.h declares
 EXPORTS = (
-    "hb_fa_fwd", "hb_fa_fwd_noalloc", "hb_status_word_noalloc", "hb_fa_bwd_preprocess", "hb_fa_bwd_dkdv", "hb_fa_bwd_dq", "hb_h2o_score", "hb_gemm_epilogue", "hb_rms_rowstat", "hb_prepare_weight", "hb_row_softmax", "hb_rowwise_program", "hb_rowwise_compiler_available", "hb_debug_rowwise_compile", "hb_status_word",
+    "hb_fa_fwd", "hb_fa_fwd_workspace", "hb_fa_fwd_ws", "hb_fa_fwd_noalloc", "hb_status_word_noalloc", "hb_fa_bwd_preprocess", "hb_fa_bwd_dkdv", "hb_fa_bwd_dq", "hb_h2o_score", "hb_gemm_epilogue", "hb_rms_rowstat", "hb_prepare_weight", "hb_row_softmax", "hb_rowwise_program", "hb_rowwise_compiler_available", "hb_debug_rowwise_compile", "hb_status_word",
     "hb_version",
     "hb_query", "hb_last_error", "hb_shutdown", "hb_debug_umma", "hb_debug_wait_timeout", "hb_debug_fa_fwd_stages",
 )
@@ -163,6 +163,10 @@ def load() -> C.CDLL:
     lib = C.CDLL(str(path))
     lib.hb_fa_fwd.argtypes = [C.POINTER(FaArgs)]
     lib.hb_fa_fwd.restype = C.c_int
+    lib.hb_fa_fwd_workspace.argtypes = [C.POINTER(FaArgs), C.POINTER(C.c_uint64)]
+    lib.hb_fa_fwd_workspace.restype = C.c_int
+    lib.hb_fa_fwd_ws.argtypes = [C.POINTER(FaArgs), C.c_void_p, C.c_uint64]
+    lib.hb_fa_fwd_ws.restype = C.c_int
     lib.hb_fa_fwd_noalloc.argtypes = [C.POINTER(FaArgs)]
     lib.hb_fa_fwd_noalloc.restype = C.c_int
     for name in ("hb_fa_bwd_preprocess", "hb_fa_bwd_dkdv", "hb_fa_bwd_dq"):

@@ -4,6 +4,7 @@
 #include "fa_fwd_sm100.cuh"
 
 #include <cstdlib>
+#include "fa_split.h"
 #include "host_common.h"
 
 #include <algorithm>
@@ -179,15 +180,30 @@ static int fa_fill_params(const hb_fa_args* a, const char* who, uint32_t* status
   return HB_OK;
 }
 
-static int fa_fwd_impl(const hb_fa_args* a) {
+static int fa_fwd_workspace_impl(const hb_fa_args* a, uint64_t* bytes) {
+  if (bytes == nullptr) return set_error(HB_ERR_BAD_ARG, "hb_fa_fwd_workspace: bytes is NULL");
+  *bytes = 0;
   bool empty = false;
-  int rc = fa_validate(a, "hb_fa_fwd", /*allow_fp8=*/true, &empty);
+  int rc = fa_validate(a, "hb_fa_fwd_workspace", /*allow_fp8=*/true, &empty);
+  if (rc != HB_OK || empty || !fa_split_takes(a)) return rc;
+  DeviceState* st = nullptr;
+  rc = get_device_state(&st);
+  if (rc != HB_OK) return rc;
+  *bytes = fa_split_workspace(a, st->sm_count);
+  return HB_OK;
+}
+
+// `ws` selects hb_fa_fwd_ws: calls with few query rows go to the split-key kernel.
+static int fa_fwd_impl(const hb_fa_args* a, const char* who, bool ws, void* workspace, uint64_t workspace_bytes) {
+  bool empty = false;
+  int rc = fa_validate(a, who, /*allow_fp8=*/true, &empty);
   if (rc != HB_OK || empty) return rc;
   DeviceState* st = nullptr;
   rc = get_device_state(&st);
   if (rc != HB_OK) return rc;
+  if (ws && fa_split_takes(a)) return fa_split_run(a, st, workspace, workspace_bytes);
   FaParams p;
-  rc = fa_fill_params(a, "hb_fa_fwd", st->status_word, &p);
+  rc = fa_fill_params(a, who, st->status_word, &p);
   if (rc != HB_OK) return rc;
   int grid = std::min(p.total_pairs, st->sm_count);
 #ifdef HB_DEBUG_GRID_ENV  // measurement builds only: fewer CTAs than SMs, to see how the per-SM rate depends on the load on L2
@@ -458,7 +474,17 @@ extern "C" {
 
 int hb_fa_fwd(const hb_fa_args* args) {
   hb::clear_error();
-  return hb::fa_fwd_impl(args);
+  return hb::fa_fwd_impl(args, "hb_fa_fwd", false, nullptr, 0);
+}
+
+int hb_fa_fwd_workspace(const hb_fa_args* args, uint64_t* bytes) {
+  hb::clear_error();
+  return hb::fa_fwd_workspace_impl(args, bytes);
+}
+
+int hb_fa_fwd_ws(const hb_fa_args* args, void* workspace, uint64_t bytes) {
+  hb::clear_error();
+  return hb::fa_fwd_impl(args, "hb_fa_fwd_ws", true, workspace, bytes);
 }
 
 #ifdef HB_FA_TRACE

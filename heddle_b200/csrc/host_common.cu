@@ -29,9 +29,10 @@ const char* describe_status(uint32_t word) {
     const uint32_t role = word & 0xffu;
     const char* kernel = role < 0x20 ? "attention forward" : role < 0x30 ? "GEMM" : role < 0x40 ? "H2O score"
                          : role < 0x50 ? "attention backward" : "probe";
-    static const char* const kFa[] = {"?", "softmax", "correction", "MMA issuer", "TMA producer", "drain"};
+    static const char* const kFa[] = {"?", "softmax", "correction", "MMA issuer", "TMA producer", "drain",
+                                      "split softmax", "split MMA issuer", "split TMA producer", "split drain"};
     static const char* const kOther[] = {"?", "TMA producer", "MMA issuer", "consumer", "drain"};
-    const char* name = role < 6 ? kFa[role] : ((role & 0xfu) < 5 && role < 0x50) ? kOther[role & 0xfu] : "?";
+    const char* name = role < 10 ? kFa[role] : ((role & 0xfu) < 5 && role < 0x50) ? kOther[role & 0xfu] : "?";
     snprintf(buf, sizeof(buf),
              "status word 0x%x: a bounded wait of the %s kernel gave up (role 0x%x, %s); that launch's outputs are incomplete",
              word, kernel, role, name);

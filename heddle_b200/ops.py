@@ -35,6 +35,9 @@ def _inner_contiguous(t: torch.Tensor) -> torch.Tensor:
     return t if t.stride(-1) == 1 else t.contiguous()
 
 
+_FA_SPLIT_MAX_ROWS = 128  # calls with more query rows never need a workspace (hb_fa_fwd_workspace)
+
+
 def fa_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal: bool = False,
            softmax_scale: Optional[float] = None, layout: str = "bhsd", return_lse: bool = False,
            out: Optional[torch.Tensor] = None,
@@ -91,7 +94,12 @@ def fa_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal: bool = 
         a.q_scale, a.k_scale, a.v_scale = (float(x) for x in scales)
     a.stream = _stream_ptr(q.device)
     with torch.cuda.device(q.device):
-        if debug_stages is None:
+        if debug_stages is None and Sq <= _FA_SPLIT_MAX_ROWS:
+            need = C.c_uint64(0)
+            _lib.check(_lib.load().hb_fa_fwd_workspace(C.byref(a), C.byref(need)))
+            ws = torch.empty(need.value, dtype=torch.uint8, device=q.device) if need.value else None
+            _lib.check(_lib.load().hb_fa_fwd_ws(C.byref(a), ws.data_ptr() if ws is not None else None, need.value))
+        elif debug_stages is None:
             _lib.check(_lib.load().hb_fa_fwd(C.byref(a)))
         else:
             _lib.check(_lib.load().hb_debug_fa_fwd_stages(C.byref(a), int(debug_stages)))

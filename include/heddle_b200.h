@@ -94,6 +94,15 @@ typedef struct hb_fa_args {
 int hb_fa_fwd(const hb_fa_args* args);
 
 /*
+ * hb_fa_fwd with a device workspace of the caller's.  With few query rows (decode, short prompts against a long cache) the
+ * keys of one (batch, KV head) are then walked by several SMs whose partial results meet in the workspace; other calls run
+ * exactly as through hb_fa_fwd.  hb_fa_fwd_workspace writes the bytes a call needs (0: none, workspace may be NULL).  The
+ * workspace must be 16-byte aligned, need not be initialised and may be reused once the call's work on `stream` is done.
+ */
+int hb_fa_fwd_workspace(const hb_fa_args* args, uint64_t* bytes);
+int hb_fa_fwd_ws(const hb_fa_args* args, void* workspace, uint64_t bytes);
+
+/*
  * hb_fa_fwd for callers that cannot allocate device memory.  No counterpart in the
  * reference (its kernels and their buffers are created by TileLang's JIT at run time).
  *
