@@ -98,7 +98,7 @@ class GemmArgs(C.Structure):
     ]
 
 
-GEMM_SCHEDULES = {"auto": 0, "single": 1, "pair": 2}
+GEMM_SCHEDULES = {"auto": 0, "single": 1, "pair": 2, "split": 3}
 
 
 class PrepareArgs(C.Structure):

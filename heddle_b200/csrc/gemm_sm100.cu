@@ -1,9 +1,10 @@
 // hb_gemm_epilogue / hb_rms_rowstat: validation, TMA descriptors and launch.
-#include "gemm_sm100.cuh"
+#include "gemm_split_sm100.cuh"
 #include "host_common.h"
 
 #include <algorithm>
 #include <cstdlib>
+#include <mutex>
 
 namespace hb {
 
@@ -61,6 +62,119 @@ static int dispatch_gemm(int epi_class, const GemmParams& p, int grid, bool pair
   }
 }
 
+// ---- the split-K kernel: which tile width and cluster size, and whether it is the one to run ----
+
+// CTAs of gemm_split_kernel that run at one time in clusters of `splits`, per device (the GPCs of the part do not hold a whole
+// number of clusters of every size).
+constexpr int kMaxSplits = 8;
+static int gemm_split_slots(const DeviceState* st, int splits) {
+  static int slots[64][kMaxSplits + 1] = {};
+  static std::mutex mutex;
+  std::lock_guard<std::mutex> lock(mutex);
+  int& n = slots[st->device & 63][splits];
+  if (n == 0) {
+    auto kernel = gemm_split_kernel<__nv_bfloat16, kEpiPlain>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(splits * st->sm_count));
+    cfg.blockDim = dim3(kGemmSplitThreads);
+    cfg.dynamicSmemBytes = kGemmSplitSmemBytes;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)splits;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSplitSmemBytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters <= 0) {
+      (void)cudaGetLastError();
+      clusters = st->sm_count / (2 * splits) > 0 ? st->sm_count / (2 * splits) : 1;
+    }
+    n = clusters * splits;
+  }
+  return n;
+}
+
+// Estimated time (ns) of one launch, fitted to a sweep of widths 64 .. 256 and clusters 1 .. 8 on 24 .. 256 x 4096 .. 22016 x
+// 4096 .. 11008 (within 10 %): an SM streams weights from HBM at 60 B/ns and all operands at 120; a 128 x 256 x 64 slab takes
+// 270 ns on the tensor cores, and never less than the 125 ns its four MMAs take to issue; HBM gives 6 KB/ns and L2 14 KB/ns in
+// all; a wave costs 5 us for its start, its first load and its stores, 450 ns more per CTA of a cluster, and 100 ns per 1000
+// accumulators read back.
+struct GemmSplitChoice {
+  int width = 0, splits = 0, slabs = 0;
+  double ns = 0.0;
+};
+
+// K slabs per stage: about 40 KB, so that four or more stages fit the ring
+static int gemm_split_slabs(int a_rows, int width, int k_steps, bool whole_slabs) {
+  if (!whole_slabs) return 1;
+  return std::max(1, std::min({4, k_steps, 40 * 1024 / ((a_rows + width) * 128)}));
+}
+
+static GemmSplitChoice gemm_split_choose(const DeviceState* st, int epi_class, int M, int n_out, int k_steps, bool whole_slabs,
+                                         int batch, int head_dim, bool w_kn) {
+  GemmSplitChoice best;
+  int slots[kMaxSplits + 1];
+  for (int splits = 1; splits <= kMaxSplits; ++splits) slots[splits] = gemm_split_slots(st, splits);
+  const int tiles_m = (M + kGemmBM - 1) / kGemmBM;
+  const int a_rows = tiles_m > 1 ? kGemmBM : (M + 7) / 8 * 8;
+  const int unit = epi_class == kEpiRope ? head_dim : w_kn ? 64 : 16;
+  const int per_col = epi_class == kEpiSwiglu ? 2 : 1;  // accumulator columns per output column
+  const double hbm = 128.0 * k_steps * batch * ((double)n_out * per_col + M) / 6000.0;
+  for (int width = unit; width <= kGemmBN; width += unit) {
+    const long long tiles = (long long)tiles_m * ((n_out * per_col + width - 1) / width) * batch;
+    const double slab = std::max({width * 128.0 / 60.0, (width + a_rows) * 128.0 / 120.0, width * (270.0 / 256.0), 125.0});
+    const int slabs = gemm_split_slabs(a_rows, width, k_steps, whole_slabs), stages = (k_steps + slabs - 1) / slabs;
+    for (int splits = 1; splits <= std::min(kMaxSplits, stages); ++splits) {
+      const long long waves = (tiles * splits + slots[splits] - 1) / slots[splits];
+      const double l2 = 128.0 * (width + a_rows) * tiles * (double)k_steps / 14000.0;
+      const double fixed = 5000.0 + (splits > 1 ? 450.0 * splits : 0.0) + std::min(M, kGemmBM) * (double)width / 10.0;
+      const double ns = std::max({hbm, l2, waves * (slab * slabs * ((stages + splits - 1) / splits))}) + waves * fixed;
+      if (best.width == 0 || ns < best.ns) best = {width, splits, slabs, ns};
+    }
+    if (tiles > 4ll * st->sm_count && width >= 128) break;  // wider tiles only leave fewer of them
+  }
+  return best;
+}
+
+template <typename T, int EPI>
+static int launch_gemm_split(const GemmSplitParams& p, int grid, const DeviceState* st, cudaStream_t stream) {
+  if (kGemmSplitSmemBytes > st->smem_optin)
+    return set_error(HB_ERR_UNSUPPORTED, "hb_gemm_epilogue: kernel needs %d bytes of shared memory, device offers %d",
+                     kGemmSplitSmemBytes, st->smem_optin);
+  auto kernel = gemm_split_kernel<T, EPI>;
+  static bool configured[64] = {};
+  if (!configured[st->device & 63]) {
+    HB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSplitSmemBytes));
+    configured[st->device & 63] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(kGemmSplitThreads);
+  cfg.dynamicSmemBytes = kGemmSplitSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)p.splits;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  HB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, p));
+  return HB_OK;
+}
+
+template <typename T>
+static int dispatch_gemm_split(int epi_class, const GemmSplitParams& p, int grid, const DeviceState* st, cudaStream_t stream) {
+  switch (epi_class) {
+    case kEpiPlain:
+      return launch_gemm_split<T, kEpiPlain>(p, grid, st, stream);
+    case kEpiSwiglu:
+      return launch_gemm_split<T, kEpiSwiglu>(p, grid, st, stream);
+    default:
+      return launch_gemm_split<T, kEpiRope>(p, grid, st, stream);
+  }
+}
+
 static bool aligned16(const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; }
 
 static int gemm_impl(const hb_gemm_args* a) {
@@ -88,7 +202,7 @@ static int gemm_impl(const hb_gemm_args* a) {
     if ((reinterpret_cast<uintptr_t>(a->rope_cos) & 15) != 0 || (reinterpret_cast<uintptr_t>(a->rope_sin) & 15) != 0)
       return set_error(HB_ERR_ALIGN, "hb_gemm_epilogue: ROPE tables need 16-byte alignment");
   }
-  if (a->schedule < HB_GEMM_AUTO || a->schedule > HB_GEMM_PAIR)
+  if (a->schedule < HB_GEMM_AUTO || a->schedule > HB_GEMM_SPLIT)
     return set_error(HB_ERR_BAD_ARG, "hb_gemm_epilogue: unknown schedule %d", a->schedule);
   const int batch = a->batch > 0 ? a->batch : 1;
   const bool w_kn = a->w_layout == HB_W_KN;
@@ -121,17 +235,65 @@ static int gemm_impl(const hb_gemm_args* a) {
   int rc = get_device_state(&st);
   if (rc != HB_OK) return rc;
 
-  GemmParams p;
-  memset(&p, 0, sizeof(p));
+  // Which kernel.  The persistent kernels (CTA pairs when a problem has more than one 128-row tile of rows, else single CTAs)
+  // win once their 256-column tiles fill the chip; with fewer than two rounds of them (eight, for a single row of tiles, which
+  // is bound by the weights) the split-K kernel runs where its estimate is the smaller one.  Theirs: 546 ns (single CTA, weights
+  // from HBM) or 290 ns (pair) a 64-wide slab of a tile, 3.5 us a round and 3 us once.  Both sides measured, us, split-K | the
+  // persistent kernel: 24 x 22016 x 4096 33 | 42; 120 x 4096 x 11008 25 | 67; 120 x 12288 x 4096 30 | 40; 1 x 4096 x 4096
+  // 11 | 28; 64 x 50000 x 4096 75 | 83; 256 x 4096 x 4096 17 | 25; 512 x 4096 x 4096 23 | 26; 1000 x 4096 x 4096 31 | 28; 256 x 22016 x 4096 61 | 56.
+  const int k_steps = (a->K + kGemmBK - 1) / kGemmBK;
+  const bool one_row = a->M <= kGemmBM;
+  const long long wide_tiles = (long long)((a->M + (one_row ? kGemmBM : kPairBM) - 1) / (one_row ? kGemmBM : kPairBM)) *
+                               ((a->N + kGemmBN - 1) / kGemmBN) * batch;
+  const int wide_slots = one_row ? st->sm_count : std::max(1, st->sm_count / 2);
+  GemmSplitChoice split;
+  if (a->schedule == HB_GEMM_SPLIT || (a->schedule == HB_GEMM_AUTO && wide_tiles < (one_row ? 8ll : 2ll) * wide_slots)) {
+    split = gemm_split_choose(st, epi_class, a->M, n_out, k_steps, a->K % kGemmBK == 0, batch, a->head_dim, w_kn);
+    const double wide_ns = (double)((wide_tiles + wide_slots - 1) / wide_slots) * (k_steps * (one_row ? 546.0 : 290.0) + 3500.0) + 3000.0;
+    if (a->schedule == HB_GEMM_AUTO && split.ns >= wide_ns) split = GemmSplitChoice();
+  }
+  const bool use_split = split.width > 0;
+
+  GemmSplitParams sp;
+  memset(&sp, 0, sizeof(sp));
+  GemmParams& p = sp.g;
   const CUtensorMapDataType dt = a->dtype == HB_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  {
+  if (use_split) {
+    sp.a_rows = a->M > kGemmBM ? kGemmBM : (a->M + 7) / 8 * 8;
+    sp.slabs = split.slabs;
+    sp.k_slabs = a->K % kGemmBK == 0 ? 1 : 0;
+    const uint64_t k_in = sp.k_slabs ? kGemmBK : a->K, k_out = sp.k_slabs ? a->K / kGemmBK : 1;
+    {
+      const uint32_t box[4] = {(uint32_t)kGemmBK, (uint32_t)sp.a_rows, (uint32_t)sp.slabs, 1};
+      const uint64_t dims[4] = {k_in, (uint64_t)a->M, k_out, (uint64_t)batch};
+      const uint64_t str[3] = {(uint64_t)a->lda * 2, kGemmBK * 2, (uint64_t)a_bs * 2};
+      rc = encode_tensor_map(&p.tm_a, dt, 4, a->a, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
+      if (rc != HB_OK) return rc;
+    }
+    if (w_kn) {
+      const uint32_t box[3] = {64, (uint32_t)(sp.slabs * kGemmBK), 1};
+      const uint64_t dims[3] = {(uint64_t)a->N, (uint64_t)a->K, (uint64_t)batch};
+      const uint64_t str[2] = {(uint64_t)a->ldw * 2, (uint64_t)w_bs * 2};
+      rc = encode_tensor_map(&p.tm_w, dt, 3, a->w, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
+    } else {
+      const uint32_t parts = epi_class == kEpiSwiglu ? 2 : 1;
+      const uint32_t box[5] = {(uint32_t)kGemmBK, (uint32_t)split.width / parts, parts, (uint32_t)sp.slabs, 1};
+      const uint64_t dims[5] = {k_in, (uint64_t)n_out, parts, k_out, (uint64_t)batch};
+      const uint64_t str[4] = {(uint64_t)a->ldw * 2, (uint64_t)n_out * a->ldw * 2, kGemmBK * 2, (uint64_t)w_bs * 2};
+      rc = encode_tensor_map(&p.tm_w, dt, 5, a->w, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B,
+                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B);  // 35.2 -> 33.5 us for 24 x 22016 x 4096
+    }
+    if (rc != HB_OK) return rc;
+  } else {
     const uint32_t box[3] = {(uint32_t)kGemmBK, 128, 1};
     const uint64_t dims[3] = {(uint64_t)a->K, (uint64_t)a->M, (uint64_t)batch};
     const uint64_t str[2] = {(uint64_t)a->lda * 2, (uint64_t)a_bs * 2};
     rc = encode_tensor_map(&p.tm_a, dt, 3, a->a, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc != HB_OK) return rc;
   }
-  if (w_kn) {
+  if (use_split) {
+    // maps are in place
+  } else if (w_kn) {
     const uint32_t box[3] = {64, (uint32_t)kGemmBK, 1};  // 64 columns (128 bytes) x 64 k-rows
     const uint64_t dims[3] = {(uint64_t)a->N, (uint64_t)a->K, (uint64_t)batch};
     const uint64_t str[2] = {(uint64_t)a->ldw * 2, (uint64_t)w_bs * 2};
@@ -144,7 +306,7 @@ static int gemm_impl(const hb_gemm_args* a) {
     rc = encode_tensor_map(&p.tm_w, dt, 3, a->w, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc != HB_OK) return rc;
   }
-  if (epi_class == kEpiPlain) {
+  if (epi_class == kEpiPlain && !use_split) {
     const uint32_t box[3] = {64, (uint32_t)kGemmBM, 1};
     const uint64_t dims[3] = {(uint64_t)n_out, (uint64_t)a->M, (uint64_t)batch};
     const uint64_t str[2] = {(uint64_t)a->ldo * 2, (uint64_t)o_bs * 2};
@@ -164,9 +326,9 @@ static int gemm_impl(const hb_gemm_args* a) {
   p.M = a->M;
   p.N_out = n_out;
   p.K = a->K;
-  p.tile_cols = epi_class == kEpiSwiglu ? 128 : kGemmBN;
-  // CTA pairs (256-row tiles) whenever a problem has more than one 128-row tile of rows
-  const bool pair = a->schedule == HB_GEMM_PAIR || (a->schedule == HB_GEMM_AUTO && a->M > kGemmBM && st->sm_count >= 2);
+  p.tile_cols = (use_split ? split.width : kGemmBN) / (epi_class == kEpiSwiglu ? 2 : 1);
+  const bool pair = !use_split &&
+                    (a->schedule == HB_GEMM_PAIR || (a->schedule == HB_GEMM_AUTO && a->M > kGemmBM && st->sm_count >= 2));
   const int tile_rows = pair ? kPairBM : kGemmBM;
   p.tiles_m = (a->M + tile_rows - 1) / tile_rows;
   p.tiles_n = (n_out + p.tile_cols - 1) / p.tile_cols;
@@ -179,7 +341,7 @@ static int gemm_impl(const hb_gemm_args* a) {
   p.w_kn = w_kn ? 1 : 0;
   p.o_batch_stride = o_bs;
   p.r_batch_stride = r_bs;
-  p.k_steps = (a->K + kGemmBK - 1) / kGemmBK;
+  p.k_steps = k_steps;
   p.act = (a->epilogue >= HB_EPI_SILU && a->epilogue <= HB_EPI_TANH) ? a->epilogue : kActNone;
   p.rope_seq = a->rope_seq;
   p.head_dim = a->head_dim;
@@ -193,6 +355,20 @@ static int gemm_impl(const hb_gemm_args* a) {
 
   const int grid = pair ? 2 * (int)std::min<long long>(tiles, st->sm_count / 2) : (int)std::min<long long>(tiles, st->sm_count);
   cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
+  if (use_split) {
+    sp.width = split.width;
+    sp.splits = split.splits;
+    p.k_steps = (k_steps + sp.slabs - 1) / sp.slabs;
+    const int stage_bytes = (sp.a_rows + sp.width) * kGemmBK * 2 * sp.slabs;
+    // the last A box of the ring is read as 128 rows: 16 KB of shared memory behind its start have to exist
+    sp.stages = std::min(kGemmSplitMaxStages, (kGemmSplitRing - 16384) / stage_bytes);
+    sp.tmem_cols = 32;
+    while (sp.tmem_cols < sp.width) sp.tmem_cols *= 2;
+    if (tiles * sp.splits > 0x7fffffffLL) return set_error(HB_ERR_UNSUPPORTED, "hb_gemm_epilogue: too many tiles");
+    const int split_grid = (int)tiles * sp.splits;
+    return a->dtype == HB_BF16 ? dispatch_gemm_split<__nv_bfloat16>(epi_class, sp, split_grid, st, stream)
+                               : dispatch_gemm_split<__half>(epi_class, sp, split_grid, st, stream);
+  }
   return a->dtype == HB_BF16 ? dispatch_gemm<__nv_bfloat16>(epi_class, p, grid, pair, st, stream)
                              : dispatch_gemm<__half>(epi_class, p, grid, pair, st, stream);
 }

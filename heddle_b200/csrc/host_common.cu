@@ -113,7 +113,8 @@ int get_device_info_noalloc(DeviceInfo* out) {
 }
 
 int encode_tensor_map(CUtensorMap* out, CUtensorMapDataType dt, int rank, const void* base, const uint64_t* dims,
-                      const uint64_t* strides_bytes, const uint32_t* box, CUtensorMapSwizzle swizzle) {
+                      const uint64_t* strides_bytes, const uint32_t* box, CUtensorMapSwizzle swizzle,
+                      CUtensorMapL2promotion promotion) {
   if (g_encode == nullptr) return set_error(HB_ERR_CUDA, "tensor-map encoder not initialised");
   if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0)
     return set_error(HB_ERR_ALIGN, "tensor base %p is not 16-byte aligned", base);
@@ -133,7 +134,7 @@ int encode_tensor_map(CUtensorMap* out, CUtensorMapDataType dt, int rank, const 
     gstr[i] = strides_bytes[i];
   }
   CUresult r = g_encode(out, dt, static_cast<cuuint32_t>(rank), const_cast<void*>(base), gdim, gstr, gbox, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, promotion,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return set_error(HB_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
   return HB_OK;

@@ -52,7 +52,8 @@ int get_device_info_noalloc(DeviceInfo* out);
 //   strides[i]  byte stride of dimension i+1
 //   box[i]      tile extent of dimension i in elements
 int encode_tensor_map(CUtensorMap* out, CUtensorMapDataType dt, int rank, const void* base, const uint64_t* dims,
-                      const uint64_t* strides_bytes, const uint32_t* box, CUtensorMapSwizzle swizzle);
+                      const uint64_t* strides_bytes, const uint32_t* box, CUtensorMapSwizzle swizzle,
+                      CUtensorMapL2promotion promotion = CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
 
 inline size_t dtype_size(int dtype) { return dtype == HB_FP8_E4M3 ? 1 : 2; }
 

@@ -226,12 +226,12 @@ def debug_umma(mode: int, a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     return out
 
 
-# Which GEMM kernel hb_gemm_epilogue runs: "auto" (CTA pairs when M > 128), "single" or "pair".
+# Which GEMM kernel hb_gemm_epilogue runs: "auto" (by the size of the problem), "single", "pair" or "split".
 _gemm_schedule = os.environ.get("HEDDLE_B200_GEMM_SCHEDULE", "auto")
 
 
 def set_gemm_schedule(name: str) -> str:
-    """Select the GEMM kernel for later calls ("auto", "single", "pair"); returns the previous choice."""
+    """Select the GEMM kernel for later calls ("auto", "single", "pair", "split"); returns the previous choice."""
     global _gemm_schedule
     if name not in _lib.GEMM_SCHEDULES:
         raise ValueError(f"unknown GEMM schedule {name!r}")

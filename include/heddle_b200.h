@@ -195,9 +195,11 @@ typedef enum hb_epilogue {
 
 typedef enum hb_w_layout { HB_W_NK = 0, HB_W_KN = 1 } hb_w_layout;
 /* Which kernel runs the product.  AUTO: CTA pairs (two CTAs share a 256 x 256 tile through
- * tcgen05.mma.cta_group::2) when M > 128, else the single-CTA kernel (128 x 256 tiles).  SINGLE and
- * PAIR force one of them; the results are identical (same accumulation order per element). */
-typedef enum hb_gemm_schedule { HB_GEMM_AUTO = 0, HB_GEMM_SINGLE = 1, HB_GEMM_PAIR = 2 } hb_gemm_schedule;
+ * tcgen05.mma.cta_group::2) when M > 128, else the single-CTA kernel (128 x 256 tiles), and for products
+ * whose tiles would leave SMs idle the split-K kernel (a cluster of up to 8 CTAs shares a tile's K range).
+ * SINGLE, PAIR and SPLIT force one of them; the results of the first two are identical (same accumulation
+ * order per element). */
+typedef enum hb_gemm_schedule { HB_GEMM_AUTO = 0, HB_GEMM_SINGLE = 1, HB_GEMM_PAIR = 2, HB_GEMM_SPLIT = 3 } hb_gemm_schedule;
 
 typedef struct hb_gemm_args {
   const void* a; /* [M, K], row stride lda */
