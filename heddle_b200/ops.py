@@ -6,8 +6,10 @@ There is no CPU or eager fallback here: CPU tensors are rejected.
 from __future__ import annotations
 
 import ctypes as C
-import os
+import functools
 import math
+import os
+import struct
 from typing import Optional, Sequence, Tuple
 
 import torch
@@ -27,8 +29,33 @@ def _require_cuda(*tensors: torch.Tensor) -> None:
                 f"{t.device} — there is no CPU fallback")
 
 
+# Host time of a call matters where its kernels take microseconds: on the host of the measurements a launch is 3 us, a
+# torch.cuda.current_stream() 2.2, a torch.cuda.device block 1.4, a reshape that changes nothing 1.0.  So the raw stream handle
+# is asked for, the device is only switched when it is another one, and views are only made where a shape needs them.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
+
+
 def _stream_ptr(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    if _raw_stream is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    return _raw_stream(device.index)
+
+
+def _call(device: torch.device, fn, *args) -> None:
+    """``fn(*args)`` with ``device`` current; raises on a non-zero status."""
+    if _current_device() == device.index:
+        rc = fn(*args)
+    else:
+        with torch.cuda.device(device):
+            rc = fn(*args)
+    if rc:
+        _lib.check(rc)
+
+
+def _as_fp32(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous fp32, the tensor itself where it is that already."""
+    return t if t.dtype is torch.float32 and t.is_contiguous() else t.to(torch.float32).contiguous()
 
 
 def _inner_contiguous(t: torch.Tensor) -> torch.Tensor:
@@ -66,43 +93,39 @@ def fa_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal: bool = 
         b_ax, h_ax, s_ax = 0, 2, 1
     else:
         raise ValueError(f"unknown layout {layout!r}")
-    B, Hq, Sq, D = q.shape[b_ax], q.shape[h_ax], q.shape[s_ax], q.shape[3]
-    Hkv, Skv = k.shape[h_ax], k.shape[s_ax]
-    if k.shape[b_ax] != B or v.shape != k.shape or k.shape[3] != D:
+    q_shape, k_shape = q.shape, k.shape
+    B, Hq, Sq, D = q_shape[b_ax], q_shape[h_ax], q_shape[s_ax], q_shape[3]
+    Hkv, Skv = k_shape[h_ax], k_shape[s_ax]
+    if k_shape[b_ax] != B or v.shape != k_shape or k_shape[3] != D:
         raise ValueError(f"shape mismatch: q {tuple(q.shape)}, k {tuple(k.shape)}, v {tuple(v.shape)}")
     out_dtype = torch.bfloat16 if q.dtype not in (torch.bfloat16, torch.float16) else q.dtype
     if out is None:
-        out = torch.empty(q.shape, dtype=out_dtype, device=q.device)
+        out = q.new_empty(q_shape, dtype=out_dtype)
     else:
         _require_cuda(out)
         if out.shape != q.shape or out.dtype != out_dtype or out.stride(-1) != 1:
             raise ValueError("out must match q's shape, have the output dtype and a contiguous last axis")
-    lse = torch.empty((B, Hq, Sq), dtype=torch.float32, device=q.device) if return_lse else None
+    lse = q.new_empty((B, Hq, Sq), dtype=torch.float32) if return_lse else None
 
-    a = _lib.FaArgs()
-    a.q, a.k, a.v, a.o = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr()
-    a.lse = lse.data_ptr() if lse is not None else None
-    a.B, a.Hq, a.Hkv, a.Sq, a.Skv, a.D = B, Hq, Hkv, Sq, Skv, D
-    a.q_stride_b, a.q_stride_h, a.q_stride_s = q.stride(b_ax), q.stride(h_ax), q.stride(s_ax)
-    a.k_stride_b, a.k_stride_h, a.k_stride_s = k.stride(b_ax), k.stride(h_ax), k.stride(s_ax)
-    a.v_stride_b, a.v_stride_h, a.v_stride_s = v.stride(b_ax), v.stride(h_ax), v.stride(s_ax)
-    a.o_stride_b, a.o_stride_h, a.o_stride_s = out.stride(b_ax), out.stride(h_ax), out.stride(s_ax)
-    a.causal = 1 if causal else 0
-    a.softmax_scale = float(softmax_scale) if softmax_scale is not None else 1.0 / math.sqrt(D)
-    a.dtype = _DTYPES[q.dtype]
-    if scales is not None:
-        a.q_scale, a.k_scale, a.v_scale = (float(x) for x in scales)
-    a.stream = _stream_ptr(q.device)
-    with torch.cuda.device(q.device):
-        if debug_stages is None and Sq <= _FA_SPLIT_MAX_ROWS:
-            need = C.c_uint64(0)
-            _lib.check(_lib.load().hb_fa_fwd_workspace(C.byref(a), C.byref(need)))
-            ws = torch.empty(need.value, dtype=torch.uint8, device=q.device) if need.value else None
-            _lib.check(_lib.load().hb_fa_fwd_ws(C.byref(a), ws.data_ptr() if ws is not None else None, need.value))
-        elif debug_stages is None:
-            _lib.check(_lib.load().hb_fa_fwd(C.byref(a)))
-        else:
-            _lib.check(_lib.load().hb_debug_fa_fwd_stages(C.byref(a), int(debug_stages)))
+    qs, ks, vs, os_ = q.stride(), k.stride(), v.stride(), out.stride()
+    q_sc, k_sc, v_sc = (float(x) for x in scales) if scales is not None else (0.0, 0.0, 0.0)
+    device = q.device
+    a = _lib.FaArgs(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr() if return_lse else None,
+        B, Hq, Hkv, Sq, Skv, D,
+        qs[b_ax], qs[h_ax], qs[s_ax], ks[b_ax], ks[h_ax], ks[s_ax], vs[b_ax], vs[h_ax], vs[s_ax], os_[b_ax], os_[h_ax], os_[s_ax],
+        1 if causal else 0, float(softmax_scale) if softmax_scale is not None else 1.0 / math.sqrt(D), _DTYPES[q.dtype],
+        q_sc, k_sc, v_sc, 0.0, 0.0, _stream_ptr(device))
+    lib = _lib.load()
+    if debug_stages is not None:
+        _call(device, lib.hb_debug_fa_fwd_stages, C.byref(a), int(debug_stages))
+    elif Sq <= _FA_SPLIT_MAX_ROWS:
+        need = C.c_uint64(0)
+        _call(device, lib.hb_fa_fwd_workspace, C.byref(a), C.byref(need))
+        ws = q.new_empty(need.value, dtype=torch.uint8) if need.value else None
+        _call(device, lib.hb_fa_fwd_ws, C.byref(a), ws.data_ptr() if ws is not None else None, need.value)
+    else:
+        _call(device, lib.hb_fa_fwd, C.byref(a))
     return (out, lse) if return_lse else out
 
 
@@ -122,31 +145,27 @@ def _bwd_args(q, k, v, o, d_o, lse, delta, causal, softmax_scale, layout):
         raise ValueError(f"unknown layout {layout!r}")
     q, k, v, d_o = (_inner_contiguous(t) for t in (q, k, v, d_o))
     o = _inner_contiguous(o) if o is not None else None
-    B, Hq, Sq, D = q.shape[b_ax], q.shape[h_ax], q.shape[s_ax], q.shape[3]
-    Hkv, Skv = k.shape[h_ax], k.shape[s_ax]
-    if k.shape[b_ax] != B or v.shape != k.shape or k.shape[3] != D or d_o.shape != q.shape or (
-            o is not None and o.shape != q.shape):
+    q_shape, k_shape = q.shape, k.shape
+    B, Hq, Sq, D = q_shape[b_ax], q_shape[h_ax], q_shape[s_ax], q_shape[3]
+    Hkv, Skv = k_shape[h_ax], k_shape[s_ax]
+    if k_shape[b_ax] != B or v.shape != k_shape or k_shape[3] != D or d_o.shape != q_shape or (
+            o is not None and o.shape != q_shape):
         raise ValueError("shape mismatch between q, k, v, o and d_o")
     keep = [q, k, v, d_o, o]
-    a = _lib.FaBwdArgs()
-    a.q, a.k, a.v, a.d_o = q.data_ptr(), k.data_ptr(), v.data_ptr(), d_o.data_ptr()
-    a.o = o.data_ptr() if o is not None else None
     for name, t in (("lse", lse), ("delta", delta)):
         if t is not None:
             if t.dtype != torch.float32 or tuple(t.shape) != (B, Hq, Sq) or not t.is_contiguous():
                 raise ValueError(f"{name} must be a contiguous fp32 [B, Hq, Sq] = {(B, Hq, Sq)} tensor")
-            setattr(a, name, t.data_ptr())
-    a.B, a.Hq, a.Hkv, a.Sq, a.Skv, a.D = B, Hq, Hkv, Sq, Skv, D
-    a.q_stride_b, a.q_stride_h, a.q_stride_s = q.stride(b_ax), q.stride(h_ax), q.stride(s_ax)
-    a.k_stride_b, a.k_stride_h, a.k_stride_s = k.stride(b_ax), k.stride(h_ax), k.stride(s_ax)
-    a.v_stride_b, a.v_stride_h, a.v_stride_s = v.stride(b_ax), v.stride(h_ax), v.stride(s_ax)
-    a.do_stride_b, a.do_stride_h, a.do_stride_s = d_o.stride(b_ax), d_o.stride(h_ax), d_o.stride(s_ax)
-    if o is not None:
-        a.o_stride_b, a.o_stride_h, a.o_stride_s = o.stride(b_ax), o.stride(h_ax), o.stride(s_ax)
-    a.causal = 1 if causal else 0
-    a.softmax_scale = float(softmax_scale) if softmax_scale is not None else 1.0 / math.sqrt(D)
-    a.dtype = _DTYPES[q.dtype]
-    a.stream = _stream_ptr(q.device)
+    qs, ks, vs, ds = q.stride(), k.stride(), v.stride(), d_o.stride()
+    os_ = o.stride() if o is not None else (0, 0, 0, 0)
+    a = _lib.FaBwdArgs(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr() if o is not None else None, d_o.data_ptr(),
+        lse.data_ptr() if lse is not None else None, delta.data_ptr() if delta is not None else None, None, None, None,
+        B, Hq, Hkv, Sq, Skv, D,
+        qs[b_ax], qs[h_ax], qs[s_ax], ks[b_ax], ks[h_ax], ks[s_ax], vs[b_ax], vs[h_ax], vs[s_ax], os_[b_ax], os_[h_ax], os_[s_ax],
+        ds[b_ax], ds[h_ax], ds[s_ax],
+        1 if causal else 0, float(softmax_scale) if softmax_scale is not None else 1.0 / math.sqrt(D), _DTYPES[q.dtype],
+        _stream_ptr(q.device))
     return a, keep, (B, Hq, Hkv, Sq, Skv, D)
 
 
@@ -155,8 +174,7 @@ def fa_bwd_preprocess(o: torch.Tensor, d_o: torch.Tensor, *, layout: str = "bhsd
     b_ax, h_ax, s_ax = (0, 1, 2) if layout == "bhsd" else (0, 2, 1)
     delta = torch.empty((o.shape[b_ax], o.shape[h_ax], o.shape[s_ax]), dtype=torch.float32, device=o.device)
     a, keep, _ = _bwd_args(o, o, o, o, d_o, None, delta, False, None, layout)
-    with torch.cuda.device(o.device):
-        _lib.check(_lib.load().hb_fa_bwd_preprocess(C.byref(a)))
+    _call(o.device, _lib.load().hb_fa_bwd_preprocess, C.byref(a))
     return delta
 
 
@@ -167,8 +185,7 @@ def fa_bwd_dkdv(q, k, v, d_o, lse, delta, *, causal: bool = False, softmax_scale
     dk = torch.empty((B, Hkv, Skv, D), dtype=q.dtype, device=q.device)
     dv = torch.empty_like(dk)
     a.dk, a.dv = dk.data_ptr(), dv.data_ptr()
-    with torch.cuda.device(q.device):
-        _lib.check(_lib.load().hb_fa_bwd_dkdv(C.byref(a)))
+    _call(q.device, _lib.load().hb_fa_bwd_dkdv, C.byref(a))
     return (dk, dv) if layout == "bhsd" else (dk.transpose(1, 2), dv.transpose(1, 2))
 
 
@@ -178,8 +195,7 @@ def fa_bwd_dq(q, k, v, d_o, lse, delta, *, causal: bool = False, softmax_scale: 
     a, keep, (B, Hq, Hkv, Sq, Skv, D) = _bwd_args(q, k, v, None, d_o, lse, delta, causal, softmax_scale, layout)
     dq = torch.empty((B, Hq, Sq, D), dtype=q.dtype, device=q.device)
     a.dq = dq.data_ptr()
-    with torch.cuda.device(q.device):
-        _lib.check(_lib.load().hb_fa_bwd_dq(C.byref(a)))
+    _call(q.device, _lib.load().hb_fa_bwd_dq, C.byref(a))
     return dq if layout == "bhsd" else dq.transpose(1, 2)
 
 
@@ -189,11 +205,19 @@ def fa_bwd(q, k, v, o, d_o, lse, *, causal: bool = False, softmax_scale: Optiona
     ``create_separated_bwd_function``, Heddle/heddle/frontend/bwd_separator.py:366-455).
 
     ``lse`` is the natural-log LSE [B, Hq, Sq] of the forward pass.  Returns (dQ, dK, dV)."""
-    lse = lse.to(torch.float32).contiguous()
-    delta = fa_bwd_preprocess(o, d_o, layout=layout)
-    dk, dv = fa_bwd_dkdv(q, k, v, d_o, lse, delta, causal=causal, softmax_scale=softmax_scale, layout=layout)
-    dq = fa_bwd_dq(q, k, v, d_o, lse, delta, causal=causal, softmax_scale=softmax_scale, layout=layout)
-    return dq, dk, dv
+    _require_cuda(q, o, d_o)
+    lse = _as_fp32(lse)
+    bshd = layout == "bshd"
+    delta = q.new_empty((q.shape[0], q.shape[2 if bshd else 1], q.shape[1 if bshd else 2]) if q.dim() == 4 else 0, dtype=torch.float32)
+    a, keep, (B, Hq, Hkv, Sq, Skv, D) = _bwd_args(q, k, v, o, d_o, lse, delta, causal, softmax_scale, layout)
+    dk = q.new_empty((B, Hkv, Skv, D))
+    dv = q.new_empty((B, Hkv, Skv, D))
+    dq = q.new_empty((B, Hq, Sq, D))
+    a.dk, a.dv, a.dq = dk.data_ptr(), dv.data_ptr(), dq.data_ptr()
+    lib, arg = _lib.load(), C.byref(a)
+    for step in (lib.hb_fa_bwd_preprocess, lib.hb_fa_bwd_dkdv, lib.hb_fa_bwd_dq):
+        _call(q.device, step, arg)
+    return (dq.transpose(1, 2), dk.transpose(1, 2), dv.transpose(1, 2)) if bshd else (dq, dk, dv)
 
 
 def status_word() -> int:
@@ -256,63 +280,73 @@ def gemm_epilogue(a: torch.Tensor, w: torch.Tensor, epilogue: str = "none", *,
         raise TypeError(f"gemm_epilogue needs matching bf16/fp16 operands, got {a.dtype} and {w.dtype}")
     if epilogue not in _lib.EPILOGUES:
         raise ValueError(f"unknown epilogue {epilogue!r}")
-    K = a.shape[-1]
-    lead = a.shape[:-1]
-    a2 = a.reshape(-1, K)
-    if a2.stride(-1) != 1:
+    shape = a.shape
+    K = shape[-1]
+    # rows of a (..., K) tensor that is contiguous lie K apart; anything else goes through a 2-D view or copy
+    if a.dim() == 2:
+        a2 = a
+    elif a.is_contiguous():
+        a2 = None
+    else:
+        a2 = a.reshape(-1, K)
+    if a2 is not None and a2.stride(-1) != 1:
         a2 = a2.contiguous()
     if w.dim() != 2 or w.shape[1] != K:
         raise ValueError(f"weight shape {tuple(w.shape)} does not match K={K}")
     if w.stride(-1) != 1:
         w = w.contiguous()
-    M, N = a2.shape[0], w.shape[0]
+    if a2 is None and K == 0:
+        a2 = a.reshape(-1, K)
+    M = a2.shape[0] if a2 is not None else a.numel() // K
+    N = w.shape[0]
     n_out = N // 2 if epilogue == "swiglu" else N
     if out is None:
-        out2 = torch.empty((M, n_out), dtype=a.dtype, device=a.device)
+        result = a.new_empty((*shape[:-1], n_out))
+        out_ptr, ldo = result.data_ptr(), n_out
     else:
         out2 = out.reshape(-1, n_out)
         if out2.data_ptr() != out.data_ptr() or out2.stride(-1) != 1:
             raise ValueError("out must be viewable as a row-major [M, N_out] matrix")
-    g = _lib.GemmArgs()
-    g.a, g.w, g.out = a2.data_ptr(), w.data_ptr(), out2.data_ptr()
-    g.M, g.N, g.K = M, N, K
-    g.lda, g.ldw, g.ldo = a2.stride(0), w.stride(0), out2.stride(0)
-    g.dtype = _DTYPES[a.dtype]
-    g.epilogue = _lib.EPILOGUES[epilogue]
+        result, out_ptr, ldo = out, out2.data_ptr(), out2.stride(0)
+    device = a.device
+    g = _lib.GemmArgs(a2.data_ptr() if a2 is not None else a.data_ptr(), w.data_ptr(), out_ptr, M, N, K,
+                      a2.stride(0) if a2 is not None else K, w.stride(0), ldo, _DTYPES[a.dtype], _lib.EPILOGUES[epilogue])
     keep = []
     if row_scale is not None:
-        rs = row_scale.reshape(-1).to(torch.float32).contiguous()
+        rs = _as_fp32(row_scale)
         if rs.numel() != M:
             raise ValueError("row_scale must have one entry per row")
         keep.append(rs)
         g.row_scale = rs.data_ptr()
     if bias is not None:
-        b = bias.to(a.dtype).contiguous()
+        b = bias if bias.dtype is a.dtype and bias.is_contiguous() else bias.to(a.dtype).contiguous()
         if b.numel() != N:
             raise ValueError("bias must have N entries")
         keep.append(b)
         g.bias = b.data_ptr()
     if residual is not None:
-        r2 = residual.reshape(-1, n_out)
-        if r2.dtype != a.dtype or r2.stride(-1) != 1:
-            r2 = r2.to(a.dtype).contiguous()
+        if residual.dtype is a.dtype and residual.is_contiguous() and residual.shape[-1:] == (n_out,):
+            r2, g.ldr = residual, n_out
+        else:
+            r2 = residual.reshape(-1, n_out)
+            if r2.dtype != a.dtype or r2.stride(-1) != 1:
+                r2 = r2.to(a.dtype).contiguous()
+            g.ldr = r2.stride(0)
         keep.append(r2)
-        g.residual, g.ldr = r2.data_ptr(), r2.stride(0)
+        g.residual = r2.data_ptr()
     if epilogue == "rope":
         if rope is None:
             raise ValueError("epilogue 'rope' needs rope=(cos, sin, head_dim, rope_cols)")
         cos, sin, hd, rope_cols = rope
-        cos = cos.to(torch.float32).contiguous()
-        sin = sin.to(torch.float32).contiguous()
+        cos, sin = _as_fp32(cos), _as_fp32(sin)
         _require_cuda(cos, sin)
         keep += [cos, sin]
         g.rope_cos, g.rope_sin = cos.data_ptr(), sin.data_ptr()
         g.rope_seq, g.head_dim, g.rope_cols = cos.shape[0], int(hd), int(rope_cols)
-    g.stream = _stream_ptr(a.device)
-    with torch.cuda.device(a.device):
-        g.schedule = _lib.GEMM_SCHEDULES[_gemm_schedule]
-        _lib.check(_lib.load().hb_gemm_epilogue(C.byref(g)))
-    return out2.reshape(*lead, n_out) if out is None else out
+    g.stream = _stream_ptr(device)
+    g.schedule = _lib.GEMM_SCHEDULES[_gemm_schedule]
+    _call(device, _lib.load().hb_gemm_epilogue, C.byref(g))
+    return result
 
 
 def _mult8(*values: int) -> bool:
@@ -345,7 +379,7 @@ def bmm(a: torch.Tensor, b: torch.Tensor, epilogue: str = "none", *, bias: Optio
         if b.stride(2) != 1 or not _mult8(b.stride(1), b.stride(0)) or b.data_ptr() % 16:
             b = b.contiguous()
         layout, ldw = _lib.HB_W_KN, b.stride(1)
-    out = torch.empty((Bn, M, N), dtype=a.dtype, device=a.device)
+    out = a.new_empty((Bn, M, N))
     if Bn == 0 or M == 0:
         return out
     g = _lib.GemmArgs()
@@ -368,9 +402,8 @@ def bmm(a: torch.Tensor, b: torch.Tensor, epilogue: str = "none", *, bias: Optio
         keep.append(r)
         g.residual, g.ldr, g.r_batch_stride = r.data_ptr(), N, M * N
     g.stream = _stream_ptr(a.device)
-    with torch.cuda.device(a.device):
-        g.schedule = _lib.GEMM_SCHEDULES[_gemm_schedule]
-        _lib.check(_lib.load().hb_gemm_epilogue(C.byref(g)))
+    g.schedule = _lib.GEMM_SCHEDULES[_gemm_schedule]
+    _call(a.device, _lib.load().hb_gemm_epilogue, C.byref(g))
     return out
 
 
@@ -394,6 +427,11 @@ def rms_rowstat(x: torch.Tensor, residual: Optional[torch.Tensor] = None, eps: f
     residual is given), rstd fp32 of shape x.shape[:-1]."""
     _require_cuda(x, residual)
     N = x.shape[-1]
+    if residual is None and not write_sum and N > 0 and x.is_contiguous():
+        rstd = x.new_empty(x.shape[:-1], dtype=torch.float32)
+        _call(x.device, _lib.load().hb_rms_rowstat, x.data_ptr(), None, None, rstd.data_ptr(), x.numel() // N, N, N, float(eps),
+              _DTYPES[x.dtype], _stream_ptr(x.device))
+        return None, rstd
     x2 = x.reshape(-1, N)
     if x2.stride(-1) != 1:
         x2 = x2.contiguous()
@@ -409,10 +447,9 @@ def rms_rowstat(x: torch.Tensor, residual: Optional[torch.Tensor] = None, eps: f
         x2 = x2.contiguous()
         y = torch.empty_like(x2)
     rstd = torch.empty((M,), dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.load().hb_rms_rowstat(x2.data_ptr(), r2.data_ptr() if r2 is not None else None,
-                                              y.data_ptr() if y is not None else None, rstd.data_ptr(), M, N,
-                                              x2.stride(0), float(eps), _DTYPES[x.dtype], _stream_ptr(x.device)))
+    _call(x.device, _lib.load().hb_rms_rowstat, x2.data_ptr(), r2.data_ptr() if r2 is not None else None,
+          y.data_ptr() if y is not None else None, rstd.data_ptr(), M, N, x2.stride(0), float(eps), _DTYPES[x.dtype],
+          _stream_ptr(x.device))
     return (y.reshape(x.shape) if y is not None else None), rstd.reshape(x.shape[:-1])
 
 
@@ -449,14 +486,23 @@ def row_softmax(x: torch.Tensor, scale: float = 1.0) -> torch.Tensor:
     multiple of 8 and at most 16384."""
     _require_cuda(x)
     cols = x.shape[-1]
-    x2 = x.reshape(-1, cols)
+    x2 = x if x.dim() == 2 else x.reshape(-1, cols)
     if x2.stride(-1) != 1 or (x2.shape[0] > 1 and x2.stride(0) % 8 != 0) or x2.data_ptr() % 16 != 0:
         x2 = x2.contiguous()
-    y = torch.empty((x2.shape[0], cols), dtype=x.dtype, device=x.device)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.load().hb_row_softmax(x2.data_ptr(), y.data_ptr(), x2.shape[0], cols, max(x2.stride(0), cols),
-                                              cols, float(scale), _DTYPES[x.dtype], _stream_ptr(x.device)))
-    return y.reshape(x.shape)
+    y = x.new_empty(x.shape)
+    _call(x.device, _lib.load().hb_row_softmax, x2.data_ptr(), y.data_ptr(), x2.shape[0], cols, max(x2.stride(0), cols),
+          cols, float(scale), _DTYPES[x.dtype], _stream_ptr(x.device))
+    return y
+
+
+@functools.lru_cache(maxsize=256)
+def _rowwise_code(heads, imms):
+    """The instruction array of a program: ``heads`` = (op, src, index) tuples, ``imms`` = the immediates as packed doubles
+    (bytes, so that -0.0 and 0.0 are two programs)."""
+    code = (_lib.EwInst * _lib.EW_MAX_INST)()
+    for pc, ((op, src, index), imm) in enumerate(zip(heads, struct.unpack(f"{len(heads)}d", imms))):
+        code[pc] = _lib.EwInst(_lib.EW_OPS[op], _lib.EW_SRCS[src or "none"], index, imm)
+    return code
 
 
 def rowwise_program(program, inputs=(), rowvecs=(), rowscalars=(), n_outputs: int = 1, mode: str = "auto"):
@@ -484,7 +530,7 @@ def rowwise_program(program, inputs=(), rowvecs=(), rowscalars=(), n_outputs: in
     for i, t in enumerate(inputs):
         if tuple(t.shape) != shape or t.dtype != x0.dtype:
             raise ValueError("rowwise_program: full-size inputs must share shape and dtype")
-        t2 = t.reshape(-1, cols)
+        t2 = t if t.dim() == 2 else t.reshape(-1, cols)
         if t2.stride(-1) != 1 or t2.stride(0) % 8 or t2.data_ptr() % 16:
             t2 = t2.contiguous()
         keep.append(t2)
@@ -502,20 +548,16 @@ def rowwise_program(program, inputs=(), rowvecs=(), rowscalars=(), n_outputs: in
             raise ValueError("rowwise_program: a per-row vector must have one entry per row")
         keep.append(t2)
         a.rowscalar[i] = t2.data_ptr()
-    outs = [torch.empty(shape, dtype=x0.dtype, device=x0.device) for _ in range(n_outputs)]
+    outs = [x0.new_empty(shape) for _ in range(n_outputs)]
     for i, o in enumerate(outs):
         a.outputs[i], a.ld_out[i] = o.data_ptr(), cols
     a.n_inputs, a.n_rowvec, a.n_rowscalar, a.n_outputs = len(inputs), len(rowvecs), len(rowscalars), n_outputs
     a.rows, a.cols, a.dtype, a.n_inst = rows, cols, _DTYPES[x0.dtype], len(program)
-    for pc, (op, src, index, imm) in enumerate(program):
-        a.program[pc].op = _lib.EW_OPS[op]
-        a.program[pc].src = _lib.EW_SRCS[src or "none"]
-        a.program[pc].index = int(index)
-        a.program[pc].imm = float(imm)
+    a.program = _rowwise_code(tuple((op, src, int(index)) for op, src, index, _ in program),
+                              struct.pack(f"{len(program)}d", *[float(inst[3]) for inst in program]))
     a.stream = _stream_ptr(x0.device)
     a.mode = {"auto": _lib.ROWWISE_AUTO, "interpret": _lib.ROWWISE_INTERPRET, "compiled": _lib.ROWWISE_COMPILED}[mode]
-    with torch.cuda.device(x0.device):
-        _lib.check(_lib.load().hb_rowwise_program(C.byref(a)))
+    _call(x0.device, _lib.load().hb_rowwise_program, C.byref(a))
     return outs[0] if n_outputs == 1 else tuple(outs)
 
 
@@ -531,19 +573,15 @@ def h2o_score(q: torch.Tensor, k: torch.Tensor, lse: torch.Tensor, *, causal: bo
     b_ax, h_ax, s_ax = (0, 1, 2) if layout == "bhsd" else (0, 2, 1)
     B, Hq, Sq, D = q.shape[b_ax], q.shape[h_ax], q.shape[s_ax], q.shape[3]
     Hkv, Skv = k.shape[h_ax], k.shape[s_ax]
-    lse = lse.to(torch.float32).contiguous()
+    lse = _as_fp32(lse)
     if tuple(lse.shape) != (B, Hq, Sq):
         raise ValueError(f"lse must be [B, Hq, Sq] = {(B, Hq, Sq)}, got {tuple(lse.shape)}")
-    score = torch.empty((B, Hq, Skv), dtype=torch.float32, device=q.device)
-    a = _lib.H2oArgs()
-    a.q, a.k, a.lse, a.score = q.data_ptr(), k.data_ptr(), lse.data_ptr(), score.data_ptr()
-    a.B, a.Hq, a.Hkv, a.Sq, a.Skv, a.D = B, Hq, Hkv, Sq, Skv, D
-    a.q_stride_b, a.q_stride_h, a.q_stride_s = q.stride(b_ax), q.stride(h_ax), q.stride(s_ax)
-    a.k_stride_b, a.k_stride_h, a.k_stride_s = k.stride(b_ax), k.stride(h_ax), k.stride(s_ax)
-    a.causal = 1 if causal else 0
-    a.softmax_scale = float(softmax_scale) if softmax_scale is not None else 1.0 / math.sqrt(D)
-    a.dtype = _DTYPES[q.dtype]
-    a.stream = _stream_ptr(q.device)
-    with torch.cuda.device(q.device):
-        _lib.check(_lib.load().hb_h2o_score(C.byref(a)))
+    score = q.new_empty((B, Hq, Skv), dtype=torch.float32)
+    qs, ks = q.stride(), k.stride()
+    a = _lib.H2oArgs(
+        q.data_ptr(), k.data_ptr(), lse.data_ptr(), score.data_ptr(), B, Hq, Hkv, Sq, Skv, D,
+        qs[b_ax], qs[h_ax], qs[s_ax], ks[b_ax], ks[h_ax], ks[s_ax],
+        1 if causal else 0, float(softmax_scale) if softmax_scale is not None else 1.0 / math.sqrt(D), _DTYPES[q.dtype],
+        _stream_ptr(q.device))
+    _call(q.device, _lib.load().hb_h2o_score, C.byref(a))
     return score
