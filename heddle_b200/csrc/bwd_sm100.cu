@@ -28,6 +28,7 @@
 // head_dim 128 or 64, bf16 / fp16.
 #include "host_common.h"
 #include "ptx_sm100.cuh"
+#include "tile_order.h"
 
 #include <algorithm>
 #include <cmath>
@@ -77,8 +78,7 @@ struct alignas(64) BwdParams {
   int B, Hq, Hkv, Sq, Skv;
   int group, causal;
   int nkb, nqb;     // 128-row key / query tiles
-  int npairs;       // pairs of tiles per head: dkdv ceil(nkb / 2), dq ceil(nqb / 2)
-  int total_items;  // pairs: dkdv B * Hkv * npairs;  dq B * Hq * npairs
+  TileOrder order;  // the work list: dkdv heads B * Hkv, blocks nkb, rank 0 = the first; dq heads B * Hq, blocks nqb, rank 0 = the last
   float scale_log2, scale;
 };
 
@@ -264,15 +264,11 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
   const bool run = (s.abort_flag == 0);
   const int past = p.Skv - p.Sq;
 
-  // Work list: entry u >> 1 is a pair of key tiles (pair, nkb-1-pair) of one (batch, kv head), u & 1 selects
-  // the tile.  Under a causal mask the two tiles of a pair together see nqb + 1 query tiles whatever the pair, so
-  // the static round-robin over pairs keeps the persistent CTAs balanced.
+  // Work list (tile_order.h): u >> 1 is the entry, u & 1 its half where entries are pairs.  Under a causal mask key tile 0 is
+  // seen by the most queries.
   auto item_of = [&](int u, int& b, int& hkv, int& k0, int& qt0) -> bool {
-    const int g = u >> 1;
-    const int pair = g % p.npairs;
-    const int bh = g / p.npairs;
-    const int kb = (u & 1) ? p.nkb - 1 - pair : pair;
-    if ((u & 1) && kb == pair) return false;  // middle tile of an odd count
+    int bh, kb;
+    if (!tile_order_get(p.order, u >> 1, u & 1, static_cast<int>(gridDim.x), bh, kb)) return false;
     b = bh / p.Hkv;
     hkv = bh - b * p.Hkv;
     k0 = kb * 128;
@@ -285,7 +281,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
       // ---------------- TMA producer ----------------
       uint32_t cnt = 0, f_phase = 1;  // cnt: steps loaded so far (stage = cnt & 1 in both rings)
       bool ok = true;
-      for (int u = 2 * blockIdx.x; ok && u < 2 * p.total_items; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1)) {
+      for (int u = 2 * blockIdx.x; ok && u < 2 * p.order.total; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1)) {
         int b, hkv, k0, qt0;
         if (!item_of(u, b, hkv, k0, qt0)) continue;
         if (!mbar_wait(&s.fixed_empty, f_phase, ctx, kBwdTma)) break;
@@ -324,7 +320,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
       BWD_PROF_DECL
       auto full_a = [&](uint32_t c) { return mbar_wait_warp(&s.a_full[c & 1u], (c >> 1) & 1u, ctx, kBwdMma); };
       auto full_b = [&](uint32_t c) { return mbar_wait_warp(&s.b_full[c & 1u], (c >> 1) & 1u, ctx, kBwdMma); };
-      for (int u = 2 * blockIdx.x; ok && u < 2 * p.total_items; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1), ++items) {
+      for (int u = 2 * blockIdx.x; ok && u < 2 * p.order.total; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1), ++items) {
         int b, hkv, k0, qt0;
         if (!item_of(u, b, hkv, k0, qt0)) {
           --items;  // not an item: keep the count of real items
@@ -437,7 +433,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
     const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2), one2 = pack_f32x2(1.0f, 1.0f);
     uint32_t cnt = 0, items = 0;
     bool ok = true;
-    for (int u = 2 * blockIdx.x; ok && u < 2 * p.total_items; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1), ++items) {
+    for (int u = 2 * blockIdx.x; ok && u < 2 * p.order.total; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1), ++items) {
       int b, hkv, k0, qt0;
       if (!item_of(u, b, hkv, k0, qt0)) {
         --items;  // not an item: keep the count of real items
@@ -622,14 +618,12 @@ __global__ void __launch_bounds__(kBwdDqThreads, 1) fa_bwd_dq_kernel(const __gri
   const bool run = (s.abort_flag == 0);
   const int past = p.Skv - p.Sq;
 
-  // Work list: entry u >> 1 is a pair of query tiles (nqb-1-pair, pair) of one (batch, head), u & 1 selects
-  // the tile; under a causal mask the two together see about the same number of key tiles for every pair.
+  // Work list (tile_order.h): u >> 1 is the entry, u & 1 its half where entries are pairs.  Under a causal mask the last query
+  // tile sees the most keys.
   auto item_of = [&](int u, int& b, int& hq, int& q0, int& nk) -> bool {
-    const int g = u >> 1;
-    const int pair = g % p.npairs;
-    const int bh = g / p.npairs;
-    const int qb = (u & 1) ? pair : p.nqb - 1 - pair;
-    if ((u & 1) && qb == p.nqb - 1 - pair) return false;  // middle tile of an odd count
+    int bh, rank;
+    if (!tile_order_get(p.order, u >> 1, u & 1, static_cast<int>(gridDim.x), bh, rank)) return false;
+    const int qb = p.nqb - 1 - rank;
     b = bh / p.Hq;
     hq = bh - b * p.Hq;
     q0 = qb * 128;
@@ -645,7 +639,7 @@ __global__ void __launch_bounds__(kBwdDqThreads, 1) fa_bwd_dq_kernel(const __gri
       // ---------------- TMA producer ----------------
       uint32_t cnt = 0, f_phase = 1;
       bool ok = true;
-      for (int u = 2 * blockIdx.x; ok && u < 2 * p.total_items; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1)) {
+      for (int u = 2 * blockIdx.x; ok && u < 2 * p.order.total; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1)) {
         int b, hq, q0, nk;
         if (!item_of(u, b, hq, q0, nk)) continue;
         const int hkv = hq / p.group;
@@ -704,7 +698,7 @@ __global__ void __launch_bounds__(kBwdDqThreads, 1) fa_bwd_dq_kernel(const __gri
         __syncwarp();
         return true;
       };
-      for (int u = 2 * blockIdx.x; ok && u < 2 * p.total_items; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1), ++items) {
+      for (int u = 2 * blockIdx.x; ok && u < 2 * p.order.total; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1), ++items) {
         int b, hq, q0, nk;
         if (!item_of(u, b, hq, q0, nk)) {
           --items;  // not an item: keep the count of real items
@@ -781,7 +775,7 @@ __global__ void __launch_bounds__(kBwdDqThreads, 1) fa_bwd_dq_kernel(const __gri
     uint32_t cnt = 0, items = 0;
     bool ok = true;
     BWD_PROF_DECL
-    for (int u = 2 * blockIdx.x; ok && u < 2 * p.total_items; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1), ++items) {
+    for (int u = 2 * blockIdx.x; ok && u < 2 * p.order.total; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1), ++items) {
       int b, hq, q0, nk;
       if (!item_of(u, b, hq, q0, nk)) {
         --items;  // not an item: keep the count of real items
@@ -1061,11 +1055,10 @@ extern "C" int hb_fa_bwd_dkdv(const hb_fa_bwd_args* a) {
   BwdParams p;
   rc = bwd_fill(a, p, st);
   if (rc != HB_OK) return rc;
-  p.npairs = (p.nkb + 1) / 2;
-  const long long total = (long long)a->B * a->Hkv * p.npairs;
+  const long long total = (long long)a->B * a->Hkv * ((p.nkb + 1) / 2);
   if (total > 0x3fffffffLL) return set_error(HB_ERR_UNSUPPORTED, "hb_fa_bwd_dkdv: problem too large");
-  p.total_items = (int)total;
-  int grid = (int)std::min<long long>(total, st->sm_count);
+  // a key tile reads Q and dO of its query heads
+  int grid = tile_order_fill(&p.order, (long long)a->B * a->Hkv, p.nkb, p.causal != 0, 4.0 * a->Sq * a->D * p.group, st->sm_count);
 #ifdef HB_DEBUG_GRID_ENV  // measurement builds only: fewer CTAs than SMs
   if (const char* e = getenv("HB_GRID")) grid = std::max(1, std::min(grid, atoi(e)));
 #endif
@@ -1095,11 +1088,9 @@ extern "C" int hb_fa_bwd_dq(const hb_fa_bwd_args* a) {
   BwdParams p;
   rc = bwd_fill(a, p, st);
   if (rc != HB_OK) return rc;
-  p.npairs = (p.nqb + 1) / 2;
-  const long long total = (long long)a->B * a->Hq * p.npairs;
+  const long long total = (long long)a->B * a->Hq * ((p.nqb + 1) / 2);
   if (total > 0x3fffffffLL) return set_error(HB_ERR_UNSUPPORTED, "hb_fa_bwd_dq: problem too large");
-  p.total_items = (int)total;
-  int grid = (int)std::min<long long>(total, st->sm_count);
+  int grid = tile_order_fill(&p.order, (long long)a->B * a->Hq, p.nqb, p.causal != 0, 4.0 * a->Skv * a->D / p.group, st->sm_count);
 #ifdef HB_DEBUG_GRID_ENV  // measurement builds only: fewer CTAs than SMs
   if (const char* e = getenv("HB_GRID")) grid = std::max(1, std::min(grid, atoi(e)));
 #endif

@@ -114,9 +114,9 @@ static int fa_validate(const hb_fa_args* a, const char* who, bool allow_fp8, boo
 }
 
 // Kernel parameters of a validated call: tensor maps over the caller's q, k, v (by strides, so
-// BHSD, BSHD and packed views need no copy), the work-list geometry and the scales.  The tensor-map
+// BHSD, BSHD and packed views need no copy), the work list and its grid size, and the scales.  The tensor-map
 // encoder must be initialised (get_device_state / get_device_info_noalloc do that).
-static int fa_fill_params(const hb_fa_args* a, const char* who, uint32_t* status, FaParams* out) {
+static int fa_fill_params(const hb_fa_args* a, const char* who, uint32_t* status, int sm_count, FaParams* out, int* grid) {
   FaParams& p = *out;
   memset(&p, 0, sizeof(p));
   const size_t es = dtype_size(a->dtype);
@@ -160,8 +160,7 @@ static int fa_fill_params(const hb_fa_args* a, const char* who, uint32_t* status
   p.group = a->Hq / a->Hkv;
   p.causal = a->causal ? 1 : 0;
   p.nqb = (a->Sq + 2 * kTileM - 1) / (2 * kTileM);
-  p.npairs = (p.nqb + 1) / 2;
-  p.total_pairs = (int)((long long)a->B * a->Hq * p.npairs);
+  *grid = tile_order_fill(&p.order, (long long)a->B * a->Hq, p.nqb, p.causal != 0, 2.0 * a->Skv * a->D * es / p.group, sm_count);
   p.nkv = (a->Skv + kTileN - 1) / kTileN;
   const float scale = a->softmax_scale > 0.f ? a->softmax_scale : 1.0f / sqrtf((float)a->D);
   p.scale_log2 = scale * 1.4426950408889634f;
@@ -203,9 +202,9 @@ static int fa_fwd_impl(const hb_fa_args* a, const char* who, bool ws, void* work
   if (rc != HB_OK) return rc;
   if (ws && fa_split_takes(a)) return fa_split_run(a, st, workspace, workspace_bytes);
   FaParams p;
-  rc = fa_fill_params(a, who, st->status_word, &p);
+  int grid = 0;
+  rc = fa_fill_params(a, who, st->status_word, st->sm_count, &p, &grid);
   if (rc != HB_OK) return rc;
-  int grid = std::min(p.total_pairs, st->sm_count);
 #ifdef HB_DEBUG_GRID_ENV  // measurement builds only: fewer CTAs than SMs, to see how the per-SM rate depends on the load on L2
   if (const char* e = getenv("HB_GRID")) grid = std::max(1, std::min(grid, atoi(e)));
 #endif
@@ -225,9 +224,9 @@ static int fa_fwd_stages_impl(const hb_fa_args* a, int stages) {
   rc = get_device_state(&st);
   if (rc != HB_OK) return rc;
   FaParams p;
-  rc = fa_fill_params(a, "hb_debug_fa_fwd_stages", st->status_word, &p);
+  int grid = 0;
+  rc = fa_fill_params(a, "hb_debug_fa_fwd_stages", st->status_word, st->sm_count, &p, &grid);
   if (rc != HB_OK) return rc;
-  const int grid = std::min(p.total_pairs, st->sm_count);
   cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
   switch (stages) {
     case 2:
@@ -295,9 +294,10 @@ static int fa_fwd_noalloc_impl(const hb_fa_args* a) {
   // hb_status_word_noalloc hands it to the host and clears it.  A time-out therefore stays
   // visible across later calls until it has been read.
   FaParams p;
-  rc = fa_fill_params(a, "hb_fa_fwd_noalloc", status, &p);
+  int grid = 0;
+  rc = fa_fill_params(a, "hb_fa_fwd_noalloc", status, info.sm_count, &p, &grid);
   if (rc != HB_OK) return rc;
-  return dispatch_fa(a, p, std::min(p.total_pairs, info.sm_count), info.smem_optin);
+  return dispatch_fa(a, p, grid, info.smem_optin);
 }
 
 // Reads (and then clears) the status word of the static scratch array on `stream`; waits for

@@ -19,12 +19,11 @@
 // written over the first 64 (16-bit) columns of S_i once the row is in registers.
 //
 // Work: a CTA handles 256 query rows of one (batch, head) at a time and walks a
-// static list of such blocks.  For causal attention block q and block (last-q) are
-// paired so that every list entry costs the same; the list is head-major so the
-// CTAs running at one time share K/V in L2.
+// static list of such blocks (tile_order.h).
 #pragma once
 
 #include "ptx_sm100.cuh"
+#include "tile_order.h"
 
 namespace hb {
 
@@ -95,8 +94,7 @@ struct alignas(64) FaParams {
   int group;        // Hq / Hkv
   int causal;
   int nqb;          // 256-row query blocks per head
-  int npairs;       // ceil(nqb / 2)
-  int total_pairs;  // B * Hq * npairs
+  TileOrder order;  // the work list: heads = B * Hq, blocks = nqb (rank 0 = the last block)
   int nkv;          // 128-key tiles
   float scale_log2; // softmax_scale * log2(e) (times q_scale * k_scale for FP8)
   float out_scale;  // multiplies O / l in the epilogue (v_scale / P scale for FP8, else 1)
@@ -125,13 +123,11 @@ struct FaItem {
   int n[2];  // key tiles each query tile visits (0 = tile entirely past Sq)
 };
 
-// Entry `g` of the static work list, first (half = 0) or second block of the pair.
+// Entry `g` of the static work list, first (half = 0) or second block where entries are pairs.
 __device__ __forceinline__ bool fa_get_item(const FaParams& p, int g, int half, FaItem& it) {
-  const int pair = g % p.npairs;
-  const int bh = g / p.npairs;
-  const int qb_hi = p.nqb - 1 - pair;
-  const int qb = half == 0 ? qb_hi : pair;
-  if (half == 1 && pair == qb_hi) return false;
+  int bh, rank;
+  if (!tile_order_get(p.order, g, half, static_cast<int>(gridDim.x), bh, rank)) return false;
+  const int qb = p.nqb - 1 - rank;
   it.b = bh / p.Hq;
   it.hq = bh - it.b * p.Hq;
   it.hkv = it.hq / p.group;
@@ -164,7 +160,7 @@ __device__ __forceinline__ void fa_softmax_role(const FaParams& p, FaSmem<T, D, 
   uint32_t s_cnt = 0, p_cnt = 0;  // completed s_full waits / own p_full arrivals
   HB_TRACE_DECL(p, warp)
 
-  for (int g = blockIdx.x; g < p.total_pairs; g += gridDim.x) {
+  for (int g = blockIdx.x; g < p.order.total; g += gridDim.x) {
     for (int half = 0; half < 2; ++half) {
       FaItem it;
       if (!fa_get_item(p, g, half, it)) continue;
@@ -315,7 +311,7 @@ __device__ __forceinline__ void fa_correction_role(const FaParams& p, FaSmem<T, 
   uint32_t c_cnt[2] = {0, 0}, o_cnt[2] = {0, 0};
   HB_TRACE_DECL(p, warp)
 
-  for (int g = blockIdx.x; g < p.total_pairs; g += gridDim.x) {
+  for (int g = blockIdx.x; g < p.order.total; g += gridDim.x) {
     for (int half = 0; half < 2; ++half) {
       FaItem it;
       if (!fa_get_item(p, g, half, it)) continue;
@@ -478,7 +474,7 @@ __device__ __forceinline__ void fa_mma_role(const FaParams& p, FaSmem<T, D, NS>&
   uint32_t q_phase = 0, p_phase = 0;  // bit i = parity of tile i's barrier
   HB_TRACE_DECL(p, 12)
 
-  for (int g = blockIdx.x; g < p.total_pairs; g += gridDim.x) {
+  for (int g = blockIdx.x; g < p.order.total; g += gridDim.x) {
     for (int half = 0; half < 2; ++half) {
       FaItem it;
       if (!fa_get_item(p, g, half, it)) continue;
@@ -554,7 +550,7 @@ __device__ __forceinline__ void fa_tma_role(const FaParams& p, FaSmem<T, D, NS>&
   constexpr int kSubElems = 128 / FaTraits<T>::kElemBytes;          // head_dim elements per sub-tile
   uint32_t slot = 0, phase = 1, q_phase[2] = {1, 1};  // "empty" barriers start out free
 
-  for (int g = blockIdx.x; g < p.total_pairs; g += gridDim.x) {
+  for (int g = blockIdx.x; g < p.order.total; g += gridDim.x) {
     for (int half = 0; half < 2; ++half) {
       FaItem it;
       if (!fa_get_item(p, g, half, it)) continue;

@@ -16,6 +16,7 @@
 // tile ahead) and reads them back as broadcast 16-byte loads.
 #include "host_common.h"
 #include "ptx_sm100.cuh"
+#include "tile_order.h"
 
 #include <algorithm>
 #include <cmath>
@@ -35,9 +36,8 @@ struct alignas(64) H2oParams {
   int B, Hq, Hkv, Sq, Skv;
   int group, causal;
   int nkb;         // 128-key tiles per head
-  int npairs;      // ceil(nkb / 2)
   int nqb;         // 128-query tiles
-  int total_items; // B * Hq * npairs
+  TileOrder order; // the work list: heads = B * Hq, blocks = nkb (rank 0 = the first)
   float scale_log2;
 };
 
@@ -58,15 +58,11 @@ struct H2oItem {
   int b, hq, hkv, k0, qt0;  // first key, first query tile that can see this key tile
 };
 
-// Entry `g` of the static work list, first (half = 0) or second key tile of the pair.  Under a
-// causal mask key tile kb is seen by nqb - qt0(kb) query tiles, so tile `pair` (many queries) and
-// tile nkb-1-pair (few) together cost the same for every pair: the persistent CTAs stay balanced.
+// Entry `g` of the static work list (tile_order.h), first (half = 0) or second key tile where entries are pairs.  Under a
+// causal mask key tile kb is seen by nqb - qt0(kb) query tiles: the first is the dearest.
 __device__ __forceinline__ bool h2o_get_item(const H2oParams& p, int g, int half, H2oItem& it) {
-  const int pair = g % p.npairs;
-  const int bh = g / p.npairs;
-  const int kb_hi = p.nkb - 1 - pair;
-  const int kb = half == 0 ? pair : kb_hi;
-  if (half == 1 && kb_hi == pair) return false;
+  int bh, kb;
+  if (!tile_order_get(p.order, g, half, static_cast<int>(gridDim.x), bh, kb)) return false;
   it.b = bh / p.Hq;
   it.hq = bh - it.b * p.Hq;
   it.hkv = it.hq / p.group;
@@ -121,7 +117,7 @@ __global__ void __launch_bounds__(kH2oThreads, 1) h2o_score_kernel(const __grid_
       // ---------------- TMA producer ----------------
       uint32_t st = 0, phase = 1, k_phase = 1;
       bool ok = true;
-      for (int u = 2 * blockIdx.x; ok && u < 2 * p.total_items; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1)) {
+      for (int u = 2 * blockIdx.x; ok && u < 2 * p.order.total; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1)) {
         H2oItem it;
         if (!h2o_get_item(p, u >> 1, u & 1, it)) continue;
         if (!mbar_wait(&s.k_empty, k_phase, ctx, kH2oTma)) break;
@@ -154,7 +150,7 @@ __global__ void __launch_bounds__(kH2oThreads, 1) h2o_score_kernel(const __grid_
       uint32_t st = 0, phase = 0, k_phase = 0, tile_i = 0;
       bool ok = true;
       const uint32_t k_lo = (smem_u32(s.k) >> 4) | kLbo;
-      for (int u = 2 * blockIdx.x; ok && u < 2 * p.total_items; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1)) {
+      for (int u = 2 * blockIdx.x; ok && u < 2 * p.order.total; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1)) {
         H2oItem it;
         if (!h2o_get_item(p, u >> 1, u & 1, it)) continue;
         if (!mbar_wait_warp(&s.k_full, k_phase, ctx, kH2oMma)) break;
@@ -205,7 +201,7 @@ __global__ void __launch_bounds__(kH2oThreads, 1) h2o_score_kernel(const __grid_
     bool ok = true;
     uint32_t tile_base = 0;  // global tile counter at the start of the item (same sequence as the MMA warp)
     const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2);
-    for (int u = 2 * blockIdx.x; ok && u < 2 * p.total_items; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1)) {
+    for (int u = 2 * blockIdx.x; ok && u < 2 * p.order.total; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1)) {
       H2oItem it;
       if (!h2o_get_item(p, u >> 1, u & 1, it)) continue;
       const int key = it.k0 + key_in_tile;
@@ -308,7 +304,6 @@ static int launch_h2o(const H2oParams& p, int grid, const DeviceState* st, cudaS
   HB_CUDA_CHECK(cudaGetLastError());
   return HB_OK;
 }
-
 static int h2o_impl(const hb_h2o_args* a) {
   if (a == nullptr) return set_error(HB_ERR_BAD_ARG, "hb_h2o_score: args is NULL");
   if (a->B < 0 || a->Hq <= 0 || a->Hkv <= 0 || a->Sq < 0 || a->Skv < 0 || a->D <= 0)
@@ -356,13 +351,11 @@ static int h2o_impl(const hb_h2o_args* a) {
   p.causal = a->causal ? 1 : 0;
   p.nkb = (a->Skv + 127) / 128;
   p.nqb = (a->Sq + 127) / 128;
-  p.npairs = (p.nkb + 1) / 2;
-  const long long total = (long long)a->B * a->Hq * p.npairs;
+  const long long total = (long long)a->B * a->Hq * ((p.nkb + 1) / 2);
   if (total > 0x3fffffffLL) return set_error(HB_ERR_UNSUPPORTED, "hb_h2o_score: problem too large");
-  p.total_items = (int)total;
   const float scale = a->softmax_scale > 0.f ? a->softmax_scale : 1.0f / sqrtf((float)a->D);
   p.scale_log2 = scale * 1.4426950408889634f;
-  const int grid = (int)std::min<long long>(total, st->sm_count);
+  const int grid = tile_order_fill(&p.order, (long long)a->B * a->Hq, p.nkb, p.causal != 0, 2.0 * a->Sq * a->D, st->sm_count);
   if (a->dtype == HB_BF16)
     return a->D == 128 ? launch_h2o<__nv_bfloat16, 128>(p, grid, st, stream) : launch_h2o<__nv_bfloat16, 64>(p, grid, st, stream);
   return a->D == 128 ? launch_h2o<__half, 128>(p, grid, st, stream) : launch_h2o<__half, 64>(p, grid, st, stream);

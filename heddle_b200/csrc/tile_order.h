@@ -1,0 +1,74 @@
+// Order in which the persistent attention kernels (forward, H2O score, both backward kernels) walk their work, one entry being
+// one block of rows or keys of one head.  Every CTA of the grid takes entries blockIdx.x, blockIdx.x + gridDim.x, ...
+//
+//   kOrderPairs   entry g is the PAIR (rank r, rank nb - 1 - r) of one head, where rank 0 is the block that costs most; under
+//                 a causal mask all pairs cost the same.  Head after head: few heads share L2 at one time.  Best when there are
+//                 many pairs per SM, else the last round of pairs leaves most of the chip idle.
+//   kOrderSnake   entries are single blocks, the dearest blocks of all heads first; odd rounds run backwards over the CTAs, so
+//                 a CTA that got a dear block gets a cheap one.  All heads are in flight at one time, so this is the order
+//                 where what they read stays in L2.
+//   kOrderHeads   single blocks, head after head (no mask: all blocks cost the same).
+//
+// us, pairs | single blocks (bf16, D 128): forward, causal, B2 Hq32 Hkv8 S3000 165 | 146, B1 H128 (Hkv16) S2023 196 | 161, B7 H8
+// S1077 on 1318 keys 72 | 43, B1 H8 S1287 43 | 30; unmasked B8 H12 S577 D64 46 | 28.  dQ, first case: 217 | 200.  With more
+// than L2 to share the pairs win: forward B8 H32 S2048 (268 MB) 291 | 310, dK/dV B1 H128 (Hkv16) S2023 (132 MB) 271 | 332.
+#pragma once
+
+#ifndef __CUDACC__
+#define HB_HD inline
+#else
+#define HB_HD __host__ __device__ __forceinline__
+#endif
+
+namespace hb {
+
+enum : int { kOrderPairs = 0, kOrderSnake = 1, kOrderHeads = 2 };
+
+struct TileOrder {
+  int heads, blocks;
+  int mode;
+  int npairs;           // kOrderPairs: ceil(blocks / 2)
+  int total;            // bound of the entry index (kOrderSnake: rounded up to whole rounds)
+};
+
+// Entry g of the list (half 0 or 1 of a pair): head and rank, or false where there is none.
+HB_HD bool tile_order_get(const TileOrder& o, int g, int half, int grid, int& head, int& rank) {
+  if (o.mode == kOrderPairs) {
+    head = g / o.npairs;
+    const int pair = g - head * o.npairs;
+    rank = half == 0 ? pair : o.blocks - 1 - pair;
+    return half == 0 || rank != pair;  // the middle block of an odd count is one entry
+  }
+  if (half != 0) return false;
+  if (o.mode == kOrderHeads) {
+    head = g / o.blocks;
+    rank = g - head * o.blocks;
+    return true;
+  }
+  const int round = g / grid, cta = g - round * grid;
+  const int u = round * grid + ((round & 1) ? grid - 1 - cta : cta);
+  if (u >= o.heads * o.blocks) return false;
+  rank = u / o.heads;
+  head = u - rank * o.heads;
+  return true;
+}
+
+// `bytes_per_head`: what the blocks of one head read in common.  Returns the grid size.
+inline int tile_order_fill(TileOrder* o, long long heads, int blocks, bool masked, double bytes_per_head, int sm_count) {
+  constexpr double kL2Budget = 96e6;  // of 126 MB: the rest is for what the blocks do not share
+  o->heads = static_cast<int>(heads);
+  o->blocks = blocks;
+  o->npairs = (blocks + 1) / 2;
+  const long long units = heads * blocks, pairs = heads * o->npairs;
+  o->mode = !masked ? kOrderHeads : heads * bytes_per_head <= kL2Budget ? kOrderSnake : kOrderPairs;
+  if (units > 0x3fff0000LL) o->mode = kOrderPairs;
+  if (o->mode == kOrderPairs) {
+    o->total = static_cast<int>(pairs);
+    return static_cast<int>(pairs < sm_count ? pairs : sm_count);
+  }
+  const int grid = static_cast<int>(units < sm_count ? units : sm_count);
+  o->total = static_cast<int>(o->mode == kOrderSnake ? (units + grid - 1) / grid * grid : units);
+  return grid;
+}
+
+}  // namespace hb
