@@ -338,6 +338,11 @@ static int gemm_impl(const hb_gemm_args* a) {
     return set_error(HB_ERR_UNSUPPORTED, "hb_gemm_epilogue: too many tiles");
   p.num_tiles = (int)tiles;
   p.batch = batch;
+  const int last_rows = p.tiles_m - (p.tiles_m - 1) / kGemmGroupM * kGemmGroupM;
+  p.div_batch = make_fast_div((uint32_t)p.tiles_per_batch);
+  p.div_group = make_fast_div((uint32_t)((long long)kGemmGroupM * p.tiles_n));
+  p.div_rows = make_fast_div(kGemmGroupM);
+  p.div_last = make_fast_div((uint32_t)last_rows);
   p.w_kn = w_kn ? 1 : 0;
   p.o_batch_stride = o_bs;
   p.r_batch_stride = r_bs;
@@ -347,10 +352,10 @@ static int gemm_impl(const hb_gemm_args* a) {
   p.head_dim = a->head_dim;
   p.rope_cols = a->rope_cols;
   p.w_row2_offset = n_out;
-  // shared-memory split of the pair kernel: a long K loop gets the deepest ring; a short one, whose time is
-  // the epilogue's, gives one stage to a second staging slab per warpgroup so that a tile's two slabs leave
-  // back to back (measured: 1, 2 and 4 slabs are within 2 % of each other, 4 costs the K = 512 case 10 %)
-  p.out_slabs = p.k_steps >= 8 ? 1 : 2;
+  // shared-memory split of the pair kernel: the deepest ring, except for a K loop of one or two steps, whose time is the
+  // epilogue's: it gives stages to staging slabs.  us with 1 | 2 | 4 slabs, 64 x [2048, K] . [K, 2048]: K = 128 125 | 123 | 114,
+  // K = 256 152 | 152 | 176, K = 384 191 | 196 | 229.
+  p.out_slabs = p.k_steps <= 2 ? 4 : 1;
   p.pair_stages = kPairSlots - p.out_slabs;
 
   const int grid = pair ? 2 * (int)std::min<long long>(tiles, st->sm_count / 2) : (int)std::min<long long>(tiles, st->sm_count);

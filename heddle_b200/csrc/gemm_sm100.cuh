@@ -47,6 +47,24 @@ enum GemmEpiClass : int { kEpiPlain = 0, kEpiSwiglu = 1, kEpiRope = 2 };
 enum GemmAct : int { kActNone = 0, kActSilu = 1, kActRelu = 2, kActGeluTanh = 3, kActSigmoid = 4, kActTanh = 5 };
 enum GemmRole : uint32_t { kGemmRoleTma = 0x21, kGemmRoleMma = 0x22, kGemmRoleEpi = 0x23, kGemmRoleDrain = 0x24 };
 
+// Exact n / d for 0 <= n < 2^31 with one high multiply (Granlund and Montgomery, "Division by invariant integers using
+// multiplication", 1994): three runtime divisions in front of every tile took each role of the persistent kernels 790 cycles,
+// 14 % of a short-K tile.
+struct FastDiv {
+  uint32_t mul, shift, d;
+};
+inline FastDiv make_fast_div(uint32_t d) {
+  FastDiv f;
+  f.d = d;
+  f.shift = 0;
+  while ((1ull << f.shift) < d) ++f.shift;
+  f.mul = static_cast<uint32_t>((((1ull << f.shift) - d) << 32) / d + 1);
+  return f;
+}
+__device__ __forceinline__ int fast_div(int n, const FastDiv& f) {
+  return static_cast<int>((__umulhi(static_cast<uint32_t>(n), f.mul) + static_cast<uint32_t>(n)) >> f.shift);
+}
+
 struct alignas(64) GemmParams {
   CUtensorMap tm_a;
   CUtensorMap tm_w;
@@ -67,11 +85,12 @@ struct alignas(64) GemmParams {
   int w_row2_offset;  // SWIGLU: first row of Wu inside the stacked weight
   int batch;          // number of independent products (>= 1)
   int tiles_per_batch;
+  FastDiv div_batch, div_group, div_rows, div_last;  // by tiles_per_batch, tiles of a rasterisation group, its M-tiles, the last group's
   int w_kn;           // 1: the second operand is [K, N] row-major
   long long o_batch_stride, r_batch_stride;  // elements between consecutive batches of out / residual
   int tma_store;      // PLAIN epilogue: results leave through shared memory and a TMA store
   int pair_stages;    // CTA-pair kernel: depth of the operand ring (3..6) ...
-  int out_slabs;      // ... and staging slabs per epilogue warpgroup (1, 2 or 4); stages + slabs = 7
+  int out_slabs;      // ... and staging slabs per epilogue warpgroup (1 or 4); stages + slabs = 7
 };
 
 struct GemmSmem {
@@ -87,15 +106,14 @@ struct GemmSmem {
 };
 
 __device__ __forceinline__ void gemm_tile_coords(const GemmParams& p, int t, int& m_t, int& n_t, int& b) {
-  b = t / p.tiles_per_batch;
+  b = fast_div(t, p.div_batch);
   t -= b * p.tiles_per_batch;
-  const int per_group = kGemmGroupM * p.tiles_n;
-  const int g = t / per_group;
+  const int g = fast_div(t, p.div_group);
   const int first_m = g * kGemmGroupM;
-  const int gsz = min(p.tiles_m - first_m, kGemmGroupM);
-  const int r = t - g * per_group;
-  m_t = first_m + r % gsz;
-  n_t = r / gsz;
+  const bool last = p.tiles_m - first_m <= kGemmGroupM;
+  const int r = t - g * static_cast<int>(p.div_group.d);
+  n_t = fast_div(r, last ? p.div_last : p.div_rows);
+  m_t = first_m + r - n_t * static_cast<int>(last ? p.div_last.d : p.div_rows.d);
 }
 
 __device__ __forceinline__ float apply_act(float v, int act) {
@@ -205,74 +223,75 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
     tc_fence_before();
     __syncwarp();
     if ((threadIdx.x & 31) == 0) mbar_arrive_cluster(release);
-    // Coalesced stores: the warpgroup's 128 rows x 64 columns go to shared memory in the 128-byte
-    // swizzled layout (a thread writes its own row: conflict-free), one thread hands the slab to the
-    // TMA, which clips rows past M and columns past N_out.  Two slabs per tile and warpgroup.
-    // The warpgroup owns a ring of `n_slabs` staging slabs; a slab is rewritten once the TMA store that
-    // last used it has read it (`wait_group.read` with n_slabs - 1 younger groups allowed in flight), so
-    // with several slabs the stores of consecutive slabs and tiles overlap (products with a short K loop
-    // are bound by this path).  Every slab commits a group, stored or not, to keep that count exact.
+    // Coalesced stores: 128 rows x 64 columns go to a slab of shared memory in the 128-byte swizzled layout (a thread writes
+    // its own row: conflict-free), one thread hands the slab to the TMA, which clips rows past M and columns past N_out.  The
+    // warpgroup owns a ring of `n_slabs` staging slabs; slabs are rewritten once the TMA store that last used them has read
+    // them.  With four, a tile's two slabs are one step (one pair of barriers, one group of stores) and the other two may
+    // still be on their way out.  Every step commits a group, stored or not, to keep the count of groups exact.
     const bool issuer = row_in_tile == 0;
     const bool raw = p.row_scale == nullptr && p.bias == nullptr && p.residual == nullptr && p.act == kActNone;
-#pragma unroll
-    for (int cc = 0; cc < 2; ++cc) {
-      const int col0 = n0 + part * (kGemmBN / 2) + cc * 64;
-      uint8_t* stage = stage_base + (slab_cursor % static_cast<uint32_t>(n_slabs)) * (kGemmBM * 128);
-      ++slab_cursor;
-      if (issuer) {
-        if (n_slabs == 1) tma_store_wait_read<0>();
-        else if (n_slabs == 2) tma_store_wait_read<1>();
-        else tma_store_wait_read<3>();
-      }
-      named_bar_sync(1 + part, 128);
+    const int per_step = n_slabs == 4 ? 2 : 1;
+    auto write_slab = [&](const uint32_t (&x)[32], const uint32_t (&y)[32], int col0, uint8_t* stage) {
       if (raw) {
         // nothing to apply: round and store (products with a short K loop are bound by this path's
         // instruction count, so it carries no scale, bias, activation or residual tests)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            const uint32_t* x = &r[cc * 2 + h][g * 8];
-            uint4 w;
-            w.x = Pack2<T>::pack(__uint_as_float(x[0]), __uint_as_float(x[1]));
-            w.y = Pack2<T>::pack(__uint_as_float(x[2]), __uint_as_float(x[3]));
-            w.z = Pack2<T>::pack(__uint_as_float(x[4]), __uint_as_float(x[5]));
-            w.w = Pack2<T>::pack(__uint_as_float(x[6]), __uint_as_float(x[7]));
-            const int chunk = (h * 4 + g) ^ (row_in_tile & 7);
-            *reinterpret_cast<uint4*>(stage + row_in_tile * 128 + chunk * 16) = w;
-          }
+        for (int g = 0; g < 8; ++g) {
+          const uint32_t* v = g < 4 ? &x[g * 8] : &y[(g - 4) * 8];
+          uint4 w;
+          w.x = Pack2<T>::pack(__uint_as_float(v[0]), __uint_as_float(v[1]));
+          w.y = Pack2<T>::pack(__uint_as_float(v[2]), __uint_as_float(v[3]));
+          w.z = Pack2<T>::pack(__uint_as_float(v[4]), __uint_as_float(v[5]));
+          w.w = Pack2<T>::pack(__uint_as_float(v[6]), __uint_as_float(v[7]));
+          *reinterpret_cast<uint4*>(stage + row_in_tile * 128 + (g ^ (row_in_tile & 7)) * 16) = w;
         }
-      } else {
+        return;
+      }
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int col = col0 + h * 32;
+      for (int g = 0; g < 8; ++g) {
+        const int col = col0 + g * 8;
+        const uint32_t* a = g < 4 ? &x[g * 8] : &y[(g - 4) * 8];
+        float v[8];
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          float v[8];
+        for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(a[e]) * rs;
+        if (p.bias != nullptr && col < p.N_out) {
+          float bb[8];
+          load_bias8<T>(p, col, bb);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[cc * 2 + h][g * 8 + e]) * rs;
-          const bool live = row_ok && col + g * 8 < p.N_out;
-          if (p.bias != nullptr && col + g * 8 < p.N_out) {
-            float bb[8];
-            load_bias8<T>(p, col + g * 8, bb);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] += bb[e];
-          }
-          if (p.act != kActNone) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] = apply_act(v[e], p.act);
-          }
-          if (live) add_residual8<T>(p, b, row, col + g * 8, v);
-          const int chunk = (h * 4 + g) ^ (row_in_tile & 7);
-          *reinterpret_cast<uint4*>(stage + row_in_tile * 128 + chunk * 16) = pack8<T>(v);
+          for (int e = 0; e < 8; ++e) v[e] += bb[e];
         }
+        if (p.act != kActNone) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] = apply_act(v[e], p.act);
+        }
+        if (row_ok && col < p.N_out) add_residual8<T>(p, b, row, col, v);
+        *reinterpret_cast<uint4*>(stage + row_in_tile * 128 + (g ^ (row_in_tile & 7)) * 16) = pack8<T>(v);
       }
+    };
+#pragma unroll
+    for (int cc = 0; cc < 2; ++cc) {
+      const int col0 = n0 + part * (kGemmBN / 2) + cc * 64;
+      const bool first = cc == 0 || per_step == 1, last = cc == 1 || per_step == 1;
+      uint8_t* stage = stage_base + (slab_cursor & static_cast<uint32_t>(n_slabs - 1)) * (kGemmBM * 128);
+      ++slab_cursor;
+      if (first) {
+        if (issuer) {
+          if (n_slabs == 1) tma_store_wait_read<0>();
+          else tma_store_wait_read<1>();
+        }
+        named_bar_sync(1 + part, 128);
       }
-      fence_proxy_async();
-      named_bar_sync(1 + part, 128);
-      if (issuer) {
-        if (col0 < p.N_out && m0 < p.M) tma_store_3d(&p.tm_out, stage, col0, m0, b);
-        tma_store_commit();
+      write_slab(r[cc * 2], r[cc * 2 + 1], col0, stage);
+      if (last) {
+        fence_proxy_async();
+        named_bar_sync(1 + part, 128);
+        if (issuer) {
+          if (m0 < p.M) {
+            if (per_step == 2 && col0 - 64 < p.N_out) tma_store_3d(&p.tm_out, stage - kGemmBM * 128, col0 - 64, m0, b);
+            if (col0 < p.N_out) tma_store_3d(&p.tm_out, stage, col0, m0, b);
+          }
+          tma_store_commit();
+        }
       }
     }
   } else if constexpr (EPI == kEpiSwiglu) {
