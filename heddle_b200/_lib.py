@@ -23,6 +23,8 @@ HB_BF16 = 0
 HB_FP16 = 1
 HB_FP8_E4M3 = 2
 
+HB_GEMM_ROPE_TABLES_16 = 0x100
+
 HB_W_NK = 0
 HB_W_KN = 1
 

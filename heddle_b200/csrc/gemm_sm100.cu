@@ -177,8 +177,12 @@ static int dispatch_gemm_split(int epi_class, const GemmSplitParams& p, int grid
 
 static bool aligned16(const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; }
 
-static int gemm_impl(const hb_gemm_args* a) {
-  if (a == nullptr) return set_error(HB_ERR_BAD_ARG, "hb_gemm_epilogue: args is NULL");
+static int gemm_impl(const hb_gemm_args* args) {
+  if (args == nullptr) return set_error(HB_ERR_BAD_ARG, "hb_gemm_epilogue: args is NULL");
+  hb_gemm_args copy = *args;
+  const hb_gemm_args* const a = &copy;
+  const bool rope16 = copy.epilogue == HB_EPI_ROPE && (copy.dtype & HB_GEMM_ROPE_TABLES_16) != 0;
+  if (rope16) copy.dtype &= ~HB_GEMM_ROPE_TABLES_16;
   if (a->M < 0 || a->N <= 0 || a->K <= 0)
     return set_error(HB_ERR_BAD_ARG, "hb_gemm_epilogue: bad extents M=%d N=%d K=%d", a->M, a->N, a->K);
   if (a->dtype != HB_BF16 && a->dtype != HB_FP16)
@@ -320,6 +324,7 @@ static int gemm_impl(const hb_gemm_args* a) {
   p.bias = a->bias;
   p.rope_cos = a->rope_cos;
   p.rope_sin = a->rope_sin;
+  p.rope16 = rope16 ? 1 : 0;
   p.status = st->status_word;
   p.ldo = a->ldo;
   p.ldr = a->ldr;

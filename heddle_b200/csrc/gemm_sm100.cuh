@@ -73,8 +73,9 @@ struct alignas(64) GemmParams {
   const float* row_scale;
   const void* residual;
   const void* bias;
-  const float* rope_cos;
-  const float* rope_sin;
+  const void* rope_cos;
+  const void* rope_sin;
+  int rope16;  // the tables are in the operands' 16-bit type, else fp32
   uint32_t* status;
   long long ldo, ldr;
   int M, N_out, K;
@@ -196,6 +197,26 @@ __device__ __forceinline__ void add_residual8(const GemmParams& p, int b, int ro
 template <typename T>
 __device__ __forceinline__ void load_bias8(const GemmParams& p, int col, float (&b)[8]) {
   unpack8<T>(*reinterpret_cast<const uint4*>(static_cast<const T*>(p.bias) + col), b);
+}
+
+// Eight consecutive entries of a cos / sin table from element `index` on (a multiple of 8: rows have head_dim / 2 entries,
+// a multiple of 32).
+template <typename T>
+__device__ __forceinline__ void load_angles8(const GemmParams& p, const void* table, long long index, float (&v)[8]) {
+  if (p.rope16) {
+    unpack8<T>(*reinterpret_cast<const uint4*>(static_cast<const T*>(table) + index), v);
+    return;
+  }
+  const float4* t = reinterpret_cast<const float4*>(static_cast<const float*>(table) + index);
+  const float4 a = t[0], b = t[1];
+  v[0] = a.x;
+  v[1] = a.y;
+  v[2] = a.z;
+  v[3] = a.w;
+  v[4] = b.x;
+  v[5] = b.y;
+  v[6] = b.z;
+  v[7] = b.w;
 }
 
 // Epilogue of one accumulator tile for the row owned by this thread.  `tacc` carries the
@@ -338,8 +359,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
   } else {  // kEpiRope
     const int hd = p.head_dim, half = hd >> 1;
     const int pos = row_ok ? (row % p.rope_seq) : 0;
-    const float* cosr = p.rope_cos + (long long)pos * half;
-    const float* sinr = p.rope_sin + (long long)pos * half;
+    const long long angles = (long long)pos * half;
     // two or more heads per tile: each warpgroup takes whole heads; one 256-wide head: each takes
     // half of the rotation pairs
     const bool split_heads = hd <= kGemmBN / 2;
@@ -369,12 +389,9 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
           }
         }
         if (rotate) {
-          // eight consecutive angles as two 16-byte loads per table (rows are 16-byte aligned:
-          // head_dim / 2 is a multiple of 32)
-          const float4 c0 = *reinterpret_cast<const float4*>(cosr + c + g * 8), c1 = *reinterpret_cast<const float4*>(cosr + c + g * 8 + 4);
-          const float4 s0 = *reinterpret_cast<const float4*>(sinr + c + g * 8), s1 = *reinterpret_cast<const float4*>(sinr + c + g * 8 + 4);
-          const float cs[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-          const float sn[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+          float cs[8], sn[8];
+          load_angles8<T>(p, p.rope_cos, angles + c + g * 8, cs);
+          load_angles8<T>(p, p.rope_sin, angles + c + g * 8, sn);
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
             const float xa = x1[e], xb = x2[e];

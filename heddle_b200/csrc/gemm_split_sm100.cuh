@@ -282,9 +282,10 @@ __global__ void __launch_bounds__(kGemmSplitThreads, 1) gemm_split_kernel(const 
         gemm_split_sum8(src + static_cast<uint32_t>(half) * 4u, part_bytes, splits, x2);
         gemm_split_scale_bias8<T>(p, rs, col + half, x2);
         if (col < p.rope_cols) {
-          const long long pos = row % p.rope_seq;
-          const float* cs = p.rope_cos + pos * half + c % half;
-          const float* sn = p.rope_sin + pos * half + c % half;
+          const long long angles = static_cast<long long>(row % p.rope_seq) * half + c % half;
+          float cs[8], sn[8];
+          load_angles8<T>(p, p.rope_cos, angles, cs);
+          load_angles8<T>(p, p.rope_sin, angles, sn);
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
             const float xa = v[e], xb = x2[e];

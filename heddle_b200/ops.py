@@ -338,7 +338,11 @@ def gemm_epilogue(a: torch.Tensor, w: torch.Tensor, epilogue: str = "none", *,
         if rope is None:
             raise ValueError("epilogue 'rope' needs rope=(cos, sin, head_dim, rope_cols)")
         cos, sin, hd, rope_cols = rope
-        cos, sin = _as_fp32(cos), _as_fp32(sin)
+        if cos.dtype is a.dtype and sin.dtype is a.dtype and cos.is_contiguous() and sin.is_contiguous() \
+                and (cos.data_ptr() | sin.data_ptr()) % 16 == 0:
+            g.dtype |= _lib.HB_GEMM_ROPE_TABLES_16  # read as they are: no conversion in front of every call
+        else:
+            cos, sin = _as_fp32(cos), _as_fp32(sin)
         _require_cuda(cos, sin)
         keep += [cos, sin]
         g.rope_cos, g.rope_sin = cos.data_ptr(), sin.data_ptr()

@@ -193,6 +193,9 @@ typedef enum hb_epilogue {
   HB_EPI_ROPE = 7
 } hb_epilogue;
 
+/* OR-ed into hb_gemm_args.dtype: the ROPE cos / sin tables are in the operands' 16-bit type instead of fp32. */
+#define HB_GEMM_ROPE_TABLES_16 0x100
+
 typedef enum hb_w_layout { HB_W_NK = 0, HB_W_KN = 1 } hb_w_layout;
 /* Which kernel runs the product.  AUTO: CTA pairs (two CTAs share a 256 x 256 tile through
  * tcgen05.mma.cta_group::2) when M > 128, else the single-CTA kernel (128 x 256 tiles), and for products
@@ -213,7 +216,7 @@ typedef struct hb_gemm_args {
   const void* bias;        /* optional [N] */
   const void* residual;    /* optional [M, N_out], row stride ldr */
   int64_t ldr;
-  const float* rope_cos;   /* ROPE: [rope_seq, head_dim/2] */
+  const float* rope_cos;   /* ROPE: [rope_seq, head_dim/2], fp32 (see HB_GEMM_ROPE_TABLES_16) */
   const float* rope_sin;
   int32_t rope_seq, head_dim;
   int32_t rope_cols;       /* ROPE: columns [0, rope_cols) are rotated, the rest copied */

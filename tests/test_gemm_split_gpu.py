@@ -83,3 +83,20 @@ def test_the_sum_over_the_cluster_has_one_order(ops):
     first = ops.gemm_epilogue(a, w)
     for _ in range(5):
         assert torch.equal(ops.gemm_epilogue(a, w), first)
+
+
+@pytest.mark.parametrize("schedule", ["single", "pair", "split"])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+def test_16_bit_rope_tables_are_read_as_they_are(ops, schedule, dt):
+    a, w, g = _mk(100, 512, 256, dt)
+    a, w, ang = a.cuda(), w.cuda(), torch.rand(40, 64, generator=g) * 6
+    cos, sin = ang.cos().to(dt).cuda(), ang.sin().to(dt).cuda()
+    prev = ops.set_gemm_schedule(schedule)
+    try:
+        out = ops.gemm_epilogue(a, w, "rope", rope=(cos, sin, 128, 384))
+        assert torch.equal(out, ops.gemm_epilogue(a, w, "rope", rope=(cos.float(), sin.float(), 128, 384)))
+        # a table that is not 16-byte aligned is converted first
+        off = torch.cat([cos.reshape(-1)[:1], cos.reshape(-1)])[1:].reshape(40, 64)
+        assert torch.equal(out, ops.gemm_epilogue(a, w, "rope", rope=(off, sin, 128, 384)))
+    finally:
+        ops.set_gemm_schedule(prev)
