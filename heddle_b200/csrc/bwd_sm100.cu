@@ -262,6 +262,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
   tc_fence_after();
   const uint32_t tmem = s.tmem_base;
   const bool run = (s.abort_flag == 0);
+  grid_launch_dependents();
+  grid_wait();
   const int past = p.Skv - p.Sq;
 
   // Work list (tile_order.h): u >> 1 is the entry, u & 1 its half where entries are pairs.  Under a causal mask key tile 0 is
@@ -616,6 +618,8 @@ __global__ void __launch_bounds__(kBwdDqThreads, 1) fa_bwd_dq_kernel(const __gri
   tc_fence_after();
   const uint32_t tmem = s.tmem_base;
   const bool run = (s.abort_flag == 0);
+  grid_launch_dependents();
+  grid_wait();
   const int past = p.Skv - p.Sq;
 
   // Work list (tile_order.h): u >> 1 is the entry, u & 1 its half where entries are pairs.  Under a causal mask the last query
@@ -885,6 +889,8 @@ __global__ void __launch_bounds__(256, 4) fa_bwd_preprocess_kernel(const T* __re
                                                                  long long o_sb, long long o_sh, long long o_ss,
                                                                  long long g_sb, long long g_sh, long long g_ss) {
   constexpr int kLanesPerRow = D / 8, kRowsPerLoad = 32 / kLanesPerRow, kRowsPerWarp = 4 * kRowsPerLoad;
+  grid_launch_dependents();
+  grid_wait();
   const int lane = threadIdx.x & 31, sub = lane / kLanesPerRow, lr = lane % kLanesPerRow;
   // the host checks that B * H * S fits 31 bits: 32-bit divisions (the 64-bit ones are emulated and were
   // a visible part of this short kernel)
@@ -982,8 +988,7 @@ static int bwd_launch(void (*kernel)(const BwdParams), const BwdParams& p, int g
     HB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
     configured[st->device & 63] = true;
   }
-  kernel<<<grid, threads, sizeof(Smem), stream>>>(p);
-  HB_CUDA_CHECK(cudaGetLastError());
+  HB_CUDA_CHECK(launch_dependent(kernel, grid, threads, sizeof(Smem), stream, 0, p));
   return HB_OK;
 }
 template <typename T, int D>
@@ -1001,10 +1006,9 @@ static int launch_preprocess(const hb_fa_bwd_args* a, cudaStream_t stream) {
   constexpr int kRowsPerBlock = 8 * 4 * (32 / (D / 8));
   const long long rows = (long long)a->B * a->Hq * a->Sq;
   const unsigned grid = (unsigned)((rows + kRowsPerBlock - 1) / kRowsPerBlock);
-  fa_bwd_preprocess_kernel<T, D><<<grid, 256, 0, stream>>>(static_cast<const T*>(a->o), static_cast<const T*>(a->d_o), a->delta,
-                                                          a->B, a->Hq, a->Sq, a->o_stride_b, a->o_stride_h, a->o_stride_s,
-                                                          a->do_stride_b, a->do_stride_h, a->do_stride_s);
-  HB_CUDA_CHECK(cudaGetLastError());
+  HB_CUDA_CHECK(launch_dependent(fa_bwd_preprocess_kernel<T, D>, grid, 256, 0, stream, 0, static_cast<const T*>(a->o),
+                                 static_cast<const T*>(a->d_o), a->delta, a->B, a->Hq, a->Sq, a->o_stride_b, a->o_stride_h,
+                                 a->o_stride_s, a->do_stride_b, a->do_stride_h, a->do_stride_s));
   return HB_OK;
 }
 

@@ -634,6 +634,8 @@ __global__ void __launch_bounds__(kFaThreads, 1) fa_fwd_kernel(const __grid_cons
   tc_fence_after();
   const uint32_t tmem = s.tmem_base;
   const bool run = (s.abort_flag == 0);
+  grid_launch_dependents();
+  grid_wait();
 #ifdef HB_FA_TRACE
   if (p.trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0) p.trace[15 * 4096 + 1] = clock64();
 #endif

@@ -79,21 +79,11 @@ static int launch_split(const FaSplitParams& p, int grid, bool combine, int smem
       configured[dev & 63] = true;
     }
   }
-  kernel<<<grid, kSplitThreads, sizeof(Smem), stream>>>(p);
-  HB_CUDA_CHECK(cudaGetLastError());
+  HB_CUDA_CHECK(launch_dependent(kernel, grid, kSplitThreads, sizeof(Smem), stream, 0, p));
   if (combine) {
-    // programmatic dependent launch: its blocks are in place when the last segment is written
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)p.items * (unsigned)p.rows);
     const long long segments = ((long long)p.pipes + p.items - 1) / p.items + 1;  // of one item, at most
-    cfg.blockDim = dim3(32 * (unsigned)std::min<long long>(kCombineMaxWarps, (segments + 3) / 4));
-    cfg.stream = stream;
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    HB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, fa_split_combine_kernel<T, D>, p));
+    const unsigned warps = (unsigned)std::min<long long>(kCombineMaxWarps, (segments + 3) / 4);
+    HB_CUDA_CHECK(launch_dependent(fa_split_combine_kernel<T, D>, (unsigned)p.items * (unsigned)p.rows, 32 * warps, 0, stream, 0, p));
   }
   return HB_OK;
 }

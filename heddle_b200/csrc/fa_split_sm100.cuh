@@ -390,8 +390,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) fa_split_kernel(const __grid
   tc_fence_after();
   const uint32_t tmem = s.tmem_base;
   const bool run = (s.abort_flag == 0);
-  // lets fa_split_combine_kernel's blocks be scheduled; they wait for this grid's results themselves
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  grid_launch_dependents();
+  grid_wait();
 
   // pipelines 0 of all CTAs come first, so a list shorter than 2 * gridDim.x runs is spread over all SMs
   const int i = warp < 8 ? warp >> 2 : (warp & 1);
@@ -431,7 +431,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) fa_split_kernel(const __grid
 constexpr int kCombineMaxWarps = 16;
 template <typename T, int D>
 __global__ void __launch_bounds__(kCombineMaxWarps * 32) fa_split_combine_kernel(const __grid_constant__ FaSplitParams p) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  grid_launch_dependents();
+  grid_wait();
   const int item = blockIdx.x / p.rows, row = blockIdx.x - item * p.rows;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const long long total = static_cast<long long>(p.items) * p.nkv, t0 = static_cast<long long>(item) * p.nkv;

@@ -19,8 +19,7 @@ static int launch_gemm(const GemmParams& p, int grid, const DeviceState* st, cud
     HB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GemmSmem)));
     configured[st->device & 63] = true;
   }
-  kernel<<<grid, kGemmThreads, sizeof(GemmSmem), stream>>>(p);
-  HB_CUDA_CHECK(cudaGetLastError());
+  HB_CUDA_CHECK(launch_dependent(kernel, grid, kGemmThreads, sizeof(GemmSmem), stream, 0, p));
   return HB_OK;
 }
 
@@ -35,8 +34,7 @@ static int launch_gemm_pair(const GemmParams& p, int grid, const DeviceState* st
     HB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes));
     configured[st->device & 63] = true;
   }
-  kernel<<<grid, kGemmThreads, kPairSmemBytes, stream>>>(p);  // clusters of two CTAs (compile-time attribute)
-  HB_CUDA_CHECK(cudaGetLastError());
+  HB_CUDA_CHECK(launch_dependent(kernel, grid, kGemmThreads, kPairSmemBytes, stream, 0, p));  // clusters of two (compile-time)
   return HB_OK;
 }
 
@@ -148,18 +146,7 @@ static int launch_gemm_split(const GemmSplitParams& p, int grid, const DeviceSta
     HB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSplitSmemBytes));
     configured[st->device & 63] = true;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3(kGemmSplitThreads);
-  cfg.dynamicSmemBytes = kGemmSplitSmemBytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr = {};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = (unsigned)p.splits;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  HB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, p));
+  HB_CUDA_CHECK(launch_dependent(kernel, grid, kGemmSplitThreads, kGemmSplitSmemBytes, stream, (unsigned)p.splits, p));
   return HB_OK;
 }
 
@@ -397,14 +384,13 @@ static int rowstat_impl(const void* x, const void* residual, void* y_out, float*
   const int grid = (M + 7) / 8;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype == HB_BF16) {
-    rms_rowstat_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(residual),
-        static_cast<__nv_bfloat16*>(y_out), rstd, M, N, ldx, eps);
+    HB_CUDA_CHECK(launch_dependent(rms_rowstat_kernel<__nv_bfloat16>, grid, 256, 0, s, 0, static_cast<const __nv_bfloat16*>(x),
+                                   static_cast<const __nv_bfloat16*>(residual), static_cast<__nv_bfloat16*>(y_out), rstd, M, N,
+                                   ldx, eps));
   } else {
-    rms_rowstat_kernel<__half><<<grid, 256, 0, s>>>(static_cast<const __half*>(x), static_cast<const __half*>(residual),
-                                                    static_cast<__half*>(y_out), rstd, M, N, ldx, eps);
+    HB_CUDA_CHECK(launch_dependent(rms_rowstat_kernel<__half>, grid, 256, 0, s, 0, static_cast<const __half*>(x),
+                                   static_cast<const __half*>(residual), static_cast<__half*>(y_out), rstd, M, N, ldx, eps));
   }
-  HB_CUDA_CHECK(cudaGetLastError());
   return HB_OK;
 }
 

@@ -474,6 +474,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
   tc_fence_after();
   const uint32_t tmem = s.tmem_base;
   const bool run = (s.abort_flag == 0);
+  grid_launch_dependents();
+  grid_wait();
 
   if (warp == 0) {
     if (run && lane == 0) {
@@ -691,6 +693,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
   tc_fence_after();
   const uint32_t tmem = s.tmem_base;
   const bool run = (s.abort_flag == 0);
+  grid_launch_dependents();
+  grid_wait();
 
   if (warp == 0) {
     if (run && lane == 0) {
@@ -850,6 +854,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) rms_rowstat_kernel(const T* __restrict__ x, const T* __restrict__ residual,
                                                           T* __restrict__ y_out, float* __restrict__ rstd, int M,
                                                           int N, long long ldx, float eps) {
+  grid_launch_dependents();
+  grid_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * 8 + warp;
   if (row >= M) return;

@@ -124,6 +124,8 @@ __global__ void __launch_bounds__(kGemmSplitThreads, 1) gemm_split_kernel(const 
   tc_fence_after();
   const uint32_t tmem = s.tmem_base;
   const bool run = (s.abort_flag == 0);
+  grid_launch_dependents();
+  grid_wait();
 
   int m_t, n_t, b;
   gemm_tile_coords(p, t, m_t, n_t, b);

@@ -107,6 +107,8 @@ __global__ void __launch_bounds__(kH2oThreads, 1) h2o_score_kernel(const __grid_
   tc_fence_after();
   const uint32_t tmem = s.tmem_base;
   const bool run = (s.abort_flag == 0);
+  grid_launch_dependents();
+  grid_wait();
   constexpr uint32_t kTileBytes = Smem::kTileBytes;
   constexpr uint32_t kHalfBytes = 128 * 128;
 
@@ -300,8 +302,7 @@ static int launch_h2o(const H2oParams& p, int grid, const DeviceState* st, cudaS
     HB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
     configured[st->device & 63] = true;
   }
-  kernel<<<grid, kH2oThreads, sizeof(Smem), stream>>>(p);
-  HB_CUDA_CHECK(cudaGetLastError());
+  HB_CUDA_CHECK(launch_dependent(kernel, grid, kH2oThreads, sizeof(Smem), stream, 0, p));
   return HB_OK;
 }
 static int h2o_impl(const hb_h2o_args* a) {

@@ -47,6 +47,31 @@ struct DeviceInfo {
 };
 int get_device_info_noalloc(DeviceInfo* out);
 
+// Launches `kernel` so that its start-up (launch latency, barrier and TMEM set-up, descriptor fetch) may run under the tail
+// of the stream's previous kernel: programmatic dependent launch.  The kernel calls grid_wait() before it touches memory.
+// `cluster` > 0 sets a run-time cluster size.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_dependent(void (*kernel)(Params...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream,
+                                    unsigned cluster, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attrs[2] = {};
+  attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attrs;
+  cfg.numAttrs = 1;
+  if (cluster > 0) {
+    attrs[1].id = cudaLaunchAttributeClusterDimension;
+    attrs[1].val.clusterDim.x = cluster;
+    attrs[1].val.clusterDim.y = attrs[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+  }
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 // 2-D .. 4-D tiled tensor map with 128-byte swizzle, zero fill out of bounds.
 //   dims[i]     extent of dimension i in elements (dimension 0 is contiguous)
 //   strides[i]  byte stride of dimension i+1

@@ -42,6 +42,14 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// Programmatic dependent launch (launch_dependent() in host_common.h): the next kernel of the stream may be scheduled from
+// grid_launch_dependents() on, and waits in grid_wait() until every earlier kernel is complete and its writes are visible.
+// No kernel touches global memory (its parameters aside) before grid_wait().  A kernel that holds TMEM calls
+// grid_launch_dependents() only after its own allocation: a dependent that took the columns first would wait for this grid,
+// and this grid for the columns.
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 template <int N>
 __device__ __forceinline__ void reg_inc() {
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(N));

@@ -82,7 +82,7 @@ bool load_nvrtc() {
 struct Driver {
   CUresult (*module_load)(CUmodule*, const void*) = nullptr;
   CUresult (*get_function)(CUfunction*, CUmodule, const char*) = nullptr;
-  CUresult (*launch)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, CUstream, void**, void**) = nullptr;
+  CUresult (*launch)(const CUlaunchConfig*, CUfunction, void**, void**) = nullptr;
   bool ok = false;
 };
 Driver g_driver;
@@ -94,7 +94,7 @@ int load_driver() {
     void** slot;
   } wanted[] = {{"cuModuleLoadData", reinterpret_cast<void**>(&g_driver.module_load)},
                 {"cuModuleGetFunction", reinterpret_cast<void**>(&g_driver.get_function)},
-                {"cuLaunchKernel", reinterpret_cast<void**>(&g_driver.launch)}};
+                {"cuLaunchKernelEx", reinterpret_cast<void**>(&g_driver.launch)}};
   for (auto& w : wanted) {
     void* fn = nullptr;
     cudaDriverEntryPointQueryResult qres;
@@ -193,6 +193,8 @@ __device__ __forceinline__ void round16(float* a) {
 
 const char* kStreamKernel = R"SRC(
 extern "C" __global__ void __launch_bounds__(THREADS) rowprog_jit(const __grid_constant__ Head p) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const unsigned groups = static_cast<unsigned>(p.cols >> 3);
   const unsigned total = static_cast<unsigned>(p.rows) * groups;
   const float red[4] = {0.f, 0.f, 0.f, 0.f};
@@ -216,6 +218,8 @@ extern "C" __global__ void __launch_bounds__(THREADS) rowprog_jit(const __grid_c
 
 const char* kReduceKernel = R"SRC(
 extern "C" __global__ void __launch_bounds__(THREADS) rowprog_jit(const __grid_constant__ Head p) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   constexpr int W = HB_WARPS_PER_ROW;
   constexpr int TPR = 32 * W;
   __shared__ float part[4];
@@ -470,9 +474,21 @@ int rowprog_jit_launch(const RowProgParams& p, bool bf16, const DeviceState& st,
   }
   RowProgHead head = p;
   void* params[] = {&head};
-  const CUresult cr = g_driver.launch(fn, grid, 1, 1, kJitThreads, 1, 1, 0, stream, params, nullptr);
+  // programmatic dependent launch: the kernel waits for its predecessors itself
+  CUlaunchAttribute attr = {};
+  attr.id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+  attr.value.programmaticStreamSerializationAllowed = 1;
+  CUlaunchConfig cfg = {};
+  cfg.gridDimX = grid;
+  cfg.gridDimY = cfg.gridDimZ = 1;
+  cfg.blockDimX = kJitThreads;
+  cfg.blockDimY = cfg.blockDimZ = 1;
+  cfg.hStream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const CUresult cr = g_driver.launch(&cfg, fn, params, nullptr);
   if (cr != CUDA_SUCCESS) {
-    set_error(HB_ERR_CUDA, "hb_rowwise_program: cuLaunchKernel failed (%d)", (int)cr);
+    set_error(HB_ERR_CUDA, "hb_rowwise_program: cuLaunchKernelEx failed (%d)", (int)cr);
     return kJitError;
   }
   return kJitLaunched;

@@ -48,6 +48,8 @@ template <typename T, int kChunks, int kWarpsPerRow>
 __global__ void __launch_bounds__(256) row_softmax_kernel(const T* __restrict__ x, T* __restrict__ y, long long rows,
                                                           int cols, long long ld_x, long long ld_y, float scale_log2) {
   constexpr int kThreadsPerRow = 32 * kWarpsPerRow;
+  grid_launch_dependents();
+  grid_wait();
   __shared__ float red[2][8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long row = kWarpsPerRow == 1 ? (blockIdx.x * 8ll + warp) : static_cast<long long>(blockIdx.x);
@@ -116,19 +118,19 @@ static int launch_row_softmax(const T* x, T* y, long long rows, int cols, long l
   if (chunks <= 32 * 8) {
     const unsigned grid = static_cast<unsigned>((rows + 7) / 8);
     if (chunks <= 32 * 2)
-      row_softmax_kernel<T, 2, 1><<<grid, 256, 0, stream>>>(x, y, rows, cols, ld_x, ld_y, scale_log2);
+      HB_CUDA_CHECK(launch_dependent(row_softmax_kernel<T, 2, 1>, grid, 256, 0, stream, 0, x, y, rows, cols, ld_x, ld_y, scale_log2));
     else if (chunks <= 32 * 4)
-      row_softmax_kernel<T, 4, 1><<<grid, 256, 0, stream>>>(x, y, rows, cols, ld_x, ld_y, scale_log2);
+      HB_CUDA_CHECK(launch_dependent(row_softmax_kernel<T, 4, 1>, grid, 256, 0, stream, 0, x, y, rows, cols, ld_x, ld_y, scale_log2));
     else
-      row_softmax_kernel<T, 8, 1><<<grid, 256, 0, stream>>>(x, y, rows, cols, ld_x, ld_y, scale_log2);
+      HB_CUDA_CHECK(launch_dependent(row_softmax_kernel<T, 8, 1>, grid, 256, 0, stream, 0, x, y, rows, cols, ld_x, ld_y, scale_log2));
   } else {
     const unsigned grid = static_cast<unsigned>(rows);
     if (chunks <= 256 * 2)
-      row_softmax_kernel<T, 2, 8><<<grid, 256, 0, stream>>>(x, y, rows, cols, ld_x, ld_y, scale_log2);
+      HB_CUDA_CHECK(launch_dependent(row_softmax_kernel<T, 2, 8>, grid, 256, 0, stream, 0, x, y, rows, cols, ld_x, ld_y, scale_log2));
     else if (chunks <= 256 * 4)
-      row_softmax_kernel<T, 4, 8><<<grid, 256, 0, stream>>>(x, y, rows, cols, ld_x, ld_y, scale_log2);
+      HB_CUDA_CHECK(launch_dependent(row_softmax_kernel<T, 4, 8>, grid, 256, 0, stream, 0, x, y, rows, cols, ld_x, ld_y, scale_log2));
     else
-      row_softmax_kernel<T, 8, 8><<<grid, 256, 0, stream>>>(x, y, rows, cols, ld_x, ld_y, scale_log2);
+      HB_CUDA_CHECK(launch_dependent(row_softmax_kernel<T, 8, 8>, grid, 256, 0, stream, 0, x, y, rows, cols, ld_x, ld_y, scale_log2));
   }
   HB_CUDA_CHECK(cudaGetLastError());
   return HB_OK;
