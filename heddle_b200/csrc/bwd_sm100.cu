@@ -78,7 +78,11 @@ struct alignas(64) BwdParams {
   int B, Hq, Hkv, Sq, Skv;
   int group, causal;
   int nkb, nqb;     // 128-row key / query tiles
-  TileOrder order;  // the work list: dkdv heads B * Hkv, blocks nkb, rank 0 = the first; dq heads B * Hq, blocks nqb, rank 0 = the last
+  // dkdv: the query heads of a KV head are dealt out to `splits` items, each with group / splits heads; with more than one, dK
+  // and dV go to `part` ([splits][dK, dV][B, Hkv, Skv, D], fp32) and fa_bwd_combine_kernel adds them up
+  int splits;
+  float* part;
+  TileOrder order;  // the work list: dkdv heads B * Hkv * splits, blocks nkb, rank 0 = the first; dq heads B * Hq, blocks nqb, rank 0 = the last
   float scale_log2, scale;
 };
 
@@ -268,9 +272,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
 
   // Work list (tile_order.h): u >> 1 is the entry, u & 1 its half where entries are pairs.  Under a causal mask key tile 0 is
   // seen by the most queries.
-  auto item_of = [&](int u, int& b, int& hkv, int& k0, int& qt0) -> bool {
+  const int heads = p.group / p.splits;  // query heads of an item
+  auto item_of = [&](int u, int& b, int& hkv, int& hq0, int& k0, int& qt0) -> bool {
     int bh, kb;
     if (!tile_order_get(p.order, u >> 1, u & 1, static_cast<int>(gridDim.x), bh, kb)) return false;
+    hq0 = bh % (p.Hkv * p.splits) * heads;
+    bh /= p.splits;
     b = bh / p.Hkv;
     hkv = bh - b * p.Hkv;
     k0 = kb * 128;
@@ -284,8 +291,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
       uint32_t cnt = 0, f_phase = 1;  // cnt: steps loaded so far (stage = cnt & 1 in both rings)
       bool ok = true;
       for (int u = 2 * blockIdx.x; ok && u < 2 * p.order.total; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1)) {
-        int b, hkv, k0, qt0;
-        if (!item_of(u, b, hkv, k0, qt0)) continue;
+        int b, hkv, hq0, k0, qt0;
+        if (!item_of(u, b, hkv, hq0, k0, qt0)) continue;
         if (!mbar_wait(&s.fixed_empty, f_phase, ctx, kBwdTma)) break;
         f_phase ^= 1;
         mbar_arrive_expect_tx(&s.fixed_full, 2 * kBwdTileBytes);
@@ -294,8 +301,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
           tma_load_4d(s.fixed[0] + hh * (128 * 128), &p.tm_k, &s.fixed_full, hh * 64, k0, hkv, b);
           tma_load_4d(s.fixed[1] + hh * (128 * 128), &p.tm_v, &s.fixed_full, hh * 64, k0, hkv, b);
         }
-        for (int hg = 0; ok && hg < p.group; ++hg) {
-          const int hq = hkv * p.group + hg;
+        for (int hg = 0; ok && hg < heads; ++hg) {
+          const int hq = hq0 + hg;
           for (int qt = qt0; qt < p.nqb; ++qt, ++cnt) {
             const uint32_t st = cnt & 1u, ph = ((cnt >> 1) & 1u) ^ 1u;
             if (!mbar_wait(&s.a_empty[st], ph, ctx, kBwdTma)) {
@@ -323,12 +330,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
       auto full_a = [&](uint32_t c) { return mbar_wait_warp(&s.a_full[c & 1u], (c >> 1) & 1u, ctx, kBwdMma); };
       auto full_b = [&](uint32_t c) { return mbar_wait_warp(&s.b_full[c & 1u], (c >> 1) & 1u, ctx, kBwdMma); };
       for (int u = 2 * blockIdx.x; ok && u < 2 * p.order.total; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1), ++items) {
-        int b, hkv, k0, qt0;
-        if (!item_of(u, b, hkv, k0, qt0)) {
+        int b, hkv, hq0, k0, qt0;
+        if (!item_of(u, b, hkv, hq0, k0, qt0)) {
           --items;  // not an item: keep the count of real items
           continue;
         }
-        const int n_steps = p.group * (p.nqb - qt0);
+        const int n_steps = heads * (p.nqb - qt0);
         if (!mbar_wait_warp(&s.fixed_full, f_phase, ctx, kBwdMma)) break;
         f_phase ^= 1;
         // prologue: S(0), dP(0)
@@ -436,14 +443,14 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
     uint32_t cnt = 0, items = 0;
     bool ok = true;
     for (int u = 2 * blockIdx.x; ok && u < 2 * p.order.total; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1), ++items) {
-      int b, hkv, k0, qt0;
-      if (!item_of(u, b, hkv, k0, qt0)) {
+      int b, hkv, hq0, k0, qt0;
+      if (!item_of(u, b, hkv, hq0, k0, qt0)) {
         --items;  // not an item: keep the count of real items
         continue;
       }
       const int key = k0 + key_in_tile;
-      for (int hg = 0; ok && hg < p.group; ++hg) {
-        const int hq = hkv * p.group + hg;
+      for (int hg = 0; ok && hg < heads; ++hg) {
+        const int hq = hq0 + hg;
         const float* lse_row = p.lse + (static_cast<long long>(b) * p.Hq + hq) * p.Sq;
         const float* dl_row = p.delta + (static_cast<long long>(b) * p.Hq + hq) * p.Sq;
         for (int qt = qt0; qt < p.nqb; ++qt, ++cnt) {
@@ -562,19 +569,28 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
       tc_fence_after();
       const bool live = key < p.Skv;
       const uint32_t col_acc = static_cast<uint32_t>(half * (D / 2));
-      T* dv_row = static_cast<T*>(p.dv) + ((static_cast<long long>(b) * p.Hkv + hkv) * p.Skv + key) * D + col_acc;
-      T* dk_row = static_cast<T*>(p.dk) + ((static_cast<long long>(b) * p.Hkv + hkv) * p.Skv + key) * D + col_acc;
+      const long long row_of = ((static_cast<long long>(b) * p.Hkv + hkv) * p.Skv + key) * D + col_acc;
+      const long long all = static_cast<long long>(p.B) * p.Hkv * p.Skv * D;
+      float* const part = p.splits > 1 ? p.part + (hq0 - hkv * p.group) / heads * 2 * all + row_of : nullptr;
 #pragma unroll 1
       for (int c = 0; c < D / 64; ++c) {
         uint32_t r[32];
-        __syncwarp();
-        tmem_ld32(tmem + lane_off + 256 + col_acc + c * 32, r);
-        tmem_wait_ld();
-        if (live) bwd_store_row<T>(dv_row + c * 32, r, 1.0f);
-        __syncwarp();
-        tmem_ld32(tmem + lane_off + 384 + col_acc + c * 32, r);
-        tmem_wait_ld();
-        if (live) bwd_store_row<T>(dk_row + c * 32, r, p.scale);
+#pragma unroll 1
+        for (int w = 0; w < 2; ++w) {  // dK, dV
+          __syncwarp();
+          tmem_ld32(tmem + lane_off + (w == 0 ? 384u : 256u) + col_acc + c * 32, r);
+          tmem_wait_ld();
+          const float scale = w == 0 ? p.scale : 1.0f;
+          if (live && part == nullptr) {
+            bwd_store_row<T>(static_cast<T*>(w == 0 ? p.dk : p.dv) + row_of + c * 32, r, scale);
+          } else if (live) {
+            float4* dst = reinterpret_cast<float4*>(part + w * all + c * 32);
+#pragma unroll
+            for (int e = 0; e < 32; e += 4)
+              dst[e / 4] = make_float4(__uint_as_float(r[e]) * scale, __uint_as_float(r[e + 1]) * scale,
+                                       __uint_as_float(r[e + 2]) * scale, __uint_as_float(r[e + 3]) * scale);
+          }
+        }
       }
       tc_fence_before();
       __syncwarp();
@@ -923,6 +939,36 @@ __global__ void __launch_bounds__(256, 4) fa_bwd_preprocess_kernel(const T* __re
   }
 }
 
+// dK, dV = the sum over the splits of fa_bwd_dkdv_kernel's partial results, in split order; blockIdx.y: 0 dK, 1 dV.
+template <typename T>
+__global__ void __launch_bounds__(256) fa_bwd_combine_kernel(const float* __restrict__ part, T* __restrict__ dk, T* __restrict__ dv,
+                                                            long long all, int splits) {
+  grid_launch_dependents();
+  grid_wait();
+  const long long i = (static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) * 8;
+  if (i >= all) return;
+  const float* src = part + blockIdx.y * all + i;
+  float v[8] = {};
+#pragma unroll 4
+  for (int k = 0; k < splits; ++k, src += 2 * all) {
+    const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+    v[0] += a.x;
+    v[1] += a.y;
+    v[2] += a.z;
+    v[3] += a.w;
+    v[4] += b.x;
+    v[5] += b.y;
+    v[6] += b.z;
+    v[7] += b.w;
+  }
+  uint4 w;
+  w.x = Pack2<T>::pack(v[0], v[1]);
+  w.y = Pack2<T>::pack(v[2], v[3]);
+  w.z = Pack2<T>::pack(v[4], v[5]);
+  w.w = Pack2<T>::pack(v[6], v[7]);
+  *reinterpret_cast<uint4*>((blockIdx.y == 0 ? dk : dv) + i) = w;
+}
+
 // ------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------
@@ -978,6 +1024,31 @@ static int bwd_fill(const hb_fa_bwd_args* a, BwdParams& p, const DeviceState* st
   return HB_OK;
 }
 
+// Into how many items the query heads of a KV head are dealt out for dK / dV (a divisor of the group size).  An item walks its
+// heads one after the other, so with few KV heads the items are few and long.  Estimated time in steps of one 128 x 128 tile
+// (1.7 us): the rounds of items, or the longest item; partial results cost a launch and their bytes (write and read in fp32,
+// about 4 MB a us).  us, one item | split: causal bf16 D128 B1 Hq32 Hkv4 S2000 189 | 75, B1 Hq8 Hkv1 S8192 729 | 220; unmasked
+// D64 B4 Hq16 Hkv2 S512 57 | 24; B2 Hq32 Hkv8 S3000 stays at one (340).
+static int bwd_dkdv_splits(const hb_fa_bwd_args* a, int sm_count) {
+  const int group = a->Hq / a->Hkv;
+  const double nkb = (a->Skv + 127) / 128, nqb = (a->Sq + 127) / 128;
+  const double mean = a->causal && a->Skv == a->Sq ? (nqb + 1) / 2 : nqb;  // query tiles that a key tile sees
+  int best = 1;
+  double best_cost = 0;
+  for (int splits = 1; splits <= group; ++splits) {
+    if (group % splits != 0) continue;
+    const double items = (double)a->B * a->Hkv * splits * nkb, heads = group / splits;
+    const double rounds = a->causal ? items / sm_count : (double)(((long long)items + sm_count - 1) / sm_count);
+    const double bytes = splits > 1 ? 16.0 * splits * a->B * a->Hkv * a->Skv * a->D : 0.0;
+    const double cost = std::max(rounds * heads * mean, heads * nqb) + (splits > 1 ? 2.0 + bytes / 4e6 / 1.7 : 0.0);
+    if (splits == 1 || cost < 0.9 * best_cost) {
+      best = splits;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
 template <typename Smem>
 static int bwd_launch(void (*kernel)(const BwdParams), const BwdParams& p, int grid, int threads, const DeviceState* st,
                       cudaStream_t stream, bool* configured) {
@@ -995,6 +1066,21 @@ template <typename T, int D>
 static int launch_dkdv(const BwdParams& p, int grid, const DeviceState* st, cudaStream_t stream) {
   static bool configured[64] = {};
   return bwd_launch<BwdSmemKv<D>>(fa_bwd_dkdv_kernel<T, D>, p, grid, kBwdThreads, st, stream, configured);
+}
+template <typename T>
+static int launch_combine(const BwdParams& p, long long all, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>((all / 8 + 255) / 256), 2);
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  HB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, fa_bwd_combine_kernel<T>, static_cast<const float*>(p.part), static_cast<T*>(p.dk),
+                                   static_cast<T*>(p.dv), all, p.splits));
+  return HB_OK;
 }
 template <typename T, int D>
 static int launch_dq(const BwdParams& p, int grid, const DeviceState* st, cudaStream_t stream) {
@@ -1035,7 +1121,7 @@ extern "C" int hb_fa_bwd_preprocess(const hb_fa_bwd_args* a) {
   return a->D == 128 ? launch_preprocess<__half, 128>(a, stream) : launch_preprocess<__half, 64>(a, stream);
 }
 
-extern "C" int hb_fa_bwd_dkdv(const hb_fa_bwd_args* a) {
+static int bwd_dkdv_impl(const hb_fa_bwd_args* a, bool ws, void* workspace, uint64_t workspace_bytes) {
   using namespace hb;
   clear_error();
   int rc = bwd_check(a, "hb_fa_bwd_dkdv");
@@ -1059,16 +1145,48 @@ extern "C" int hb_fa_bwd_dkdv(const hb_fa_bwd_args* a) {
   BwdParams p;
   rc = bwd_fill(a, p, st);
   if (rc != HB_OK) return rc;
-  const long long total = (long long)a->B * a->Hkv * ((p.nkb + 1) / 2);
-  if (total > 0x3fffffffLL) return set_error(HB_ERR_UNSUPPORTED, "hb_fa_bwd_dkdv: problem too large");
+  p.splits = ws ? bwd_dkdv_splits(a, st->sm_count) : 1;
+  const long long all = (long long)a->B * a->Hkv * a->Skv * a->D;
+  const uint64_t need = p.splits > 1 ? 8ull * p.splits * all : 0;
+  if (need > 0 && (workspace == nullptr || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15) != 0))
+    return set_error(HB_ERR_BAD_ARG, "hb_fa_bwd_dkdv_ws: needs a 16-byte aligned workspace of %llu bytes, got %llu",
+                     (unsigned long long)need, (unsigned long long)workspace_bytes);
+  p.part = static_cast<float*>(workspace);
+  const long long heads = (long long)a->B * a->Hkv * p.splits;
+  if (heads * ((p.nkb + 1) / 2) > 0x3fffffffLL) return set_error(HB_ERR_UNSUPPORTED, "hb_fa_bwd_dkdv: problem too large");
   // a key tile reads Q and dO of its query heads
-  int grid = tile_order_fill(&p.order, (long long)a->B * a->Hkv, p.nkb, p.causal != 0, 4.0 * a->Sq * a->D * p.group, st->sm_count);
+  int grid = tile_order_fill(&p.order, heads, p.nkb, p.causal != 0, 4.0 * a->Sq * a->D * p.group / p.splits, st->sm_count);
 #ifdef HB_DEBUG_GRID_ENV  // measurement builds only: fewer CTAs than SMs
   if (const char* e = getenv("HB_GRID")) grid = std::max(1, std::min(grid, atoi(e)));
 #endif
   if (a->dtype == HB_BF16)
-    return a->D == 128 ? launch_dkdv<__nv_bfloat16, 128>(p, grid, st, stream) : launch_dkdv<__nv_bfloat16, 64>(p, grid, st, stream);
-  return a->D == 128 ? launch_dkdv<__half, 128>(p, grid, st, stream) : launch_dkdv<__half, 64>(p, grid, st, stream);
+    rc = a->D == 128 ? launch_dkdv<__nv_bfloat16, 128>(p, grid, st, stream) : launch_dkdv<__nv_bfloat16, 64>(p, grid, st, stream);
+  else
+    rc = a->D == 128 ? launch_dkdv<__half, 128>(p, grid, st, stream) : launch_dkdv<__half, 64>(p, grid, st, stream);
+  if (rc != HB_OK || p.splits == 1) return rc;
+  return a->dtype == HB_BF16 ? launch_combine<__nv_bfloat16>(p, all, stream) : launch_combine<__half>(p, all, stream);
+}
+
+extern "C" int hb_fa_bwd_dkdv(const hb_fa_bwd_args* a) { return bwd_dkdv_impl(a, false, nullptr, 0); }
+
+extern "C" int hb_fa_bwd_dkdv_ws(const hb_fa_bwd_args* a, void* workspace, uint64_t bytes) {
+  return bwd_dkdv_impl(a, true, workspace, bytes);
+}
+
+extern "C" int hb_fa_bwd_dkdv_workspace(const hb_fa_bwd_args* a, uint64_t* bytes) {
+  using namespace hb;
+  clear_error();
+  int rc = bwd_check(a, "hb_fa_bwd_dkdv_workspace");
+  if (rc != HB_OK) return rc;
+  if (bytes == nullptr) return set_error(HB_ERR_BAD_ARG, "hb_fa_bwd_dkdv_workspace: bytes is NULL");
+  *bytes = 0;
+  if (a->B == 0 || a->Skv == 0 || a->Sq == 0 || a->Hq == a->Hkv) return HB_OK;
+  DeviceState* st = nullptr;
+  rc = get_device_state(&st);
+  if (rc != HB_OK) return rc;
+  const int splits = bwd_dkdv_splits(a, st->sm_count);
+  if (splits > 1) *bytes = 8ull * splits * a->B * a->Hkv * a->Skv * a->D;
+  return HB_OK;
 }
 
 extern "C" int hb_fa_bwd_dq(const hb_fa_bwd_args* a) {

@@ -178,6 +178,16 @@ def fa_bwd_preprocess(o: torch.Tensor, d_o: torch.Tensor, *, layout: str = "bhsd
     return delta
 
 
+def _bwd_dkdv_call(q, a, grouped: bool) -> None:
+    lib, arg = _lib.load(), C.byref(a)
+    if not grouped:
+        return _call(q.device, lib.hb_fa_bwd_dkdv, arg)
+    need = C.c_uint64(0)
+    _call(q.device, lib.hb_fa_bwd_dkdv_workspace, arg, C.byref(need))
+    ws = q.new_empty(need.value, dtype=torch.uint8) if need.value else None
+    _call(q.device, lib.hb_fa_bwd_dkdv_ws, arg, ws.data_ptr() if ws is not None else None, need.value)
+
+
 def fa_bwd_dkdv(q, k, v, d_o, lse, delta, *, causal: bool = False, softmax_scale: Optional[float] = None,
                 layout: str = "bhsd") -> Tuple[torch.Tensor, torch.Tensor]:
     """dK, dV through ``hb_fa_bwd_dkdv``; contiguous [B, Hkv, Skv, D] (a transposed view for "bshd")."""
@@ -185,7 +195,7 @@ def fa_bwd_dkdv(q, k, v, d_o, lse, delta, *, causal: bool = False, softmax_scale
     dk = torch.empty((B, Hkv, Skv, D), dtype=q.dtype, device=q.device)
     dv = torch.empty_like(dk)
     a.dk, a.dv = dk.data_ptr(), dv.data_ptr()
-    _call(q.device, _lib.load().hb_fa_bwd_dkdv, C.byref(a))
+    _bwd_dkdv_call(q, a, Hq != Hkv)
     return (dk, dv) if layout == "bhsd" else (dk.transpose(1, 2), dv.transpose(1, 2))
 
 
@@ -215,8 +225,9 @@ def fa_bwd(q, k, v, o, d_o, lse, *, causal: bool = False, softmax_scale: Optiona
     dq = q.new_empty((B, Hq, Sq, D))
     a.dk, a.dv, a.dq = dk.data_ptr(), dv.data_ptr(), dq.data_ptr()
     lib, arg = _lib.load(), C.byref(a)
-    for step in (lib.hb_fa_bwd_preprocess, lib.hb_fa_bwd_dkdv, lib.hb_fa_bwd_dq):
-        _call(q.device, step, arg)
+    _call(q.device, lib.hb_fa_bwd_preprocess, arg)
+    _bwd_dkdv_call(q, a, Hq != Hkv)
+    _call(q.device, lib.hb_fa_bwd_dq, arg)
     return (dq.transpose(1, 2), dk.transpose(1, 2), dv.transpose(1, 2)) if bshd else (dq, dk, dv)
 
 

@@ -313,6 +313,11 @@ typedef struct hb_fa_bwd_args {
 
 int hb_fa_bwd_preprocess(const hb_fa_bwd_args* args);
 int hb_fa_bwd_dkdv(const hb_fa_bwd_args* args);
+/* hb_fa_bwd_dkdv with a device workspace of the caller's: with grouped queries and few KV heads the query heads of a KV head
+ * are then dealt out to several SMs, whose fp32 partial results meet in the workspace.  hb_fa_bwd_dkdv_workspace writes the
+ * bytes a call needs (0: none); 16-byte aligned, need not be initialised, reusable once the work on `stream` is done. */
+int hb_fa_bwd_dkdv_workspace(const hb_fa_bwd_args* args, uint64_t* bytes);
+int hb_fa_bwd_dkdv_ws(const hb_fa_bwd_args* args, void* workspace, uint64_t bytes);
 int hb_fa_bwd_dq(const hb_fa_bwd_args* args);
 
 /*

@@ -231,3 +231,27 @@ def test_bshd_strided_gqa_backward(ops):
     for name, got, ref in (("dq", dq, rq), ("dk", dk, rk), ("dv", dv, rv)):
         err = (t(got) - ref).abs().max().item()
         assert err <= _tol(torch.bfloat16, ref), f"{name}: {err} (reference max {ref.abs().max().item()})"
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,Sq,Skv,D,causal,dtype", [
+    (1, 8, 1, 300, 300, 128, True, torch.bfloat16),    # eight heads of one KV head: one item each
+    (1, 12, 2, 200, 500, 64, True, torch.float16),     # a group of six, causal with more keys than queries
+    (2, 16, 4, 129, 257, 128, False, torch.bfloat16),  # ragged last tiles
+    (1, 6, 2, 1, 130, 64, False, torch.float16),       # one query row
+])
+def test_grouped_heads_over_several_sms(ops, B, Hq, Hkv, Sq, Skv, D, causal, dtype):
+    """dK / dV of grouped queries with few KV heads: the heads of a group go to several items, whose fp32 parts are added."""
+    q, k, v = O.make_qkv(B, Hq, Hkv, Sq, Skv, D, seed=Sq + Skv, dtype=dtype)
+    d_o = torch.randn(q.shape, generator=torch.Generator().manual_seed(5)).to(dtype)
+    qc, kc, vc, gc = (t.cuda() for t in (q, k, v, d_o))
+    out, lse = ops.fa_fwd(qc, kc, vc, causal=causal, return_lse=True)
+    dq, dk, dv = ops.fa_bwd(qc, kc, vc, out, gc, lse, causal=causal)
+    torch.cuda.synchronize()
+    assert ops.status_word() == 0
+    for got, ref in zip((dq, dk, dv), O.attention_backward(q, k, v, d_o, causal=causal)[:3]):
+        # 16-bit P and dS in the products, one rounding of the result
+        tol = (2e-2 if dtype == torch.bfloat16 else 4e-3) * max(1.0, ref.abs().max().item())
+        assert (got.cpu().float() - ref).abs().max().item() <= tol
+    delta = ops.fa_bwd_preprocess(out, gc)
+    again = ops.fa_bwd_dkdv(qc, kc, vc, gc, lse, delta, causal=causal)
+    assert torch.equal(again[0], dk) and torch.equal(again[1], dv)
