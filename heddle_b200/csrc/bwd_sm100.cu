@@ -83,6 +83,7 @@ struct alignas(64) BwdParams {
   int splits;
   float* part;
   TileOrder order;  // the work list: dkdv heads B * Hkv * splits, blocks nkb, rank 0 = the first; dq heads B * Hq, blocks nqb, rank 0 = the last
+  FastDiv by_heads, by_splits, by_group;  // dkdv: Hkv (of B * Hkv), splits;  dq: Hq, group
   float scale_log2, scale;
 };
 
@@ -272,14 +273,15 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
 
   // Work list (tile_order.h): u >> 1 is the entry, u & 1 its half where entries are pairs.  Under a causal mask key tile 0 is
   // seen by the most queries.
-  const int heads = p.group / p.splits;  // query heads of an item
+  const int heads = fast_div(p.group, p.by_splits);  // query heads of an item
   auto item_of = [&](int u, int& b, int& hkv, int& hq0, int& k0, int& qt0) -> bool {
     int bh, kb;
-    if (!tile_order_get(p.order, u >> 1, u & 1, static_cast<int>(gridDim.x), bh, kb)) return false;
-    hq0 = bh % (p.Hkv * p.splits) * heads;
-    bh /= p.splits;
-    b = bh / p.Hkv;
+    if (!tile_order_get(p.order, u >> 1, u & 1, bh, kb)) return false;
+    const int virtual_head = bh;  // (b * Hkv + hkv) * splits + split
+    bh = fast_div(bh, p.by_splits);
+    b = fast_div(bh, p.by_heads);
     hkv = bh - b * p.Hkv;
+    hq0 = hkv * p.group + (virtual_head - bh * p.splits) * heads;
     k0 = kb * 128;
     qt0 = p.causal ? max(0, (k0 - past) / 128) : 0;
     return true;
@@ -571,7 +573,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
       const uint32_t col_acc = static_cast<uint32_t>(half * (D / 2));
       const long long row_of = ((static_cast<long long>(b) * p.Hkv + hkv) * p.Skv + key) * D + col_acc;
       const long long all = static_cast<long long>(p.B) * p.Hkv * p.Skv * D;
-      float* const part = p.splits > 1 ? p.part + (hq0 - hkv * p.group) / heads * 2 * all + row_of : nullptr;
+      const int split = p.splits > 1 ? (hq0 - hkv * p.group) / heads : 0;
+      float* const part = p.splits > 1 ? p.part + split * 2 * all + row_of : nullptr;
 #pragma unroll 1
       for (int c = 0; c < D / 64; ++c) {
         uint32_t r[32];
@@ -642,9 +645,9 @@ __global__ void __launch_bounds__(kBwdDqThreads, 1) fa_bwd_dq_kernel(const __gri
   // tile sees the most keys.
   auto item_of = [&](int u, int& b, int& hq, int& q0, int& nk) -> bool {
     int bh, rank;
-    if (!tile_order_get(p.order, u >> 1, u & 1, static_cast<int>(gridDim.x), bh, rank)) return false;
+    if (!tile_order_get(p.order, u >> 1, u & 1, bh, rank)) return false;
     const int qb = p.nqb - 1 - rank;
-    b = bh / p.Hq;
+    b = fast_div(bh, p.by_heads);
     hq = bh - b * p.Hq;
     q0 = qb * 128;
     nk = p.causal ? min(p.nkb, (min(q0 + 127, p.Sq - 1) + past) / 128 + 1) : p.nkb;
@@ -662,7 +665,7 @@ __global__ void __launch_bounds__(kBwdDqThreads, 1) fa_bwd_dq_kernel(const __gri
       for (int u = 2 * blockIdx.x; ok && u < 2 * p.order.total; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1)) {
         int b, hq, q0, nk;
         if (!item_of(u, b, hq, q0, nk)) continue;
-        const int hkv = hq / p.group;
+        const int hkv = fast_div(hq, p.by_group);
         if (!mbar_wait(&s.fixed_empty, f_phase, ctx, kBwdTma)) break;
         f_phase ^= 1;
         mbar_arrive_expect_tx(&s.fixed_full, 2 * kBwdTileBytes);
@@ -1152,6 +1155,8 @@ static int bwd_dkdv_impl(const hb_fa_bwd_args* a, bool ws, void* workspace, uint
     return set_error(HB_ERR_BAD_ARG, "hb_fa_bwd_dkdv_ws: needs a 16-byte aligned workspace of %llu bytes, got %llu",
                      (unsigned long long)need, (unsigned long long)workspace_bytes);
   p.part = static_cast<float*>(workspace);
+  p.by_heads = make_fast_div((uint32_t)a->Hkv);
+  p.by_splits = make_fast_div((uint32_t)p.splits);
   const long long heads = (long long)a->B * a->Hkv * p.splits;
   if (heads * ((p.nkb + 1) / 2) > 0x3fffffffLL) return set_error(HB_ERR_UNSUPPORTED, "hb_fa_bwd_dkdv: problem too large");
   // a key tile reads Q and dO of its query heads
@@ -1212,6 +1217,8 @@ extern "C" int hb_fa_bwd_dq(const hb_fa_bwd_args* a) {
   if (rc != HB_OK) return rc;
   const long long total = (long long)a->B * a->Hq * ((p.nqb + 1) / 2);
   if (total > 0x3fffffffLL) return set_error(HB_ERR_UNSUPPORTED, "hb_fa_bwd_dq: problem too large");
+  p.by_heads = make_fast_div((uint32_t)a->Hq);
+  p.by_group = make_fast_div((uint32_t)p.group);
   int grid = tile_order_fill(&p.order, (long long)a->B * a->Hq, p.nqb, p.causal != 0, 4.0 * a->Skv * a->D / p.group, st->sm_count);
 #ifdef HB_DEBUG_GRID_ENV  // measurement builds only: fewer CTAs than SMs
   if (const char* e = getenv("HB_GRID")) grid = std::max(1, std::min(grid, atoi(e)));

@@ -156,6 +156,8 @@ static int fa_fill_params(const hb_fa_args* a, const char* who, uint32_t* status
   p.Sq = a->Sq;
   p.Skv = a->Skv;
   p.group = a->Hq / a->Hkv;
+  p.by_hq = make_fast_div((uint32_t)a->Hq);
+  p.by_group = make_fast_div((uint32_t)p.group);
   p.causal = a->causal ? 1 : 0;
   p.nqb = (a->Sq + 2 * kTileM - 1) / (2 * kTileM);
   *grid = tile_order_fill(&p.order, (long long)a->B * a->Hq, p.nqb, p.causal != 0, 2.0 * a->Skv * a->D * es / p.group, sm_count);

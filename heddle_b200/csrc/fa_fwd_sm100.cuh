@@ -96,6 +96,7 @@ struct alignas(64) FaParams {
   int nqb;          // 256-row query blocks per head
   TileOrder order;  // the work list: heads = B * Hq, blocks = nqb (rank 0 = the last block)
   int nkv;          // 128-key tiles
+  FastDiv by_hq, by_group;
   float scale_log2; // softmax_scale * log2(e) (times q_scale * k_scale for FP8)
   float out_scale;  // multiplies O / l in the epilogue (v_scale / P scale for FP8, else 1)
 };
@@ -126,11 +127,11 @@ struct FaItem {
 // Entry `g` of the static work list, first (half = 0) or second block where entries are pairs.
 __device__ __forceinline__ bool fa_get_item(const FaParams& p, int g, int half, FaItem& it) {
   int bh, rank;
-  if (!tile_order_get(p.order, g, half, static_cast<int>(gridDim.x), bh, rank)) return false;
+  if (!tile_order_get(p.order, g, half, bh, rank)) return false;
   const int qb = p.nqb - 1 - rank;
-  it.b = bh / p.Hq;
+  it.b = fast_div(bh, p.by_hq);
   it.hq = bh - it.b * p.Hq;
-  it.hkv = it.hq / p.group;
+  it.hkv = fast_div(it.hq, p.by_group);
   it.q0 = qb * (2 * kTileM);
 #pragma unroll
   for (int i = 0; i < 2; ++i) {

@@ -29,6 +29,7 @@
 //   ROPE    rotate-half rotary embedding on head_dim-wide column groups
 #pragma once
 
+#include "fast_div.h"
 #include "ptx_sm100.cuh"
 
 namespace hb {
@@ -46,24 +47,6 @@ constexpr int kGemmGroupM = HB_GEMM_GROUP_M;  // M-tiles per rasterisation group
 enum GemmEpiClass : int { kEpiPlain = 0, kEpiSwiglu = 1, kEpiRope = 2 };
 enum GemmAct : int { kActNone = 0, kActSilu = 1, kActRelu = 2, kActGeluTanh = 3, kActSigmoid = 4, kActTanh = 5 };
 enum GemmRole : uint32_t { kGemmRoleTma = 0x21, kGemmRoleMma = 0x22, kGemmRoleEpi = 0x23, kGemmRoleDrain = 0x24 };
-
-// Exact n / d for 0 <= n < 2^31 with one high multiply (Granlund and Montgomery, "Division by invariant integers using
-// multiplication", 1994): three runtime divisions in front of every tile took each role of the persistent kernels 790 cycles,
-// 14 % of a short-K tile.
-struct FastDiv {
-  uint32_t mul, shift, d;
-};
-inline FastDiv make_fast_div(uint32_t d) {
-  FastDiv f;
-  f.d = d;
-  f.shift = 0;
-  while ((1ull << f.shift) < d) ++f.shift;
-  f.mul = static_cast<uint32_t>((((1ull << f.shift) - d) << 32) / d + 1);
-  return f;
-}
-__device__ __forceinline__ int fast_div(int n, const FastDiv& f) {
-  return static_cast<int>((__umulhi(static_cast<uint32_t>(n), f.mul) + static_cast<uint32_t>(n)) >> f.shift);
-}
 
 struct alignas(64) GemmParams {
   CUtensorMap tm_a;

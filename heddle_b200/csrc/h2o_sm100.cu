@@ -38,6 +38,7 @@ struct alignas(64) H2oParams {
   int nkb;         // 128-key tiles per head
   int nqb;         // 128-query tiles
   TileOrder order; // the work list: heads = B * Hq, blocks = nkb (rank 0 = the first)
+  FastDiv by_hq, by_group;
   float scale_log2;
 };
 
@@ -62,10 +63,10 @@ struct H2oItem {
 // causal mask key tile kb is seen by nqb - qt0(kb) query tiles: the first is the dearest.
 __device__ __forceinline__ bool h2o_get_item(const H2oParams& p, int g, int half, H2oItem& it) {
   int bh, kb;
-  if (!tile_order_get(p.order, g, half, static_cast<int>(gridDim.x), bh, kb)) return false;
-  it.b = bh / p.Hq;
+  if (!tile_order_get(p.order, g, half, bh, kb)) return false;
+  it.b = fast_div(bh, p.by_hq);
   it.hq = bh - it.b * p.Hq;
-  it.hkv = it.hq / p.group;
+  it.hkv = fast_div(it.hq, p.by_group);
   it.k0 = kb * 128;
   // h2o_attention.py:99-101: q_start = max(0, (k0 - past_len) / block_M)
   it.qt0 = p.causal ? max(0, (it.k0 - (p.Skv - p.Sq)) / 128) : 0;
@@ -349,6 +350,8 @@ static int h2o_impl(const hb_h2o_args* a) {
   p.Sq = a->Sq;
   p.Skv = a->Skv;
   p.group = a->Hq / a->Hkv;
+  p.by_hq = make_fast_div((uint32_t)a->Hq);
+  p.by_group = make_fast_div((uint32_t)p.group);
   p.causal = a->causal ? 1 : 0;
   p.nkb = (a->Skv + 127) / 128;
   p.nqb = (a->Sq + 127) / 128;
