@@ -14,7 +14,8 @@
 // interpreter's structure one to one:
 //   * no reductions: a grid-stride stream over groups of 8 columns, kG groups per thread;
 //   * reductions: one row per warp (cols <= 1024) or per 128-thread CTA, R + 1 passes, pass r runs
-//     the program up to the r-th reduction and reduces the accumulator over the row.
+//     the program up to the r-th reduction and reduces the accumulator over the row; where they fit,
+//     the row's inputs are read once and kept in registers (cached_iterations).
 #include "rowprog_sm100.cuh"
 
 #include <dlfcn.h>
@@ -210,7 +211,7 @@ extern "C" __global__ void __launch_bounds__(THREADS) rowprog_jit(const __grid_c
       col[g] = ok[g] ? static_cast<int>(idx - r * groups) << 3 : 0;
     }
     float a[E];
-    rp_body(p, 0, row, col, ok, red, a);
+    rp_body(p, 0, row, col, ok, red, a, nullptr);
     if (g0 + stride < g0) break;  // the next index would wrap 32 bits: this was the last batch
   }
 }
@@ -229,13 +230,37 @@ extern "C" __global__ void __launch_bounds__(THREADS) rowprog_jit(const __grid_c
   const bool row_ok = row < p.rows;
   const int groups = p.cols >> 3;
   float red[4] = {0.f, 0.f, 0.f, 0.f};
+#if HB_ITERS > 0
+  // the row's inputs are read once, all loads in flight together, and stay packed in registers for every pass
+  uint4 cin[HB_ITERS][HB_NIN * G];
+#pragma unroll
+  for (int it = 0; it < HB_ITERS; ++it)
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const int gi = t + TPR * (it * G + g);
+#pragma unroll
+      for (int i = 0; i < HB_NIN; ++i)
+        cin[it][i * G + g] = (row_ok && gi < groups && ((HB_IN_USED >> i) & 1))
+                                 ? *reinterpret_cast<const uint4*>(static_cast<const unsigned short*>(p.in[i]) + row * p.ld_in[i] + (gi << 3))
+                                 : make_uint4(0, 0, 0, 0);
+    }
+#endif
 #pragma unroll
   for (int pass = 0; pass <= HB_NRED; ++pass) {
     const bool last = pass == HB_NRED;
     const int kind = last ? 0 : RED_KIND(pass);
     float partial = (kind == 1) ? __int_as_float(0xff800000) : 0.f;
     if (row_ok) {
+#if HB_ITERS > 0
+#pragma unroll
+      for (int it = 0; it < HB_ITERS; ++it) {
+        const int g0 = t + it * TPR * G;
+        if (g0 >= groups) break;
+        const uint4* const cached = cin[it];
+#else
       for (int g0 = t; g0 < groups; g0 += TPR * G) {
+        const uint4* const cached = nullptr;
+#endif
         long long rows_[G]; int col[G]; bool ok[G];
 #pragma unroll
         for (int g = 0; g < G; ++g) {
@@ -245,7 +270,7 @@ extern "C" __global__ void __launch_bounds__(THREADS) rowprog_jit(const __grid_c
           col[g] = ok[g] ? gi << 3 : 0;
         }
         float a[E];
-        rp_body(p, pass, rows_, col, ok, red, a);
+        rp_body(p, pass, rows_, col, ok, red, a, cached);
         if (!last) {
 #pragma unroll
           for (int g = 0; g < G; ++g) {
@@ -289,10 +314,41 @@ std::string fmt_float(float x) {
   return buf;
 }
 
+// Bit i: the program reads input i.  *n: one more than the highest such index.
+unsigned inputs_used(const RowProgParams& p, int* n) {
+  unsigned used = 0;
+  *n = 0;
+  for (int pc = 0; pc < p.n_inst; ++pc) {
+    const hb_ew_inst& in = p.prog[pc];
+    if (in.op < HB_EW_LOAD || in.op > HB_EW_POW || in.src != HB_SRC_INPUT) continue;
+    used |= 1u << in.index;
+    *n = std::max(*n, in.index + 1);
+  }
+  return used;
+}
+
+// Iterations of the reduce kernel's column loop when the row's inputs stay in registers between the passes, rounded up to a
+// power of two (one kernel per power, not per width), or 0 where they would take more than 64 registers a thread.  A program
+// with R reductions otherwise reads its inputs R + 1 times, from L1 or L2.
+int cached_iterations(const RowProgParams& p, int warps_per_row) {
+  int n_in = 0;
+  inputs_used(p, &n_in);
+  if (warps_per_row == 0 || n_in == 0) return 0;
+  const int per_iter = 32 * warps_per_row * kJitG;
+  int iters = 1;
+  while (iters * per_iter < p.cols / 8) iters *= 2;
+  return iters * kJitG * n_in <= 16 ? iters : 0;
+}
+
 // One line of rp_body per instruction; the formulas are those of the interpreter's op switch.
 std::string generate(const RowProgParams& p, bool bf16, int warps_per_row) {
   std::string s;
   char line[256];
+  int n_in = 0;
+  const unsigned used = inputs_used(p, &n_in);
+  const int iters = cached_iterations(p, warps_per_row);
+  snprintf(line, sizeof(line), "#define HB_ITERS %d\n#define HB_NIN %d\n#define HB_IN_USED %uu\n", iters, n_in, used);
+  s += line;
   snprintf(line, sizeof(line), "#define HB_T_BF16 %d\n#define HB_G %d\n#define HB_NRED %d\n#define HB_WARPS_PER_ROW %d\n", bf16 ? 1 : 0, kJitG,
            p.n_red, warps_per_row);
   s += line;
@@ -309,7 +365,7 @@ std::string generate(const RowProgParams& p, bool bf16, int warps_per_row) {
     s += kinds + "0)\n" + slots + "0)\n";
   }
   s += "__device__ __forceinline__ void rp_body(const Head& p, int pass, const long long* row, const int* col, const bool* ok,\n"
-       "                                        const float* red, float* a) {\n  float v[E];\n";
+       "                                        const float* red, float* a, const uint4* cached) {\n  float v[E];\n";
   bool tmp_used[HB_EW_MAX_TMP] = {};
   for (int pc = 0; pc < p.n_inst; ++pc)
     if (p.prog[pc].op == HB_EW_STORE_TMP) tmp_used[p.prog[pc].index] = true;
@@ -322,7 +378,12 @@ std::string generate(const RowProgParams& p, bool bf16, int warps_per_row) {
     const bool binary = in.op >= HB_EW_LOAD && in.op <= HB_EW_POW;
     if (binary) {
       switch (in.src) {
-        case HB_SRC_INPUT: s += "  ld_in(p.in[" + idx + "], p.ld_in[" + idx + "], row, col, ok, v);\n"; break;
+        case HB_SRC_INPUT:
+          if (iters > 0) {
+            s += "  _Pragma(\"unroll\") for (int g = 0; g < G; ++g) unpack8(cached[" + idx + " * G + g], v + 8 * g);\n";
+            break;
+          }
+          s += "  ld_in(p.in[" + idx + "], p.ld_in[" + idx + "], row, col, ok, v);\n"; break;
         case HB_SRC_ROWVEC: s += "  ld_rowvec(p.rowvec[" + idx + "], col, ok, v);\n"; break;
         case HB_SRC_ROWSCALAR: s += "  ld_rowscalar(p.rowscalar[" + idx + "], row, ok, v);\n"; break;
         case HB_SRC_TMP: s += "  _Pragma(\"unroll\") for (int e = 0; e < E; ++e) v[e] = t" + idx + "[e];\n"; break;
@@ -448,6 +509,7 @@ int rowprog_jit_launch(const RowProgParams& p, bool bf16, const DeviceState& st,
     std::string key(reinterpret_cast<const char*>(p.prog), sizeof(hb_ew_inst) * p.n_inst);
     key += static_cast<char>(bf16 ? 1 : 0);
     key += static_cast<char>(warps_per_row);
+    key += static_cast<char>(cached_iterations(p, warps_per_row));
     key += static_cast<char>(st.device);
     auto it = g_cache.find(key);
     if (it == g_cache.end()) {
