@@ -1054,7 +1054,7 @@ static int bwd_dkdv_splits(const hb_fa_bwd_args* a, int sm_count) {
 
 template <typename Smem>
 static int bwd_launch(void (*kernel)(const BwdParams), const BwdParams& p, int grid, int threads, const DeviceState* st,
-                      cudaStream_t stream, bool* configured) {
+                      cudaStream_t stream, bool* configured, double steps_per_block) {
   if ((int)sizeof(Smem) > st->smem_optin)
     return set_error(HB_ERR_UNSUPPORTED, "attention backward needs %d bytes of shared memory per CTA, the device offers %d",
                      (int)sizeof(Smem), st->smem_optin);
@@ -1062,13 +1062,15 @@ static int bwd_launch(void (*kernel)(const BwdParams), const BwdParams& p, int g
     HB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
     configured[st->device & 63] = true;
   }
-  HB_CUDA_CHECK(launch_dependent(kernel, grid, threads, sizeof(Smem), stream, 0, p));
+  HB_CUDA_CHECK(launch_dependent_if(launch_early(tile_order_steps(p.order, p.causal != 0, steps_per_block)), kernel, grid, threads,
+                                    sizeof(Smem), stream, 0, p));
   return HB_OK;
 }
 template <typename T, int D>
 static int launch_dkdv(const BwdParams& p, int grid, const DeviceState* st, cudaStream_t stream) {
   static bool configured[64] = {};
-  return bwd_launch<BwdSmemKv<D>>(fa_bwd_dkdv_kernel<T, D>, p, grid, kBwdThreads, st, stream, configured);
+  return bwd_launch<BwdSmemKv<D>>(fa_bwd_dkdv_kernel<T, D>, p, grid, kBwdThreads, st, stream, configured,
+                                   static_cast<double>(p.group / p.splits) * p.nqb);
 }
 template <typename T>
 static int launch_combine(const BwdParams& p, long long all, cudaStream_t stream) {
@@ -1088,7 +1090,7 @@ static int launch_combine(const BwdParams& p, long long all, cudaStream_t stream
 template <typename T, int D>
 static int launch_dq(const BwdParams& p, int grid, const DeviceState* st, cudaStream_t stream) {
   static bool configured[64] = {};
-  return bwd_launch<BwdSmemQ<D>>(fa_bwd_dq_kernel<T, D>, p, grid, kBwdDqThreads, st, stream, configured);
+  return bwd_launch<BwdSmemQ<D>>(fa_bwd_dq_kernel<T, D>, p, grid, kBwdDqThreads, st, stream, configured, p.nkb);
 }
 template <typename T, int D>
 static int launch_preprocess(const hb_fa_bwd_args* a, cudaStream_t stream) {

@@ -39,7 +39,8 @@ static int launch_fa(const FaParams& p, int grid, int smem_optin, cudaStream_t s
       configured[dev & 63] = true;
     }
   }
-  HB_CUDA_CHECK(launch_dependent(kernel, grid, kFaThreads, sizeof(Smem), stream, 0, p));
+  HB_CUDA_CHECK(launch_dependent_if(launch_early(tile_order_steps(p.order, p.causal != 0, p.nkv)), kernel, grid, kFaThreads,
+                                    sizeof(Smem), stream, 0, p));
   return HB_OK;
 }
 
@@ -50,7 +51,8 @@ static int launch_fa_stages(const FaParams& p, int grid, int smem_optin, cudaStr
   auto kernel = fa_fwd_kernel<T, D, NS>;
   // set on every call: this is a diagnostic path, not worth a per-device table
   HB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
-  HB_CUDA_CHECK(launch_dependent(kernel, grid, kFaThreads, sizeof(Smem), stream, 0, p));
+  HB_CUDA_CHECK(launch_dependent_if(launch_early(tile_order_steps(p.order, p.causal != 0, p.nkv)), kernel, grid, kFaThreads,
+                                    sizeof(Smem), stream, 0, p));
   return HB_OK;
 }
 

@@ -303,7 +303,8 @@ static int launch_h2o(const H2oParams& p, int grid, const DeviceState* st, cudaS
     HB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
     configured[st->device & 63] = true;
   }
-  HB_CUDA_CHECK(launch_dependent(kernel, grid, kH2oThreads, sizeof(Smem), stream, 0, p));
+  HB_CUDA_CHECK(launch_dependent_if(launch_early(tile_order_steps(p.order, p.causal != 0, p.nqb)), kernel, grid, kH2oThreads,
+                                    sizeof(Smem), stream, 0, p));
   return HB_OK;
 }
 static int h2o_impl(const hb_h2o_args* a) {

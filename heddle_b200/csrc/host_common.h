@@ -50,9 +50,12 @@ int get_device_info_noalloc(DeviceInfo* out);
 // Launches `kernel` so that its start-up (launch latency, barrier and TMEM set-up, descriptor fetch) may run under the tail
 // of the stream's previous kernel: programmatic dependent launch.  The kernel calls grid_wait() before it touches memory.
 // `cluster` > 0 sets a run-time cluster size.
+// Worth it while a kernel's start-up is visible in its time (6 % of a four-kernel train step of 114 us); the attention kernels
+// of a long problem start in order instead (`early` false): waiting CTAs cost the step of B4 H32 S4096 0.4 % (2133 -> 2143 us).
+inline bool launch_early(double steps_per_cta) { return steps_per_cta <= 100.0; }
 template <typename... Params, typename... Args>
-inline cudaError_t launch_dependent(void (*kernel)(Params...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream,
-                                    unsigned cluster, Args... args) {
+inline cudaError_t launch_dependent_if(bool early, void (*kernel)(Params...), unsigned grid, unsigned threads, size_t smem,
+                                       cudaStream_t stream, unsigned cluster, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
@@ -60,7 +63,7 @@ inline cudaError_t launch_dependent(void (*kernel)(Params...), unsigned grid, un
   cfg.stream = stream;
   cudaLaunchAttribute attrs[2] = {};
   attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attrs[0].val.programmaticStreamSerializationAllowed = 1;
+  attrs[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
   cfg.attrs = attrs;
   cfg.numAttrs = 1;
   if (cluster > 0) {
@@ -70,6 +73,11 @@ inline cudaError_t launch_dependent(void (*kernel)(Params...), unsigned grid, un
     cfg.numAttrs = 2;
   }
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+template <typename... Params, typename... Args>
+inline cudaError_t launch_dependent(void (*kernel)(Params...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream,
+                                    unsigned cluster, Args... args) {
+  return launch_dependent_if(true, kernel, grid, threads, smem, stream, cluster, args...);
 }
 
 // 2-D .. 4-D tiled tensor map with 128-byte swizzle, zero fill out of bounds.

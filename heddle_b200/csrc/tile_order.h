@@ -74,4 +74,9 @@ inline int tile_order_fill(TileOrder* o, long long heads, int blocks, bool maske
   return grid;
 }
 
+// Steps of 128 keys (or queries) of an average CTA: `per_block` is the most a block has, a masked one half of that on average.
+inline double tile_order_steps(const TileOrder& o, bool masked, double per_block) {
+  return static_cast<double>(o.heads) * o.blocks * per_block * (masked ? 0.5 : 1.0) / o.by_grid.d;
+}
+
 }  // namespace hb
