@@ -127,7 +127,8 @@ static GemmSplitChoice gemm_split_choose(const DeviceState* st, int epi_class, i
       const long long waves = (tiles * splits + slots[splits] - 1) / slots[splits];
       const double l2 = 128.0 * (width + a_rows) * tiles * (double)k_steps / 14000.0;
       const double fixed = 5000.0 + (splits > 1 ? 450.0 * splits : 0.0) + std::min(M, kGemmBM) * (double)width / 10.0;
-      const double ns = std::max({hbm, l2, waves * (slab * slabs * ((stages + splits - 1) / splits))}) + waves * fixed;
+      // CTAs of later waves start as SMs come free, so most of their fixed time hides under the others' streaming
+      const double ns = std::max({hbm, l2, waves * (slab * slabs * ((stages + splits - 1) / splits))}) + fixed * (0.7 + 0.3 * waves);
       if (best.width == 0 || ns < best.ns) best = {width, splits, slabs, ns};
     }
     if (tiles > 4ll * st->sm_count && width >= 128) break;  // wider tiles only leave fewer of them
