@@ -58,6 +58,12 @@ def _as_fp32(t: torch.Tensor) -> torch.Tensor:
     return t if t.dtype is torch.float32 and t.is_contiguous() else t.to(torch.float32).contiguous()
 
 
+def _row_stride(t2: torch.Tensor) -> int:
+    """Row stride of a [rows, cols] view for the library.  A single row may carry any stride (a slice of a wider buffer, the
+    transpose of a column), and ``contiguous()`` leaves it: sizes of one do not count.  No second row is read, so it is cols."""
+    return t2.stride(0) if t2.shape[0] > 1 else t2.shape[1]
+
+
 def _inner_contiguous(t: torch.Tensor) -> torch.Tensor:
     return t if t.stride(-1) == 1 else t.contiguous()
 
@@ -321,7 +327,7 @@ def gemm_epilogue(a: torch.Tensor, w: torch.Tensor, epilogue: str = "none", *,
         result, out_ptr, ldo = out, out2.data_ptr(), out2.stride(0)
     device = a.device
     g = _lib.GemmArgs(a2.data_ptr() if a2 is not None else a.data_ptr(), w.data_ptr(), out_ptr, M, N, K,
-                      a2.stride(0) if a2 is not None else K, w.stride(0), ldo, _DTYPES[a.dtype], _lib.EPILOGUES[epilogue])
+                      _row_stride(a2) if a2 is not None else K, w.stride(0), ldo, _DTYPES[a.dtype], _lib.EPILOGUES[epilogue])
     keep = []
     if row_scale is not None:
         rs = _as_fp32(row_scale)
@@ -505,7 +511,7 @@ def row_softmax(x: torch.Tensor, scale: float = 1.0) -> torch.Tensor:
     if x2.stride(-1) != 1 or (x2.shape[0] > 1 and x2.stride(0) % 8 != 0) or x2.data_ptr() % 16 != 0:
         x2 = x2.contiguous()
     y = x.new_empty(x.shape)
-    _call(x.device, _lib.load().hb_row_softmax, x2.data_ptr(), y.data_ptr(), x2.shape[0], cols, max(x2.stride(0), cols),
+    _call(x.device, _lib.load().hb_row_softmax, x2.data_ptr(), y.data_ptr(), x2.shape[0], cols, max(_row_stride(x2), cols),
           cols, float(scale), _DTYPES[x.dtype], _stream_ptr(x.device))
     return y
 
@@ -546,10 +552,10 @@ def rowwise_program(program, inputs=(), rowvecs=(), rowscalars=(), n_outputs: in
         if tuple(t.shape) != shape or t.dtype != x0.dtype:
             raise ValueError("rowwise_program: full-size inputs must share shape and dtype")
         t2 = t if t.dim() == 2 else t.reshape(-1, cols)
-        if t2.stride(-1) != 1 or t2.stride(0) % 8 or t2.data_ptr() % 16:
+        if t2.stride(-1) != 1 or _row_stride(t2) % 8 or t2.data_ptr() % 16:
             t2 = t2.contiguous()
         keep.append(t2)
-        a.inputs[i], a.ld_in[i] = t2.data_ptr(), t2.stride(0)
+        a.inputs[i], a.ld_in[i] = t2.data_ptr(), _row_stride(t2)
     rows = keep[0].shape[0]
     for i, t in enumerate(rowvecs):
         t2 = t.reshape(-1).to(x0.dtype).contiguous()
