@@ -508,10 +508,10 @@ def row_softmax(x: torch.Tensor, scale: float = 1.0) -> torch.Tensor:
     _require_cuda(x)
     cols = x.shape[-1]
     x2 = x if x.dim() == 2 else x.reshape(-1, cols)
-    if x2.stride(-1) != 1 or (x2.shape[0] > 1 and x2.stride(0) % 8 != 0) or x2.data_ptr() % 16 != 0:
+    if x2.stride(-1) != 1 or _row_stride(x2) < cols or _row_stride(x2) % 8 or x2.data_ptr() % 16:
         x2 = x2.contiguous()
     y = x.new_empty(x.shape)
-    _call(x.device, _lib.load().hb_row_softmax, x2.data_ptr(), y.data_ptr(), x2.shape[0], cols, max(_row_stride(x2), cols),
+    _call(x.device, _lib.load().hb_row_softmax, x2.data_ptr(), y.data_ptr(), x2.shape[0], cols, _row_stride(x2),
           cols, float(scale), _DTYPES[x.dtype], _stream_ptr(x.device))
     return y
 
