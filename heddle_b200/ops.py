@@ -392,8 +392,11 @@ def bmm(a: torch.Tensor, b: torch.Tensor, epilogue: str = "none", *, bias: Optio
     N = b.shape[2]
     if not _mult8(K, N):
         raise ValueError(f"bmm needs K and N to be multiples of 8 (K={K}, N={N})")
-    if a.stride(2) != 1 or not _mult8(a.stride(1), a.stride(0)) or a.data_ptr() % 16:
+    # the library reads a batch stride of 0 as densely packed batches: one broadcast batch becomes dense first
+    if a.stride(2) != 1 or not _mult8(a.stride(1), a.stride(0)) or a.data_ptr() % 16 or (Bn > 1 and a.stride(0) == 0):
         a = a.contiguous()
+    if Bn > 1 and b.stride(0) == 0:
+        b = b.contiguous()
     if b.stride(1) == 1 and b.stride(2) >= K and _mult8(b.stride(2), b.stride(0)) and b.data_ptr() % 16 == 0 and K > 1:
         layout, ldw = _lib.HB_W_NK, b.stride(2)   # a transposed view of [B, N, K] storage
     else:

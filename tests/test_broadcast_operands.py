@@ -27,6 +27,17 @@ def test_row_softmax_reads_inside_a_broadcast_row(built_lib, handed_over):
     assert ld == 4096 and x != row.data_ptr()  # a dense copy: 16 rows of 4096 do not fit behind the row itself
 
 
+@pytest.mark.parametrize("which", ["a", "b"])
+def test_bmm_reads_inside_a_broadcast_batch(built_lib, handed_over, which):
+    ops, calls = handed_over
+    a, b = torch.randn(1, 24, 64).to(BF16), torch.randn(1, 64, 40).to(BF16)
+    wide = {"a": (a.expand(8, 24, 64), b.repeat(8, 1, 1)), "b": (a.repeat(8, 1, 1), b.expand(8, 64, 40))}[which]
+    ops.bmm(*wide)
+    g = calls[0][0]._obj
+    assert g.batch == 8 and g.a_batch_stride == 24 * 64 and g.w_batch_stride == 64 * 40
+    assert (g.a != a.data_ptr()) if which == "a" else (g.w != b.data_ptr())  # 0 would select densely packed batches
+
+
 @pytest.mark.gpu
 def test_results_equal_those_of_a_dense_copy(built_lib):
     from heddle_b200 import ops
@@ -34,3 +45,7 @@ def test_results_equal_those_of_a_dense_copy(built_lib):
     g = torch.Generator().manual_seed(4)
     x = torch.randn(4096, generator=g).to(BF16).cuda().expand(16, 4096)
     assert torch.equal(ops.row_softmax(x), ops.row_softmax(x.contiguous()))
+    a, b = torch.randn(1, 24, 64, generator=g).to(BF16).cuda(), torch.randn(1, 64, 40, generator=g).to(BF16).cuda()
+    for wide in ((a.expand(8, 24, 64), b.repeat(8, 1, 1)), (a.repeat(8, 1, 1), b.expand(8, 64, 40)),
+                 (a.repeat(8, 1, 1), b.transpose(1, 2).contiguous().expand(8, 40, 64).transpose(1, 2))):
+        assert torch.equal(ops.bmm(*wide), ops.bmm(*(t.contiguous() for t in wide)))
