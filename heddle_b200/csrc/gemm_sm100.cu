@@ -1,4 +1,5 @@
 // hb_gemm_epilogue / hb_rms_rowstat: validation, TMA descriptors and launch.
+#include "gemm_split_plan.h"
 #include "gemm_split_sm100.cuh"
 #include "host_common.h"
 
@@ -60,11 +61,10 @@ static int dispatch_gemm(int epi_class, const GemmParams& p, int grid, bool pair
   }
 }
 
-// ---- the split-K kernel: which tile width and cluster size, and whether it is the one to run ----
+// ---- the split-K kernel (gemm_split_plan.h: whether it is the one to run) ----
 
 // CTAs of gemm_split_kernel that run at one time in clusters of `splits`, per device (the GPCs of the part do not hold a whole
 // number of clusters of every size).
-constexpr int kMaxSplits = 8;
 static int gemm_split_slots(const DeviceState* st, int splits) {
   static int slots[64][kMaxSplits + 1] = {};
   static std::mutex mutex;
@@ -91,49 +91,6 @@ static int gemm_split_slots(const DeviceState* st, int splits) {
     n = clusters * splits;
   }
   return n;
-}
-
-// Estimated time (ns) of one launch, fitted to a sweep of widths 64 .. 256 and clusters 1 .. 8 on 24 .. 256 x 4096 .. 22016 x
-// 4096 .. 11008 (within 10 %): an SM streams weights from HBM at 60 B/ns and all operands at 120; a 128 x 256 x 64 slab takes
-// 270 ns on the tensor cores, and never less than the 125 ns its four MMAs take to issue; HBM gives 6 KB/ns and L2 14 KB/ns in
-// all; a wave costs 5 us for its start, its first load and its stores, 450 ns more per CTA of a cluster, and 100 ns per 1000
-// accumulators read back.
-struct GemmSplitChoice {
-  int width = 0, splits = 0, slabs = 0;
-  double ns = 0.0;
-};
-
-// K slabs per stage: about 40 KB, so that four or more stages fit the ring
-static int gemm_split_slabs(int a_rows, int width, int k_steps, bool whole_slabs) {
-  if (!whole_slabs) return 1;
-  return std::max(1, std::min({4, k_steps, 40 * 1024 / ((a_rows + width) * 128)}));
-}
-
-static GemmSplitChoice gemm_split_choose(const DeviceState* st, int epi_class, int M, int n_out, int k_steps, bool whole_slabs,
-                                         int batch, int head_dim, bool w_kn) {
-  GemmSplitChoice best;
-  int slots[kMaxSplits + 1];
-  for (int splits = 1; splits <= kMaxSplits; ++splits) slots[splits] = gemm_split_slots(st, splits);
-  const int tiles_m = (M + kGemmBM - 1) / kGemmBM;
-  const int a_rows = tiles_m > 1 ? kGemmBM : (M + 7) / 8 * 8;
-  const int unit = epi_class == kEpiRope ? head_dim : w_kn ? 64 : 16;
-  const int per_col = epi_class == kEpiSwiglu ? 2 : 1;  // accumulator columns per output column
-  const double hbm = 128.0 * k_steps * batch * ((double)n_out * per_col + M) / 6000.0;
-  for (int width = unit; width <= kGemmBN; width += unit) {
-    const long long tiles = (long long)tiles_m * ((n_out * per_col + width - 1) / width) * batch;
-    const double slab = std::max({width * 128.0 / 60.0, (width + a_rows) * 128.0 / 120.0, width * (270.0 / 256.0), 125.0});
-    const int slabs = gemm_split_slabs(a_rows, width, k_steps, whole_slabs), stages = (k_steps + slabs - 1) / slabs;
-    for (int splits = 1; splits <= std::min(kMaxSplits, stages); ++splits) {
-      const long long waves = (tiles * splits + slots[splits] - 1) / slots[splits];
-      const double l2 = 128.0 * (width + a_rows) * tiles * (double)k_steps / 14000.0;
-      const double fixed = 5000.0 + (splits > 1 ? 450.0 * splits : 0.0) + std::min(M, kGemmBM) * (double)width / 10.0;
-      // CTAs of later waves start as SMs come free, so most of their fixed time hides under the others' streaming
-      const double ns = std::max({hbm, l2, waves * (slab * slabs * ((stages + splits - 1) / splits))}) + fixed * (0.7 + 0.3 * waves);
-      if (best.width == 0 || ns < best.ns) best = {width, splits, slabs, ns};
-    }
-    if (tiles > 4ll * st->sm_count && width >= 128) break;  // wider tiles only leave fewer of them
-  }
-  return best;
 }
 
 template <typename T, int EPI>
@@ -227,22 +184,18 @@ static int gemm_impl(const hb_gemm_args* args) {
   int rc = get_device_state(&st);
   if (rc != HB_OK) return rc;
 
-  // Which kernel.  The persistent kernels (CTA pairs when a problem has more than one 128-row tile of rows, else single CTAs)
-  // win once their 256-column tiles fill the chip; with fewer than two rounds of them (eight, for a single row of tiles, which
-  // is bound by the weights) the split-K kernel runs where its estimate is the smaller one.  Theirs: 546 ns (single CTA, weights
-  // from HBM) or 290 ns (pair) a 64-wide slab of a tile, 3.5 us a round and 3 us once.  Both sides measured, us, split-K | the
-  // persistent kernel: 24 x 22016 x 4096 33 | 42; 120 x 4096 x 11008 25 | 67; 120 x 12288 x 4096 30 | 40; 1 x 4096 x 4096
-  // 11 | 28; 64 x 50000 x 4096 75 | 83; 256 x 4096 x 4096 17 | 25; 512 x 4096 x 4096 23 | 26; 1000 x 4096 x 4096 31 | 28; 256 x 22016 x 4096 61 | 56.
+  // Which kernel.  The persistent kernels win once their 256-column tiles fill the chip; below that the split-K kernel runs where
+  // its estimate is the smaller one (gemm_split_plan.h).
   const int k_steps = (a->K + kGemmBK - 1) / kGemmBK;
-  const bool one_row = a->M <= kGemmBM;
-  const long long wide_tiles = (long long)((a->M + (one_row ? kGemmBM : kPairBM) - 1) / (one_row ? kGemmBM : kPairBM)) *
-                               ((a->N + kGemmBN - 1) / kGemmBN) * batch;
-  const int wide_slots = one_row ? st->sm_count : std::max(1, st->sm_count / 2);
+  const GemmWide wide = gemm_wide(st->sm_count, a->M, a->N, batch);
   GemmSplitChoice split;
-  if (a->schedule == HB_GEMM_SPLIT || (a->schedule == HB_GEMM_AUTO && wide_tiles < (one_row ? 8ll : 2ll) * wide_slots)) {
-    split = gemm_split_choose(st, epi_class, a->M, n_out, k_steps, a->K % kGemmBK == 0, batch, a->head_dim, w_kn);
-    const double wide_ns = (double)((wide_tiles + wide_slots - 1) / wide_slots) * (k_steps * (one_row ? 546.0 : 290.0) + 3500.0) + 3000.0;
-    if (a->schedule == HB_GEMM_AUTO && split.ns >= wide_ns) split = GemmSplitChoice();
+  if (a->schedule == HB_GEMM_SPLIT || (a->schedule == HB_GEMM_AUTO && gemm_split_eligible(wide))) {
+    int slots[kMaxSplits + 1] = {};
+    for (int splits = 1; splits <= kMaxSplits; ++splits) slots[splits] = gemm_split_slots(st, splits);
+    split = gemm_split_choose(slots, st->sm_count, epi_class, a->M, n_out, k_steps, a->K % kGemmBK == 0, batch, a->head_dim, w_kn);
+    const bool plain = epi_class == kEpiPlain && a->epilogue == HB_EPI_NONE;
+    const double bytes = 2.0 * batch * ((double)a->M * a->K + (double)a->N * a->K + (double)a->M * n_out);
+    if (a->schedule == HB_GEMM_AUTO && !gemm_split_wins(split, wide, k_steps, plain, bytes)) split = GemmSplitChoice();
   }
   const bool use_split = split.width > 0;
 

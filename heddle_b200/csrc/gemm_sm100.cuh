@@ -30,21 +30,18 @@
 #pragma once
 
 #include "fast_div.h"
+#include "gemm_shape.h"
 #include "ptx_sm100.cuh"
 
 namespace hb {
 
 constexpr int kGemmThreads = 320;  // TMA warp, MMA warp, two epilogue warpgroups
-constexpr int kGemmBM = 128;
-constexpr int kGemmBN = 256;
-constexpr int kGemmBK = 64;
 constexpr int kGemmStages = 4;
 #ifndef HB_GEMM_GROUP_M
 #define HB_GEMM_GROUP_M 16
 #endif
 constexpr int kGemmGroupM = HB_GEMM_GROUP_M;  // M-tiles per rasterisation group (L2 reuse of the weight slabs)
 
-enum GemmEpiClass : int { kEpiPlain = 0, kEpiSwiglu = 1, kEpiRope = 2 };
 enum GemmAct : int { kActNone = 0, kActSilu = 1, kActRelu = 2, kActGeluTanh = 3, kActSigmoid = 4, kActTanh = 5 };
 enum GemmRole : uint32_t { kGemmRoleTma = 0x21, kGemmRoleMma = 0x22, kGemmRoleEpi = 0x23, kGemmRoleDrain = 0x24 };
 
@@ -593,7 +590,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
 // commit aimed at its ring, the leader has seen every release aimed at it, and the pair meets at a
 // cluster barrier, so nothing can arrive at shared memory that is gone.
 // ------------------------------------------------------------------------------------------
-constexpr int kPairBM = 256;  // rows of a pair's tile (128 per CTA)
 constexpr int kPairMaxStages = 6;
 constexpr int kPairSlots = 7;              // 32 KB slots of shared memory: ring stages + staging slabs per warpgroup
 constexpr int kPairStageA = kGemmBM * kGemmBK * 2;        // 16 KB
