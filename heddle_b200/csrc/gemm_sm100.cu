@@ -63,14 +63,14 @@ static int dispatch_gemm(int epi_class, const GemmParams& p, int grid, bool pair
 
 // ---- the split-K kernel (gemm_split_plan.h: whether it is the one to run) ----
 
-// CTAs of gemm_split_kernel that run at one time in clusters of `splits`, per device (the GPCs of the part do not hold a whole
-// number of clusters of every size).
-static int gemm_split_slots(const DeviceState* st, int splits) {
+// CTAs of gemm_split_kernel that run at one time in clusters of 1 .. kMaxSplits, per device (the GPCs of the part do not hold a
+// whole number of clusters of every size).  Asked for once; the entries do not change after that.
+static const int* gemm_split_slots(const DeviceState* st) {
   static int slots[64][kMaxSplits + 1] = {};
   static std::mutex mutex;
   std::lock_guard<std::mutex> lock(mutex);
-  int& n = slots[st->device & 63][splits];
-  if (n == 0) {
+  int* const table = slots[st->device & 63];
+  for (int splits = 1; splits <= kMaxSplits && table[kMaxSplits] == 0; ++splits) {
     auto kernel = gemm_split_kernel<__nv_bfloat16, kEpiPlain>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(splits * st->sm_count));
@@ -88,9 +88,9 @@ static int gemm_split_slots(const DeviceState* st, int splits) {
       (void)cudaGetLastError();
       clusters = st->sm_count / (2 * splits) > 0 ? st->sm_count / (2 * splits) : 1;
     }
-    n = clusters * splits;
+    table[splits] = clusters * splits;
   }
-  return n;
+  return table;
 }
 
 template <typename T, int EPI>
@@ -190,9 +190,7 @@ static int gemm_impl(const hb_gemm_args* args) {
   const GemmWide wide = gemm_wide(st->sm_count, a->M, a->N, batch);
   GemmSplitChoice split;
   if (a->schedule == HB_GEMM_SPLIT || (a->schedule == HB_GEMM_AUTO && gemm_split_eligible(wide))) {
-    int slots[kMaxSplits + 1] = {};
-    for (int splits = 1; splits <= kMaxSplits; ++splits) slots[splits] = gemm_split_slots(st, splits);
-    split = gemm_split_choose(slots, st->sm_count, epi_class, a->M, n_out, k_steps, a->K % kGemmBK == 0, batch, a->head_dim, w_kn);
+    split = gemm_split_choose(gemm_split_slots(st), st->sm_count, epi_class, a->M, n_out, k_steps, a->K % kGemmBK == 0, batch, a->head_dim, w_kn);
     const bool plain = epi_class == kEpiPlain && a->epilogue == HB_EPI_NONE;
     const double bytes = 2.0 * batch * ((double)a->M * a->K + (double)a->N * a->K + (double)a->M * n_out);
     if (a->schedule == HB_GEMM_AUTO && !gemm_split_wins(split, wide, k_steps, plain, bytes)) split = GemmSplitChoice();

@@ -38,11 +38,14 @@ inline GemmSplitChoice gemm_split_choose(const int* slots, int sm_count, int epi
   for (int width = unit; width <= kGemmBN; width += unit) {
     const long long tiles = (long long)tiles_m * ((n_out * per_col + width - 1) / width) * batch;
     const double slab = std::max({width * 128.0 / 60.0, (width + a_rows) * 128.0 / 120.0, width * (270.0 / 256.0), 125.0});
+    const double l2 = 128.0 * (width + a_rows) * tiles * (double)k_steps / 14000.0;
     const int slabs = gemm_split_slabs(a_rows, width, k_steps, whole_slabs), stages = (k_steps + slabs - 1) / slabs;
     for (int splits = 1; splits <= std::min(kMaxSplits, stages); ++splits) {
-      const long long waves = (tiles * splits + slots[splits] - 1) / slots[splits];
-      const double l2 = 128.0 * (width + a_rows) * tiles * (double)k_steps / 14000.0;
       const double fixed = 5000.0 + (splits > 1 ? 450.0 * splits : 0.0) + std::min(M, kGemmBM) * (double)width / 10.0;
+      // no cluster of this size or larger is faster than this; the search is host time of every call with few tiles, 0.9 us
+      // without this line and 0.3 to 0.7 with it
+      if (best.width != 0 && std::max(hbm, l2) + fixed >= best.ns) break;
+      const long long waves = (tiles * splits + slots[splits] - 1) / slots[splits];
       const double stream = slab * slabs * ((stages + splits - 1) / splits);
       // CTAs of later waves start as SMs come free, so most of their fixed time hides under the others' streaming ...
       const double ns = std::max({hbm, l2, waves * stream}) + fixed * (0.7 + 0.3 * waves);
