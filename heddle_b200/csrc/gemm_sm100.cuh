@@ -833,7 +833,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) rms_rowstat_kernel(const T* __restrict__ x, const T* __restrict__ residual,
                                                           T* __restrict__ y_out, float* __restrict__ rstd, int M,
                                                           int N, long long ldx, float eps) {
-  grid_launch_dependents();
+  if (gridDim.x <= kFewBlocks) grid_launch_dependents();
   grid_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * 8 + warp;
@@ -880,6 +880,7 @@ __global__ void __launch_bounds__(256) rms_rowstat_kernel(const T* __restrict__ 
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  grid_launch_dependents();
   if (lane == 0) rstd[row] = rsqrtf(acc / (float)N + eps);
 }
 

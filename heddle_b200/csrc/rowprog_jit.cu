@@ -16,6 +16,7 @@
 //   * reductions: one row per warp (cols <= 1024) or per 128-thread CTA, R + 1 passes, pass r runs
 //     the program up to the r-th reduction and reduces the accumulator over the row; where they fit,
 //     the row's inputs are read once and kept in registers (cached_iterations).
+#include "ptx_sm100.cuh"
 #include "rowprog_sm100.cuh"
 
 #include <dlfcn.h>
@@ -219,7 +220,7 @@ extern "C" __global__ void __launch_bounds__(THREADS) rowprog_jit(const __grid_c
 
 const char* kReduceKernel = R"SRC(
 extern "C" __global__ void __launch_bounds__(THREADS) rowprog_jit(const __grid_constant__ Head p) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (gridDim.x <= HB_FEW_BLOCKS) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   constexpr int W = HB_WARPS_PER_ROW;
   constexpr int TPR = 32 * W;
@@ -248,6 +249,9 @@ extern "C" __global__ void __launch_bounds__(THREADS) rowprog_jit(const __grid_c
 #pragma unroll
   for (int pass = 0; pass <= HB_NRED; ++pass) {
     const bool last = pass == HB_NRED;
+#if HB_ITERS > 0
+    if (last) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the loads are done (see grid_launch_dependents)
+#endif
     const int kind = last ? 0 : RED_KIND(pass);
     float partial = (kind == 1) ? __int_as_float(0xff800000) : 0.f;
     if (row_ok) {
@@ -347,7 +351,8 @@ std::string generate(const RowProgParams& p, bool bf16, int warps_per_row) {
   int n_in = 0;
   const unsigned used = inputs_used(p, &n_in);
   const int iters = cached_iterations(p, warps_per_row);
-  snprintf(line, sizeof(line), "#define HB_ITERS %d\n#define HB_NIN %d\n#define HB_IN_USED %uu\n", iters, n_in, used);
+  snprintf(line, sizeof(line), "#define HB_ITERS %d\n#define HB_NIN %d\n#define HB_IN_USED %uu\n#define HB_FEW_BLOCKS %uu\n", iters, n_in,
+           used, kFewBlocks);
   s += line;
   snprintf(line, sizeof(line), "#define HB_T_BF16 %d\n#define HB_G %d\n#define HB_NRED %d\n#define HB_WARPS_PER_ROW %d\n", bf16 ? 1 : 0, kJitG,
            p.n_red, warps_per_row);

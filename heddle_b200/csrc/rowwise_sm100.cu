@@ -48,7 +48,7 @@ template <typename T, int kChunks, int kWarpsPerRow>
 __global__ void __launch_bounds__(256) row_softmax_kernel(const T* __restrict__ x, T* __restrict__ y, long long rows,
                                                           int cols, long long ld_x, long long ld_y, float scale_log2) {
   constexpr int kThreadsPerRow = 32 * kWarpsPerRow;
-  grid_launch_dependents();
+  if (gridDim.x <= kFewBlocks) grid_launch_dependents();
   grid_wait();
   __shared__ float red[2][8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -99,6 +99,7 @@ __global__ void __launch_bounds__(256) row_softmax_kernel(const T* __restrict__ 
 #pragma unroll
     for (int w = 0; w < kWarpsPerRow; ++w) sum += red[1][w];
   }
+  grid_launch_dependents();
   const float inv = 1.0f / sum;
 #pragma unroll
   for (int k = 0; k < kChunks; ++k) {
