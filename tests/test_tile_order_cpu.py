@@ -52,3 +52,37 @@ def test_every_block_is_taken_once(tmp_path):
     r = subprocess.run([str(tmp_path / "t")], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
     assert r.stdout.strip() == "432 lists"
+
+
+MODES = r'''
+#include <cstdio>
+#include "heddle_b200/csrc/tile_order.h"
+int main() {
+  struct { int heads, blocks; double bytes, from; int mode; } cases[] = {
+      {320, 10, 2.0 * 1166 * 128, hb::kPairsFromH2o, hb::kOrderPairs},   // pairs fill their rounds: 92 us, snake 107
+      {128, 16, 2.0 * 1931 * 128, hb::kPairsFromH2o, hb::kOrderPairs},   // 88 | 99
+      {64, 24, 2.0 * 3000 * 128, hb::kPairsFromH2o, hb::kOrderSnake},    // 102 | 92
+      {192, 11, 2.0 * 1361 * 64, hb::kPairsFromH2o, hb::kOrderSnake},    // 82 | 80
+      {144, 10, 4.0 * 1264 * 128, hb::kPairsFromDkdv, hb::kOrderPairs},  // 134 | 150
+      {48, 23, 4.0 * 2881 * 64 * 2, hb::kPairsFromDkdv, hb::kOrderSnake},  // 316 | 309
+      {144, 10, 4.0 * 1264 * 128, hb::kPairsFromDq128, hb::kOrderPairs},   // 103 | 111
+      {128, 31, 4.0 * 3852 * 128 / 4, hb::kPairsFromDq128, hb::kOrderSnake},  // 628 | 616
+      {96, 7, 4.0 * 1600 * 128, hb::kPairsNever, hb::kOrderSnake},
+      {128, 16, 4.0 * 4096 * 128, hb::kPairsNever, hb::kOrderPairs},     // 268 MB: more than L2
+  };
+  int i = 0;
+  for (auto& c : cases) {
+    hb::TileOrder o;
+    hb::tile_order_fill(&o, c.heads, c.blocks, true, c.bytes, 148, c.from);
+    if (o.mode != c.mode) return printf("case %d: mode %d\n", i, o.mode), 1;
+    ++i;
+  }
+}
+'''
+
+
+def test_the_order_is_the_one_that_was_measured_faster(tmp_path):
+    (tmp_path / "m.cpp").write_text(MODES)
+    subprocess.run(["g++", "-std=c++17", "-I", str(ROOT), str(tmp_path / "m.cpp"), "-o", str(tmp_path / "m")], check=True)
+    r = subprocess.run([str(tmp_path / "m")], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
