@@ -16,43 +16,8 @@ bool fa_split_takes(const hb_fa_args* a) {
   return (a->dtype == HB_BF16 || a->dtype == HB_FP16) && a->Sq > 0 && a->Sq <= kTileM;
 }
 
-struct FaSplitPlan {
-  int hb, hgroups, rows, nkv, items, pipes;
-  bool cuts;  // a run may start or end inside an item
-};
-
 static FaSplitPlan fa_split_plan(const hb_fa_args* a, int sm_count) {
-  FaSplitPlan pl;
-  const int group = a->Hq / a->Hkv;
-  pl.hgroups = (group + kTileM / a->Sq - 1) / (kTileM / a->Sq);
-  pl.hb = (group + pl.hgroups - 1) / pl.hgroups;
-  pl.hgroups = (group + pl.hb - 1) / pl.hb;
-  pl.rows = pl.hb * a->Sq;
-  pl.nkv = (a->Skv + kTileN - 1) / kTileN;
-  pl.items = a->B * a->Hkv * pl.hgroups;  // fits: fa_validate bounds B * Hq
-  // How many runs: the tiles of the longest one, plus what partial results cost in tiles (the combine launch, and each
-  // partial segment's rows written and read again).  Items left whole; every item cut into the same number of runs; all
-  // pipelines an equal share whatever the items.
-  const long long total = (long long)pl.items * pl.nkv, cap = 2ll * sm_count;
-  const long long whole = (pl.items + cap - 1) / cap * pl.nkv;
-  pl.pipes = (int)std::min<long long>(cap, pl.items);
-  pl.cuts = false;
-  long long best = whole;
-  const long long even = std::min<long long>(cap / pl.items, pl.nkv);
-  if (even > 1) {
-    const long long cost = (pl.nkv + even - 1) / even + 3 + pl.rows / 12;
-    if (cost < best) {
-      best = cost;
-      pl.pipes = (int)(pl.items * even);
-      pl.cuts = true;
-    }
-  }
-  const long long flat = std::min(cap, total);
-  if ((total + flat - 1) / flat + 3 + pl.rows / 10 < best) {
-    pl.pipes = (int)flat;
-    pl.cuts = true;
-  }
-  return pl;
+  return fa_split_plan(a->B, a->Hq, a->Hkv, a->Sq, a->Skv, sm_count);
 }
 
 uint64_t fa_split_workspace(const hb_fa_args* a, int sm_count) {
@@ -81,9 +46,10 @@ static int launch_split(const FaSplitParams& p, int grid, bool combine, int smem
   }
   HB_CUDA_CHECK(launch_dependent(kernel, grid, kSplitThreads, sizeof(Smem), stream, 0, p));
   if (combine) {
-    const long long segments = ((long long)p.pipes + p.items - 1) / p.items + 1;  // of one item, at most
+    const FaSplitPlan& pl = p.plan;
+    const long long segments = ((long long)pl.pipes + pl.items - 1) / pl.items + 1;  // of one item, at most
     const unsigned warps = (unsigned)std::min<long long>(kCombineMaxWarps, (segments + 3) / 4);
-    HB_CUDA_CHECK(launch_dependent(fa_split_combine_kernel<T, D>, (unsigned)p.items * (unsigned)p.rows, 32 * warps, 0, stream, 0, p));
+    HB_CUDA_CHECK(launch_dependent(fa_split_combine_kernel<T, D>, (unsigned)(fa_split_candidates(pl) * pl.rows), 32 * warps, 0, stream, 0, p));
   }
   return HB_OK;
 }
@@ -91,15 +57,15 @@ static int launch_split(const FaSplitParams& p, int grid, bool combine, int smem
 template <typename T>
 static int launch_split_d(const FaSplitParams& p, int D, int grid, bool combine, int smem_optin, cudaStream_t stream) {
   if (D == 128)
-    return p.rows <= 64 ? launch_split<T, 128, 64>(p, grid, combine, smem_optin, stream)
+    return p.plan.rows <= 64 ? launch_split<T, 128, 64>(p, grid, combine, smem_optin, stream)
                         : launch_split<T, 128, 128>(p, grid, combine, smem_optin, stream);
-  return p.rows <= 64 ? launch_split<T, 64, 64>(p, grid, combine, smem_optin, stream)
+  return p.plan.rows <= 64 ? launch_split<T, 64, 64>(p, grid, combine, smem_optin, stream)
                       : launch_split<T, 64, 128>(p, grid, combine, smem_optin, stream);
 }
 
 int fa_split_run(const hb_fa_args* a, const DeviceState* st, void* workspace, uint64_t workspace_bytes) {
   const FaSplitPlan pl = fa_split_plan(a, st->sm_count);
-  const bool cuts = pl.cuts;
+  const bool cuts = pl.cuts != 0;
   const uint64_t need = fa_split_workspace(a, st->sm_count);
   if (cuts && (workspace == nullptr || workspace_bytes < need))
     return set_error(HB_ERR_BAD_ARG, "hb_fa_fwd_ws: needs a workspace of %llu bytes, got %llu", (unsigned long long)need,
@@ -143,13 +109,7 @@ int fa_split_run(const hb_fa_args* a, const DeviceState* st, void* workspace, ui
   p.Skv = a->Skv;
   p.group = a->Hq / a->Hkv;
   p.causal = a->causal ? 1 : 0;
-  p.hb = pl.hb;
-  p.hgroups = pl.hgroups;
-  p.rows = pl.rows;
-  p.nkv = pl.nkv;
-  p.items = pl.items;
-  p.pipes = pl.pipes;
-  p.cuts = cuts ? 1 : 0;
+  p.plan = pl;
   const float scale = a->softmax_scale > 0.f ? a->softmax_scale : 1.0f / sqrtf((float)a->D);
   p.scale_log2 = scale * 1.4426950408889634f;
   const int grid = std::min(pl.pipes, st->sm_count);

@@ -18,9 +18,11 @@
 #pragma once
 
 #include "fa_fwd_sm100.cuh"
+#include "fa_split_plan.h"
 
 namespace hb {
 
+static_assert(kFaSplitTile == kTileM && kFaSplitTile == kTileN, "the plan and the kernel cut the same tiles");
 constexpr int kSplitThreads = 384;  // 2 softmax warpgroups, 2 MMA warps, 2 TMA warps
 enum FaSplitRole : uint32_t { kRoleSplitSoftmax = 6, kRoleSplitMma = 7, kRoleSplitTma = 8, kRoleSplitDrain = 9 };
 
@@ -35,13 +37,7 @@ struct alignas(64) FaSplitParams {
   int B, Hq, Hkv, Sq, Skv;
   int group;     // Hq / Hkv
   int causal;
-  int hb;        // query heads of a row tile
-  int hgroups;   // row tiles per (batch, kv head) = ceil(group / hb)
-  int rows;      // hb * Sq <= 128
-  int nkv;       // 128-key tiles
-  int items;     // B * Hkv * hgroups
-  int pipes;     // runs the tile list is cut into
-  int cuts;      // 0: every run is a run of whole items
+  FaSplitPlan plan;
   float scale_log2;
 };
 
@@ -70,25 +66,19 @@ struct FaSegment {
   int j0, j1;  // key tiles [j0, j1)
 };
 
-// Run of pipeline w: key tiles [begin, end) of the global list.
-__device__ __forceinline__ long long fa_split_begin(const FaSplitParams& p, int w) {
-  const long long n = static_cast<long long>(w) * p.items;
-  return p.cuts ? n * p.nkv / p.pipes : n / p.pipes * p.nkv;
-}
 __device__ __forceinline__ void fa_split_item(const FaSplitParams& p, int item, FaSegment& g) {
   g.item = item;
-  const int hg = item % p.hgroups, bk = item / p.hgroups;
+  const int hg = item % p.plan.hgroups, bk = item / p.plan.hgroups;
   g.b = bk / p.Hkv;
   g.hkv = bk - g.b * p.Hkv;
-  g.hq0 = g.hkv * p.group + hg * p.hb;
-  g.heads = min(p.hb, p.group - hg * p.hb);
+  g.hq0 = g.hkv * p.group + hg * p.plan.hb;
+  g.heads = min(p.plan.hb, p.group - hg * p.plan.hb);
 }
 __device__ __forceinline__ FaSegment fa_split_segment(const FaSplitParams& p, long long t, long long end) {
   FaSegment g;
-  const int item = static_cast<int>(t / p.nkv);
+  int item;
+  fa_split_segment(p.plan, t, end, item, g.j0, g.j1);
   fa_split_item(p, item, g);
-  g.j0 = static_cast<int>(t - static_cast<long long>(item) * p.nkv);
-  g.j1 = static_cast<int>(min(static_cast<long long>(p.nkv), g.j0 + (end - t)));
   return g;
 }
 
@@ -111,9 +101,9 @@ __device__ __forceinline__ void fa_split_softmax_role(const FaSplitParams& p, Fa
   const int past = p.Skv - p.Sq;
   uint32_t s_phase = 0, o_phase = 0;
 
-  const long long end = fa_split_begin(p, w + 1);
+  const long long end = fa_split_begin(p.plan, w + 1);
   bool first = true;
-  for (long long t = fa_split_begin(p, w); t < end; first = false) {
+  for (long long t = fa_split_begin(p.plan, w); t < end; first = false) {
     const FaSegment g = fa_split_segment(p, t, end);
     t += g.j1 - g.j0;
     float m = -INFINITY, l = 0.f;
@@ -150,7 +140,7 @@ __device__ __forceinline__ void fa_split_softmax_role(const FaSplitParams& p, Fa
       // the same rule as the general kernel: a maximum that grew by less than 2^8 is not adopted
       const float m_cand = fmaxf(m, row_max);
       const float diff = (m - m_cand) * scale_log2;
-      const bool adopt = row < p.rows && diff < -FaTraits<T>::kRescaleThreshold;  // padding rows never ask for a rescale
+      const bool adopt = row < p.plan.rows && diff < -FaTraits<T>::kRescaleThreshold;  // padding rows never ask for a rescale
       const float alpha = adopt ? fast_exp2(diff) : 1.f;
       m = adopt ? m_cand : m;
       const float m_scaled = (m == -INFINITY) ? 0.f : m * scale_log2;
@@ -206,13 +196,13 @@ __device__ __forceinline__ void fa_split_softmax_role(const FaSplitParams& p, Fa
     if (!mbar_wait_warp(&s.o_full[i], o_phase, ctx, kRoleSplitSoftmax)) return;
     o_phase ^= 1;
     tc_fence_after();
-    const bool whole = g.j0 == 0 && g.j1 == p.nkv;
-    const bool live = row < p.rows && head < g.heads;
+    const bool whole = g.j0 == 0 && g.j1 == p.plan.nkv;
+    const bool live = row < p.plan.rows && head < g.heads;
     const float inv_l = (l > 0.f) ? (1.0f / l) : 0.f;
     const float lse2 = (l > 0.f) ? (m * scale_log2 + fast_log2(l)) : -INFINITY;
     const long long slot = 2ll * w + (first ? 0 : 1);
     T* orow = static_cast<T*>(p.o) + g.b * p.o_sb + (g.hq0 + head) * p.o_sh + static_cast<long long>(pos) * p.o_ss;
-    float* prow = p.part_o + (slot * p.rows + row) * D;
+    float* prow = p.part_o + (slot * p.plan.rows + row) * D;
 #pragma unroll
     for (int c = 0; c < D / 32; ++c) {
       uint32_t r[32];
@@ -242,7 +232,7 @@ __device__ __forceinline__ void fa_split_softmax_role(const FaSplitParams& p, Fa
       if (p.lse != nullptr)
         p.lse[(static_cast<long long>(g.b) * p.Hq + g.hq0 + head) * p.Sq + pos] = lse2 * 0.6931471805599453f;
     } else if (live) {
-      p.part_lse[slot * p.rows + row] = lse2;
+      p.part_lse[slot * p.plan.rows + row] = lse2;
     }
     // the next segment's first product overwrites O: it waits for this thread's next arrival on p_full
     tc_fence_before();
@@ -275,8 +265,8 @@ __device__ __forceinline__ void fa_split_mma_role(const FaSplitParams& p, FaSpli
     }
   };
 
-  const long long end = fa_split_begin(p, w + 1);
-  for (long long t = fa_split_begin(p, w); t < end;) {
+  const long long end = fa_split_begin(p.plan, w + 1);
+  for (long long t = fa_split_begin(p.plan, w); t < end;) {
     const FaSegment g = fa_split_segment(p, t, end);
     t += g.j1 - g.j0;
     if (!mbar_wait_warp(&s.q_full[i], q_phase, ctx, kRoleSplitMma)) return;
@@ -323,8 +313,8 @@ __device__ __forceinline__ void fa_split_tma_role(const FaSplitParams& p, FaSpli
                                                   int w) {
   using Smem = FaSplitSmem<T, D, RC>;
   uint32_t slot = 0, phase = 1, q_phase = 1;  // "empty" barriers start out free
-  const long long end = fa_split_begin(p, w + 1);
-  for (long long t = fa_split_begin(p, w); t < end;) {
+  const long long end = fa_split_begin(p.plan, w + 1);
+  for (long long t = fa_split_begin(p.plan, w); t < end;) {
     const FaSegment g = fa_split_segment(p, t, end);
     t += g.j1 - g.j0;
     auto load_kv = [&](const CUtensorMap* tm, int j) -> bool {
@@ -341,7 +331,7 @@ __device__ __forceinline__ void fa_split_tma_role(const FaSplitParams& p, FaSpli
     };
     if (!mbar_wait(&s.q_empty[i], q_phase, ctx, kRoleSplitTma)) return;
     q_phase ^= 1;
-    mbar_arrive_expect_tx(&s.q_full[i], static_cast<uint32_t>(p.rows) * D * 2u);
+    mbar_arrive_expect_tx(&s.q_full[i], static_cast<uint32_t>(p.plan.rows) * D * 2u);
 #pragma unroll
     for (int h = 0; h < D / 64; ++h) tma_load_4d(s.q[i] + h * (RC * 128), &p.tm_q, &s.q_full[i], h * 64, 0, g.hq0, g.b);
     if (!load_kv(&p.tm_k, g.j0)) return;
@@ -359,7 +349,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) fa_split_kernel(const __grid
   Smem& s = *reinterpret_cast<Smem*>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   AbortCtx ctx{&s.abort_flag, p.status};
-  const int softmax_warps = (p.rows + 31) / 32;  // per pipeline; the others have no live row
+  const int softmax_warps = (p.plan.rows + 31) / 32;  // per pipeline; the others have no live row
 
   if (threadIdx.x == 0) {
     s.abort_flag = 0;
@@ -401,18 +391,18 @@ __global__ void __launch_bounds__(kSplitThreads, 1) fa_split_kernel(const __grid
   if (warp < 8) {
     reg_inc<200>();
     const int first_warp = fa_split_row0<RC>(i) / 32;
-    if (run && w < p.pipes && (warp & 3) >= first_warp && (warp & 3) < first_warp + softmax_warps)
+    if (run && w < p.plan.pipes && (warp & 3) >= first_warp && (warp & 3) < first_warp + softmax_warps)
       fa_split_softmax_role<T, D, RC>(p, s, ctx, tmem, i, w);
   } else {
     reg_dec<96>();
-    if (run && w < p.pipes && warp < 10) {
+    if (run && w < p.plan.pipes && warp < 10) {
       fa_split_mma_role<T, D, RC>(p, s, ctx, tmem, i, w);
       __syncwarp();
       if (s.abort_flag && lane == 0) {
         umma_commit(&s.drain[i]);  // aborting: let the tensor pipe drain before TMEM is released
         mbar_wait(&s.drain[i], 0, ctx, kRoleSplitDrain);
       }
-    } else if (run && w < p.pipes && lane == 0) {
+    } else if (run && w < p.plan.pipes && lane == 0) {
       fa_split_tma_role<T, D, RC>(p, s, ctx, i, w);
     }
   }
@@ -425,30 +415,32 @@ __global__ void __launch_bounds__(kSplitThreads, 1) fa_split_kernel(const __grid
   }
 }
 
-// Merges the partial segments of an item: one block per (item, row), its warps deal the segments out, a lane has D / 32
+// Merges the partial segments of an item: one block per (candidate, row), its warps deal the segments out, a lane has D / 32
 // columns; weights exp2(lse - max lse).  Items that one pipeline covered are already written.  It is bound by the latency of
-// its loads: the block has a warp per four segments (one item over 256 runs: 21.5 us a call with 4 warps, 15.3 with 16).
+// its loads: the block has a warp per four segments (one item over 256 runs: 21.5 us a call with 4 warps, 15.3 with 16).  With
+// fewer runs than items the candidates are the boundaries between runs: one block per (item, row) was 155648 blocks for 295 items
+// in parts (B38 Hq256 Hkv32, 16 rows, 4096 keys: 564 -> 457 us).
 constexpr int kCombineMaxWarps = 16;
 template <typename T, int D>
 __global__ void __launch_bounds__(kCombineMaxWarps * 32) fa_split_combine_kernel(const __grid_constant__ FaSplitParams p) {
   grid_launch_dependents();
   grid_wait();
-  const int item = blockIdx.x / p.rows, row = blockIdx.x - item * p.rows;
+  const int candidate = blockIdx.x / p.plan.rows, row = blockIdx.x - candidate * p.plan.rows;
+  const int item = fa_split_candidate(p.plan, candidate);
+  if (item < 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  const long long total = static_cast<long long>(p.items) * p.nkv, t0 = static_cast<long long>(item) * p.nkv;
-  // pipeline of tile t: the last w with w * total / pipes <= t
-  const int w0 = static_cast<int>(((t0 + 1) * p.pipes - 1) / total);
-  const int w1 = static_cast<int>(((t0 + p.nkv) * p.pipes - 1) / total);
+  int w0, w1;
+  fa_split_pipes_of(p.plan, item, w0, w1);
   FaSegment g;
   fa_split_item(p, item, g);
   const int head = row / p.Sq, pos = row - head * p.Sq;
   if (w0 == w1 || head >= g.heads) return;
-  // an item that does not start its pipeline's run left its segment in that pipeline's second slot (only w0 can)
-  const int first_slot = fa_split_begin(p, w0) / p.nkv == item ? 2 * w0 : 2 * w0 + 1;
-  auto slot_of = [&](int w) -> long long { return w == w0 ? first_slot : 2 * w; };
+  // only the first pipeline's part can be its second segment
+  const long long first_slot = fa_split_slot(p.plan, w0, item);
+  auto slot_of = [&](int w) -> long long { return w == w0 ? first_slot : 2ll * w; };
 
   float mx = -INFINITY;
-  for (int w = w0 + lane; w <= w1; w += 32) mx = fmaxf(mx, p.part_lse[slot_of(w) * p.rows + row]);
+  for (int w = w0 + lane; w <= w1; w += 32) mx = fmaxf(mx, p.part_lse[slot_of(w) * p.plan.rows + row]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   if (mx == -INFINITY) mx = 0.f;  // no visible key at all: every weight is 0
@@ -457,7 +449,7 @@ __global__ void __launch_bounds__(kCombineMaxWarps * 32) fa_split_combine_kernel
   float acc[kCols] = {}, sum = 0.f;
 #pragma unroll 4
   for (int w = w0 + warp; w <= w1; w += warps) {
-    const long long r = slot_of(w) * p.rows + row;
+    const long long r = slot_of(w) * p.plan.rows + row;
     const float wt = fast_exp2(p.part_lse[r] - mx);
     const float* src = p.part_o + r * D + lane * kCols;
     sum += wt;
