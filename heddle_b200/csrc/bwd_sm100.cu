@@ -572,26 +572,40 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
       const bool live = key < p.Skv;
       const uint32_t col_acc = static_cast<uint32_t>(half * (D / 2));
       const long long row_of = ((static_cast<long long>(b) * p.Hkv + hkv) * p.Skv + key) * D + col_acc;
-      const long long all = static_cast<long long>(p.B) * p.Hkv * p.Skv * D;
-      const int split = p.splits > 1 ? (hq0 - hkv * p.group) / heads : 0;
-      float* const part = p.splits > 1 ? p.part + split * 2 * all + row_of : nullptr;
+      if (p.splits == 1) {  // straight on: as one loop with the other form, 1.5 % of a call of short items
+        T* dv_row = static_cast<T*>(p.dv) + row_of;
+        T* dk_row = static_cast<T*>(p.dk) + row_of;
 #pragma unroll 1
-      for (int c = 0; c < D / 64; ++c) {
-        uint32_t r[32];
-#pragma unroll 1
-        for (int w = 0; w < 2; ++w) {  // dK, dV
+        for (int c = 0; c < D / 64; ++c) {
+          uint32_t r[32];
           __syncwarp();
-          tmem_ld32(tmem + lane_off + (w == 0 ? 384u : 256u) + col_acc + c * 32, r);
+          tmem_ld32(tmem + lane_off + 256 + col_acc + c * 32, r);
           tmem_wait_ld();
-          const float scale = w == 0 ? p.scale : 1.0f;
-          if (live && part == nullptr) {
-            bwd_store_row<T>(static_cast<T*>(w == 0 ? p.dk : p.dv) + row_of + c * 32, r, scale);
-          } else if (live) {
-            float4* dst = reinterpret_cast<float4*>(part + w * all + c * 32);
+          if (live) bwd_store_row<T>(dv_row + c * 32, r, 1.0f);
+          __syncwarp();
+          tmem_ld32(tmem + lane_off + 384 + col_acc + c * 32, r);
+          tmem_wait_ld();
+          if (live) bwd_store_row<T>(dk_row + c * 32, r, p.scale);
+        }
+      } else {
+        const long long all = static_cast<long long>(p.B) * p.Hkv * p.Skv * D;
+        float* const part = p.part + (hq0 - hkv * p.group) / heads * 2 * all + row_of;
+#pragma unroll 1
+        for (int c = 0; c < D / 64; ++c) {
+          uint32_t r[32];
+#pragma unroll 1
+          for (int w = 0; w < 2; ++w) {  // dK, dV
+            __syncwarp();
+            tmem_ld32(tmem + lane_off + (w == 0 ? 384u : 256u) + col_acc + c * 32, r);
+            tmem_wait_ld();
+            const float scale = w == 0 ? p.scale : 1.0f;
+            if (live) {
+              float4* dst = reinterpret_cast<float4*>(part + w * all + c * 32);
 #pragma unroll
-            for (int e = 0; e < 32; e += 4)
-              dst[e / 4] = make_float4(__uint_as_float(r[e]) * scale, __uint_as_float(r[e + 1]) * scale,
-                                       __uint_as_float(r[e + 2]) * scale, __uint_as_float(r[e + 3]) * scale);
+              for (int e = 0; e < 32; e += 4)
+                dst[e / 4] = make_float4(__uint_as_float(r[e]) * scale, __uint_as_float(r[e + 1]) * scale,
+                                         __uint_as_float(r[e + 2]) * scale, __uint_as_float(r[e + 3]) * scale);
+            }
           }
         }
       }
