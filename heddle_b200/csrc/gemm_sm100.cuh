@@ -223,7 +223,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
     tmem_wait_ld();
     tc_fence_before();
     __syncwarp();
-    if ((threadIdx.x & 31) == 0) mbar_arrive_cluster(release);
+    if ((threadIdx.x & 31) == 0) mbar_arrive_cluster_relaxed(release);
     // Coalesced stores: 128 rows x 64 columns go to a slab of shared memory in the 128-byte swizzled layout (a thread writes
     // its own row: conflict-free), one thread hands the slab to the TMA, which clips rows past M and columns past N_out.  The
     // warpgroup owns a ring of `n_slabs` staging slabs; slabs are rewritten once the TMA store that last used them has read
@@ -307,7 +307,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
     tmem_wait_ld();
     tc_fence_before();
     __syncwarp();
-    if ((threadIdx.x & 31) == 0) mbar_arrive_cluster(release);
+    if ((threadIdx.x & 31) == 0) mbar_arrive_cluster_relaxed(release);
 #pragma unroll
     for (int cc = 0; cc < 2; ++cc) {
       const int col = n0 + (part * 2 + cc) * 32;
@@ -386,7 +386,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
     auto release_acc = [&]() {
       tc_fence_before();
       __syncwarp();
-      if ((threadIdx.x & 31) == 0) mbar_arrive_cluster(release);
+      if ((threadIdx.x & 31) == 0) mbar_arrive_cluster_relaxed(release);
     };
     if (split_heads) {
       // head_dim 64 or 128: the warpgroup's 128 columns are read with one wait and the accumulator is

@@ -350,10 +350,10 @@ __device__ __forceinline__ void cluster_sync_relaxed() {
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
 // Arrive on a barrier given by its shared::cluster address (this CTA's or the peer's) to say that TMEM has been read: no
-// memory is handed over, so CTA-scope release is enough (tcgen05.fence::before_thread_sync orders the TMEM reads).  A
+// memory is handed over, and tcgen05.fence::before_thread_sync in front orders the TMEM reads, so the arrival is relaxed.  A
 // cluster-scope release waits for every earlier store of the thread: 1400-2900 cycles a tile in the GEMM epilogue.
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // try_wait that also orders against arrivals from the peer CTA
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
