@@ -171,7 +171,7 @@ def load() -> C.CDLL:
     lib.hb_fa_fwd_ws.restype = C.c_int
     lib.hb_fa_fwd_noalloc.argtypes = [C.POINTER(FaArgs)]
     lib.hb_fa_fwd_noalloc.restype = C.c_int
-    for name in ("hb_fa_bwd_preprocess", "hb_fa_bwd_dkdv", "hb_fa_bwd_dkdv_workspace", "hb_fa_bwd_dkdv_ws", "hb_fa_bwd_dq"):
+    for name in ("hb_fa_bwd_preprocess", "hb_fa_bwd_dkdv", "hb_fa_bwd_dq"):
         getattr(lib, name).argtypes = [C.POINTER(FaBwdArgs)]
         getattr(lib, name).restype = C.c_int
     lib.hb_fa_bwd_dkdv_workspace.argtypes = [C.POINTER(FaBwdArgs), C.POINTER(C.c_uint64)]

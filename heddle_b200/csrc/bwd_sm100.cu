@@ -1088,17 +1088,9 @@ static int launch_dkdv(const BwdParams& p, int grid, const DeviceState* st, cuda
 }
 template <typename T>
 static int launch_combine(const BwdParams& p, long long all, cudaStream_t stream) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>((all / 8 + 255) / 256), 2);
-  cfg.blockDim = dim3(256);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr = {};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  HB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, fa_bwd_combine_kernel<T>, static_cast<const float*>(p.part), static_cast<T*>(p.dk),
-                                   static_cast<T*>(p.dv), all, p.splits));
+  const dim3 grid(static_cast<unsigned>((all / 8 + 255) / 256), 2);
+  HB_CUDA_CHECK(launch_dependent(fa_bwd_combine_kernel<T>, grid, 256, 0, stream, 0, static_cast<const float*>(p.part),
+                                 static_cast<T*>(p.dk), static_cast<T*>(p.dv), all, p.splits));
   return HB_OK;
 }
 template <typename T, int D>

@@ -54,10 +54,10 @@ int get_device_info_noalloc(DeviceInfo* out);
 // of a long problem start in order instead (`early` false): waiting CTAs cost the step of B4 H32 S4096 0.4 % (2133 -> 2143 us).
 inline bool launch_early(double steps_per_cta) { return steps_per_cta <= 100.0; }
 template <typename... Params, typename... Args>
-inline cudaError_t launch_dependent_if(bool early, void (*kernel)(Params...), unsigned grid, unsigned threads, size_t smem,
+inline cudaError_t launch_dependent_if(bool early, void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem,
                                        cudaStream_t stream, unsigned cluster, Args... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -75,12 +75,12 @@ inline cudaError_t launch_dependent_if(bool early, void (*kernel)(Params...), un
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 template <typename... Params, typename... Args>
-inline cudaError_t launch_dependent(void (*kernel)(Params...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream,
+inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream,
                                     unsigned cluster, Args... args) {
   return launch_dependent_if(true, kernel, grid, threads, smem, stream, cluster, args...);
 }
 
-// 2-D .. 4-D tiled tensor map with 128-byte swizzle, zero fill out of bounds.
+// 2-D .. 5-D tiled tensor map with 128-byte swizzle, zero fill out of bounds.
 //   dims[i]     extent of dimension i in elements (dimension 0 is contiguous)
 //   strides[i]  byte stride of dimension i+1
 //   box[i]      tile extent of dimension i in elements
