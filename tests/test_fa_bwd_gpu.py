@@ -7,6 +7,8 @@ and 5e-3 * max(1, max|reference|) for fp16.  delta is an fp32 sum of 128 product
 <= 1e-4 relative to the same sum formed in fp32 from the kernel's own (rounded) O, and <= 1e-1 (bf16) /
 1e-2 (fp16) absolute against the oracle's delta, which uses the unrounded O.
 """
+import ctypes
+
 import pytest
 import torch
 
@@ -237,9 +239,9 @@ def test_bshd_strided_gqa_backward(ops):
     (1, 8, 1, 300, 300, 128, True, torch.bfloat16),    # eight heads of one KV head: one item each
     (1, 12, 2, 200, 500, 64, True, torch.float16),     # a group of six, causal with more keys than queries
     (2, 16, 4, 129, 257, 128, False, torch.bfloat16),  # ragged last tiles
-    (1, 6, 2, 1, 130, 64, False, torch.float16),       # one query row
+    (1, 16, 2, 1, 130, 64, False, torch.float16),      # one query row
 ])
-def test_grouped_heads_over_several_sms(ops, B, Hq, Hkv, Sq, Skv, D, causal, dtype):
+def test_grouped_heads_over_several_sms(ops, built_lib, B, Hq, Hkv, Sq, Skv, D, causal, dtype):
     """dK / dV of grouped queries with few KV heads: the heads of a group go to several items, whose fp32 parts are added."""
     q, k, v = O.make_qkv(B, Hq, Hkv, Sq, Skv, D, seed=Sq + Skv, dtype=dtype)
     d_o = torch.randn(q.shape, generator=torch.Generator().manual_seed(5)).to(dtype)
@@ -255,3 +257,17 @@ def test_grouped_heads_over_several_sms(ops, B, Hq, Hkv, Sq, Skv, D, causal, dty
     delta = ops.fa_bwd_preprocess(out, gc)
     again = ops.fa_bwd_dkdv(qc, kc, vc, gc, lse, delta, causal=causal)
     assert torch.equal(again[0], dk) and torch.equal(again[1], dv)
+    # the heads were dealt out (a workspace is asked for), and one item a KV head gives the same sums but for their order: fp32
+    # parts of up to 1e-4 of the largest sum, and one rounding to 16 bits
+    a, keep, _ = ops._bwd_args(qc, kc, vc, None, gc, lse, delta, causal, None, "bhsd")
+    one = torch.empty_like(dk), torch.empty_like(dv)
+    a.dk, a.dv = one[0].data_ptr(), one[1].data_ptr()
+    need = ctypes.c_uint64(0)
+    assert built_lib.hb_fa_bwd_dkdv_workspace(ctypes.byref(a), ctypes.byref(need)) == 0
+    assert need.value >= 2 * 8 * dk.numel()  # two parts or more of dK and dV in fp32
+    assert built_lib.hb_fa_bwd_dkdv(ctypes.byref(a)) == 0
+    torch.cuda.synchronize()
+    unit = 2.0**-7 if dtype == torch.bfloat16 else 2.0**-10
+    for got, ref in zip((dk, dv), one):
+        ref = ref.float()
+        assert ((got.float() - ref).abs() <= unit * ref.abs() + 1e-4 * ref.abs().max()).all()
