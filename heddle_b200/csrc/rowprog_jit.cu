@@ -471,6 +471,14 @@ int compile_image(const std::string& src, std::vector<char>* image) {
   return HB_OK;
 }
 
+// A program that was called before may meet a width that needs a kernel of its own inside a stream capture.  Loading a module touches
+// no stream, but a capture forbids such calls to the capturing thread unless the thread says that it knows.
+struct AllowedInCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  AllowedInCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~AllowedInCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 int compile(const std::string& src, CUfunction* out) {
   std::vector<char> image;
   const int rc = compile_image(src, &image);
@@ -518,6 +526,7 @@ int rowprog_jit_launch(const RowProgParams& p, bool bf16, const DeviceState& st,
     key += static_cast<char>(st.device);
     auto it = g_cache.find(key);
     if (it == g_cache.end()) {
+      const AllowedInCapture allowed;
       // the primary context of the current device must be current for the module load
       if (cudaFree(nullptr) != cudaSuccess) {
         set_error(HB_ERR_CUDA, "hb_rowwise_program: no CUDA context");

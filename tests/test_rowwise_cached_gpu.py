@@ -31,3 +31,20 @@ def test_against_the_oracle(built_lib, cols, program, n_in, dtype):
     # most 2^-7 (bf16) or 2^-10 (fp16) of it; the fp32 reductions themselves are within 1e-5
     tol = (2.0**-7 if dtype == torch.bfloat16 else 2.0**-10) * ref.abs() + 1e-5
     assert ((out.float().cpu() - ref).abs() <= tol).all()
+
+
+def test_a_width_met_first_inside_a_capture(built_lib):
+    """Each power of two of the width has a kernel of its own, so a program that has run may still compile inside a capture."""
+    from heddle_b200 import ops
+
+    if not built_lib.hb_rowwise_compiler_available():
+        pytest.skip("libnvrtc cannot be loaded in this process")
+    program = (("load", "input", 0, 0.0), ("mul", "imm", 0, 1.37), *NORM[1:])  # no other test's program
+    x = {cols: torch.randn(6, cols, generator=torch.Generator().manual_seed(cols)).to(torch.bfloat16).cuda() for cols in (2048, 16384)}
+    ops.rowwise_program(program, [x[2048]], mode="compiled")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = ops.rowwise_program(program, [x[16384]], mode="compiled")
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, ops.rowwise_program(program, [x[16384]], mode="compiled"))
