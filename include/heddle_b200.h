@@ -96,7 +96,10 @@ int hb_fa_fwd(const hb_fa_args* args);
 /*
  * hb_fa_fwd with a device workspace of the caller's.  With few query rows (decode, short prompts against a long cache) the
  * keys of one (batch, KV head) are then walked by several SMs whose partial results meet in the workspace; other calls run
- * exactly as through hb_fa_fwd.  hb_fa_fwd_workspace writes the bytes a call needs (0: none, workspace may be NULL).  The
+ * exactly as through hb_fa_fwd.  Where keys are shared out follows from B, Hkv, the group, Sq, Skv and the device's SMs, and
+ * each part rounds P to 16 bits against its own maximum: a row's result repeats for equal shapes, and between shapes (a batch
+ * and a shard of it) it is the same within rounding, not bit for bit.  hb_fa_fwd walks a row's keys in one order whatever else
+ * is in the call.  hb_fa_fwd_workspace writes the bytes a call needs (0: none, workspace may be NULL).  The
  * workspace must be 16-byte aligned, need not be initialised and may be reused once the call's work on `stream` is done.
  */
 int hb_fa_fwd_workspace(const hb_fa_args* args, uint64_t* bytes);
@@ -201,7 +204,9 @@ typedef enum hb_w_layout { HB_W_NK = 0, HB_W_KN = 1 } hb_w_layout;
  * tcgen05.mma.cta_group::2) when M > 128, else the single-CTA kernel (128 x 256 tiles), and for products
  * whose tiles would leave SMs idle the split-K kernel (a cluster of up to 8 CTAs shares a tile's K range).
  * SINGLE, PAIR and SPLIT force one of them; the results of the first two are identical (same accumulation
- * order per element). */
+ * order per element).  SPLIT sums parts of K, how many depends on M, N, K, the batch and the epilogue: under
+ * AUTO and SPLIT a row's result repeats for equal shapes and agrees within fp32 rounding of the sum between
+ * shapes (a row alone and in a larger M); SINGLE and PAIR give a row the same bits for every M. */
 typedef enum hb_gemm_schedule { HB_GEMM_AUTO = 0, HB_GEMM_SINGLE = 1, HB_GEMM_PAIR = 2, HB_GEMM_SPLIT = 3 } hb_gemm_schedule;
 
 typedef struct hb_gemm_args {
@@ -314,7 +319,9 @@ typedef struct hb_fa_bwd_args {
 int hb_fa_bwd_preprocess(const hb_fa_bwd_args* args);
 int hb_fa_bwd_dkdv(const hb_fa_bwd_args* args);
 /* hb_fa_bwd_dkdv with a device workspace of the caller's: with grouped queries and few KV heads the query heads of a KV head
- * are then dealt out to several SMs, whose fp32 partial results meet in the workspace.  hb_fa_bwd_dkdv_workspace writes the
+ * are then dealt out to several SMs, whose fp32 partial results meet in the workspace.  Into how many parts follows from B, Hkv,
+ * the group, Sq, Skv and the device's SMs: results repeat for equal shapes and agree within fp32 rounding of the sums between
+ * shapes; hb_fa_bwd_dkdv always sums in one order.  hb_fa_bwd_dkdv_workspace writes the
  * bytes a call needs (0: none); 16-byte aligned, need not be initialised, reusable once the work on `stream` is done. */
 int hb_fa_bwd_dkdv_workspace(const hb_fa_bwd_args* args, uint64_t* bytes);
 int hb_fa_bwd_dkdv_ws(const hb_fa_bwd_args* args, void* workspace, uint64_t bytes);
@@ -430,7 +437,9 @@ typedef struct hb_rowwise_args {
  * (nothing is compiled).  COMPILED: the specialised kernel or HB_ERR_UNSUPPORTED.  All three give
  * the same results.  HEDDLE_B200_ROWWISE_JIT=0 in the environment turns the compiler off;
  * HEDDLE_B200_NVRTC names the library file to load.  The first call with a new program compiles and
- * loads a module (0.1-0.7 s) and must not be made inside a stream capture; later calls only launch. */
+ * loads a module (0.1-0.7 s); later calls only launch.  A program with reductions whose inputs stay in
+ * registers between them has a kernel for each power of two of its width, compiled (0.1-0.4 s) when a
+ * width of that power is met first; inside a stream capture too. */
 typedef enum hb_rowwise_mode { HB_ROWWISE_AUTO = 0, HB_ROWWISE_INTERPRET = 1, HB_ROWWISE_COMPILED = 2 } hb_rowwise_mode;
 
 int hb_rowwise_program(const hb_rowwise_args* args);
