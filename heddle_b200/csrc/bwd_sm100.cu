@@ -1169,7 +1169,7 @@ static int bwd_dkdv_impl(const hb_fa_bwd_args* a, bool ws, void* workspace, uint
   if (heads * ((p.nkb + 1) / 2) > 0x3fffffffLL) return set_error(HB_ERR_UNSUPPORTED, "hb_fa_bwd_dkdv: problem too large");
   // a key tile reads Q and dO of its query heads
   int grid = tile_order_fill(&p.order, heads, p.nkb, p.causal != 0, 4.0 * a->Sq * a->D * p.group / p.splits, st->sm_count,
-                             kPairsFromDkdv);
+                             pairs_from(kPairsFromDkdv, a->Sq, a->Skv));
 #ifdef HB_DEBUG_GRID_ENV  // measurement builds only: fewer CTAs than SMs
   if (const char* e = getenv("HB_GRID")) grid = std::max(1, std::min(grid, atoi(e)));
 #endif
@@ -1229,7 +1229,7 @@ extern "C" int hb_fa_bwd_dq(const hb_fa_bwd_args* a) {
   p.by_heads = make_fast_div((uint32_t)a->Hq);
   p.by_group = make_fast_div((uint32_t)p.group);
   int grid = tile_order_fill(&p.order, (long long)a->B * a->Hq, p.nqb, p.causal != 0, 4.0 * a->Skv * a->D / p.group, st->sm_count,
-                             a->D == 128 ? kPairsFromDq128 : kPairsNever);
+                             pairs_from(a->D == 128 ? kPairsFromDq128 : kPairsNever, a->Sq, a->Skv));
 #ifdef HB_DEBUG_GRID_ENV  // measurement builds only: fewer CTAs than SMs
   if (const char* e = getenv("HB_GRID")) grid = std::max(1, std::min(grid, atoi(e)));
 #endif

@@ -361,7 +361,7 @@ static int h2o_impl(const hb_h2o_args* a) {
   const float scale = a->softmax_scale > 0.f ? a->softmax_scale : 1.0f / sqrtf((float)a->D);
   p.scale_log2 = scale * 1.4426950408889634f;
   const int grid = tile_order_fill(&p.order, (long long)a->B * a->Hq, p.nkb, p.causal != 0, 2.0 * a->Sq * a->D, st->sm_count,
-                                   kPairsFromH2o);
+                                   pairs_from(kPairsFromH2o, a->Sq, a->Skv));
   if (a->dtype == HB_BF16)
     return a->D == 128 ? launch_h2o<__nv_bfloat16, 128>(p, grid, st, stream) : launch_h2o<__nv_bfloat16, 64>(p, grid, st, stream);
   return a->D == 128 ? launch_h2o<__half, 128>(p, grid, st, stream) : launch_h2o<__half, 64>(p, grid, st, stream);

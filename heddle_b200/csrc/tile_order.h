@@ -53,17 +53,25 @@ HB_HD bool tile_order_get(const TileOrder& o, int g, int half, int& head, int& r
 }
 
 // From which fill of the rounds of pairs on pairs are the faster order under a mask: snake then gains little and its heads, all in
-// flight, share L2 worse.  The forward kernel stays with snake whatever the fill (0.81 to 1.03 of the pairs' time at fills of 0.93
-// to 1); dQ with D 64 too (0.92 to 0.99, one 1.003).  us, pairs | snake, bf16: H2O score B10 Hq32 Hkv16 S1166 D128 (fill 0.98) 92 |
-// 107, B4 H32 S1931 D128 (0.99) 88 | 99, B10 H32 S955 D64 (0.96) 64 | 68, below it B3 Hq64 Hkv16 S1361 D64 (0.89) 82 | 80; dK/dV B9 H16
+// flight, share L2 worse, the more so the more of it they need.  That is for the mask of a square problem: with more than a block
+// of earlier keys pairs cost unequal amounts, and snake is the better balance (dK/dV B5 Hq32 Hkv16 S823 on 1775 keys D64, fill
+// 0.95: 181 | 164 us).  The forward kernel stays with snake whatever the fill (0.81 to 1.03 of the pairs' time at fills of 0.93 to
+// 1); dQ with D 64 too (0.92 to 0.99, one 1.003).  us, pairs | snake, bf16: H2O score B10 Hq32 Hkv16 S1166 D128 (fill 0.98) 92 | 107,
+// B4 H32 S1931 D128 (0.99) 88 | 99, B10 H32 S955 D64 (0.96) 64 | 68, below it B3 Hq64 Hkv16 S1361 D64 (0.89) 82 | 80; dK/dV B9 H16
 // S1264 D128 (0.97) 134 | 150, B3 H32 S3735 D64 (0.97) 522 | 552, below it B6 Hq16 Hkv8 S2881 D64 (0.93) 316 | 309; dQ B9 H16 S1264
-// D128 (0.97) 103 | 111, below it B1 Hq128 Hkv32 S3852 D128 (0.96) 628 | 616.
-constexpr double kPairsFromH2o = 0.945, kPairsFromDkdv = 0.94, kPairsFromDq128 = 0.965, kPairsNever = 2.0;
+// D128 (0.97) 103 | 111, below it B1 Hq128 Hkv32 S3852 D128 (0.96) 628 | 616.  Over 75 MB: H2O B3 Hq256 Hkv32 S425 D128 (0.94) 50 | 54,
+// B5 Hq32 Hkv16 S1891 D128 (0.90) 105 | 108, dK/dV B2 H32 S2614 D128 (0.91) 228 | 237.
+struct PairsFrom {
+  double fill, crowded;  // up to 75 MB of common operands, and over it
+};
+constexpr PairsFrom kPairsFromH2o = {0.945, 0.90}, kPairsFromDkdv = {0.94, 0.90}, kPairsFromDq128 = {0.965, 0.965}, kPairsNever = {2.0, 2.0};
+inline PairsFrom pairs_from(const PairsFrom& square, int Sq, int Skv) { return Skv - Sq <= 128 ? square : kPairsNever; }
 
 // `bytes_per_head`: what the blocks of one head read in common.  Returns the grid size.
 inline int tile_order_fill(TileOrder* o, long long heads, int blocks, bool masked, double bytes_per_head, int sm_count,
-                           double pairs_from = kPairsNever) {
+                           const PairsFrom& pairs_from = kPairsNever) {
   constexpr double kL2Budget = 96e6;  // of 126 MB: the rest is for what the blocks do not share
+  constexpr double kL2Crowded = 75e6;
   o->heads = static_cast<int>(heads);
   o->blocks = blocks;
   o->npairs = (blocks + 1) / 2;
@@ -71,7 +79,8 @@ inline int tile_order_fill(TileOrder* o, long long heads, int blocks, bool maske
   // rounds of the longest CTA, in blocks
   const long long rounds = (units + sm_count - 1) / sm_count, pair_rounds = 2 * ((pairs + sm_count - 1) / sm_count);
   const double pairs_fill = (double)units / ((double)pair_rounds * sm_count);
-  if (masked) o->mode = heads * bytes_per_head <= kL2Budget && pairs_fill < pairs_from ? kOrderSnake : kOrderPairs;
+  const double common = heads * bytes_per_head, limit = common > kL2Crowded ? pairs_from.crowded : pairs_from.fill;
+  if (masked) o->mode = common <= kL2Budget && pairs_fill < limit ? kOrderSnake : kOrderPairs;
   else o->mode = rounds < pair_rounds ? kOrderHeads : kOrderPairs;
   if (units > 0x3fff0000LL) o->mode = kOrderPairs;
   const long long entries = o->mode == kOrderPairs ? pairs : units;

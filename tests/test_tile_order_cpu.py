@@ -58,7 +58,7 @@ MODES = r'''
 #include <cstdio>
 #include "heddle_b200/csrc/tile_order.h"
 int main() {
-  struct { int heads, blocks; double bytes, from; int mode; } cases[] = {
+  struct { int heads, blocks; double bytes; hb::PairsFrom from; int mode; } cases[] = {
       {320, 10, 2.0 * 1166 * 128, hb::kPairsFromH2o, hb::kOrderPairs},   // pairs fill their rounds: 92 us, snake 107
       {128, 16, 2.0 * 1931 * 128, hb::kPairsFromH2o, hb::kOrderPairs},   // 88 | 99
       {64, 24, 2.0 * 3000 * 128, hb::kPairsFromH2o, hb::kOrderSnake},    // 102 | 92
@@ -67,6 +67,10 @@ int main() {
       {48, 23, 4.0 * 2881 * 64 * 2, hb::kPairsFromDkdv, hb::kOrderSnake},  // 316 | 309
       {144, 10, 4.0 * 1264 * 128, hb::kPairsFromDq128, hb::kOrderPairs},   // 103 | 111
       {128, 31, 4.0 * 3852 * 128 / 4, hb::kPairsFromDq128, hb::kOrderSnake},  // 628 | 616
+      {768, 4, 2.0 * 425 * 128, hb::kPairsFromH2o, hb::kOrderPairs},        // 84 MB: 50 | 54
+      {64, 21, 4.0 * 2614 * 128, hb::kPairsFromDkdv, hb::kOrderPairs},      // 86 MB: 228 | 237
+      {80, 14, 4.0 * 823 * 64 * 2, hb::pairs_from(hb::kPairsFromDkdv, 823, 1775), hb::kOrderSnake},  // not square: 181 | 164
+      {256, 28, 2.0 * 3562 * 64 / 2, hb::pairs_from(hb::kPairsFromH2o, 3562, 3587), hb::kOrderPairs},
       {96, 7, 4.0 * 1600 * 128, hb::kPairsNever, hb::kOrderSnake},
       {128, 16, 4.0 * 4096 * 128, hb::kPairsNever, hb::kOrderPairs},     // 268 MB: more than L2
   };
