@@ -48,11 +48,11 @@ __device__ __forceinline__ bool elect_one() {
 // grid_launch_dependents() only after its own allocation: a dependent that took the columns first would wait for this grid,
 // and this grid for the columns.
 //
-// The kernels that give a row to a warp or a small block let their dependents in only when their own loads are done, unless the
+// The row kernels and compiled pointwise programs let their dependents in only when their own loads are done, unless the
 // grid is a few blocks: dependents that are let in at the start take the free slots next to a grid that does not fill the chip
 // evenly, and theirs do the same, so that such kernels in a row end up two to an SM beside idle ones.  us a call back to back, let
 // in at the start | when loaded | never: RMS statistic 1095 x 6240 8.7 | 6.9 | 7.0, three-input program 1096 x 600 2.65 | 1.8 | 2.3,
-// softmax 118 x 14880 5.3 | 4.6 | 4.6; with 3 blocks, RMS 22 x 8240 4.65 | 4.8 | 5.2.
+// softmax 118 x 14880 5.3 | 4.6 | 4.6, silu(x) y 69 x 12048 2.8 | 1.9 | 2.4; with 3 blocks, RMS 22 x 8240 4.65 | 4.8 | 5.2.
 constexpr unsigned kFewBlocks = 37;  // a quarter of the SMs
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

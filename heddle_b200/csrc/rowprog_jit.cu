@@ -195,7 +195,7 @@ __device__ __forceinline__ void round16(float* a) {
 
 const char* kStreamKernel = R"SRC(
 extern "C" __global__ void __launch_bounds__(THREADS) rowprog_jit(const __grid_constant__ Head p) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (gridDim.x <= HB_FEW_BLOCKS) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const unsigned groups = static_cast<unsigned>(p.cols >> 3);
   const unsigned total = static_cast<unsigned>(p.rows) * groups;
@@ -212,7 +212,8 @@ extern "C" __global__ void __launch_bounds__(THREADS) rowprog_jit(const __grid_c
       col[g] = ok[g] ? static_cast<int>(idx - r * groups) << 3 : 0;
     }
     float a[E];
-    rp_body(p, 0, row, col, ok, red, a, nullptr);
+    const bool last = total - g0 <= stride;  // of this thread's batches: its dependents are let in in front of the last store
+    rp_body(p, 0, row, col, ok, red, a, nullptr, last);
     if (g0 + stride < g0) break;  // the next index would wrap 32 bits: this was the last batch
   }
 }
@@ -274,7 +275,7 @@ extern "C" __global__ void __launch_bounds__(THREADS) rowprog_jit(const __grid_c
           col[g] = ok[g] ? gi << 3 : 0;
         }
         float a[E];
-        rp_body(p, pass, rows_, col, ok, red, a, cached);
+        rp_body(p, pass, rows_, col, ok, red, a, cached, false);
         if (!last) {
 #pragma unroll
           for (int g = 0; g < G; ++g) {
@@ -370,7 +371,10 @@ std::string generate(const RowProgParams& p, bool bf16, int warps_per_row) {
     s += kinds + "0)\n" + slots + "0)\n";
   }
   s += "__device__ __forceinline__ void rp_body(const Head& p, int pass, const long long* row, const int* col, const bool* ok,\n"
-       "                                        const float* red, float* a, const uint4* cached) {\n  float v[E];\n";
+       "                                        const float* red, float* a, const uint4* cached, bool let_in) {\n  float v[E];\n";
+  int last_store = -1;
+  for (int pc = 0; pc < p.n_inst; ++pc)
+    if (p.prog[pc].op == HB_EW_STORE_OUT) last_store = pc;
   bool tmp_used[HB_EW_MAX_TMP] = {};
   for (int pc = 0; pc < p.n_inst; ++pc)
     if (p.prog[pc].op == HB_EW_STORE_TMP) tmp_used[p.prog[pc].index] = true;
@@ -431,6 +435,7 @@ std::string generate(const RowProgParams& p, bool bf16, int warps_per_row) {
     } else if (in.op == HB_EW_STORE_TMP) {
       s += "  _Pragma(\"unroll\") for (int e = 0; e < E; ++e) t" + idx + "[e] = a[e];\n";
     } else if (in.op == HB_EW_STORE_OUT) {
+      if (p.n_red == 0 && pc == last_store) s += "  if (let_in) asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");  // see grid_launch_dependents\n";
       s += "  if (pass == HB_NRED) st_out(p.out[" + idx + "], p.ld_out[" + idx + "], row, col, ok, a);\n";
     } else {  // a reduction: the pass that ends here returns with the accumulator to reduce
       s += "  if (pass == " + std::to_string(reductions_seen) + ") return;\n";
