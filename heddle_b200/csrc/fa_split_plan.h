@@ -74,8 +74,8 @@ HB_HD void fa_split_pipes_of(const FaSplitPlan& p, int item, int& w0, int& w1) {
 }
 // Workspace slot of pipeline w's part of an item.  A run has at most two parts of items: its first segment and, where that is
 // another one, its last.
-HB_HD long long fa_split_slot(const FaSplitPlan& p, int w, int item) {
-  return 2ll * w + (fa_split_begin(p, w) < static_cast<long long>(item) * p.nkv ? 1 : 0);
+HB_HD int fa_split_slot(const FaSplitPlan& p, int w, int item) {
+  return fa_split_begin(p, w) / p.nkv == item ? 2 * w : 2 * w + 1;
 }
 // Candidates for an item in parts: every item, or, where there are fewer, every boundary between two runs.
 HB_HD int fa_split_candidates(const FaSplitPlan& p) { return p.pipes <= p.items ? p.pipes - 1 : p.items; }

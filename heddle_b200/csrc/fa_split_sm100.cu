@@ -49,7 +49,8 @@ static int launch_split(const FaSplitParams& p, int grid, bool combine, int smem
     const FaSplitPlan& pl = p.plan;
     const long long segments = ((long long)pl.pipes + pl.items - 1) / pl.items + 1;  // of one item, at most
     const unsigned warps = (unsigned)std::min<long long>(kCombineMaxWarps, (segments + 3) / 4);
-    HB_CUDA_CHECK(launch_dependent(fa_split_combine_kernel<T, D>, (unsigned)(fa_split_candidates(pl) * pl.rows), 32 * warps, 0, stream, 0, p));
+    auto merge = pl.pipes <= pl.items ? fa_split_combine_kernel<T, D, true> : fa_split_combine_kernel<T, D, false>;
+    HB_CUDA_CHECK(launch_dependent(merge, (unsigned)(fa_split_candidates(pl) * pl.rows), 32 * warps, 0, stream, 0, p));
   }
   return HB_OK;
 }

@@ -419,15 +419,16 @@ __global__ void __launch_bounds__(kSplitThreads, 1) fa_split_kernel(const __grid
 // columns; weights exp2(lse - max lse).  Items that one pipeline covered are already written.  It is bound by the latency of
 // its loads: the block has a warp per four segments (one item over 256 runs: 21.5 us a call with 4 warps, 15.3 with 16).  With
 // fewer runs than items the candidates are the boundaries between runs: one block per (item, row) was 155648 blocks for 295 items
-// in parts (B38 Hq256 Hkv32, 16 rows, 4096 keys: 564 -> 457 us).
+// in parts (B38 Hq256 Hkv32, 16 rows, 4096 keys: 564 -> 457 us).  The two forms are two kernels: as one it took 40 registers
+// instead of 32, and three blocks of 16 warps on an SM instead of four (B4 H1, 128 rows, 13208 keys: 24.2 -> 27.7 us).
 constexpr int kCombineMaxWarps = 16;
-template <typename T, int D>
+template <typename T, int D, bool kBoundaries>
 __global__ void __launch_bounds__(kCombineMaxWarps * 32) fa_split_combine_kernel(const __grid_constant__ FaSplitParams p) {
   grid_launch_dependents();
   grid_wait();
   const int candidate = blockIdx.x / p.plan.rows, row = blockIdx.x - candidate * p.plan.rows;
-  const int item = fa_split_candidate(p.plan, candidate);
-  if (item < 0) return;
+  const int item = kBoundaries ? fa_split_candidate(p.plan, candidate) : candidate;
+  if (kBoundaries && item < 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   int w0, w1;
   fa_split_pipes_of(p.plan, item, w0, w1);
@@ -436,8 +437,8 @@ __global__ void __launch_bounds__(kCombineMaxWarps * 32) fa_split_combine_kernel
   const int head = row / p.Sq, pos = row - head * p.Sq;
   if (w0 == w1 || head >= g.heads) return;
   // only the first pipeline's part can be its second segment
-  const long long first_slot = fa_split_slot(p.plan, w0, item);
-  auto slot_of = [&](int w) -> long long { return w == w0 ? first_slot : 2ll * w; };
+  const int first_slot = fa_split_slot(p.plan, w0, item);
+  auto slot_of = [&](int w) -> long long { return w == w0 ? first_slot : 2 * w; };
 
   float mx = -INFINITY;
   for (int w = w0 + lane; w <= w1; w += 32) mx = fmaxf(mx, p.part_lse[slot_of(w) * p.plan.rows + row]);
