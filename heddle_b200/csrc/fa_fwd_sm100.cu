@@ -186,11 +186,11 @@ static int fa_fwd_workspace_impl(const hb_fa_args* a, uint64_t* bytes) {
   *bytes = 0;
   bool empty = false;
   int rc = fa_validate(a, "hb_fa_fwd_workspace", /*allow_fp8=*/true, &empty);
-  if (rc != HB_OK || empty || !fa_split_takes(a)) return rc;
+  if (rc != HB_OK || empty) return rc;
   DeviceState* st = nullptr;
   rc = get_device_state(&st);
   if (rc != HB_OK) return rc;
-  *bytes = fa_split_workspace(a, st->sm_count);
+  if (fa_split_takes(a, st->sm_count)) *bytes = fa_split_workspace(a, st->sm_count);
   return HB_OK;
 }
 
@@ -202,7 +202,7 @@ static int fa_fwd_impl(const hb_fa_args* a, const char* who, bool ws, void* work
   DeviceState* st = nullptr;
   rc = get_device_state(&st);
   if (rc != HB_OK) return rc;
-  if (ws && fa_split_takes(a)) return fa_split_run(a, st, workspace, workspace_bytes);
+  if (ws && fa_split_takes(a, st->sm_count)) return fa_split_run(a, st, workspace, workspace_bytes);
   FaParams p;
   int grid = 0;
   rc = fa_fill_params(a, who, st->status_word, st->sm_count, &p, &grid);

@@ -54,6 +54,16 @@ inline FaSplitPlan fa_split_plan(int B, int Hq, int Hkv, int Sq, int Skv, int sm
   return pl;
 }
 
+// Whether the general kernel (a 256-row block per query head, an SM each) is the faster one for a call of at most 128 query rows.
+// Where one head fills a row tile nothing is packed, and where items stay whole nothing is shared out; then the general kernel's
+// rounds of blocks are finer than this kernel's, two items an SM at a time.  It matters where three of them stand against two of
+// these: us, here | general, D 128: 368 prompts of 128 rows 16.0 | 12.9, 384 of 100 rows 15.7 | 13.7, 352 of 100 rows on 442 keys 33.8
+// | 30.2, 304 on 357 27.0 | 22.9.  Elsewhere a round here is 0.8 of the time (608 prompts of 128 rows on 413 keys 45 | 47, 2100 on 314
+// 91 | 109), less with up to 96 rows (1552 of 65 rows 34 | 45) and with D 64 (1600 of 120 rows 30 | 40).
+inline bool fa_split_general_wins(const FaSplitPlan& p, int D, int sm_count) {
+  return D == 128 && p.hb == 1 && p.rows > 96 && !p.cuts && p.items > 2 * sm_count && p.items <= 3 * sm_count;
+}
+
 // Run of pipeline w: key tiles [begin(w), begin(w + 1)) of the list.
 HB_HD long long fa_split_begin(const FaSplitPlan& p, int w) {
   const long long n = static_cast<long long>(w) * p.items;

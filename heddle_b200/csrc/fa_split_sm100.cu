@@ -11,13 +11,14 @@
 
 namespace hb {
 
-bool fa_split_takes(const hb_fa_args* a) {
-  // The query rows of at least one head fit one 128-row tile.  Longer prompts fill the general kernel's 256-row blocks.
-  return (a->dtype == HB_BF16 || a->dtype == HB_FP16) && a->Sq > 0 && a->Sq <= kTileM;
-}
-
 static FaSplitPlan fa_split_plan(const hb_fa_args* a, int sm_count) {
   return fa_split_plan(a->B, a->Hq, a->Hkv, a->Sq, a->Skv, sm_count);
+}
+
+bool fa_split_takes(const hb_fa_args* a, int sm_count) {
+  // The query rows of at least one head fit one 128-row tile.  Longer prompts fill the general kernel's 256-row blocks.
+  if ((a->dtype != HB_BF16 && a->dtype != HB_FP16) || a->Sq <= 0 || a->Sq > kTileM) return false;
+  return !fa_split_general_wins(fa_split_plan(a, sm_count), a->D, sm_count);
 }
 
 uint64_t fa_split_workspace(const hb_fa_args* a, int sm_count) {

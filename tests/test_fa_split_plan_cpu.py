@@ -81,6 +81,14 @@ int main() {
             }
   if (!whole || !even || !flat || !few || !crossing || !middle) return fail("a form is missing", 0, 0, 0, 0, 0);
   printf("whole %d even %d flat %d, fewer runs than items %d\n", whole, even, flat, few);
+  // whole items of one head each between two and three rounds of SMs: the general kernel (us here | there in the header)
+  struct { int B, Hq, Hkv, Sq, Skv, D; bool general; } calls[] = {
+      {23, 16, 4, 128, 128, 128, true}, {3, 128, 16, 100, 100, 128, true}, {22, 16, 16, 100, 442, 128, true}, {19, 16, 16, 100, 357, 128, true},
+      {76, 8, 2, 128, 413, 128, false}, {1050, 2, 2, 128, 314, 128, false}, {97, 16, 16, 65, 65, 128, false}, {25, 64, 16, 120, 120, 64, false},
+      {18, 16, 16, 128, 128, 128, false}, {23, 16, 4, 128, 128, 64, false}, {40, 32, 4, 1, 300, 128, false}, {16, 64, 8, 1, 6001, 128, false}};
+  for (auto& c : calls)
+    if (fa_split_general_wins(fa_split_plan(c.B, c.Hq, c.Hkv, c.Sq, c.Skv, 148), c.D, 148) != c.general)
+      return fail("general", c.B, c.Hq, c.Hkv, c.Sq, c.Skv);
   // the merge is as large as what there is to merge, not as the number of items
   const FaSplitPlan p = fa_split_plan(38, 256, 32, 16, 4096, 148);
   if (!p.cuts || fa_split_candidates(p) * p.rows > 2 * 148 * 128) return fail("merge", 38, 256, 32, 16, 4096);
