@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
   using Smem = BwdSmemKv<D>;
   constexpr uint32_t kBwdTileBytes = bwd_tile_bytes(D);
   Smem& s = *reinterpret_cast<Smem*>(smem_raw);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   AbortCtx ctx{&s.abort_flag, p.status};
   if (threadIdx.x == 0) {
     bwd_init(s, ctx, smem_raw, 8);
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = s.tmem_base;
+  const uint32_t tmem = warp_uniform(s.tmem_base);
   const bool run = (s.abort_flag == 0);
   grid_launch_dependents();
   grid_wait();
@@ -633,7 +633,7 @@ __global__ void __launch_bounds__(kBwdDqThreads, 1) fa_bwd_dq_kernel(const __gri
   using Smem = BwdSmemQ<D>;
   constexpr uint32_t kBwdTileBytes = bwd_tile_bytes(D);
   Smem& s = *reinterpret_cast<Smem*>(smem_raw);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   AbortCtx ctx{&s.abort_flag, p.status};
   if (threadIdx.x == 0) {
     bwd_init(s, ctx, smem_raw, 4);
@@ -649,7 +649,7 @@ __global__ void __launch_bounds__(kBwdDqThreads, 1) fa_bwd_dq_kernel(const __gri
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = s.tmem_base;
+  const uint32_t tmem = warp_uniform(s.tmem_base);
   const bool run = (s.abort_flag == 0);
   grid_launch_dependents();
   grid_wait();

@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) fa_split_kernel(const __grid
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   using Smem = FaSplitSmem<T, D, RC>;
   Smem& s = *reinterpret_cast<Smem*>(smem_raw);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   AbortCtx ctx{&s.abort_flag, p.status};
   const int softmax_warps = (p.plan.rows + 31) / 32;  // per pipeline; the others have no live row
 
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) fa_split_kernel(const __grid
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = s.tmem_base;
+  const uint32_t tmem = warp_uniform(s.tmem_base);
   const bool run = (s.abort_flag == 0);
   grid_launch_dependents();
   grid_wait();

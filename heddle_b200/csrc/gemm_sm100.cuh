@@ -447,7 +447,7 @@ template <typename T, int EPI>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_constant__ GemmParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   GemmSmem& s = *reinterpret_cast<GemmSmem*>(smem_raw);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   AbortCtx ctx{&s.abort_flag, p.status};
 
   if (threadIdx.x == 0) {
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = s.tmem_base;
+  const uint32_t tmem = warp_uniform(s.tmem_base);
   const bool run = (s.abort_flag == 0);
   grid_launch_dependents();
   grid_wait();
@@ -663,7 +663,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
   uint8_t* const ring_b = ring_a + kStages * kPairStageA;
   uint8_t* const slabs = ring_b + kStages * kPairStageB;
   GemmPairCtrl& s = *reinterpret_cast<GemmPairCtrl*>(smem_raw + kPairSlots * 32768);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   AbortCtx ctx{&s.abort_flag, p.status};
@@ -692,7 +692,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
   tc_fence_before();
   cluster_sync_all();  // both CTAs' barriers are initialised before anything arrives at them
   tc_fence_after();
-  const uint32_t tmem = s.tmem_base;
+  const uint32_t tmem = warp_uniform(s.tmem_base);
   const bool run = (s.abort_flag == 0);
   grid_launch_dependents();
   grid_wait();

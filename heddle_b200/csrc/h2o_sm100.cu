@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(kH2oThreads, 1) h2o_score_kernel(const __grid_
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   using Smem = H2oSmem<D>;
   Smem& s = *reinterpret_cast<Smem*>(smem_raw);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   AbortCtx ctx{&s.abort_flag, p.status};
 
   if (threadIdx.x == 0) {
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kH2oThreads, 1) h2o_score_kernel(const __grid_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = s.tmem_base;
+  const uint32_t tmem = warp_uniform(s.tmem_base);
   const bool run = (s.abort_flag == 0);
   grid_launch_dependents();
   grid_wait();

@@ -42,6 +42,13 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// A value that every lane of the warp has, in a form the compiler knows to be the same: the branches between roles are then uniform
+// and what the MMA and TMA warps compute can stay in uniform registers, which is where tcgen05.mma takes its operands from.
+// us without -> with, back to back: H2O B2 Hq32 Hkv8 S3000 276 -> 271, B8 H32 S454 64.0 -> 62.9; train step B5 H16 S101 28.9 -> 27.5; FP8
+// attention B3 Hq32 Hkv8 S335 17.4 -> 17.1; bf16 B4 H32 S4096 570 -> 564.  Not in the split-K GEMM (512 x 4096 x 4096 24.0 -> 24.5).
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ int uniform_warp() { return static_cast<int>(warp_uniform(threadIdx.x >> 5)); }
+
 // Programmatic dependent launch (launch_dependent() in host_common.h): the next kernel of the stream may be scheduled from
 // grid_launch_dependents() on, and waits in grid_wait() until every earlier kernel is complete and its writes are visible.
 // No kernel touches global memory (its parameters aside) before grid_wait().  A kernel that holds TMEM calls
