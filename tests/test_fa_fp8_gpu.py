@@ -65,3 +65,15 @@ def test_fp8_rejects_other_head_dims(ops):
     x = torch.zeros(1, 1, 128, 64, device="cuda").to(torch.float8_e4m3fn)
     with pytest.raises(RuntimeError, match="head_dim 128"):
         ops.fa_fwd(x, x, x)
+
+
+@pytest.mark.parametrize("Skv", [1, 63, 64, 65, 128, 192, 193])
+def test_fp8_halves_of_a_key_tile(ops, Skv):
+    """P reaches the MMA in two halves of 64 keys: tiles that end in, at and behind either half, against the same oracle and bounds."""
+    (qq, kq, vq), scales, (qd, kd, vd) = _quantised(2, 2, 1, 300, Skv, 128, seed=Skv)
+    out = ops.fa_fwd(qq.cuda(), kq.cuda(), vq.cuda(), causal=False, scales=scales)
+    torch.cuda.synchronize()
+    assert ops.status_word() == 0
+    ref, _ = O.attention_eager(qd, kd, vd, causal=False)
+    # one key: O = V, exact but for the rounding to bf16; else P in e4m3, 2^-4 relative per weight
+    assert (out.float().cpu() - ref).abs().max().item() <= (6e-2 if Skv > 1 else 2.0**-8 * vd.abs().max().item())
