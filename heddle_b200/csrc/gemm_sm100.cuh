@@ -99,25 +99,28 @@ __device__ __forceinline__ void gemm_tile_coords(const GemmParams& p, int t, int
   m_t = first_m + r - n_t * static_cast<int>(last ? p.div_last.d : p.div_rows.d);
 }
 
-// 1 / (1 + e^-v): one ex2, one rcp (1 ulp), so no call and no branch; e^-v = inf gives 0
-__device__ __forceinline__ float sigmoid_f32(float v) { return fast_rcp(1.0f + __expf(-v)); }
+// x / (1 + e^-v) with one ex2 and one rcp (1 ulp) of a number in [1, 2]: no call, no branch, nothing overflows or is flushed on the
+// way (e^-v for v < -88 would be, and 1 / (1 + e^-v) be 0 where the product is a normal number)
+__device__ __forceinline__ float times_sigmoid(float x, float v) {
+  const float t = __expf(-fabsf(v));
+  return x * fast_rcp(1.0f + t) * (v >= 0.0f ? 1.0f : t);
+}
 
 template <int ACT>
 __device__ __forceinline__ float apply_act(float v) {
-  if constexpr (ACT == kActSilu) return v * sigmoid_f32(v);
+  if constexpr (ACT == kActSilu) return times_sigmoid(v, v);
   if constexpr (ACT == kActRelu) return fmaxf(v, 0.0f);
   // 0.5 (1 + tanh u) = sigmoid(2 u), which does not cancel for u << 0
-  if constexpr (ACT == kActGeluTanh) return v * sigmoid_f32(1.5957691216f * (v + 0.044715f * v * v * v));
-  if constexpr (ACT == kActSigmoid) return sigmoid_f32(v);
+  if constexpr (ACT == kActGeluTanh) return times_sigmoid(v, 1.5957691216f * (v + 0.044715f * v * v * v));
+  if constexpr (ACT == kActSigmoid) return times_sigmoid(1.0f, v);
   if constexpr (ACT == kActTanh) return tanhf(v);
   return v;
 }
 
 // f(std::integral_constant<int, ACT>) for the activation `act`.  A product chooses once per slab of 64 columns: a choice per element
 // put all five functions, and their branches, behind each of 128 unrolled elements.
-// us, 408 x 17024 x 3232: SiLU 117 -> 45, GELU 159 -> 46, none 42; 14368 x 14144 x 4480 +
-// GELU 2860 -> 1335, none 1350; 4000 x 8192 x 640 + bias and row scale 56 -> 47.  The division went with it: 2722 x 3200 x 2640 +
-// SwiGLU 38.0 -> 35.4.
+// us, 408 x 17024 x 3232: SiLU 117 -> 55, GELU 159 -> 56, none 52; 14368 x 14144 x 4480 + GELU 3180 -> 1506; 4000 x 8192 x 640:
+// SiLU 238 -> 56, GELU 324 -> 63, bias and row scale 56 -> 51.  The division went with it: 2722 x 3200 x 2640 + SwiGLU 46.5 -> 44.6.
 template <typename F>
 __device__ __forceinline__ void with_act(int act, F&& f) {
   switch (act) {
