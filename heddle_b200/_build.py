@@ -1,4 +1,5 @@
-"""Build the C-ABI shared library ``libheddle_b200.so`` in-tree with nvcc for sm_100a.
+"""Build the C-ABI shared library ``libheddle_b200.so`` in-tree with nvcc for sm_100a, and ``_native.so``, the host path of the
+tensor-level calls (csrc/ops_native.cpp), with g++ against PyTorch's headers.
 
 nvcc cross-compiles without a GPU, so this runs on a CPU-only host as well.
 ``python -m heddle_b200._build`` rebuilds; ``build(force=False)`` rebuilds only
@@ -11,12 +12,15 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 OBJ_DIR = CSRC / "build"
 LIB_PATH = PKG_DIR / "libheddle_b200.so"
+NATIVE_SRC = CSRC / "ops_native.cpp"
+NATIVE_PATH = PKG_DIR / "_native.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -38,10 +42,10 @@ def sources() -> list[Path]:
 
 
 def _stale() -> bool:
-    if not LIB_PATH.exists():
+    if not LIB_PATH.exists() or not NATIVE_PATH.exists():
         return True
-    t = LIB_PATH.stat().st_mtime
-    deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h"))
+    t = min(LIB_PATH.stat().st_mtime, NATIVE_PATH.stat().st_mtime)
+    deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + [NATIVE_SRC]
     deps.append(PKG_DIR.parent / "include" / "heddle_b200.h")
     return any(d.stat().st_mtime > t for d in deps)
 
@@ -55,12 +59,30 @@ def _compile_one(src: Path) -> tuple[Path, str]:
     return obj, proc.stderr
 
 
+def _build_native() -> None:
+    """``_native.so``: PyTorch's libraries are the ones that ``import torch`` has loaded."""
+    import torch
+
+    torch_dir = Path(torch.__file__).resolve().parent
+    cxx = shutil.which("g++") or "g++"
+    cuda_include = Path(_nvcc()).resolve().parent.parent / "include"
+    includes = [torch_dir / "include", torch_dir / "include/torch/csrc/api/include", cuda_include, sysconfig.get_paths()["include"]]
+    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[f for d in includes for f in ("-isystem", str(d))], str(NATIVE_SRC), "-o", str(NATIVE_PATH),
+           f"-L{torch_dir / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError(f"g++ failed for {NATIVE_SRC.name}:\n{proc.stdout}\n{proc.stderr}")
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     if not force and not _stale():
         return LIB_PATH
     OBJ_DIR.mkdir(parents=True, exist_ok=True)
     with concurrent.futures.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as pool:
+        native = pool.submit(_build_native)
         results = list(pool.map(_compile_one, sources()))
+        native.result()
     log = "".join(text for _, text in results)
     (OBJ_DIR / "ptxas.log").write_text(log)
     if verbose:

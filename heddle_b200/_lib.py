@@ -150,6 +150,19 @@ EXPORTS = (
 )
 
 _lib = None
+native = None  # heddle_b200._native, bound to the library, once load() has run
+
+
+def _load_native(lib: C.CDLL) -> None:
+    """The host path of the tensor-level calls (csrc/ops_native.cpp), calling into ``lib``."""
+    global native
+    try:
+        from . import _native
+    except ImportError as e:
+        raise RuntimeError(f"heddle_b200._native cannot be loaded ({e}): build it with `python -m heddle_b200._build`") from e
+    addresses = {name: C.cast(getattr(lib, name), C.c_void_p).value for name in EXPORTS}
+    _native.bind(addresses, check, EW_OPS, EW_SRCS)
+    native = _native
 
 
 def load() -> C.CDLL:
@@ -214,6 +227,7 @@ def load() -> C.CDLL:
     lib.hb_debug_fa_fwd_stages.restype = C.c_int
     lib.hb_debug_wait_timeout.argtypes = [C.c_uint32, C.POINTER(C.c_uint32), C.POINTER(C.c_uint64)]
     lib.hb_debug_wait_timeout.restype = C.c_int
+    _load_native(lib)
     _lib = lib
     return lib
 

@@ -83,14 +83,11 @@ def _tilelang_sdpa_direct(q, k, v, is_causal=None, scale=None, out_bshd=False):
     """
     if is_causal is None:
         is_causal = q.shape[2] == k.shape[2]
-    out = None
-    if out_bshd:
-        out_dtype = q.dtype if q.dtype in (torch.bfloat16, torch.float16) else torch.bfloat16
-        out = torch.empty((q.shape[0], q.shape[2], q.shape[1], q.shape[3]), dtype=out_dtype,
-                          device=q.device).transpose(1, 2)
     if torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad):
-        return _SdpaFunc.apply(q, k, v, bool(is_causal), scale, out)
-    return ops.fa_fwd(q, k, v, causal=bool(is_causal), softmax_scale=scale, out=out)
+        return _SdpaFunc.apply(q, k, v, bool(is_causal), scale, ops.empty_bshd(q) if out_bshd else None)
+    if out_bshd:
+        return ops.fa_fwd_stored_bshd(q, k, v, bool(is_causal), scale)
+    return ops.fa_fwd(q, k, v, causal=bool(is_causal), softmax_scale=scale)
 
 
 @torch.fx.wrap

@@ -25,7 +25,7 @@ from typing import Dict, List, Optional, Tuple
 import torch
 import torch.fx as fx
 
-from .. import ops
+from .. import _lib, ops
 
 _ACT_NAMES = {"silu": "silu", "relu": "relu", "sigmoid": "sigmoid", "tanh": "tanh"}
 
@@ -54,9 +54,19 @@ class _PreparedWeights:
             version = -1
         return (t.data_ptr(), version, tuple(t.shape), tuple(t.stride()), t.dtype, str(t.device))
 
+    @classmethod
+    def _states(cls, sources):
+        if _lib.native is None and sources[0].is_cuda:
+            _lib.load()  # one form of the state from the first call on
+        if _lib.native is not None:
+            state = _lib.native.tensors_state(sources)
+            if state is not NotImplemented:
+                return state
+        return tuple(cls._state(t) for t in sources)
+
     def get(self, sources, build):
         key = tuple(id(t) for t in sources)
-        state = tuple(self._state(t) for t in sources)
+        state = self._states(sources)
         entry = self._entries.get(key)
         if entry is not None:
             refs, old_state, value = entry

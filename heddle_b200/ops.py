@@ -29,7 +29,9 @@ def _require_cuda(*tensors: torch.Tensor) -> None:
                 f"{t.device} — there is no CPU fallback")
 
 
-# Host time of a call matters where its kernels take microseconds: on the host of the measurements a launch is 3 us, a
+# Plain calls run through ``_lib.native`` (csrc/ops_native.cpp), which does what the functions below do in Python, from the second
+# call of a process on (the first one loads the library); it returns NotImplemented for everything else, and the general path
+# here goes on.  Host time of a call matters where its kernels take microseconds: on the host of the measurements a launch is 3 us, a
 # torch.cuda.current_stream() 2.2, a torch.cuda.device block 1.4, a reshape that changes nothing 1.0.  So the raw stream handle
 # is asked for, the device is only switched when it is another one, and views are only made where a shape needs them.
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
@@ -87,6 +89,10 @@ def fa_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal: bool = 
     ``debug_stages`` (2, 3 or 5; bf16, head_dim 128) runs the kernel built with that depth of the K/V
     ring (``hb_debug_fa_fwd_stages``): results must not depend on it.
     """
+    if _lib.native is not None and debug_stages is None:
+        r = _lib.native.fa_fwd(q, k, v, causal, softmax_scale, layout, return_lse, out, scales, False)
+        if r is not NotImplemented:
+            return r
     _require_cuda(q, k, v)
     if q.dim() != 4 or k.dim() != 4 or v.dim() != 4:
         raise ValueError("q, k, v must be 4-D")
@@ -133,6 +139,21 @@ def fa_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal: bool = 
     else:
         _call(device, lib.hb_fa_fwd, C.byref(a))
     return (out, lse) if return_lse else out
+
+
+def fa_fwd_stored_bshd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool, softmax_scale: Optional[float]) -> torch.Tensor:
+    """``fa_fwd`` of [B, H, S, D] tensors whose result is stored as [B, S, H, D] and returned as its [B, H, S, D] view."""
+    if _lib.native is not None:
+        r = _lib.native.fa_fwd(q, k, v, causal, softmax_scale, "bhsd", False, None, None, True)
+        if r is not NotImplemented:
+            return r
+    return fa_fwd(q, k, v, causal=causal, softmax_scale=softmax_scale, out=empty_bshd(q))
+
+
+def empty_bshd(q: torch.Tensor) -> torch.Tensor:
+    """An attention result for ``q`` [B, H, S, D], stored as [B, S, H, D]."""
+    out_dtype = q.dtype if q.dtype in (torch.bfloat16, torch.float16) else torch.bfloat16
+    return torch.empty((q.shape[0], q.shape[2], q.shape[1], q.shape[3]), dtype=out_dtype, device=q.device).transpose(1, 2)
 
 
 def _bwd_args(q, k, v, o, d_o, lse, delta, causal, softmax_scale, layout):
@@ -221,6 +242,10 @@ def fa_bwd(q, k, v, o, d_o, lse, *, causal: bool = False, softmax_scale: Optiona
     ``create_separated_bwd_function``, Heddle/heddle/frontend/bwd_separator.py:366-455).
 
     ``lse`` is the natural-log LSE [B, Hq, Sq] of the forward pass.  Returns (dQ, dK, dV)."""
+    if _lib.native is not None:
+        r = _lib.native.fa_bwd(q, k, v, o, d_o, lse, causal, softmax_scale, layout)
+        if r is not NotImplemented:
+            return r
     _require_cuda(q, o, d_o)
     lse = _as_fp32(lse)
     bshd = layout == "bshd"
@@ -292,6 +317,10 @@ def gemm_epilogue(a: torch.Tensor, w: torch.Tensor, epilogue: str = "none", *,
     ``residual`` (..., N_out); ``rope`` = (cos [S, hd/2] fp32, sin, head_dim, rope_cols)
     with position = row index mod S.  Returns (..., N_out) in a's dtype.
     """
+    if _lib.native is not None and out is None and epilogue in _lib.EPILOGUES:
+        r = _lib.native.gemm_epilogue(a, w, _lib.EPILOGUES[epilogue], bias, row_scale, residual, rope, _lib.GEMM_SCHEDULES[_gemm_schedule])
+        if r is not NotImplemented:
+            return r
     _require_cuda(a, w, bias, row_scale, residual)
     if a.dtype not in (torch.bfloat16, torch.float16) or w.dtype != a.dtype:
         raise TypeError(f"gemm_epilogue needs matching bf16/fp16 operands, got {a.dtype} and {w.dtype}")
@@ -374,6 +403,9 @@ def _mult8(*values: int) -> bool:
     return all(int(v) % 8 == 0 for v in values)
 
 
+_UNARY = ("none", "silu", "relu", "gelu_tanh", "sigmoid", "tanh")
+
+
 def bmm(a: torch.Tensor, b: torch.Tensor, epilogue: str = "none", *, bias: Optional[torch.Tensor] = None,
         residual: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``epilogue(a @ b)`` for a [B, M, K] and b [B, K, N] (``torch.bmm``) in one launch of the tcgen05 GEMM:
@@ -381,12 +413,16 @@ def bmm(a: torch.Tensor, b: torch.Tensor, epilogue: str = "none", *, bias: Optio
     the MN-major operand path, ``w.transpose(-1, -2)`` views of [N, K] storage through the K-major one — so
     neither layout is copied.  Replaces the reference's batched kernel
     (Heddle/heddle/frontend/backend.py:491-536).  K, N and the strides must be multiples of 8 elements."""
+    if _lib.native is not None and bias is None and residual is None and epilogue in _UNARY:
+        r = _lib.native.bmm(a, b, _lib.EPILOGUES[epilogue], _lib.GEMM_SCHEDULES[_gemm_schedule])
+        if r is not NotImplemented:
+            return r
     _require_cuda(a, b, bias, residual)
     if a.dim() != 3 or b.dim() != 3 or a.shape[0] != b.shape[0] or a.shape[2] != b.shape[1]:
         raise ValueError(f"bmm needs [B, M, K] x [B, K, N], got {tuple(a.shape)} and {tuple(b.shape)}")
     if a.dtype not in (torch.bfloat16, torch.float16) or b.dtype != a.dtype:
         raise TypeError(f"bmm needs matching bf16/fp16 operands, got {a.dtype} and {b.dtype}")
-    if epilogue not in ("none", "silu", "relu", "gelu_tanh", "sigmoid", "tanh"):
+    if epilogue not in _UNARY:
         raise ValueError(f"bmm takes the unary epilogues only, not {epilogue!r}")
     Bn, M, K = a.shape
     N = b.shape[2]
@@ -449,6 +485,10 @@ def rms_rowstat(x: torch.Tensor, residual: Optional[torch.Tensor] = None, eps: f
 
     Returns (y, rstd): y = x + residual in x's dtype (None unless ``write_sum`` or a
     residual is given), rstd fp32 of shape x.shape[:-1]."""
+    if _lib.native is not None and residual is None and not write_sum:
+        r = _lib.native.rms_rowstat(x, eps)
+        if r is not NotImplemented:
+            return None, r
     _require_cuda(x, residual)
     N = x.shape[-1]
     if residual is None and not write_sum and N > 0 and x.is_contiguous():
@@ -508,6 +548,10 @@ def prepare_weight(weights: "Sequence[torch.Tensor]", gamma: Optional[torch.Tens
 def row_softmax(x: torch.Tensor, scale: float = 1.0) -> torch.Tensor:
     """softmax(scale * x) over the last dimension (``hb_row_softmax``): bf16 / fp16, last dimension a
     multiple of 8 and at most 16384."""
+    if _lib.native is not None:
+        r = _lib.native.row_softmax(x, scale)
+        if r is not NotImplemented:
+            return r
     _require_cuda(x)
     cols = x.shape[-1]
     x2 = x if x.dim() == 2 else x.reshape(-1, cols)
@@ -529,6 +573,9 @@ def _rowwise_code(heads, imms):
     return code
 
 
+_ROWWISE_MODES = {"auto": _lib.ROWWISE_AUTO, "interpret": _lib.ROWWISE_INTERPRET, "compiled": _lib.ROWWISE_COMPILED}
+
+
 def rowwise_program(program, inputs=(), rowvecs=(), rowscalars=(), n_outputs: int = 1, mode: str = "auto"):
     """Run an accumulator-machine program over [rows, cols] views of ``inputs`` (``hb_rowwise_program``).
 
@@ -538,6 +585,10 @@ def rowwise_program(program, inputs=(), rowvecs=(), rowscalars=(), n_outputs: in
     (shape (..., 1) or (...)), converted to fp32.  Returns ``n_outputs`` new tensors shaped like the
     inputs (a tuple when ``n_outputs`` > 1).  ``mode``: "auto" (a kernel compiled for this program at
     run time and cached; the interpreter kernel where NVRTC cannot be loaded), "interpret" or "compiled"."""
+    if _lib.native is not None and mode in _ROWWISE_MODES:
+        r = _lib.native.rowwise_program(program, inputs, rowvecs, rowscalars, n_outputs, _ROWWISE_MODES[mode])
+        if r is not NotImplemented:
+            return r
     if not inputs:
         raise ValueError("rowwise_program needs at least one full-size input")
     _require_cuda(*inputs, *rowvecs, *rowscalars)
@@ -580,7 +631,7 @@ def rowwise_program(program, inputs=(), rowvecs=(), rowscalars=(), n_outputs: in
     a.program = _rowwise_code(tuple((op, src, int(index)) for op, src, index, _ in program),
                               struct.pack(f"{len(program)}d", *[float(inst[3]) for inst in program]))
     a.stream = _stream_ptr(x0.device)
-    a.mode = {"auto": _lib.ROWWISE_AUTO, "interpret": _lib.ROWWISE_INTERPRET, "compiled": _lib.ROWWISE_COMPILED}[mode]
+    a.mode = _ROWWISE_MODES[mode]
     _call(x0.device, _lib.load().hb_rowwise_program, C.byref(a))
     return outs[0] if n_outputs == 1 else tuple(outs)
 
@@ -590,6 +641,10 @@ def h2o_score(q: torch.Tensor, k: torch.Tensor, lse: torch.Tensor, *, causal: bo
     """H2O score through ``hb_h2o_score``: score[b,h,j] = sum_i exp(s_ij - lse_i), fp32 [B, Hq, Skv].
 
     ``lse`` is the natural-log LSE [B, Hq, Sq] that ``fa_fwd(..., return_lse=True)`` returns."""
+    if _lib.native is not None:
+        r = _lib.native.h2o_score(q, k, lse, causal, softmax_scale, layout)
+        if r is not NotImplemented:
+            return r
     _require_cuda(q, k, lse)
     if q.dtype not in (torch.bfloat16, torch.float16) or k.dtype != q.dtype:
         raise TypeError(f"unsupported or mismatched dtypes: {q.dtype}, {k.dtype}")
