@@ -144,7 +144,7 @@ ROWWISE_AUTO, ROWWISE_INTERPRET, ROWWISE_COMPILED = 0, 1, 2
 
 # every symbol include/heddle_b200.h declares
 EXPORTS = (
-    "hb_fa_fwd", "hb_fa_fwd_workspace", "hb_fa_fwd_ws", "hb_fa_fwd_noalloc", "hb_status_word_noalloc", "hb_fa_bwd_preprocess", "hb_fa_bwd_dkdv", "hb_fa_bwd_dkdv_workspace", "hb_fa_bwd_dkdv_ws", "hb_fa_bwd_dq", "hb_h2o_score", "hb_gemm_epilogue", "hb_rms_rowstat", "hb_prepare_weight", "hb_row_softmax", "hb_rowwise_program", "hb_rowwise_compiler_available", "hb_debug_rowwise_compile", "hb_status_word",
+    "hb_fa_fwd", "hb_fa_fwd_workspace", "hb_fa_fwd_ws", "hb_fa_fwd_noalloc", "hb_status_word_noalloc", "hb_fa_bwd_preprocess", "hb_fa_bwd_dkdv", "hb_fa_bwd_dkdv_workspace", "hb_fa_bwd_dkdv_ws", "hb_fa_bwd_dq", "hb_fa_bwd", "hb_h2o_score", "hb_gemm_epilogue", "hb_rms_rowstat", "hb_prepare_weight", "hb_row_softmax", "hb_rowwise_program", "hb_rowwise_compiler_available", "hb_debug_rowwise_compile", "hb_status_word",
     "hb_version",
     "hb_query", "hb_last_error", "hb_shutdown", "hb_debug_umma", "hb_debug_wait_timeout", "hb_debug_fa_fwd_stages",
 )
@@ -191,6 +191,8 @@ def load() -> C.CDLL:
     lib.hb_fa_bwd_dkdv_workspace.restype = C.c_int
     lib.hb_fa_bwd_dkdv_ws.argtypes = [C.POINTER(FaBwdArgs), C.c_void_p, C.c_uint64]
     lib.hb_fa_bwd_dkdv_ws.restype = C.c_int
+    lib.hb_fa_bwd.argtypes = [C.POINTER(FaBwdArgs), C.c_void_p, C.c_uint64]
+    lib.hb_fa_bwd.restype = C.c_int
     lib.hb_h2o_score.argtypes = [C.POINTER(H2oArgs)]
     lib.hb_h2o_score.restype = C.c_int
     lib.hb_gemm_epilogue.argtypes = [C.POINTER(GemmArgs)]

@@ -82,6 +82,13 @@ struct alignas(64) BwdParams {
   // and dV go to `part` ([splits][dK, dV][B, Hkv, Skv, D], fp32) and fa_bwd_combine_kernel adds them up
   int splits;
   float* part;
+  // A kernel of hb_fa_bwd, whose three kernels follow one another in the stream.  The preprocess kernel lets its dependents in once all
+  // earlier kernels are complete, so dK/dV may load its inputs beside it: only its consumers, who read delta, wait for it.  They let
+  // dQ in behind that wait, so dQ has nothing to wait for at its start: its CTAs run beside those of dK/dV where the latter leave SMs
+  // free or finish early, and dQ waits for dK/dV at its end, so that a kernel that waits for dQ has both.
+  // us of a train step, one after the other -> chained: D64 B1 H1 S333 causal 26.6 -> 18.8, D128 B5 H16 S101 27.5 -> 22.1, D128 B3 H4 S941
+  // causal 60.6 -> 43.6, D64 B1 Hq4 Hkv1 S1844 causal 81.4 -> 60.4, D64 B8 H12 S577 101.9 -> 98.6, D128 B16 H16 S700 causal 327 -> 322.
+  int chained;
   TileOrder order;  // the work list: dkdv heads B * Hkv * splits, blocks nkb, rank 0 = the first; dq heads B * Hq, blocks nqb, rank 0 = the last
   FastDiv by_heads, by_splits, by_group;  // dkdv: Hkv (of B * Hkv), splits;  dq: Hq, group
   float scale_log2, scale;
@@ -267,8 +274,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
   tc_fence_after();
   const uint32_t tmem = warp_uniform(s.tmem_base);
   const bool run = (s.abort_flag == 0);
-  grid_launch_dependents();
-  grid_wait();
+  if (!p.chained) {
+    grid_launch_dependents();
+    grid_wait();
+  }
   const int past = p.Skv - p.Sq;
 
   // Work list (tile_order.h): u >> 1 is the entry, u & 1 its half where entries are pairs.  Under a causal mask key tile 0 is
@@ -436,6 +445,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
     __syncwarp();
   } else if (run) {
     // ---------------- consumers: one key per pair of threads ----------------
+    if (p.chained) {
+      grid_wait();
+      grid_launch_dependents();
+    }
     const int slab = warp & 3, half = warp >> 2;
     const int key_in_tile = slab * 32 + lane;
     const uint32_t lane_off = static_cast<uint32_t>(slab * 32) << 16;
@@ -652,7 +665,7 @@ __global__ void __launch_bounds__(kBwdDqThreads, 1) fa_bwd_dq_kernel(const __gri
   const uint32_t tmem = warp_uniform(s.tmem_base);
   const bool run = (s.abort_flag == 0);
   grid_launch_dependents();
-  grid_wait();
+  if (!p.chained) grid_wait();
   const int past = p.Skv - p.Sq;
 
   // Work list (tile_order.h): u >> 1 is the entry, u & 1 its half where entries are pairs.  Under a causal mask the last query
@@ -821,8 +834,9 @@ __global__ void __launch_bounds__(kBwdDqThreads, 1) fa_bwd_dq_kernel(const __gri
       const int q = q0 + row_in_tile;
       const bool live = q < p.Sq;
       const long long stat = (static_cast<long long>(b) * p.Hq + hq) * p.Sq + q;
-      const float nlse2 = live ? -__ldg(p.lse + stat) * 1.4426950408889634f : -INFINITY;
-      const float dlt = live ? __ldg(p.delta + stat) : 0.f;
+      // from L2: a chained call has not waited in front of these reads, and an earlier kernel may have left lines in L1
+      const float nlse2 = live ? -__ldcg(p.lse + stat) * 1.4426950408889634f : -INFINITY;
+      const float dlt = live ? __ldcg(p.delta + stat) : 0.f;
       const float4 l4 = make_float4(nlse2, nlse2, nlse2, nlse2);
       const uint64_t ndl2 = pack_f32x2(-dlt, -dlt);
       for (int kt = 0; kt < nk; ++kt, ++cnt) {
@@ -910,6 +924,7 @@ __global__ void __launch_bounds__(kBwdDqThreads, 1) fa_bwd_dq_kernel(const __gri
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
+  if (p.chained) grid_wait();
 }
 
 // ------------------------------------------------------------------------------------------
@@ -922,8 +937,8 @@ __global__ void __launch_bounds__(256, 4) fa_bwd_preprocess_kernel(const T* __re
                                                                  long long o_sb, long long o_sh, long long o_ss,
                                                                  long long g_sb, long long g_sh, long long g_ss) {
   constexpr int kLanesPerRow = D / 8, kRowsPerLoad = 32 / kLanesPerRow, kRowsPerWarp = 4 * kRowsPerLoad;
-  grid_launch_dependents();
   grid_wait();
+  grid_launch_dependents();  // behind the wait: see BwdParams::chained
   const int lane = threadIdx.x & 31, sub = lane / kLanesPerRow, lr = lane % kLanesPerRow;
   // the host checks that B * H * S fits 31 bits: 32-bit divisions (the 64-bit ones are emulated and were
   // a visible part of this short kernel)
@@ -1076,8 +1091,8 @@ static int bwd_launch(void (*kernel)(const BwdParams), const BwdParams& p, int g
     HB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
     configured[st->device & 63] = true;
   }
-  HB_CUDA_CHECK(launch_dependent_if(launch_early(tile_order_steps(p.order, p.causal != 0, steps_per_block)), kernel, grid, threads,
-                                    sizeof(Smem), stream, 0, p));
+  const bool early = p.chained != 0 || launch_early(tile_order_steps(p.order, p.causal != 0, steps_per_block));
+  HB_CUDA_CHECK(launch_dependent_if(early, kernel, grid, threads, sizeof(Smem), stream, 0, p));
   return HB_OK;
 }
 template <typename T, int D>
@@ -1111,6 +1126,14 @@ static int launch_preprocess(const hb_fa_bwd_args* a, cudaStream_t stream) {
 
 }  // namespace hb
 
+static int bwd_combine(const hb_fa_bwd_args* a, const hb::BwdParams& p) {
+  using namespace hb;
+  if (p.splits == 1) return HB_OK;
+  const long long all = (long long)a->B * a->Hkv * a->Skv * a->D;
+  cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
+  return a->dtype == HB_BF16 ? launch_combine<__nv_bfloat16>(p, all, stream) : launch_combine<__half>(p, all, stream);
+}
+
 extern "C" int hb_fa_bwd_preprocess(const hb_fa_bwd_args* a) {
   using namespace hb;
   clear_error();
@@ -1132,7 +1155,9 @@ extern "C" int hb_fa_bwd_preprocess(const hb_fa_bwd_args* a) {
   return a->D == 128 ? launch_preprocess<__half, 128>(a, stream) : launch_preprocess<__half, 64>(a, stream);
 }
 
-static int bwd_dkdv_impl(const hb_fa_bwd_args* a, bool ws, void* workspace, uint64_t workspace_bytes) {
+// `chained`: a call of hb_fa_bwd, which has `combine` launched later (a no-op where there are no parts)
+static int bwd_dkdv_impl(const hb_fa_bwd_args* a, bool ws, void* workspace, uint64_t workspace_bytes, bool chained = false,
+                         hb::BwdParams* combine = nullptr) {
   using namespace hb;
   clear_error();
   int rc = bwd_check(a, "hb_fa_bwd_dkdv");
@@ -1163,6 +1188,7 @@ static int bwd_dkdv_impl(const hb_fa_bwd_args* a, bool ws, void* workspace, uint
     return set_error(HB_ERR_BAD_ARG, "hb_fa_bwd_dkdv_ws: needs a 16-byte aligned workspace of %llu bytes, got %llu",
                      (unsigned long long)need, (unsigned long long)workspace_bytes);
   p.part = static_cast<float*>(workspace);
+  p.chained = chained ? 1 : 0;
   p.by_heads = make_fast_div((uint32_t)a->Hkv);
   p.by_splits = make_fast_div((uint32_t)p.splits);
   const long long heads = (long long)a->B * a->Hkv * p.splits;
@@ -1177,8 +1203,8 @@ static int bwd_dkdv_impl(const hb_fa_bwd_args* a, bool ws, void* workspace, uint
     rc = a->D == 128 ? launch_dkdv<__nv_bfloat16, 128>(p, grid, st, stream) : launch_dkdv<__nv_bfloat16, 64>(p, grid, st, stream);
   else
     rc = a->D == 128 ? launch_dkdv<__half, 128>(p, grid, st, stream) : launch_dkdv<__half, 64>(p, grid, st, stream);
-  if (rc != HB_OK || p.splits == 1) return rc;
-  return a->dtype == HB_BF16 ? launch_combine<__nv_bfloat16>(p, all, stream) : launch_combine<__half>(p, all, stream);
+  if (combine != nullptr) *combine = p;
+  return rc != HB_OK || combine != nullptr ? rc : bwd_combine(a, p);
 }
 
 extern "C" int hb_fa_bwd_dkdv(const hb_fa_bwd_args* a) { return bwd_dkdv_impl(a, false, nullptr, 0); }
@@ -1203,7 +1229,7 @@ extern "C" int hb_fa_bwd_dkdv_workspace(const hb_fa_bwd_args* a, uint64_t* bytes
   return HB_OK;
 }
 
-extern "C" int hb_fa_bwd_dq(const hb_fa_bwd_args* a) {
+static int bwd_dq_impl(const hb_fa_bwd_args* a, bool chained) {
   using namespace hb;
   clear_error();
   int rc = bwd_check(a, "hb_fa_bwd_dq");
@@ -1226,6 +1252,7 @@ extern "C" int hb_fa_bwd_dq(const hb_fa_bwd_args* a) {
   if (rc != HB_OK) return rc;
   const long long total = (long long)a->B * a->Hq * ((p.nqb + 1) / 2);
   if (total > 0x3fffffffLL) return set_error(HB_ERR_UNSUPPORTED, "hb_fa_bwd_dq: problem too large");
+  p.chained = chained ? 1 : 0;
   p.by_heads = make_fast_div((uint32_t)a->Hq);
   p.by_group = make_fast_div((uint32_t)p.group);
   int grid = tile_order_fill(&p.order, (long long)a->B * a->Hq, p.nqb, p.causal != 0, 4.0 * a->Skv * a->D / p.group, st->sm_count,
@@ -1236,6 +1263,27 @@ extern "C" int hb_fa_bwd_dq(const hb_fa_bwd_args* a) {
   if (a->dtype == HB_BF16)
     return a->D == 128 ? launch_dq<__nv_bfloat16, 128>(p, grid, st, stream) : launch_dq<__nv_bfloat16, 64>(p, grid, st, stream);
   return a->D == 128 ? launch_dq<__half, 128>(p, grid, st, stream) : launch_dq<__half, 64>(p, grid, st, stream);
+}
+
+extern "C" int hb_fa_bwd_dq(const hb_fa_bwd_args* a) { return bwd_dq_impl(a, false); }
+
+extern "C" int hb_fa_bwd(const hb_fa_bwd_args* a, void* workspace, uint64_t bytes) {
+  using namespace hb;
+  int rc = hb_fa_bwd_preprocess(a);
+  if (rc != HB_OK) return rc;
+  DeviceState* st = nullptr;
+  rc = get_device_state(&st);
+  if (rc != HB_OK) return rc;
+  // Chained unless the kernels are long (as with early starts, launch_early()): 64 heads of 2048 keys unmasked 618 | 622 us, B2 Hq32 Hkv8
+  // S3000 773 | 787.  An empty problem launches no kernel, or a memset in place of one: nothing to chain.
+  const double nqb = (a->Sq + 127) / 128, nkb = (a->Skv + 127) / 128;
+  const double steps = (double)a->B * a->Hq * nqb * (a->causal ? nkb - (nqb - 1) / 2 : nkb) / st->sm_count;
+  const bool chained = a->B > 0 && a->Sq > 0 && a->Skv > 0 && launch_early(steps);
+  BwdParams parts;
+  parts.splits = 1;
+  rc = bwd_dkdv_impl(a, a->Hq != a->Hkv, workspace, bytes, chained, &parts);
+  if (rc == HB_OK) rc = bwd_dq_impl(a, chained);
+  return rc == HB_OK ? bwd_combine(a, parts) : rc;
 }
 
 #ifdef HB_BWD_PROF

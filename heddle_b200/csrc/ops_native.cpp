@@ -34,11 +34,8 @@ struct Lib {
   decltype(&hb_fa_fwd) fa_fwd;
   decltype(&hb_fa_fwd_workspace) fa_fwd_workspace;
   decltype(&hb_fa_fwd_ws) fa_fwd_ws;
-  decltype(&hb_fa_bwd_preprocess) fa_bwd_preprocess;
-  decltype(&hb_fa_bwd_dkdv) fa_bwd_dkdv;
   decltype(&hb_fa_bwd_dkdv_workspace) fa_bwd_dkdv_workspace;
-  decltype(&hb_fa_bwd_dkdv_ws) fa_bwd_dkdv_ws;
-  decltype(&hb_fa_bwd_dq) fa_bwd_dq;
+  decltype(&hb_fa_bwd) fa_bwd;
   decltype(&hb_h2o_score) h2o_score;
   decltype(&hb_gemm_epilogue) gemm_epilogue;
   decltype(&hb_rms_rowstat) rms_rowstat;
@@ -320,17 +317,12 @@ PyObject* fa_bwd(PyObject*, PyObject* const* args, Py_ssize_t n) {
   fill_dims(a, d, causal != 0, scale, dtype, dev);
   at::Tensor ws;
   uint64_t need = 0;
-  const bool grouped = d.Hq != d.Hkv;
-  if (grouped) {
+  if (d.Hq != d.Hkv) {
     const int rc = lib.fa_bwd_dkdv_workspace(&a, &need);
     if (rc != HB_OK) return raise_status(rc);
     if (need > 0) ws = empty_like_options(q, {static_cast<int64_t>(need)}, at::kByte);
   }
-  const int rc = unlocked([&] {
-    int r = lib.fa_bwd_preprocess(&a);
-    if (r == HB_OK) r = grouped ? lib.fa_bwd_dkdv_ws(&a, need > 0 ? ws.data_ptr() : nullptr, need) : lib.fa_bwd_dkdv(&a);
-    return r == HB_OK ? lib.fa_bwd_dq(&a) : r;
-  });
+  const int rc = unlocked([&] { return lib.fa_bwd(&a, need > 0 ? ws.data_ptr() : nullptr, need); });
   if (rc != HB_OK) return raise_status(rc);
   if (layout == 1) {
     dq = dq.transpose(1, 2);
@@ -702,11 +694,8 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HB_BIND(fa_fwd)
   HB_BIND(fa_fwd_workspace)
   HB_BIND(fa_fwd_ws)
-  HB_BIND(fa_bwd_preprocess)
-  HB_BIND(fa_bwd_dkdv)
   HB_BIND(fa_bwd_dkdv_workspace)
-  HB_BIND(fa_bwd_dkdv_ws)
-  HB_BIND(fa_bwd_dq)
+  HB_BIND(fa_bwd)
   HB_BIND(h2o_score)
   HB_BIND(gemm_epilogue)
   HB_BIND(rms_rowstat)

@@ -255,10 +255,11 @@ def fa_bwd(q, k, v, o, d_o, lse, *, causal: bool = False, softmax_scale: Optiona
     dv = q.new_empty((B, Hkv, Skv, D))
     dq = q.new_empty((B, Hq, Sq, D))
     a.dk, a.dv, a.dq = dk.data_ptr(), dv.data_ptr(), dq.data_ptr()
-    lib, arg = _lib.load(), C.byref(a)
-    _call(q.device, lib.hb_fa_bwd_preprocess, arg)
-    _bwd_dkdv_call(q, a, Hq != Hkv)
-    _call(q.device, lib.hb_fa_bwd_dq, arg)
+    lib, arg, need = _lib.load(), C.byref(a), C.c_uint64(0)
+    if Hq != Hkv:
+        _call(q.device, lib.hb_fa_bwd_dkdv_workspace, arg, C.byref(need))
+    ws = q.new_empty(need.value, dtype=torch.uint8) if need.value else None
+    _call(q.device, lib.hb_fa_bwd, arg, ws.data_ptr() if ws is not None else None, need.value)
     return (dq.transpose(1, 2), dk.transpose(1, 2), dv.transpose(1, 2)) if bshd else (dq, dk, dv)
 
 

@@ -326,6 +326,9 @@ int hb_fa_bwd_dkdv(const hb_fa_bwd_args* args);
 int hb_fa_bwd_dkdv_workspace(const hb_fa_bwd_args* args, uint64_t* bytes);
 int hb_fa_bwd_dkdv_ws(const hb_fa_bwd_args* args, void* workspace, uint64_t bytes);
 int hb_fa_bwd_dq(const hb_fa_bwd_args* args);
+/* The whole backward pass: hb_fa_bwd_preprocess, hb_fa_bwd_dkdv_ws and hb_fa_bwd_dq, with the same results; the kernels overlap
+ * where they leave SMs free, which separate calls cannot.  The workspace is hb_fa_bwd_dkdv_workspace's. */
+int hb_fa_bwd(const hb_fa_bwd_args* args, void* workspace, uint64_t bytes);
 
 /*
  * y = softmax(scale * x) over the last axis of a [rows, cols] matrix (bf16 / fp16, fp32 math,
