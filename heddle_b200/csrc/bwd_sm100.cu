@@ -178,19 +178,6 @@ __device__ __forceinline__ void bwd_load_tile(void* dst, const CUtensorMap* tm, 
     tma_load_4d(static_cast<uint8_t*>(dst) + hh * (128 * 128), tm, bar, hh * 64, row0, h, b);
 }
 
-template <typename T>
-__device__ __forceinline__ void bwd_store_row(T* dst, const uint32_t (&r)[32], float mul) {
-#pragma unroll
-  for (int e = 0; e < 32; e += 8) {
-    uint4 w;
-    w.x = Pack2<T>::pack(__uint_as_float(r[e]) * mul, __uint_as_float(r[e + 1]) * mul);
-    w.y = Pack2<T>::pack(__uint_as_float(r[e + 2]) * mul, __uint_as_float(r[e + 3]) * mul);
-    w.z = Pack2<T>::pack(__uint_as_float(r[e + 4]) * mul, __uint_as_float(r[e + 5]) * mul);
-    w.w = Pack2<T>::pack(__uint_as_float(r[e + 6]) * mul, __uint_as_float(r[e + 7]) * mul);
-    *reinterpret_cast<uint4*>(dst + e) = w;
-  }
-}
-
 // Four probabilities 2^(s * scale_log2 + nl) of one thread's row; with HB_BWD_POLY part of them on the FMA pipe.
 __device__ __forceinline__ void bwd_exp4(const uint32_t* sv, int e, uint64_t sc2, float4 l4, float* out) {
 #ifdef HB_BWD_KO_EXP  // measurement builds only: no exponentials (wrong results)
@@ -582,49 +569,41 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
       // read-out: dV as is, dK times the softmax scale; each thread stores its half of the row's head_dim columns
       if (!mbar_wait_warp(&s.acc_full, items & 1u, ctx, kBwdCons)) break;
       tc_fence_after();
-      const bool live = key < p.Skv;
+      const int quad_key = key - (lane & 3), rows = p.Skv - quad_key;
       const uint32_t col_acc = static_cast<uint32_t>(half * (D / 2));
-      const long long row_of = ((static_cast<long long>(b) * p.Hkv + hkv) * p.Skv + key) * D + col_acc;
-      if (p.splits == 1) {  // straight on: as one loop with the other form, 1.5 % of a call of short items
+      const long long row_of = ((static_cast<long long>(b) * p.Hkv + hkv) * p.Skv + quad_key) * D + col_acc;
+      // the thread's part of both accumulators is read before anything is stored: the next item's first dV product waits for them
+      uint32_t rv[D / 2], rk[D / 2];
+#pragma unroll
+      for (int c = 0; c < D / 64; ++c) {
+        tmem_ld32(tmem + lane_off + 256 + col_acc + c * 32, rv + c * 32);
+        tmem_ld32(tmem + lane_off + 384 + col_acc + c * 32, rk + c * 32);
+      }
+      tmem_wait_ld();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s.acc_empty);
+      __syncwarp();
+      if (p.splits == 1) {
         T* dv_row = static_cast<T*>(p.dv) + row_of;
         T* dk_row = static_cast<T*>(p.dk) + row_of;
-#pragma unroll 1
+#pragma unroll
         for (int c = 0; c < D / 64; ++c) {
-          uint32_t r[32];
-          __syncwarp();
-          tmem_ld32(tmem + lane_off + 256 + col_acc + c * 32, r);
-          tmem_wait_ld();
-          if (live) bwd_store_row<T>(dv_row + c * 32, r, 1.0f);
-          __syncwarp();
-          tmem_ld32(tmem + lane_off + 384 + col_acc + c * 32, r);
-          tmem_wait_ld();
-          if (live) bwd_store_row<T>(dk_row + c * 32, r, p.scale);
+          uint4 w[4];
+          pack_row32<T>(rv + c * 32, 1.0f, w);
+          store_rows32(dv_row + c * 32, D, rows, w);
+          pack_row32<T>(rk + c * 32, p.scale, w);
+          store_rows32(dk_row + c * 32, D, rows, w);
         }
       } else {
         const long long all = static_cast<long long>(p.B) * p.Hkv * p.Skv * D;
         float* const part = p.part + (hq0 - hkv * p.group) / heads * 2 * all + row_of;
-#pragma unroll 1
-        for (int c = 0; c < D / 64; ++c) {
-          uint32_t r[32];
-#pragma unroll 1
-          for (int w = 0; w < 2; ++w) {  // dK, dV
-            __syncwarp();
-            tmem_ld32(tmem + lane_off + (w == 0 ? 384u : 256u) + col_acc + c * 32, r);
-            tmem_wait_ld();
-            const float scale = w == 0 ? p.scale : 1.0f;
-            if (live) {
-              float4* dst = reinterpret_cast<float4*>(part + w * all + c * 32);
 #pragma unroll
-              for (int e = 0; e < 32; e += 4)
-                dst[e / 4] = make_float4(__uint_as_float(r[e]) * scale, __uint_as_float(r[e + 1]) * scale,
-                                         __uint_as_float(r[e + 2]) * scale, __uint_as_float(r[e + 3]) * scale);
-            }
-          }
+        for (int c = 0; c < D / 64; ++c) {  // dK, dV
+          store_rows32_f32(part + c * 32, D, rows, rk + c * 32, p.scale);
+          store_rows32_f32(part + all + c * 32, D, rows, rv + c * 32, 1.0f);
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&s.acc_empty);
     }
   }
 
@@ -900,18 +879,21 @@ __global__ void __launch_bounds__(kBwdDqThreads, 1) fa_bwd_dq_kernel(const __gri
       if (!mbar_wait_warp(&s.acc_full, items & 1u, ctx, kBwdCons)) break;
       tc_fence_after();
       const uint32_t col_acc = static_cast<uint32_t>(grp * (D / 2));
-      T* dq_row = static_cast<T*>(p.dq) + stat * D + col_acc;
-#pragma unroll 1
-      for (int c = 0; c < D / 64; ++c) {
-        uint32_t r[32];
-        __syncwarp();
-        tmem_ld32(tmem + lane_off + 384 + col_acc + c * 32, r);
-        tmem_wait_ld();
-        if (live) bwd_store_row<T>(dq_row + c * 32, r, p.scale);
-      }
+      T* const dq_row = static_cast<T*>(p.dq) + (stat - (lane & 3)) * D + col_acc;
+      uint32_t r[D / 2];
+#pragma unroll
+      for (int c = 0; c < D / 64; ++c) tmem_ld32(tmem + lane_off + 384 + col_acc + c * 32, r + c * 32);
+      tmem_wait_ld();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&s.acc_empty);
+      __syncwarp();
+#pragma unroll
+      for (int c = 0; c < D / 64; ++c) {
+        uint4 w[4];
+        pack_row32<T>(r + c * 32, p.scale, w);
+        store_rows32(dq_row + c * 32, D, p.Sq - q + (lane & 3), w);
+      }
       BWD_PROF(0)
     }
     BWD_PROF_FLUSH

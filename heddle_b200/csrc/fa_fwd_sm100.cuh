@@ -385,7 +385,11 @@ __device__ __forceinline__ void fa_correction_role(const FaParams& p, FaSmem<T, 
         const bool live = qrow < p.Sq;
         using Out = typename FaTraits<T>::Out;
         const float inv_l = (l > 0.f) ? (p.out_scale / l) : 0.f;
-        Out* orow = static_cast<Out*>(p.o) + it.b * p.o_sb + it.hq * p.o_sh + static_cast<long long>(qrow) * p.o_ss;
+        Out* const orow = static_cast<Out*>(p.o) + it.b * p.o_sb + it.hq * p.o_sh + static_cast<long long>(qrow) * p.o_ss;
+        // Stores in full lines (store_rows32) leave the memory pipe to the loads of the blocks around; with few steps a block the
+        // exchange in front of them is in the way of the next block's first product instead.  us direct |
+        // exchanged: bf16 B4 H32 S4096 causal 567 | 558, unmasked 1005 | 996; B16 H16 S300 causal 31.2 | 32.5, FP8 B3 Hq256 Hkv32 S1003 228 | 236.
+        const bool exchange = it.n[i] >= 12;
         const uint32_t tO = tmem + lane_off + 256u + static_cast<uint32_t>(i * 128);
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
@@ -393,16 +397,14 @@ __device__ __forceinline__ void fa_correction_role(const FaParams& p, FaSmem<T, 
           __syncwarp();  // reconverge after the predicated stores of the previous chunk
           tmem_ld32(tO + c * 32, r);
           tmem_wait_ld();
-          if (live) {
+          uint4 w[4];
+          pack_row32<Out>(r, inv_l, w);
+          if (exchange) {
+            const int up = lane & 3;
+            store_rows32(orow - up * p.o_ss + c * 32, p.o_ss, p.Sq - qrow + up, w);
+          } else if (live) {
 #pragma unroll
-            for (int e = 0; e < 32; e += 8) {
-              uint4 w;
-              w.x = Pack2<Out>::pack(__uint_as_float(r[e]) * inv_l, __uint_as_float(r[e + 1]) * inv_l);
-              w.y = Pack2<Out>::pack(__uint_as_float(r[e + 2]) * inv_l, __uint_as_float(r[e + 3]) * inv_l);
-              w.z = Pack2<Out>::pack(__uint_as_float(r[e + 4]) * inv_l, __uint_as_float(r[e + 5]) * inv_l);
-              w.w = Pack2<Out>::pack(__uint_as_float(r[e + 6]) * inv_l, __uint_as_float(r[e + 7]) * inv_l);
-              *reinterpret_cast<uint4*>(orow + c * 32 + e) = w;
-            }
+            for (int e = 0; e < 4; ++e) *reinterpret_cast<uint4*>(orow + c * 32 + e * 8) = w[e];
           }
         }
         if (live && p.lse != nullptr) {

