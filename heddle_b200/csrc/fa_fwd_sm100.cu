@@ -21,14 +21,14 @@ struct FaConfig {
 
 static std::mutex g_fa_mutex;  // guards the per-device set-up tables below
 
-template <typename T, int D>
-static int launch_fa(const FaParams& p, int grid, int smem_optin, cudaStream_t stream) {
+template <typename T, int D, bool Long>
+static int launch_fa_form(const FaParams& p, int grid, int smem_optin, cudaStream_t stream) {
   constexpr int NS = FaConfig<T, D>::kStages;
   using Smem = FaSmem<T, D, NS>;
   if ((int)sizeof(Smem) > smem_optin)
     return set_error(HB_ERR_UNSUPPORTED, "hb_fa_fwd: kernel needs %d bytes of shared memory, device offers %d",
                      (int)sizeof(Smem), smem_optin);
-  auto kernel = fa_fwd_kernel<T, D, NS>;
+  auto kernel = fa_fwd_kernel<T, D, NS, Long>;
   static bool configured[64] = {};
   int dev = 0;
   HB_CUDA_CHECK(cudaGetDevice(&dev));
@@ -44,11 +44,17 @@ static int launch_fa(const FaParams& p, int grid, int smem_optin, cudaStream_t s
   return HB_OK;
 }
 
+template <typename T, int D>
+static int launch_fa(const FaParams& p, int grid, int smem_optin, cudaStream_t stream) {
+  return p.nkv >= kFaLongFrom ? launch_fa_form<T, D, true>(p, grid, smem_optin, stream)
+                              : launch_fa_form<T, D, false>(p, grid, smem_optin, stream);
+}
+
 template <typename T, int D, int NS>
 static int launch_fa_stages(const FaParams& p, int grid, int smem_optin, cudaStream_t stream) {
   using Smem = FaSmem<T, D, NS>;
   if ((int)sizeof(Smem) > smem_optin) return set_error(HB_ERR_UNSUPPORTED, "hb_debug_fa_fwd_stages: not enough shared memory");
-  auto kernel = fa_fwd_kernel<T, D, NS>;
+  auto kernel = fa_fwd_kernel<T, D, NS, false>;
   // set on every call: this is a diagnostic path, not worth a per-device table
   HB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
   HB_CUDA_CHECK(launch_dependent_if(launch_early(tile_order_steps(p.order, p.causal != 0, p.nkv)), kernel, grid, kFaThreads,

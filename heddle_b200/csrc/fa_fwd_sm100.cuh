@@ -45,7 +45,6 @@ struct FaTraits {
   static constexpr uint32_t kFormat = Pack2<T>::kFormat;
   static constexpr float kRescaleThreshold = 8.0f;  // log2 units
   static constexpr float kPScale = 1.0f;
-  static constexpr bool kSplitP = false;
 };
 template <>
 struct FaTraits<__nv_fp8_e4m3> {
@@ -55,13 +54,23 @@ struct FaTraits<__nv_fp8_e4m3> {
   static constexpr uint32_t kFormat = 0;  // e4m3 in kind::f8f6f4
   static constexpr float kRescaleThreshold = 3.0f;
   static constexpr float kPScale = 32.0f;
-  // P is handed to the MMA warp in two halves, so that half of P V runs beside the second half's exponentials: what bounds the
-  // step is the softmax, and this takes a part of the products out of its chain.  With 16-bit inputs, whose products are twice
-  // as long, the MMA warp's second wait costs more than that gives.  us without -> with:
-  // B4 H32 S8192 3086 -> 2994, B3 H12 S3020 causal 78.3 -> 76.4, B3 Hq64 Hkv8 S1003 causal 65.2 -> 64.8; bf16 with three quarters
-  // of P first, B4 H32 S4096: 482 -> 486.
-  static constexpr bool kSplitP = true;
 };
+
+// The kernel has two forms, for few and for many key tiles (`Long`, from kFaLongFrom on).  They differ in what pays off only where a
+// block has steps enough to hide it; as one kernel with a choice inside, short blocks paid 2 to 4 % for it.
+//   FP8, split P: P is handed to the MMA warp in two halves, so that half of P V runs beside the second half's exponentials.  What
+//     bounds the step is the softmax, and this takes a part of the products out of its chain.  With 16-bit inputs, whose products are
+//     twice as long, the MMA warp's second wait costs more than that gives (bf16 B4 H32 S4096, three quarters of P first: 482 -> 486 us).
+//   D = 128, full line stores: O leaves through store_rows32.  The exchange in front of the stores delays the next block's first
+//     product, full lines leave the memory pipe to the loads of the blocks around (rows of 64 columns are half as many lines).
+// us, short form | long form: FP8 B3 Hq128 Hkv32 S291 causal 39.0 | 44.7, B16 Hq32 Hkv8 S500 causal 57.8 | 65.5, B3 H12 S3020 causal
+// 79.4 | 77.1, B4 H32 S8192 3192 | 3042; bf16 D128 B16 H16 S300 causal 30.8 | 32.3, B3 Hq32 Hkv8 S1003 causal 39.8 | 40.6, B4 H16 S1400
+// causal 51.4 | 50.1, B4 H32 S4096 1020 | 1010.
+constexpr int kFaLongFrom = 12;  // key tiles
+template <typename T, bool Long>
+constexpr bool fa_split_p = Long && FaTraits<T>::kFp8;
+template <int D, bool Long>
+constexpr bool fa_full_lines = Long && D == 128;
 
 // Optional phase tracing (compiled in with -DHB_FA_TRACE only): lane 0 of selected warps of
 // CTA 0 appends (clock64 << 8 | code) records to a caller-provided, zero-filled buffer, 4096 slots
@@ -123,8 +132,8 @@ struct FaSmem {
   uint64_t q_full[2], q_empty[2];
   uint64_t kv_full[NS], kv_empty[NS];
   uint64_t s_full[2];     // MMA -> softmax: S_i holds the scores of the next step
-  uint64_t p_full[2];     // softmax + correction -> MMA: P_i (kSplitP: its first half) written and O_i rescaled
-  uint64_t p_rest[2];     // softmax -> MMA: the second half of P_i written (kSplitP)
+  uint64_t p_full[2];     // softmax + correction -> MMA: P_i (split P: its first half) written and O_i rescaled
+  uint64_t p_rest[2];     // softmax -> MMA: the second half of P_i written (split P)
   uint64_t corr_full[2];  // softmax -> correction: alpha (or final l, m) published
   uint64_t o_full[2];     // MMA -> correction: O_i complete
   uint64_t drain;
@@ -164,7 +173,7 @@ __device__ __forceinline__ bool fa_get_item(const FaParams& p, int g, int half, 
 // ------------------------------------------------------------------------------------
 // softmax warpgroup (tile i): one query row per thread
 // ------------------------------------------------------------------------------------
-template <typename T, int D, int NS>
+template <typename T, int D, int NS, bool Long>
 __device__ __forceinline__ void fa_softmax_role(const FaParams& p, FaSmem<T, D, NS>& s, const AbortCtx& ctx,
                                                 uint32_t tmem, int i) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -286,7 +295,7 @@ __device__ __forceinline__ void fa_softmax_role(const FaParams& p, FaSmem<T, D, 
               }
             }
             tmem_st16(tS + q * 16, pk);
-            if (FaTraits<T>::kSplitP && (q + 1) * kChunk == kTileN / 2) {
+            if (fa_split_p<T, Long> && (q + 1) * kChunk == kTileN / 2) {
               tmem_wait_st();
               tc_fence_before();
               __syncwarp();
@@ -302,7 +311,7 @@ __device__ __forceinline__ void fa_softmax_role(const FaParams& p, FaSmem<T, D, 
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(FaTraits<T>::kSplitP ? &s.p_rest[i] : &s.p_full[i]);
+        if (lane == 0) mbar_arrive(fa_split_p<T, Long> ? &s.p_rest[i] : &s.p_full[i]);
         ++p_cnt;
         HB_TRACE(p, warp, 5);
       }
@@ -322,7 +331,7 @@ __device__ __forceinline__ void fa_softmax_role(const FaParams& p, FaSmem<T, D, 
 // ------------------------------------------------------------------------------------
 // correction warpgroup
 // ------------------------------------------------------------------------------------
-template <typename T, int D, int NS>
+template <typename T, int D, int NS, bool Long>
 __device__ __forceinline__ void fa_correction_role(const FaParams& p, FaSmem<T, D, NS>& s, const AbortCtx& ctx,
                                                    uint32_t tmem) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -386,10 +395,6 @@ __device__ __forceinline__ void fa_correction_role(const FaParams& p, FaSmem<T, 
         using Out = typename FaTraits<T>::Out;
         const float inv_l = (l > 0.f) ? (p.out_scale / l) : 0.f;
         Out* const orow = static_cast<Out*>(p.o) + it.b * p.o_sb + it.hq * p.o_sh + static_cast<long long>(qrow) * p.o_ss;
-        // Stores in full lines (store_rows32) leave the memory pipe to the loads of the blocks around; with few steps a block the
-        // exchange in front of them is in the way of the next block's first product instead.  us direct |
-        // exchanged: bf16 B4 H32 S4096 causal 567 | 558, unmasked 1005 | 996; B16 H16 S300 causal 31.2 | 32.5, FP8 B3 Hq256 Hkv32 S1003 228 | 236.
-        const bool exchange = it.n[i] >= 12;
         const uint32_t tO = tmem + lane_off + 256u + static_cast<uint32_t>(i * 128);
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
@@ -399,7 +404,7 @@ __device__ __forceinline__ void fa_correction_role(const FaParams& p, FaSmem<T, 
           tmem_wait_ld();
           uint4 w[4];
           pack_row32<Out>(r, inv_l, w);
-          if (exchange) {
+          if constexpr (fa_full_lines<D, Long>) {
             const int up = lane & 3;
             store_rows32(orow - up * p.o_ss + c * 32, p.o_ss, p.Sq - qrow + up, w);
           } else if (live) {
@@ -420,7 +425,7 @@ __device__ __forceinline__ void fa_correction_role(const FaParams& p, FaSmem<T, 
 // ------------------------------------------------------------------------------------
 // MMA issuer (one warp; an elected lane issues)
 // ------------------------------------------------------------------------------------
-template <typename T, int D, int NS>
+template <typename T, int D, int NS, bool Long>
 __device__ __forceinline__ void fa_mma_role(const FaParams& p, FaSmem<T, D, NS>& s, const AbortCtx& ctx,
                                             uint32_t tmem) {
   using Tr = FaTraits<T>;
@@ -430,7 +435,8 @@ __device__ __forceinline__ void fa_mma_role(const FaParams& p, FaSmem<T, D, NS>&
   constexpr uint32_t kSubBytes = kTileM * 128;            // one 128-byte-wide, 128-row sub-tile
   constexpr int kQkSteps = D * Tr::kElemBytes / 32;       // each MMA consumes 32 bytes of head_dim
   constexpr int kPvSteps = kTileN * Tr::kElemBytes / 32;  // ... and 32 bytes' worth of keys of P
-  constexpr int kPvFirst = Tr::kSplitP ? kPvSteps / 2 : kPvSteps;  // of them, those that wait for p_full only
+  constexpr bool kSplitP = fa_split_p<T, Long>;
+  constexpr int kPvFirst = kSplitP ? kPvSteps / 2 : kPvSteps;  // of them, those that wait for p_full only
   constexpr uint32_t kVStep16 = (32u / Tr::kElemBytes) * 128u >> 4;  // V rows per MMA x 128 B, in 16-byte units
   // Shared-memory descriptors: the high word (SBO = 1024 B, version 1, SWIZZLE_128B) is constant;
   // the low word is (address >> 4) | (LBO >> 4) << 16 and only its address field moves per MMA.
@@ -539,7 +545,7 @@ __device__ __forceinline__ void fa_mma_role(const FaParams& p, FaSmem<T, D, NS>&
             tc_fence_after();
             HB_TRACE(p, 12, 12 + i);
             issue_pv(i, slot_v, j > 0 ? 1u : 0u, Int<0>{}, Int<kPvFirst>{});
-            if constexpr (Tr::kSplitP) {
+            if constexpr (kSplitP) {
               if (!mbar_wait_warp(&s.p_rest[i], ((p_phase >> i) & 1u) ^ 1u, ctx, kRoleMma)) return;
               tc_fence_after();
               issue_pv(i, slot_v, 1u, Int<kPvFirst>{}, Int<kPvSteps>{});
@@ -623,7 +629,7 @@ __device__ __forceinline__ void fa_tma_role(const FaParams& p, FaSmem<T, D, NS>&
 // ------------------------------------------------------------------------------------
 // kernel
 // ------------------------------------------------------------------------------------
-template <typename T, int D, int NS>
+template <typename T, int D, int NS, bool Long>
 __global__ void __launch_bounds__(kFaThreads, 1) fa_fwd_kernel(const __grid_constant__ FaParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   using Smem = FaSmem<T, D, NS>;
@@ -676,14 +682,14 @@ __global__ void __launch_bounds__(kFaThreads, 1) fa_fwd_kernel(const __grid_cons
   static_assert(8 * 32 * (184 - 128) <= 4 * 32 * (128 - 80) + 4 * 32 * (128 - 64), "setmaxnreg budget does not balance");
   if (warp < 8) {
     reg_inc<184>();
-    if (run) fa_softmax_role<T, D, NS>(p, s, ctx, tmem, warp >> 2);
+    if (run) fa_softmax_role<T, D, NS, Long>(p, s, ctx, tmem, warp >> 2);
   } else if (warp < 12) {
     reg_dec<80>();
-    if (run) fa_correction_role<T, D, NS>(p, s, ctx, tmem);
+    if (run) fa_correction_role<T, D, NS, Long>(p, s, ctx, tmem);
   } else {
     reg_dec<64>();
     if (run && warp == 12) {
-      fa_mma_role<T, D, NS>(p, s, ctx, tmem);
+      fa_mma_role<T, D, NS, Long>(p, s, ctx, tmem);
       __syncwarp();
       if (s.abort_flag && lane == 0) {
         // aborting: let the tensor pipe drain before TMEM is released
