@@ -25,6 +25,7 @@ namespace hb {
 
 constexpr int kH2oThreads = 384;  // warps 10, 11 only complete the third warpgroup for setmaxnreg
 constexpr int kH2oStages = 4;
+constexpr int kH2oParts = 8;
 enum H2oRole : uint32_t { kH2oTma = 0x31, kH2oMma = 0x32, kH2oCons = 0x33, kH2oDrain = 0x34 };
 
 struct alignas(64) H2oParams {
@@ -53,6 +54,11 @@ struct H2oSmem {
   uint64_t drain;
   uint32_t tmem_base, abort_flag;
   alignas(16) float nlse[8][2][128];  // per consumer warp, double-buffered: -LSE * log2(e) of a query tile
+  // Sums of the two groups over an item's keys, and per 32 keys whether the first of the two has come.  A ring: neither group gets more
+  // than three items ahead, since the products are issued in order, every item here has a tile of both groups, and a group that
+  // has not summed an item up holds the products at two tiles behind it.
+  float part[kH2oParts][2][128];
+  uint32_t part_first[kH2oParts][4];
 };
 
 struct H2oItem {
@@ -89,6 +95,7 @@ __global__ void __launch_bounds__(kH2oThreads, 1) h2o_score_kernel(const __grid_
       mbar_init(&s.q_full[i], 1);
       mbar_init(&s.q_empty[i], 1);
     }
+    for (int i = 0; i < kH2oParts * 4; ++i) s.part_first[i / 4][i % 4] = 0;
     for (int i = 0; i < 4; ++i) {
       mbar_init(&s.acc_full[i], 1);
       mbar_init(&s.acc_empty[i], 4);
@@ -202,6 +209,7 @@ __global__ void __launch_bounds__(kH2oThreads, 1) h2o_score_kernel(const __grid_
     const int past = p.Skv - p.Sq;
     uint32_t cg = 0, buf = 0;  // cg: tiles this group has consumed (selects buffer and parity)
     bool ok = true;
+    uint32_t paired = 0;     // items of more than one tile
     uint32_t tile_base = 0;  // global tile counter at the start of the item (same sequence as the MMA warp)
     const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2);
     for (int u = 2 * blockIdx.x; ok && u < 2 * p.order.total; u += ((u & 1) ? 2 * (int)gridDim.x - 1 : 1)) {
@@ -280,8 +288,28 @@ __global__ void __launch_bounds__(kH2oThreads, 1) h2o_score_kernel(const __grid_
       unpack_f32x2(sa, s0, s1);
       unpack_f32x2(sb, s2, s3);
       const float sum = (s0 + s1) + (s2 + s3);
-      // the two groups add their halves into the zero-initialised output (two commutative adds)
-      if (key < p.Skv) atomicAdd(p.score + (static_cast<long long>(it.b) * p.Hq + it.hq) * p.Skv + key, sum);
+      // The groups' halves meet in shared memory: whichever of the two warps of these keys comes second adds and stores.  (Two
+      // atomic adds into the output needed a memset in front of the kernel, which also kept it from starting early: us of attention +
+      // score B4 H1 S115 14.2 -> 9.6, B4 Hq4 Hkv1 S511 20.5 -> 18.8, B8 H32 S454 61.8 -> 61.1.)
+      float total = sum;
+      bool store = true;
+      if (ntiles > 1) {  // else the other group has no tile of the item, and nothing to add
+        const uint32_t slot = paired++ % kH2oParts, slab = warp & 3u;
+        s.part[slot][grp][key_in_tile] = sum;
+        __syncwarp();
+        uint32_t second = 0;
+        if (lane == 0) {
+          __threadfence_block();
+          second = atomicXor(&s.part_first[slot][slab], 1u);
+          __threadfence_block();
+        }
+        second = __shfl_sync(0xffffffffu, second, 0);
+        store = second != 0;
+        if (store) total += s.part[slot][grp ^ 1][key_in_tile];
+      } else {
+        store = t_first == 0;
+      }
+      if (store && key < p.Skv) p.score[(static_cast<long long>(it.b) * p.Hq + it.hq) * p.Skv + key] = total;
     }
    }
   }
@@ -323,8 +351,10 @@ static int h2o_impl(const hb_h2o_args* a) {
   int rc = get_device_state(&st);
   if (rc != HB_OK) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
-  HB_CUDA_CHECK(cudaMemsetAsync(a->score, 0, sizeof(float) * (size_t)a->B * a->Hq * a->Skv, stream));
-  if (a->Sq == 0) return HB_OK;
+  if (a->Sq == 0) {
+    HB_CUDA_CHECK(cudaMemsetAsync(a->score, 0, sizeof(float) * (size_t)a->B * a->Hq * a->Skv, stream));
+    return HB_OK;
+  }
   H2oParams p;
   memset(&p, 0, sizeof(p));
   const size_t es = 2;
