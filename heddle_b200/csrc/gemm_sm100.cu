@@ -71,7 +71,7 @@ static const int* gemm_split_slots(const DeviceState* st) {
   std::lock_guard<std::mutex> lock(mutex);
   int* const table = slots[st->device & 63];
   for (int splits = 1; splits <= kMaxSplits && table[kMaxSplits] == 0; ++splits) {
-    auto kernel = gemm_split_kernel<__nv_bfloat16, kEpiPlain>;
+    auto kernel = gemm_split_kernel<__nv_bfloat16, kEpiPlain, false>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(splits * st->sm_count));
     cfg.blockDim = dim3(kGemmSplitThreads);
@@ -93,12 +93,12 @@ static const int* gemm_split_slots(const DeviceState* st) {
   return table;
 }
 
-template <typename T, int EPI>
-static int launch_gemm_split(const GemmSplitParams& p, int grid, const DeviceState* st, cudaStream_t stream) {
+template <typename T, int EPI, bool Tail>
+static int launch_gemm_split(const GemmSplitArgs<Tail>& p, int grid, const DeviceState* st, cudaStream_t stream) {
   if (kGemmSplitSmemBytes > st->smem_optin)
     return set_error(HB_ERR_UNSUPPORTED, "hb_gemm_epilogue: kernel needs %d bytes of shared memory, device offers %d",
                      kGemmSplitSmemBytes, st->smem_optin);
-  auto kernel = gemm_split_kernel<T, EPI>;
+  auto kernel = gemm_split_kernel<T, EPI, Tail>;
   static bool configured[64] = {};
   if (!configured[st->device & 63]) {
     HB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSplitSmemBytes));
@@ -108,15 +108,15 @@ static int launch_gemm_split(const GemmSplitParams& p, int grid, const DeviceSta
   return HB_OK;
 }
 
-template <typename T>
-static int dispatch_gemm_split(int epi_class, const GemmSplitParams& p, int grid, const DeviceState* st, cudaStream_t stream) {
+template <typename T, bool Tail>
+static int dispatch_gemm_split(int epi_class, const GemmSplitArgs<Tail>& p, int grid, const DeviceState* st, cudaStream_t stream) {
   switch (epi_class) {
     case kEpiPlain:
-      return launch_gemm_split<T, kEpiPlain>(p, grid, st, stream);
+      return launch_gemm_split<T, kEpiPlain, Tail>(p, grid, st, stream);
     case kEpiSwiglu:
-      return launch_gemm_split<T, kEpiSwiglu>(p, grid, st, stream);
+      return launch_gemm_split<T, kEpiSwiglu, Tail>(p, grid, st, stream);
     default:
-      return launch_gemm_split<T, kEpiRope>(p, grid, st, stream);
+      return launch_gemm_split<T, kEpiRope, Tail>(p, grid, st, stream);
   }
 }
 
@@ -197,34 +197,50 @@ static int gemm_impl(const hb_gemm_args* args) {
   }
   const bool use_split = split.width > 0;
 
-  GemmSplitParams sp;
+  GemmSplitArgs<true> sp;
   memset(&sp, 0, sizeof(sp));
   GemmParams& p = sp.g;
   const CUtensorMapDataType dt = a->dtype == HB_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  bool split_tail = false;
   if (use_split) {
     sp.a_rows = a->M > kGemmBM ? kGemmBM : (a->M + 7) / 8 * 8;
     sp.slabs = split.slabs;
-    sp.k_slabs = a->K % kGemmBK == 0 ? 1 : 0;
-    const uint64_t k_in = sp.k_slabs ? kGemmBK : a->K, k_out = sp.k_slabs ? a->K / kGemmBK : 1;
-    {
-      const uint32_t box[4] = {(uint32_t)kGemmBK, (uint32_t)sp.a_rows, (uint32_t)sp.slabs, 1};
-      const uint64_t dims[4] = {k_in, (uint64_t)a->M, k_out, (uint64_t)batch};
+    const bool tail = a->K % kGemmBK != 0;
+    sp.k_slabs = tail && sp.slabs == 1 ? 0 : 1;  // stages of one slab need no tail of their own: the plain map fills up
+    // `whole`: slabs of 64 along a third dimension; else K as it is
+    auto a_map = [&](CUtensorMap* tm, bool whole) {
+      const uint32_t box[4] = {(uint32_t)kGemmBK, (uint32_t)sp.a_rows, whole ? (uint32_t)sp.slabs : 1u, 1};
+      const uint64_t dims[4] = {whole ? (uint64_t)kGemmBK : (uint64_t)a->K, (uint64_t)a->M, whole ? (uint64_t)(a->K / kGemmBK) : 1, (uint64_t)batch};
       const uint64_t str[3] = {(uint64_t)a->lda * 2, kGemmBK * 2, (uint64_t)a_bs * 2};
-      rc = encode_tensor_map(&p.tm_a, dt, 4, a->a, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
-      if (rc != HB_OK) return rc;
-    }
+      return encode_tensor_map(tm, dt, 4, a->a, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
+    };
+    auto w_map = [&](CUtensorMap* tm, bool whole) {
+      const uint32_t parts = epi_class == kEpiSwiglu ? 2 : 1;
+      const uint32_t box[5] = {(uint32_t)kGemmBK, (uint32_t)split.width / parts, parts, whole ? (uint32_t)sp.slabs : 1u, 1};
+      const uint64_t dims[5] = {whole ? (uint64_t)kGemmBK : (uint64_t)a->K, (uint64_t)n_out, parts, whole ? (uint64_t)(a->K / kGemmBK) : 1, (uint64_t)batch};
+      const uint64_t str[4] = {(uint64_t)a->ldw * 2, (uint64_t)n_out * a->ldw * 2, kGemmBK * 2, (uint64_t)w_bs * 2};
+      return encode_tensor_map(tm, dt, 5, a->w, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B,
+                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B);  // 35.2 -> 33.5 us for 24 x 22016 x 4096
+    };
+    rc = a_map(&p.tm_a, sp.k_slabs != 0);
+    if (rc != HB_OK) return rc;
     if (w_kn) {
       const uint32_t box[3] = {64, (uint32_t)(sp.slabs * kGemmBK), 1};
       const uint64_t dims[3] = {(uint64_t)a->N, (uint64_t)a->K, (uint64_t)batch};
       const uint64_t str[2] = {(uint64_t)a->ldw * 2, (uint64_t)w_bs * 2};
       rc = encode_tensor_map(&p.tm_w, dt, 3, a->w, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
     } else {
-      const uint32_t parts = epi_class == kEpiSwiglu ? 2 : 1;
-      const uint32_t box[5] = {(uint32_t)kGemmBK, (uint32_t)split.width / parts, parts, (uint32_t)sp.slabs, 1};
-      const uint64_t dims[5] = {k_in, (uint64_t)n_out, parts, k_out, (uint64_t)batch};
-      const uint64_t str[4] = {(uint64_t)a->ldw * 2, (uint64_t)n_out * a->ldw * 2, kGemmBK * 2, (uint64_t)w_bs * 2};
-      rc = encode_tensor_map(&p.tm_w, dt, 5, a->w, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B);  // 35.2 -> 33.5 us for 24 x 22016 x 4096
+      rc = w_map(&p.tm_w, sp.k_slabs != 0);
+    }
+    if (rc != HB_OK) return rc;
+    const GemmSplitStages stages = gemm_split_stages(sp.a_rows, split.width, k_steps, !tail);
+    p.k_steps = stages.stages;
+    split_tail = tail && sp.k_slabs;
+    if (split_tail) {
+      sp.tail_stage = stages.stages - 1;
+      sp.last_slabs = a->K / kGemmBK - (sp.tail_stage - 1) * sp.slabs;
+      rc = a_map(&sp.tm_a_tail, false);
+      if (rc == HB_OK && !w_kn) rc = w_map(&sp.tm_w_tail, false);
     }
     if (rc != HB_OK) return rc;
   } else {
@@ -290,7 +306,7 @@ static int gemm_impl(const hb_gemm_args* args) {
   p.w_kn = w_kn ? 1 : 0;
   p.o_batch_stride = o_bs;
   p.r_batch_stride = r_bs;
-  p.k_steps = k_steps;
+  if (!use_split) p.k_steps = k_steps;
   p.act = (a->epilogue >= HB_EPI_SILU && a->epilogue <= HB_EPI_TANH) ? a->epilogue : kActNone;
   p.rope_seq = a->rope_seq;
   p.head_dim = a->head_dim;
@@ -307,7 +323,6 @@ static int gemm_impl(const hb_gemm_args* args) {
   if (use_split) {
     sp.width = split.width;
     sp.splits = split.splits;
-    p.k_steps = (k_steps + sp.slabs - 1) / sp.slabs;
     const int stage_bytes = (sp.a_rows + sp.width) * kGemmBK * 2 * sp.slabs;
     // the last A box of the ring is read as 128 rows: 16 KB of shared memory behind its start have to exist
     sp.stages = std::min(kGemmSplitMaxStages, (kGemmSplitRing - 16384) / stage_bytes);
@@ -315,8 +330,13 @@ static int gemm_impl(const hb_gemm_args* args) {
     while (sp.tmem_cols < sp.width) sp.tmem_cols *= 2;
     if (tiles * sp.splits > 0x7fffffffLL) return set_error(HB_ERR_UNSUPPORTED, "hb_gemm_epilogue: too many tiles");
     const int split_grid = (int)tiles * sp.splits;
-    return a->dtype == HB_BF16 ? dispatch_gemm_split<__nv_bfloat16>(epi_class, sp, split_grid, st, stream)
-                               : dispatch_gemm_split<__half>(epi_class, sp, split_grid, st, stream);
+    if (split_tail)
+      return a->dtype == HB_BF16 ? dispatch_gemm_split<__nv_bfloat16, true>(epi_class, sp, split_grid, st, stream)
+                                 : dispatch_gemm_split<__half, true>(epi_class, sp, split_grid, st, stream);
+    GemmSplitArgs<false> plain;
+    static_cast<GemmSplitParams&>(plain) = sp;
+    return a->dtype == HB_BF16 ? dispatch_gemm_split<__nv_bfloat16, false>(epi_class, plain, split_grid, st, stream)
+                               : dispatch_gemm_split<__half, false>(epi_class, plain, split_grid, st, stream);
   }
   return a->dtype == HB_BF16 ? dispatch_gemm<__nv_bfloat16>(epi_class, p, grid, pair, st, stream)
                              : dispatch_gemm<__half>(epi_class, p, grid, pair, st, stream);

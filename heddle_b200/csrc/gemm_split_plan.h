@@ -16,10 +16,15 @@ struct GemmSplitChoice {
   double rule_ns = 0.0;  // what the split-K kernel is compared with a persistent one by
 };
 
-// K slabs per stage: about 40 KB, so that four or more stages fit the ring
-inline int gemm_split_slabs(int a_rows, int width, int k_steps, bool whole_slabs) {
-  if (!whole_slabs) return 1;
-  return std::max(1, std::min({4, k_steps, 40 * 1024 / ((a_rows + width) * 128)}));
+// K slabs per stage: about 40 KB, so that four or more stages fit the ring.  A K that is not a multiple of 64 leaves a tail, which is a
+// stage of its own behind the whole slabs.
+struct GemmSplitStages {
+  int slabs, stages;
+};
+inline GemmSplitStages gemm_split_stages(int a_rows, int width, int k_steps, bool whole_slabs) {
+  const int whole = whole_slabs ? k_steps : k_steps - 1;
+  const int slabs = std::max(1, std::min({4, whole, 40 * 1024 / ((a_rows + width) * 128)}));
+  return {slabs, (whole + slabs - 1) / slabs + (k_steps - whole)};
 }
 
 // Estimated time (ns) of one launch, fitted to a sweep of widths 64 .. 256 and clusters 1 .. 8 on 24 .. 256 x 4096 .. 22016 x
@@ -39,7 +44,7 @@ inline GemmSplitChoice gemm_split_choose(const int* slots, int sm_count, int epi
     const long long tiles = (long long)tiles_m * ((n_out * per_col + width - 1) / width) * batch;
     const double slab = std::max({width * 128.0 / 60.0, (width + a_rows) * 128.0 / 120.0, width * (270.0 / 256.0), 125.0});
     const double l2 = 128.0 * (width + a_rows) * tiles * (double)k_steps / 14000.0;
-    const int slabs = gemm_split_slabs(a_rows, width, k_steps, whole_slabs), stages = (k_steps + slabs - 1) / slabs;
+    const auto [slabs, stages] = gemm_split_stages(a_rows, width, k_steps, whole_slabs);
     for (int splits = 1; splits <= std::min(kMaxSplits, stages); ++splits) {
       const double fixed = 5000.0 + (splits > 1 ? 450.0 * splits : 0.0) + std::min(M, kGemmBM) * (double)width / 10.0;
       // no cluster of this size or larger is faster than this; the search is host time of every call with few tiles, 0.9 us

@@ -26,13 +26,26 @@ struct GemmSplitParams {
   GemmParams g;    // tile_cols = output columns of a tile
   int width;       // accumulator columns of a tile (= tile_cols, twice that for SWIGLU)
   int a_rows;      // rows of the A box (multiple of 8, <= 128)
-  int slabs;       // 64-wide K slabs per stage (1 unless K is a multiple of 64); g.k_steps counts stages
+  int slabs;       // 64-wide K slabs per stage; g.k_steps counts stages
   // 1: the maps are A [64, rows, K / 64, batch] and W [64, rows, parts, K / 64, batch], 0: [K, rows, ..., 1, batch].  A SWIGLU
   // weight has two parts, gate and up: one copy brings both.
   int k_slabs;
   int stages;
   int splits;      // cluster size
   int tmem_cols;   // power of two >= width
+};
+
+// With `Tail`, what a K that is not a multiple of 64 leaves behind its whole slabs is the last stage, one slab brought by maps of the
+// second kind, which fill it up with zeros.  (A kernel of its own: with the choice at run time the others paid 3 to 4 %.)
+// us with one slab per stage for such a K -> with the tail apart: 17 x 5344 x 3056 16.8 -> 11.4, 8 x 1392 x 11616 16.4 -> 11.7, 28 x 7120 x
+// 5416 26.6 -> 22.4, 1 x 1360 x 5912 10.9 -> 8.7, 2 x 1120 x 1160 7.1 -> 5.8.
+template <bool Tail>
+struct GemmSplitArgs : GemmSplitParams {};
+template <>
+struct GemmSplitArgs<true> : GemmSplitParams {
+  int tail_stage;
+  int last_slabs;  // whole slabs in the stage in front of it
+  CUtensorMap tm_a_tail, tm_w_tail;
 };
 
 struct GemmSplitCtrl {
@@ -86,8 +99,8 @@ __device__ __forceinline__ void gemm_split_scale_bias8(const GemmParams& p, floa
   }
 }
 
-template <typename T, int EPI>
-__global__ void __launch_bounds__(kGemmSplitThreads, 1) gemm_split_kernel(const __grid_constant__ GemmSplitParams sp) {
+template <typename T, int EPI, bool Tail>
+__global__ void __launch_bounds__(kGemmSplitThreads, 1) gemm_split_kernel(const __grid_constant__ GemmSplitArgs<Tail> sp) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const GemmParams& p = sp.g;
   const uint32_t a_slab = static_cast<uint32_t>(sp.a_rows) * 128u, b_slab = static_cast<uint32_t>(sp.width) * 128u;
@@ -114,6 +127,10 @@ __global__ void __launch_bounds__(kGemmSplitThreads, 1) gemm_split_kernel(const 
     if ((smem_u32(smem_raw) & 1023u) != 0u) raise_abort(ctx, kStatusSmemMisaligned);
     prefetch_tensormap(&p.tm_a);
     prefetch_tensormap(&p.tm_w);
+    if constexpr (Tail) {
+      prefetch_tensormap(&sp.tm_a_tail);
+      if (!p.w_kn) prefetch_tensormap(&sp.tm_w_tail);
+    }
   }
   if (warp == 1) {
     tmem_alloc(&s.tmem_base, static_cast<uint32_t>(sp.tmem_cols));
@@ -138,8 +155,22 @@ __global__ void __launch_bounds__(kGemmSplitThreads, 1) gemm_split_kernel(const 
       uint32_t st = 0, phase = 1;
       for (int ks = k_begin; ks < k_end; ++ks) {
         if (!mbar_wait(&s.empty[st], phase, ctx, kGemmRoleTma)) break;
-        mbar_arrive_expect_tx(&s.full[st], a_bytes + b_bytes);
         uint8_t* const sb = ring_b + st * b_bytes;
+        if constexpr (Tail) {
+          if (ks == sp.tail_stage) {
+            const int k0 = p.K / kGemmBK * kGemmBK;
+            mbar_arrive_expect_tx(&s.full[st], a_slab + (p.w_kn ? b_bytes : b_slab));
+            if (p.w_kn) {  // rows past K are zeros
+              for (int i = 0; i < sp.width / 64; ++i)
+                tma_load_3d(sb + i * (sp.slabs * kGemmBK * 128), &p.tm_w, &s.full[st], n0 + i * 64, k0, b);
+            } else {
+              tma_load_5d(sb, &sp.tm_w_tail, &s.full[st], k0, n0, 0, 0, b);
+            }
+            tma_load_4d(ring_a + st * a_bytes, &sp.tm_a_tail, &s.full[st], k0, m0, 0, b);
+            break;
+          }
+        }
+        mbar_arrive_expect_tx(&s.full[st], a_bytes + b_bytes);
         const int kc = sp.k_slabs ? 0 : ks * kGemmBK, slab = sp.k_slabs ? ks * sp.slabs : 0;
         if (p.w_kn) {
           for (int i = 0; i < sp.width / 64; ++i)
@@ -175,7 +206,12 @@ __global__ void __launch_bounds__(kGemmSplitThreads, 1) gemm_split_kernel(const 
         tc_fence_after();
         const uint32_t a_lo = (smem_u32(ring_a + st * a_bytes) >> 4) | kLbo, b_lo = (smem_u32(ring_b + st * b_bytes) >> 4) | b_lbo;
         if (leader) {
-          for (int sl = 0; sl < sp.slabs; ++sl) {
+          int slabs = sp.slabs;
+          if constexpr (Tail) {
+            // the last stage of whole slabs may hold fewer: with a [K, N] operand the rest of its box are the tail's rows
+            if (ks >= sp.tail_stage - 1) slabs = ks == sp.tail_stage ? 1 : sp.last_slabs;
+          }
+          for (int sl = 0; sl < slabs; ++sl) {
             const uint32_t a = a_lo + static_cast<uint32_t>(sl) * (a_slab >> 4), w = b_lo + static_cast<uint32_t>(sl) * b_next;
 #pragma unroll
             for (int kk = 0; kk < kGemmBK / 16; ++kk) {

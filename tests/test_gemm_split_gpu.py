@@ -100,3 +100,25 @@ def test_16_bit_rope_tables_are_read_as_they_are(ops, schedule, dt):
         assert torch.equal(out, ops.gemm_epilogue(a, w, "rope", rope=(off, sin, 128, 384)))
     finally:
         ops.set_gemm_schedule(prev)
+
+
+@pytest.mark.parametrize("K", [72, 136, 184, 248, 264, 320, 520, 1000, 2040])
+@pytest.mark.parametrize("w_layout", ["nk", "kn"])
+def test_tail_of_k(ops, K, w_layout):
+    """A K that is not a multiple of 64 is whole slabs, several to a stage, and a tail of its own.  What lies behind K in either operand
+    is NaN: nothing of it may be read into a product."""
+    dt, B, M, N = torch.bfloat16, 3, 40, 144
+    g = torch.Generator().manual_seed(K)
+    a = torch.full((B, M, K + 64), float("nan"), dtype=dt)
+    a[:, :, :K] = torch.randn(B, M, K, generator=g).to(dt)
+    w = torch.full((B, N, K + 64), float("nan"), dtype=dt)
+    w[:, :, :K] = (torch.randn(B, N, K, generator=g) * 0.05).to(dt)
+    ref = a[:, :, :K].float() @ w[:, :, :K].float().transpose(1, 2)
+    if w_layout == "nk":
+        b = w.cuda()[:, :, :K].transpose(1, 2)
+    else:
+        b = w.transpose(1, 2).contiguous().cuda()[:, :K]
+    _check(ops, ops.bmm(a.cuda()[:, :, :K], b), ref, dt)
+    if w_layout == "nk":
+        one = ops.gemm_epilogue(a[0].cuda()[:, :K], w[0].cuda()[:, :K], "swiglu")
+        _check(ops, one, torch.nn.functional.silu(ref[0][:, : N // 2]) * ref[0][:, N // 2:], dt)
