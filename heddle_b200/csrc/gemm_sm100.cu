@@ -24,12 +24,12 @@ static int launch_gemm(const GemmParams& p, int grid, const DeviceState* st, cud
   return HB_OK;
 }
 
-template <typename T, int EPI>
-static int launch_gemm_pair(const GemmParams& p, int grid, const DeviceState* st, cudaStream_t stream) {
+template <typename T, int EPI, bool Residual>
+static int launch_gemm_pair(const GemmPairParams<Residual>& p, int grid, const DeviceState* st, cudaStream_t stream) {
   if (kPairSmemBytes > st->smem_optin)
     return set_error(HB_ERR_UNSUPPORTED, "hb_gemm_epilogue: kernel needs %d bytes of shared memory, device offers %d",
                      kPairSmemBytes, st->smem_optin);
-  auto kernel = gemm_pair_kernel<T, EPI>;
+  auto kernel = gemm_pair_kernel<T, EPI, Residual>;
   static bool configured[64] = {};
   if (!configured[st->device & 63]) {
     HB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes));
@@ -40,17 +40,28 @@ static int launch_gemm_pair(const GemmParams& p, int grid, const DeviceState* st
 }
 
 template <typename T>
-static int dispatch_gemm(int epi_class, const GemmParams& p, int grid, bool pair, const DeviceState* st, cudaStream_t stream) {
-  if (pair) {
-    switch (epi_class) {
-      case kEpiPlain:
-        return launch_gemm_pair<T, kEpiPlain>(p, grid, st, stream);
-      case kEpiSwiglu:
-        return launch_gemm_pair<T, kEpiSwiglu>(p, grid, st, stream);
-      default:
-        return launch_gemm_pair<T, kEpiRope>(p, grid, st, stream);
-    }
+static int dispatch_gemm_pair(int epi_class, const GemmParams& base, const CUtensorMap* residual, int grid, const DeviceState* st,
+                              cudaStream_t stream) {
+  if (residual != nullptr) {
+    GemmPairParams<true> p;
+    static_cast<GemmParams&>(p) = base;
+    p.tm_res = *residual;
+    return launch_gemm_pair<T, kEpiPlain, true>(p, grid, st, stream);
   }
+  GemmPairParams<false> p;
+  static_cast<GemmParams&>(p) = base;
+  switch (epi_class) {
+    case kEpiPlain:
+      return launch_gemm_pair<T, kEpiPlain, false>(p, grid, st, stream);
+    case kEpiSwiglu:
+      return launch_gemm_pair<T, kEpiSwiglu, false>(p, grid, st, stream);
+    default:
+      return launch_gemm_pair<T, kEpiRope, false>(p, grid, st, stream);
+  }
+}
+
+template <typename T>
+static int dispatch_gemm(int epi_class, const GemmParams& p, int grid, const DeviceState* st, cudaStream_t stream) {
   switch (epi_class) {
     case kEpiPlain:
       return launch_gemm<T, kEpiPlain>(p, grid, st, stream);
@@ -265,6 +276,10 @@ static int gemm_impl(const hb_gemm_args* args) {
     rc = encode_tensor_map(&p.tm_w, dt, 3, a->w, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc != HB_OK) return rc;
   }
+  const bool pair = !use_split &&
+                    (a->schedule == HB_GEMM_PAIR || (a->schedule == HB_GEMM_AUTO && a->M > kGemmBM && st->sm_count >= 2));
+  const bool res_tma = pair && epi_class == kEpiPlain && a->residual != nullptr;
+  CUtensorMap tm_res;
   if (epi_class == kEpiPlain && !use_split) {
     const uint32_t box[3] = {64, (uint32_t)kGemmBM, 1};
     const uint64_t dims[3] = {(uint64_t)n_out, (uint64_t)a->M, (uint64_t)batch};
@@ -272,6 +287,11 @@ static int gemm_impl(const hb_gemm_args* args) {
     rc = encode_tensor_map(&p.tm_out, dt, 3, a->out, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc != HB_OK) return rc;
     p.tma_store = 1;
+    if (res_tma) {
+      const uint64_t res_str[2] = {(uint64_t)a->ldr * 2, (uint64_t)r_bs * 2};
+      rc = encode_tensor_map(&tm_res, dt, 3, a->residual, dims, res_str, box, CU_TENSOR_MAP_SWIZZLE_128B);
+      if (rc != HB_OK) return rc;
+    }
   }
   p.out = a->out;
   p.row_scale = a->row_scale;
@@ -287,8 +307,6 @@ static int gemm_impl(const hb_gemm_args* args) {
   p.N_out = n_out;
   p.K = a->K;
   p.tile_cols = (use_split ? split.width : kGemmBN) / (epi_class == kEpiSwiglu ? 2 : 1);
-  const bool pair = !use_split &&
-                    (a->schedule == HB_GEMM_PAIR || (a->schedule == HB_GEMM_AUTO && a->M > kGemmBM && st->sm_count >= 2));
   const int tile_rows = pair ? kPairBM : kGemmBM;
   p.tiles_m = (a->M + tile_rows - 1) / tile_rows;
   p.tiles_n = (n_out + p.tile_cols - 1) / p.tile_cols;
@@ -315,7 +333,8 @@ static int gemm_impl(const hb_gemm_args* args) {
   // shared-memory split of the pair kernel: the deepest ring, except for a K loop of one or two steps, whose time is the
   // epilogue's: it gives stages to staging slabs.  us with 1 | 2 | 4 slabs, 64 x [2048, K] . [K, 2048]: K = 128 125 | 123 | 114,
   // K = 256 152 | 152 | 176, K = 384 191 | 196 | 229.
-  p.out_slabs = p.k_steps <= 2 ? 4 : 1;
+  // With a residual, two slabs hold a tile's part of it (GemmPairParams).
+  p.out_slabs = res_tma ? 2 : p.k_steps <= 2 ? 4 : 1;
   p.pair_stages = kPairSlots - p.out_slabs;
 
   const int grid = pair ? 2 * (int)std::min<long long>(tiles, st->sm_count / 2) : (int)std::min<long long>(tiles, st->sm_count);
@@ -338,8 +357,13 @@ static int gemm_impl(const hb_gemm_args* args) {
     return a->dtype == HB_BF16 ? dispatch_gemm_split<__nv_bfloat16, false>(epi_class, plain, split_grid, st, stream)
                                : dispatch_gemm_split<__half, false>(epi_class, plain, split_grid, st, stream);
   }
-  return a->dtype == HB_BF16 ? dispatch_gemm<__nv_bfloat16>(epi_class, p, grid, pair, st, stream)
-                             : dispatch_gemm<__half>(epi_class, p, grid, pair, st, stream);
+  if (pair) {
+    const CUtensorMap* const res = res_tma ? &tm_res : nullptr;
+    return a->dtype == HB_BF16 ? dispatch_gemm_pair<__nv_bfloat16>(epi_class, p, res, grid, st, stream)
+                               : dispatch_gemm_pair<__half>(epi_class, p, res, grid, st, stream);
+  }
+  return a->dtype == HB_BF16 ? dispatch_gemm<__nv_bfloat16>(epi_class, p, grid, st, stream)
+                             : dispatch_gemm<__half>(epi_class, p, grid, st, stream);
 }
 
 static int rowstat_impl(const void* x, const void* residual, void* y_out, float* rstd, int M, int N, long long ldx,

@@ -73,7 +73,17 @@ struct alignas(64) GemmParams {
   long long o_batch_stride, r_batch_stride;  // elements between consecutive batches of out / residual
   int tma_store;      // PLAIN epilogue: results leave through shared memory and a TMA store
   int pair_stages;    // CTA-pair kernel: depth of the operand ring (3..6) ...
-  int out_slabs;      // ... and staging slabs per epilogue warpgroup (1 or 4); stages + slabs = 7
+  int out_slabs;      // ... and staging slabs per epilogue warpgroup (1, 2 or 4); stages + slabs = 7
+};
+// The pair kernel brings a plain product's residual by TMA, into the staging slabs that its results leave through (out_slabs = 2), while
+// the main loop runs.  Read by its threads, a row each (32 lines a load), it cost 14 us of 36: us without a residual | read by threads |
+// by TMA: 1203 x 4464 x 1552 21.5 | 35.9 | 24.1, 5094 x 864 x 1016 18.2 | 32.7 | 20.8, 16384 x 2048 x 128 - | 84.0 | 35.3, 2000 x 4096 x 4096
+// - | 66.3 | 59.7, 16384 x 4096 x 11008 - | 1175 | 1180 (its ring is five stages deep instead of six).
+template <bool Residual>
+struct GemmPairParams : GemmParams {};
+template <>
+struct GemmPairParams<true> : GemmParams {
+  CUtensorMap tm_res;  // as tm_out
 };
 
 struct GemmSmem {
@@ -123,6 +133,7 @@ __device__ __forceinline__ float apply_act(float v) {
 // SiLU 238 -> 56, GELU 324 -> 63, bias and row scale 56 -> 51.  The division went with it: 2722 x 3200 x 2640 + SwiGLU 46.5 -> 44.6.
 template <typename F>
 __device__ __forceinline__ void with_act(int act, F&& f) {
+  if (act == kActNone) return f(std::integral_constant<int, kActNone>{});  // no jump table in the way of most products
   switch (act) {
     case kActSilu:
       return f(std::integral_constant<int, kActSilu>{});
@@ -132,10 +143,8 @@ __device__ __forceinline__ void with_act(int act, F&& f) {
       return f(std::integral_constant<int, kActGeluTanh>{});
     case kActSigmoid:
       return f(std::integral_constant<int, kActSigmoid>{});
-    case kActTanh:
-      return f(std::integral_constant<int, kActTanh>{});
     default:
-      return f(std::integral_constant<int, kActNone>{});
+      return f(std::integral_constant<int, kActTanh>{});
   }
 }
 
@@ -229,7 +238,7 @@ __device__ __forceinline__ void load_angles8(const GemmParams& p, const void* ta
 // tile: `part` (0 or 1) selects this thread's half of the output columns.  `release` is the
 // shared::cluster address of the barrier that hands the accumulator buffer back to the MMA warp
 // (this CTA's own, or the leader's when a CTA pair shares the MMA).
-template <typename T, int EPI>
+template <typename T, int EPI, bool ResInSlabs = false>
 __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t tacc, int b, int m0, int n0,
                                                   int row_in_tile, int part, uint8_t* stage_base, int n_slabs, uint32_t& slab_cursor,
                                                   uint32_t release) {
@@ -253,7 +262,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
     // its own row: conflict-free), one thread hands the slab to the TMA, which clips rows past M and columns past N_out.  The
     // warpgroup owns a ring of `n_slabs` staging slabs; slabs are rewritten once the TMA store that last used them has read
     // them.  With four, a tile's two slabs are one step (one pair of barriers, one group of stores) and the other two may
-    // still be on their way out.  Every step commits a group, stored or not, to keep the count of groups exact.
+    // still be on their way out.  With two, each holds the residual of one of the tile's slabs (GemmPairParams).  Every step commits a group, stored or not, to keep the count of groups exact.
     const bool issuer = row_in_tile == 0;
     const bool raw = p.row_scale == nullptr && p.bias == nullptr && p.residual == nullptr && p.act == kActNone;
     const int per_step = n_slabs == 4 ? 2 : 1;
@@ -289,8 +298,16 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
           }
 #pragma unroll
           for (int e = 0; e < 8; ++e) v[e] = apply_act<decltype(act)::value>(v[e]);
-          if (row_ok && col < p.N_out) add_residual8<T>(p, b, row, col, v);
-          *reinterpret_cast<uint4*>(stage + row_in_tile * 128 + (g ^ (row_in_tile & 7)) * 16) = pack8<T>(v);
+          uint4* const chunk = reinterpret_cast<uint4*>(stage + row_in_tile * 128 + (g ^ (row_in_tile & 7)) * 16);
+          if constexpr (ResInSlabs) {
+            float res[8];
+            unpack8<T>(*chunk, res);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] += res[e];
+          } else if (row_ok && col < p.N_out) {
+            add_residual8<T>(p, b, row, col, v);
+          }
+          *chunk = pack8<T>(v);
         }
       });
     };
@@ -300,7 +317,7 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
       const bool first = cc == 0 || per_step == 1, last = cc == 1 || per_step == 1;
       uint8_t* stage = stage_base + (slab_cursor & static_cast<uint32_t>(n_slabs - 1)) * (kGemmBM * 128);
       ++slab_cursor;
-      if (first) {
+      if (first && !ResInSlabs) {  // a slab that a residual was loaded into is free
         if (issuer) {
           if (n_slabs == 1) tma_store_wait_read<0>();
           else tma_store_wait_read<1>();
@@ -627,6 +644,7 @@ constexpr int kPairSlab = kGemmBM * 128;                  // 16 KB: 128 rows x 6
 struct GemmPairCtrl {
   uint64_t full[kPairMaxStages], empty[kPairMaxStages];
   uint64_t acc_full[2], acc_empty[2];
+  uint64_t res_full[2];  // per epilogue warpgroup
   uint64_t drain;
   uint32_t tmem_base;
   uint32_t abort_flag;
@@ -658,8 +676,8 @@ __device__ __forceinline__ void gemm_pair_tile_coords(const GemmParams& p, int t
   gemm_tile_coords(p, t, m_t, n_t, b);
 }
 
-template <typename T, int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gemm_pair_kernel(const __grid_constant__ GemmParams p) {
+template <typename T, int EPI, bool Residual>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gemm_pair_kernel(const __grid_constant__ GemmPairParams<Residual> p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int kStages = p.pair_stages;
   uint8_t* const ring_a = smem_raw;
@@ -680,6 +698,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s.acc_full[i], 1);
       mbar_init(&s.acc_empty[i], 16);  // 8 epilogue warps of each CTA (used in the leader only)
+      mbar_init(&s.res_full[i], 1);
     }
     mbar_init(&s.drain, 1);
     fence_mbar_init();
@@ -818,16 +837,28 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
     const int quarter = warp & 3;
     const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
     uint32_t tile_i = 0, slab_cursor = 0;
-    uint8_t* const my_slabs = slabs + ((warp - 2) >> 2) * p.out_slabs * kPairSlab;
+    const int part = (warp - 2) >> 2;
+    uint8_t* const my_slabs = slabs + part * p.out_slabs * kPairSlab;
     for (int t = pair; t < p.num_tiles; t += n_pairs, ++tile_i) {
       int m_t, n_t, b;
       gemm_pair_tile_coords(p, t, m_t, n_t, b);
       const uint32_t acc = tile_i & 1;
+      const int m0 = m_t * kPairBM + static_cast<int>(rank) * kGemmBM;
+      if constexpr (Residual) {
+        if (quarter == 0 && lane == 0) {
+          tma_store_wait_read<0>();  // the last tile's results have left the slabs
+          const int col0 = n_t * p.tile_cols + part * (kGemmBN / 2);
+          const int n = m0 >= p.M ? 0 : (col0 < p.N_out ? 1 : 0) + (col0 + 64 < p.N_out ? 1 : 0);
+          mbar_arrive_expect_tx(&s.res_full[part], static_cast<uint32_t>(n) * kPairSlab);
+          for (int i = 0; i < n; ++i) tma_load_3d(my_slabs + i * kPairSlab, &p.tm_res, &s.res_full[part], col0 + i * 64, m0, b);
+        }
+        __syncwarp();
+      }
       if (!mbar_wait_warp(&s.acc_full[acc], (tile_i >> 1) & 1, ctx, kGemmRoleEpi)) break;
+      if (Residual && !mbar_wait_warp(&s.res_full[part], tile_i & 1, ctx, kGemmRoleEpi)) break;
       tc_fence_after();
-      gemm_epilogue_row<T, EPI>(p, tmem + lane_off + acc * kGemmBN, b, m_t * kPairBM + static_cast<int>(rank) * kGemmBM,
-                                n_t * p.tile_cols, quarter * 32 + lane, (warp - 2) >> 2, my_slabs, p.out_slabs, slab_cursor,
-                                mapa_u32(smem_u32(&s.acc_empty[acc]), 0));
+      gemm_epilogue_row<T, EPI, Residual>(p, tmem + lane_off + acc * kGemmBN, b, m0, n_t * p.tile_cols, quarter * 32 + lane, part,
+                                          my_slabs, p.out_slabs, slab_cursor, mapa_u32(smem_u32(&s.acc_empty[acc]), 0));
     }
     if (p.tma_store && quarter == 0 && lane == 0) tma_store_wait_all<0>();
   }

@@ -206,12 +206,12 @@ __global__ void __launch_bounds__(kGemmSplitThreads, 1) gemm_split_kernel(const 
         tc_fence_after();
         const uint32_t a_lo = (smem_u32(ring_a + st * a_bytes) >> 4) | kLbo, b_lo = (smem_u32(ring_b + st * b_bytes) >> 4) | b_lbo;
         if (leader) {
-          int slabs = sp.slabs;
-          if constexpr (Tail) {
+          auto slabs = [&]() -> int {
             // the last stage of whole slabs may hold fewer: with a [K, N] operand the rest of its box are the tail's rows
-            if (ks >= sp.tail_stage - 1) slabs = ks == sp.tail_stage ? 1 : sp.last_slabs;
-          }
-          for (int sl = 0; sl < slabs; ++sl) {
+            if constexpr (Tail) return ks == sp.tail_stage ? 1 : ks == sp.tail_stage - 1 ? sp.last_slabs : sp.slabs;
+            else return sp.slabs;
+          };
+          for (int sl = 0; sl < slabs(); ++sl) {
             const uint32_t a = a_lo + static_cast<uint32_t>(sl) * (a_slab >> 4), w = b_lo + static_cast<uint32_t>(sl) * b_next;
 #pragma unroll
             for (int kk = 0; kk < kGemmBK / 16; ++kk) {

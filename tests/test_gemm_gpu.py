@@ -344,3 +344,23 @@ def test_full_size_projection_by_size_independent_properties(ops):
     assert float((got - checksum).abs().max()) <= float(bound)
     twice = ops.gemm_epilogue(a * 2, w)
     assert torch.equal(twice, out * 2)
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 136, 64), (300, 520, 200), (513, 264, 1000), (1500, 3080, 72), (9000, 512, 136)])
+@pytest.mark.parametrize("form", ["dense", "wide rows", "in place"])
+def test_residual(ops, M, N, K, form):
+    """A residual that is read tile by tile beside the products: tails in every dimension, several tiles a CTA, rows of a wider tensor with
+    NaN around them, and the result written over it."""
+    dt = torch.float16
+    a, w = _mk(M, N, K, seed=M + N, dtype=dt)
+    g = torch.Generator().manual_seed(K)
+    res = torch.randn(M, N, generator=g).to(dt)
+    wide = torch.full((M, N + 16), float("nan"), dtype=dt)
+    wide[:, 8:8 + N] = res
+    r = wide.cuda()[:, 8:8 + N] if form == "wide rows" else res.cuda()
+    rs = torch.rand(M, generator=g) + 0.5
+    out = ops.gemm_epilogue(a.cuda(), w.cuda(), "silu", row_scale=rs.cuda(), residual=r, out=r if form == "in place" else None)
+    torch.cuda.synchronize()
+    assert ops.status_word() == 0
+    ref = O.epilogue_fp32((a.float() @ w.float().t()) * rs[:, None], "silu") + res.float()
+    _close(out, ref, tol=2e-3)  # fp32 sums, rounded once to fp16
