@@ -28,13 +28,13 @@ uint64_t fa_split_workspace(const hb_fa_args* a, int sm_count) {
 
 static std::mutex g_split_mutex;
 
-template <typename T, int D, int RC>
+template <typename T, int D, int RC, int NH>
 static int launch_split(const FaSplitParams& p, int grid, bool combine, int smem_optin, cudaStream_t stream) {
   using Smem = FaSplitSmem<T, D, RC>;
   if ((int)sizeof(Smem) > smem_optin)
     return set_error(HB_ERR_UNSUPPORTED, "hb_fa_fwd_ws: kernel needs %d bytes of shared memory, device offers %d",
                      (int)sizeof(Smem), smem_optin);
-  auto kernel = fa_split_kernel<T, D, RC>;
+  auto kernel = fa_split_kernel<T, D, RC, NH>;
   static bool configured[64] = {};
   int dev = 0;
   HB_CUDA_CHECK(cudaGetDevice(&dev));
@@ -56,13 +56,16 @@ static int launch_split(const FaSplitParams& p, int grid, bool combine, int smem
   return HB_OK;
 }
 
+template <typename T, int D>
+static int launch_split_rows(const FaSplitParams& p, int grid, bool combine, int smem_optin, cudaStream_t stream) {
+  if (p.plan.rows <= 8) return launch_split<T, D, 64, 1>(p, grid, combine, smem_optin, stream);
+  if (p.plan.rows <= 16) return launch_split<T, D, 64, 2>(p, grid, combine, smem_optin, stream);
+  if (p.plan.rows <= 64) return launch_split<T, D, 64, 0>(p, grid, combine, smem_optin, stream);
+  return launch_split<T, D, 128, 0>(p, grid, combine, smem_optin, stream);
+}
 template <typename T>
 static int launch_split_d(const FaSplitParams& p, int D, int grid, bool combine, int smem_optin, cudaStream_t stream) {
-  if (D == 128)
-    return p.plan.rows <= 64 ? launch_split<T, 128, 64>(p, grid, combine, smem_optin, stream)
-                        : launch_split<T, 128, 128>(p, grid, combine, smem_optin, stream);
-  return p.plan.rows <= 64 ? launch_split<T, 64, 64>(p, grid, combine, smem_optin, stream)
-                      : launch_split<T, 64, 128>(p, grid, combine, smem_optin, stream);
+  return D == 128 ? launch_split_rows<T, 128>(p, grid, combine, smem_optin, stream) : launch_split_rows<T, 64>(p, grid, combine, smem_optin, stream);
 }
 
 int fa_split_run(const hb_fa_args* a, const DeviceState* st, void* workspace, uint64_t workspace_bytes) {

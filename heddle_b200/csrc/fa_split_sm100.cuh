@@ -89,6 +89,195 @@ __device__ __forceinline__ constexpr int fa_split_row0(int i) {
   return RC == 64 ? 64 * i : 0;
 }
 
+// End of a segment: O / l of the thread's row (its lane of O at tO) to the output, or as a partial result.
+template <typename T, int D>
+__device__ __forceinline__ void fa_split_store_segment(const FaSplitParams& p, const FaSegment& g, uint32_t tO, int w, bool first, int row,
+                                                       int head, int pos, float m, float l) {
+  const bool whole = g.j0 == 0 && g.j1 == p.plan.nkv;
+  const bool live = row < p.plan.rows && head < g.heads;
+  const float inv_l = (l > 0.f) ? (1.0f / l) : 0.f;
+  const float lse2 = (l > 0.f) ? (m * p.scale_log2 + fast_log2(l)) : -INFINITY;
+  const long long slot = 2ll * w + (first ? 0 : 1);
+  T* orow = static_cast<T*>(p.o) + g.b * p.o_sb + (g.hq0 + head) * p.o_sh + static_cast<long long>(pos) * p.o_ss;
+  float* prow = p.part_o + (slot * p.plan.rows + row) * D;
+#pragma unroll
+  for (int c = 0; c < D / 32; ++c) {
+    uint32_t r[32];
+    __syncwarp();
+    tmem_ld32(tO + c * 32, r);
+    tmem_wait_ld();
+    if (live && whole) {
+#pragma unroll
+      for (int e = 0; e < 32; e += 8) {
+        uint4 o;
+        o.x = Pack2<T>::pack(__uint_as_float(r[e]) * inv_l, __uint_as_float(r[e + 1]) * inv_l);
+        o.y = Pack2<T>::pack(__uint_as_float(r[e + 2]) * inv_l, __uint_as_float(r[e + 3]) * inv_l);
+        o.z = Pack2<T>::pack(__uint_as_float(r[e + 4]) * inv_l, __uint_as_float(r[e + 5]) * inv_l);
+        o.w = Pack2<T>::pack(__uint_as_float(r[e + 6]) * inv_l, __uint_as_float(r[e + 7]) * inv_l);
+        *reinterpret_cast<uint4*>(orow + c * 32 + e) = o;
+      }
+    } else if (live) {
+#pragma unroll
+      for (int e = 0; e < 32; e += 4) {
+        *reinterpret_cast<float4*>(prow + c * 32 + e) =
+            make_float4(__uint_as_float(r[e]) * inv_l, __uint_as_float(r[e + 1]) * inv_l, __uint_as_float(r[e + 2]) * inv_l,
+                        __uint_as_float(r[e + 3]) * inv_l);
+      }
+    }
+  }
+  if (live && whole) {
+    if (p.lse != nullptr)
+      p.lse[(static_cast<long long>(g.b) * p.Hq + g.hq0 + head) * p.Sq + pos] = lse2 * 0.6931471805599453f;
+  } else if (live) {
+    p.part_lse[slot * p.plan.rows + row] = lse2;
+  }
+}
+
+// The softmax of calls with at most 8 NH rows (NH 1 or 2), decode above all.  With a thread a row, one warp turned 128 columns over for
+// a handful of live lanes: 1500 cycles of the 2500 to 2900 that a step of such a pipeline took, which with 64-wide heads (32 KB a step)
+// is slower than HBM.  Here a row lies on the four lanes of a quad, 32 columns each: a quarter of the exponentials (half, with 9 to 16
+// rows), two shuffles for the maximum, the sum put together at the end of the segment.
+// us a thread a row -> a quad a row: D 64 B54 H12 393 keys 26.0 -> 21.1, B2 H32 Sq 2 15777 keys 55.0 -> 50.9, B25 Hq32 Hkv8 2189 keys
+// 29.5 -> 27.0, B32 H4 559 keys 12.3 -> 9.6; D 128 B62 H16 Sq 3 442 keys 48.0 -> 44.7, B13 Hq32 Hkv4 6060 keys 36.6 -> 35.5, B14 H1 Sq 8 146
+// keys 7.5 -> 6.2, B16 Hq64 Hkv8 6001 keys 70.2 -> 69.3.
+template <typename T, int D, int NH, int RC>
+__device__ __forceinline__ void fa_split_softmax_few(const FaSplitParams& p, FaSplitSmem<T, D, RC>& s, const AbortCtx& ctx, uint32_t tmem,
+                                                     int i, int w) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
+  const uint32_t tS = tmem + lane_off + static_cast<uint32_t>(i * 256), tO = tS + 128;
+  const int c = lane & 3, lane_head = lane / p.Sq;
+  const float scale_log2 = p.scale_log2;
+  const int past = p.Skv - p.Sq;
+  uint32_t s_phase = 0, o_phase = 0;
+  int row[NH], pos[NH];
+#pragma unroll
+  for (int h = 0; h < NH; ++h) {
+    row[h] = (lane >> 2) + 8 * h;
+    pos[h] = row[h] % p.Sq;
+  }
+  // the value of the lane's own row, for whole rows on lanes
+  auto of_row = [&](const float (&x)[NH]) {
+    float y = __shfl_sync(0xffffffffu, x[0], (lane & 7) * 4);
+    if constexpr (NH == 2) {
+      const float z = __shfl_sync(0xffffffffu, x[1], (lane & 7) * 4);
+      if (lane & 8) y = z;
+    }
+    return y;
+  };
+
+  const long long end = fa_split_begin(p.plan, w + 1);
+  bool first = true;
+  for (long long t = fa_split_begin(p.plan, w); t < end; first = false) {
+    const FaSegment g = fa_split_segment(p, t, end);
+    t += g.j1 - g.j0;
+    float m[NH], l[NH];
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
+      m[h] = -INFINITY;
+      l[h] = 0.f;
+    }
+
+    for (int j = g.j0; j < g.j1; ++j) {
+      if (!mbar_wait_warp(&s.s_full[i], s_phase, ctx, kRoleSplitSoftmax)) return;
+      s_phase ^= 1;
+      tc_fence_after();
+      uint32_t r[64], pk[32];
+      tmem_ld_16x128cols(tS, r);
+      tmem_wait_ld();
+      const int col0 = j * kTileN;
+      const bool need_mask = col0 + kTileN > p.Skv || (p.causal && col0 + kTileN - 1 > past);
+      float alpha[NH];
+#pragma unroll
+      for (int h = 0; h < NH; ++h) {
+        if (need_mask) {
+          int lim = p.Skv - 1 - col0;
+          if (p.causal) lim = min(lim, past + pos[h] - col0);
+          lim -= 2 * c;
+#pragma unroll
+          for (int q = 0; q < 16; ++q) {
+            uint32_t* x = &r[4 * q + 2 * h];
+            x[0] = 8 * q <= lim ? x[0] : 0xff800000u;  // -inf
+            x[1] = 8 * q + 1 <= lim ? x[1] : 0xff800000u;
+          }
+        }
+        float mx[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) mx[q] = fmaxf(__uint_as_float(r[4 * q + 2 * h]), __uint_as_float(r[4 * q + 2 * h + 1]));
+#pragma unroll
+        for (int q = 4; q < 16; ++q)
+          mx[q & 3] = max3(mx[q & 3], __uint_as_float(r[4 * q + 2 * h]), __uint_as_float(r[4 * q + 2 * h + 1]));
+        float row_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+        row_max = fmaxf(row_max, __shfl_xor_sync(0xffffffffu, row_max, 1));
+        row_max = fmaxf(row_max, __shfl_xor_sync(0xffffffffu, row_max, 2));
+
+        // the same rule as the general kernel: a maximum that grew by less than 2^8 is not adopted
+        const float m_cand = fmaxf(m[h], row_max);
+        const float diff = (m[h] - m_cand) * scale_log2;
+        const bool adopt = row[h] < p.plan.rows && diff < -FaTraits<T>::kRescaleThreshold;  // padding rows never ask for a rescale
+        alpha[h] = adopt ? fast_exp2(diff) : 1.f;
+        m[h] = adopt ? m_cand : m[h];
+        const float m_scaled = (m[h] == -INFINITY) ? 0.f : m[h] * scale_log2;
+
+        const uint64_t sc2 = pack_f32x2(scale_log2, scale_log2), nm2 = pack_f32x2(-m_scaled, -m_scaled);
+        uint64_t sa = pack_f32x2(0.f, 0.f), sb = sa;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+          const uint64_t x =
+              fma_f32x2(pack_f32x2(__uint_as_float(r[4 * q + 2 * h]), __uint_as_float(r[4 * q + 2 * h + 1])), sc2, nm2);
+          float a, b;
+          unpack_f32x2(x, a, b);
+          a = fast_exp2(a);
+          b = fast_exp2(b);
+          if (q & 1) sb = add_f32x2(sb, pack_f32x2(a, b));
+          else sa = add_f32x2(sa, pack_f32x2(a, b));
+          pk[2 * q + h] = Pack2<T>::pack(a, b);
+          if (NH == 1) pk[2 * q + 1] = 0u;
+        }
+        float sum0, sum1, sum2, sum3;
+        unpack_f32x2(sa, sum0, sum1);
+        unpack_f32x2(sb, sum2, sum3);
+        l[h] = l[h] * alpha[h] + ((sum0 + sum1) + (sum2 + sum3));  // of this lane's columns
+      }
+      tmem_st_16x64cols(tS, pk);
+      // O is rescaled a row a lane: S(j) was committed behind PV(j - 1), so that product is complete, and PV(j) is only issued after
+      // this warp's arrival on p_full
+      bool moved = alpha[0] != 1.f;
+      if constexpr (NH == 2) moved = moved || alpha[1] != 1.f;
+      if (j > g.j0 && __any_sync(0xffffffffu, moved)) {
+        const float a = of_row(alpha);
+#pragma unroll
+        for (int q = 0; q < D / 32; ++q) {
+          uint32_t o[32];
+          tmem_ld32(tO + q * 32, o);
+          tmem_wait_ld();
+#pragma unroll
+          for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * a);
+          tmem_st32(tO + q * 32, o);
+        }
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s.p_full[i]);
+    }
+
+    if (!mbar_wait_warp(&s.o_full[i], o_phase, ctx, kRoleSplitSoftmax)) return;
+    o_phase ^= 1;
+    tc_fence_after();
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
+      l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
+      l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
+    }
+    const float m_row = of_row(m), l_row = of_row(l);
+    fa_split_store_segment<T, D>(p, g, tO, w, first, lane, lane_head, lane - lane_head * p.Sq, m_row, l_row);
+    // the next segment's first product overwrites O: it waits for this warp's next arrival on p_full
+    tc_fence_before();
+    __syncwarp();
+  }
+}
+
 template <typename T, int D, int RC>
 __device__ __forceinline__ void fa_split_softmax_role(const FaSplitParams& p, FaSplitSmem<T, D, RC>& s, const AbortCtx& ctx,
                                                       uint32_t tmem, int i, int w) {
@@ -196,44 +385,7 @@ __device__ __forceinline__ void fa_split_softmax_role(const FaSplitParams& p, Fa
     if (!mbar_wait_warp(&s.o_full[i], o_phase, ctx, kRoleSplitSoftmax)) return;
     o_phase ^= 1;
     tc_fence_after();
-    const bool whole = g.j0 == 0 && g.j1 == p.plan.nkv;
-    const bool live = row < p.plan.rows && head < g.heads;
-    const float inv_l = (l > 0.f) ? (1.0f / l) : 0.f;
-    const float lse2 = (l > 0.f) ? (m * scale_log2 + fast_log2(l)) : -INFINITY;
-    const long long slot = 2ll * w + (first ? 0 : 1);
-    T* orow = static_cast<T*>(p.o) + g.b * p.o_sb + (g.hq0 + head) * p.o_sh + static_cast<long long>(pos) * p.o_ss;
-    float* prow = p.part_o + (slot * p.plan.rows + row) * D;
-#pragma unroll
-    for (int c = 0; c < D / 32; ++c) {
-      uint32_t r[32];
-      __syncwarp();
-      tmem_ld32(tO + c * 32, r);
-      tmem_wait_ld();
-      if (live && whole) {
-#pragma unroll
-        for (int e = 0; e < 32; e += 8) {
-          uint4 o;
-          o.x = Pack2<T>::pack(__uint_as_float(r[e]) * inv_l, __uint_as_float(r[e + 1]) * inv_l);
-          o.y = Pack2<T>::pack(__uint_as_float(r[e + 2]) * inv_l, __uint_as_float(r[e + 3]) * inv_l);
-          o.z = Pack2<T>::pack(__uint_as_float(r[e + 4]) * inv_l, __uint_as_float(r[e + 5]) * inv_l);
-          o.w = Pack2<T>::pack(__uint_as_float(r[e + 6]) * inv_l, __uint_as_float(r[e + 7]) * inv_l);
-          *reinterpret_cast<uint4*>(orow + c * 32 + e) = o;
-        }
-      } else if (live) {
-#pragma unroll
-        for (int e = 0; e < 32; e += 4) {
-          *reinterpret_cast<float4*>(prow + c * 32 + e) =
-              make_float4(__uint_as_float(r[e]) * inv_l, __uint_as_float(r[e + 1]) * inv_l, __uint_as_float(r[e + 2]) * inv_l,
-                          __uint_as_float(r[e + 3]) * inv_l);
-        }
-      }
-    }
-    if (live && whole) {
-      if (p.lse != nullptr)
-        p.lse[(static_cast<long long>(g.b) * p.Hq + g.hq0 + head) * p.Sq + pos] = lse2 * 0.6931471805599453f;
-    } else if (live) {
-      p.part_lse[slot * p.plan.rows + row] = lse2;
-    }
+    fa_split_store_segment<T, D>(p, g, tO, w, first, row, head, pos, m, l);
     // the next segment's first product overwrites O: it waits for this thread's next arrival on p_full
     tc_fence_before();
     __syncwarp();
@@ -342,7 +494,15 @@ __device__ __forceinline__ void fa_split_tma_role(const FaSplitParams& p, FaSpli
   }
 }
 
-template <typename T, int D, int RC>
+template <typename T, int D, int RC, int NH>
+__device__ __forceinline__ void fa_split_softmax(const FaSplitParams& p, FaSplitSmem<T, D, RC>& s, const AbortCtx& ctx, uint32_t tmem, int i,
+                                                 int w) {
+  if constexpr (NH > 0) fa_split_softmax_few<T, D, NH, RC>(p, s, ctx, tmem, i, w);
+  else fa_split_softmax_role<T, D, RC>(p, s, ctx, tmem, i, w);
+}
+
+// NH: 0, or 1 or 2 for at most 8 NH rows (fa_split_softmax_few)
+template <typename T, int D, int RC, int NH>
 __global__ void __launch_bounds__(kSplitThreads, 1) fa_split_kernel(const __grid_constant__ FaSplitParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   using Smem = FaSplitSmem<T, D, RC>;
@@ -392,7 +552,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) fa_split_kernel(const __grid
     reg_inc<200>();
     const int first_warp = fa_split_row0<RC>(i) / 32;
     if (run && w < p.plan.pipes && (warp & 3) >= first_warp && (warp & 3) < first_warp + softmax_warps)
-      fa_split_softmax_role<T, D, RC>(p, s, ctx, tmem, i, w);
+      fa_split_softmax<T, D, RC, NH>(p, s, ctx, tmem, i, w);
   } else {
     reg_dec<96>();
     if (run && w < p.plan.pipes && warp < 10) {

@@ -113,3 +113,25 @@ def test_workspace_is_asked_for_and_checked(ops, built_lib):
     assert built_lib.hb_fa_fwd_ws(C.byref(a), ws.data_ptr(), need.value - 4) == _lib.HB_ERR_BAD_ARG
     assert built_lib.hb_fa_fwd_ws(C.byref(a), ws.data_ptr(), need.value) == _lib.HB_OK
     assert torch.equal(out, ops.fa_fwd(q, k, k))
+
+
+@pytest.mark.parametrize("group,Sq", [(1, 1), (7, 1), (2, 4), (9, 1), (3, 5), (8, 2), (17, 1)])
+@pytest.mark.parametrize("Skv", [5, 130, 1100])
+@pytest.mark.parametrize("D,dt", [(64, torch.float16), (128, torch.bfloat16)])
+def test_few_rows(ops, group, Sq, Skv, D, dt):
+    """Up to 8, up to 16 and more rows a tile, which three softmax forms turn over: masks inside a tile for every row, maxima that grow along the
+    keys and rows whose maxima differ, partial segments and whole ones (two heads of keys on two pipelines, and twelve)."""
+    for B, Hkv in ((1, 2), (6, 2)):
+        q, k, v = O.make_qkv(B, group * Hkv, Hkv, Sq, Skv, D, seed=Skv + group, dtype=dt)
+        q = (q.float() * torch.linspace(0.2, 3.0, group * Hkv)[:, None, None]).to(dt)
+        k = (k.float() * torch.linspace(0.3, 2.0, Skv)[:, None]).to(dt)
+        ref, ref_lse = O.attention_eager(q, k, v, causal=True)
+        mass, _ = O.attention_eager(q, k, v.abs(), causal=True)
+        out, lse = ops.fa_fwd(q.cuda(), k.cuda(), v.cuda(), causal=True, return_lse=True)
+        torch.cuda.synchronize()
+        assert ops.status_word() == 0
+        # as in test_against_the_oracle
+        unit = 2.0**-8 if dt == torch.bfloat16 else 2.0**-11
+        tol = unit * (mass + ref.abs()) + 1e-4 * mass + (Skv * 2.0**-25 * 4.5 if dt == torch.float16 else 0.0)
+        assert ((out.float().cpu() - ref).abs() / tol).max().item() <= 1.0
+        assert (lse.cpu() - ref_lse).abs().max().item() <= 2e-3
