@@ -115,6 +115,15 @@ __global__ void __launch_bounds__(kGemmSplitThreads, 1) gemm_split_kernel(const 
   const int rank = static_cast<int>(blockIdx.x) % splits, t = static_cast<int>(blockIdx.x) / splits;
   AbortCtx ctx{&s.abort_flag, p.status};
 
+  int m_t, n_t, b;
+  gemm_tile_coords(p, t, m_t, n_t, b);
+  const int m0 = m_t * kGemmBM, n0 = n_t * p.tile_cols;
+  const int k_begin = p.k_steps * rank / splits, k_end = p.k_steps * (rank + 1) / splits;  // at most 2^25 stages, 8 ranks
+  // In front of the wait for the predecessor, where the time is free: a 64-bit division and first reads of the parameters, which miss the
+  // constant cache, lay 0.7 us between that and the first copies, 0.3 us now.  us back to back, before -> after: 1 x 4096 x 4096 10.2 ->
+  // 9.9, 64 x 1024 x 512 4.4 -> 4.1, 1 x 640 x 720 4.9 -> 4.5, batch of 3 67 x 280 x 1392 6.0 -> 5.5.
+  computed(m0, n0, b, k_begin, k_end, a_bytes, b_bytes, p.w_kn, sp.k_slabs);
+
   if (threadIdx.x == 0) {
     s.abort_flag = 0;
     for (int i = 0; i < sp.stages; ++i) {
@@ -143,12 +152,6 @@ __global__ void __launch_bounds__(kGemmSplitThreads, 1) gemm_split_kernel(const 
   const bool run = (s.abort_flag == 0);
   grid_launch_dependents();
   grid_wait();
-
-  int m_t, n_t, b;
-  gemm_tile_coords(p, t, m_t, n_t, b);
-  const int m0 = m_t * kGemmBM, n0 = n_t * p.tile_cols;
-  const int k_begin = static_cast<int>(static_cast<long long>(p.k_steps) * rank / splits);
-  const int k_end = static_cast<int>(static_cast<long long>(p.k_steps) * (rank + 1) / splits);
 
   if (warp == 0) {
     if (run && lane == 0) {

@@ -64,6 +64,13 @@ constexpr unsigned kFewBlocks = 37;  // a quarter of the SMs
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Keeps what is computed of x in front of what follows, as of grid_wait().  (Working out the first block ahead of the wait was neutral to
+// slower in the attention kernels and their merge, D 64 B1 H4 Sq 8 17594 keys 13.5 -> 14.3 us: only the split-K GEMM does.)
+template <typename... X>
+__device__ __forceinline__ void computed(X... x) {
+  ((void)[](uint32_t v) { asm volatile("" ::"r"(v)); }(static_cast<uint32_t>(x)), ...);
+}
+
 template <int N>
 __device__ __forceinline__ void reg_inc() {
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(N));
