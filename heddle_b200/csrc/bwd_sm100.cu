@@ -462,10 +462,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) fa_bwd_dkdv_kernel(const __gri
           {
             const int q = qt * 128 + half * 64 + lane * 2;
             float2 nv, dv;
-            nv.x = (q < p.Sq) ? -__ldg(lse_row + q) * 1.4426950408889634f : -INFINITY;
-            nv.y = (q + 1 < p.Sq) ? -__ldg(lse_row + q + 1) * 1.4426950408889634f : -INFINITY;
-            dv.x = (q < p.Sq) ? __ldg(dl_row + q) : 0.f;
-            dv.y = (q + 1 < p.Sq) ? __ldg(dl_row + q + 1) : 0.f;
+            nv.x = (q < p.Sq) ? -lse_row[q] * 1.4426950408889634f : -INFINITY;
+            nv.y = (q + 1 < p.Sq) ? -lse_row[q + 1] * 1.4426950408889634f : -INFINITY;
+            dv.x = (q < p.Sq) ? dl_row[q] : 0.f;
+            dv.y = (q + 1 < p.Sq) ? dl_row[q + 1] : 0.f;
             nl2[lane] = nv;
             dl2[lane] = dv;
           }
@@ -914,8 +914,7 @@ __global__ void __launch_bounds__(kBwdDqThreads, 1) fa_bwd_dq_kernel(const __gri
 // (16 bytes each); a warp covers 4 * 256 / D rows with all eight 16-byte loads of a lane in flight at once.
 // ------------------------------------------------------------------------------------------
 template <typename T, int D>
-__global__ void __launch_bounds__(256, 4) fa_bwd_preprocess_kernel(const T* __restrict__ o, const T* __restrict__ d_o,
-                                                                 float* __restrict__ delta, int B, int H, int S,
+__global__ void __launch_bounds__(256, 4) fa_bwd_preprocess_kernel(const T* o, const T* d_o, float* delta, int B, int H, int S,
                                                                  long long o_sb, long long o_sh, long long o_ss,
                                                                  long long g_sb, long long g_sh, long long g_ss) {
   constexpr int kLanesPerRow = D / 8, kRowsPerLoad = 32 / kLanesPerRow, kRowsPerWarp = 4 * kRowsPerLoad;
@@ -955,7 +954,7 @@ __global__ void __launch_bounds__(256, 4) fa_bwd_preprocess_kernel(const T* __re
 
 // dK, dV = the sum over the splits of fa_bwd_dkdv_kernel's partial results, in split order; blockIdx.y: 0 dK, 1 dV.
 template <typename T>
-__global__ void __launch_bounds__(256) fa_bwd_combine_kernel(const float* __restrict__ part, T* __restrict__ dk, T* __restrict__ dv,
+__global__ void __launch_bounds__(256) fa_bwd_combine_kernel(const float* part, T* dk, T* dv,
                                                             long long all, int splits) {
   grid_launch_dependents();
   grid_wait();

@@ -886,9 +886,8 @@ __device__ __forceinline__ uint4 ld_stream(const T* ptr) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) rms_rowstat_kernel(const T* __restrict__ x, const T* __restrict__ residual,
-                                                          T* __restrict__ y_out, float* __restrict__ rstd, int M,
-                                                          int N, long long ldx, float eps) {
+__global__ void __launch_bounds__(256) rms_rowstat_kernel(const T* x, const T* residual, T* y_out, float* rstd, int M, int N,
+                                                          long long ldx, float eps) {
   if (gridDim.x <= kFewBlocks) grid_launch_dependents();
   grid_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kH2oThreads, 1) h2o_score_kernel(const __grid_
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const int q = (it.qt0 + t) * 128 + lane * 4 + u;
-          v[u] = (q < p.Sq) ? -__ldg(lse_row + q) * 1.4426950408889634f : -INFINITY;
+          v[u] = (q < p.Sq) ? -lse_row[q] * 1.4426950408889634f : -INFINITY;
         }
       };
       // this group's tiles of the item: t = t_first, t_first + 2, ...

@@ -53,7 +53,8 @@ __device__ __forceinline__ int uniform_warp() { return static_cast<int>(warp_uni
 // grid_launch_dependents() on, and waits in grid_wait() until every earlier kernel is complete and its writes are visible.
 // No kernel touches global memory (its parameters aside) before grid_wait().  A kernel that holds TMEM calls
 // grid_launch_dependents() only after its own allocation: a dependent that took the columns first would wait for this grid,
-// and this grid for the columns.
+// and this grid for the columns.  Global memory is read by plain loads: what a kernel waits for is written during its own lifetime, which the
+// read-only path (__ldg, const __restrict__ parameters) does not allow; its loads may be moved in front of the wait.
 //
 // The row kernels and compiled pointwise programs let their dependents in only when their own loads are done, unless the
 // grid is a few blocks: dependents that are let in at the start take the free slots next to a grid that does not fill the chip

@@ -45,7 +45,7 @@ __device__ __forceinline__ uint4 rs_pack8(const float (&f)[8]) {
 
 // kChunks 16-byte chunks per thread; kWarpsPerRow warps cooperate on a row (1 or 8).
 template <typename T, int kChunks, int kWarpsPerRow>
-__global__ void __launch_bounds__(256) row_softmax_kernel(const T* __restrict__ x, T* __restrict__ y, long long rows,
+__global__ void __launch_bounds__(256) row_softmax_kernel(const T* x, T* y, long long rows,
                                                           int cols, long long ld_x, long long ld_y, float scale_log2) {
   constexpr int kThreadsPerRow = 32 * kWarpsPerRow;
   if (gridDim.x <= kFewBlocks) grid_launch_dependents();
