@@ -304,6 +304,7 @@ __global__ void __launch_bounds__(kH2oThreads, 1) h2o_score_kernel(const __grid_
           __threadfence_block();
         }
         second = __shfl_sync(0xffffffffu, second, 0);
+        __syncwarp();  // a shuffle orders no memory: lane 0's fence in front of the other lanes' reads
         store = second != 0;
         if (store) total += s.part[slot][grp ^ 1][key_in_tile];
       } else {

@@ -81,7 +81,7 @@ def test_h2o_full_length_properties(ops):
     assert (sc.sum(-1) - S).abs().max().item() <= 2e-3 * S
     # the last key is only seen by the last query, the first key by every query
     assert (sc[..., -1] <= 1.0 + 1e-3).all() and (sc[..., 0] >= sc[..., -1]).all()
-    # two commutative atomic adds per key: the result does not depend on their order
+    # two halves per key, one commutative add: the result does not depend on which comes first
     assert torch.equal(score, again)
     _, ref_lse = O.attention_eager(q[:1, :1], k[:1, :1], v[:1, :1], causal=True)
     ref = O.h2o_score(q[:1, :1], k[:1, :1], ref_lse, causal=True)
