@@ -278,7 +278,9 @@ static int gemm_impl(const hb_gemm_args* args) {
   }
   const bool pair = !use_split &&
                     (a->schedule == HB_GEMM_PAIR || (a->schedule == HB_GEMM_AUTO && a->M > kGemmBM && st->sm_count >= 2));
-  const bool res_tma = pair && epi_class == kEpiPlain && a->residual != nullptr;
+  // A tensor map has strides of 16 bytes to 2^40, forward only: a residual with others (its batches may lie in any order) is read by threads.
+  const bool res_strides = a->ldr < (1ll << 39) && (batch == 1 || (r_bs > 0 && r_bs < (1ll << 39)));
+  const bool res_tma = pair && epi_class == kEpiPlain && a->residual != nullptr && res_strides;
   CUtensorMap tm_res;
   if (epi_class == kEpiPlain && !use_split) {
     const uint32_t box[3] = {64, (uint32_t)kGemmBM, 1};
@@ -288,7 +290,7 @@ static int gemm_impl(const hb_gemm_args* args) {
     if (rc != HB_OK) return rc;
     p.tma_store = 1;
     if (res_tma) {
-      const uint64_t res_str[2] = {(uint64_t)a->ldr * 2, (uint64_t)r_bs * 2};
+      const uint64_t res_str[2] = {(uint64_t)a->ldr * 2, (uint64_t)(batch == 1 ? a->ldr : r_bs) * 2};  // one batch: any
       rc = encode_tensor_map(&tm_res, dt, 3, a->residual, dims, res_str, box, CU_TENSOR_MAP_SWIZZLE_128B);
       if (rc != HB_OK) return rc;
     }

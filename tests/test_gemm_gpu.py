@@ -364,3 +364,30 @@ def test_residual(ops, M, N, K, form):
     assert ops.status_word() == 0
     ref = O.epilogue_fp32((a.float() @ w.float().t()) * rs[:, None], "silu") + res.float()
     _close(out, ref, tol=2e-3)  # fp32 sums, rounded once to fp16
+
+
+@pytest.mark.parametrize("schedule", ["single", "pair", "split"])
+@pytest.mark.parametrize("batch,stride", [(1, 4), (1, -136 * 264), (3, -300 * 264), (3, 8)])
+def test_residual_batch_strides(ops, schedule, batch, stride):
+    """r_batch_stride of the C ABI: not looked at with one batch; else any multiple of 8 elements whose rows exist, backward and overlapping
+    ones too."""
+    from heddle_b200 import _lib
+
+    M, N, K = 300, 264, 136
+    gen = torch.Generator().manual_seed(batch)
+    a = torch.randn(batch, M, K, generator=gen).half().cuda()
+    w = (torch.randn(batch, N, K, generator=gen) * 0.1).half().cuda()
+    rows = torch.randn(batch * M * N + 64, generator=gen).half().cuda()
+    out = torch.empty(batch, M, N, dtype=torch.float16, device="cuda")
+    first = -stride * (batch - 1) if batch > 1 and stride < 0 else 0
+    g = _lib.GemmArgs()
+    g.a, g.w, g.out, g.residual = a.data_ptr(), w.data_ptr(), out.data_ptr(), rows.data_ptr() + 2 * first
+    g.M, g.N, g.K, g.lda, g.ldw, g.ldo, g.ldr = M, N, K, K, K, N, N
+    g.dtype, g.batch, g.r_batch_stride, g.schedule = _lib.HB_FP16, batch, stride, _lib.GEMM_SCHEDULES[schedule]
+    g.stream = torch.cuda.current_stream().cuda_stream
+    _lib.check(_lib.load().hb_gemm_epilogue(g))
+    assert ops.status_word() == 0
+    for b in range(batch):
+        at = first + b * (stride if batch > 1 else 0)
+        ref = a[b].float() @ w[b].float().t() + rows[at:at + M * N].reshape(M, N).float()
+        _close(out[b], ref.cpu(), tol=2e-3)  # fp32 sums, rounded once to fp16
