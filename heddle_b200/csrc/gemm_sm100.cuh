@@ -854,8 +854,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) gem
         }
         __syncwarp();
       }
-      if (!mbar_wait_warp(&s.acc_full[acc], (tile_i >> 1) & 1, ctx, kGemmRoleEpi)) break;
-      if (Residual && !mbar_wait_warp(&s.res_full[part], tile_i & 1, ctx, kGemmRoleEpi)) break;
+      bool ok = mbar_wait_warp(&s.acc_full[acc], (tile_i >> 1) & 1, ctx, kGemmRoleEpi);
+      // also where the first wait gave up: the CTA may not leave while its copy is on the way
+      if constexpr (Residual) ok = mbar_wait_warp(&s.res_full[part], tile_i & 1, ctx, kGemmRoleEpi) && ok;
+      if (!ok) break;
       tc_fence_after();
       gemm_epilogue_row<T, EPI, Residual>(p, tmem + lane_off + acc * kGemmBN, b, m0, n_t * p.tile_cols, quarter * 32 + lane, part,
                                           my_slabs, p.out_slabs, slab_cursor, mapa_u32(smem_u32(&s.acc_empty[acc]), 0));
