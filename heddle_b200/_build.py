@@ -13,6 +13,7 @@ import shutil
 import subprocess
 import sys
 import sysconfig
+import warnings
 from pathlib import Path
 
 PKG_DIR = Path(__file__).resolve().parent
@@ -41,13 +42,20 @@ def sources() -> list[Path]:
     return sorted(CSRC.glob("*.cu"))
 
 
+def _older(target: Path, deps: list[Path]) -> bool:
+    return not target.exists() or any(d.stat().st_mtime > target.stat().st_mtime for d in deps)
+
+
+def _header() -> Path:
+    return PKG_DIR.parent / "include" / "heddle_b200.h"
+
+
 def _stale() -> bool:
-    if not LIB_PATH.exists() or not NATIVE_PATH.exists():
-        return True
-    t = min(LIB_PATH.stat().st_mtime, NATIVE_PATH.stat().st_mtime)
-    deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + [NATIVE_SRC]
-    deps.append(PKG_DIR.parent / "include" / "heddle_b200.h")
-    return any(d.stat().st_mtime > t for d in deps)
+    return _older(LIB_PATH, [*CSRC.glob("*.cu"), *CSRC.glob("*.cuh"), *CSRC.glob("*.h"), _header()])
+
+
+def _native_stale() -> bool:
+    return _older(NATIVE_PATH, [NATIVE_SRC, _header()])
 
 
 def _compile_one(src: Path) -> tuple[Path, str]:
@@ -59,7 +67,7 @@ def _compile_one(src: Path) -> tuple[Path, str]:
     return obj, proc.stderr
 
 
-def _build_native() -> None:
+def _compile_native() -> None:
     """``_native.so``: PyTorch's libraries are the ones that ``import torch`` has loaded."""
     import torch
 
@@ -75,14 +83,23 @@ def _build_native() -> None:
         raise RuntimeError(f"g++ failed for {NATIVE_SRC.name}:\n{proc.stdout}\n{proc.stderr}")
 
 
+def _build_native() -> None:
+    """Without it (no g++, no headers of Python or PyTorch) the tensor-level calls do in Python what it does, at more host time."""
+    NATIVE_PATH.unlink(missing_ok=True)  # one built from other sources may not stay behind
+    try:
+        _compile_native()
+    except Exception as e:
+        warnings.warn(f"heddle_b200._native was not built, its host path stays in Python: {e}", RuntimeWarning, stacklevel=2)
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
+    if force or _native_stale():
+        _build_native()
     if not force and not _stale():
         return LIB_PATH
     OBJ_DIR.mkdir(parents=True, exist_ok=True)
     with concurrent.futures.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as pool:
-        native = pool.submit(_build_native)
         results = list(pool.map(_compile_one, sources()))
-        native.result()
     log = "".join(text for _, text in results)
     (OBJ_DIR / "ptxas.log").write_text(log)
     if verbose:

@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import warnings
 from pathlib import Path
 
 _PKG_DIR = Path(__file__).resolve().parent
@@ -154,12 +155,17 @@ native = None  # heddle_b200._native, bound to the library, once load() has run
 
 
 def _load_native(lib: C.CDLL) -> None:
-    """The host path of the tensor-level calls (csrc/ops_native.cpp), calling into ``lib``."""
+    """The host path of the tensor-level calls (csrc/ops_native.cpp), calling into ``lib``.  It saves host time only: without it
+    ops.py does the same in Python."""
     global native
     try:
+        import torch  # noqa: F401  (its libraries are those the module needs)
+
         from . import _native
     except ImportError as e:
-        raise RuntimeError(f"heddle_b200._native cannot be loaded ({e}): build it with `python -m heddle_b200._build`") from e
+        warnings.warn(f"heddle_b200._native cannot be loaded, calls take the host path in Python: {e} "
+                      "(`python -m heddle_b200._build` builds it)", RuntimeWarning, stacklevel=3)
+        return
     addresses = {name: C.cast(getattr(lib, name), C.c_void_p).value for name in EXPORTS}
     _native.bind(addresses, check, EW_OPS, EW_SRCS)
     native = _native
