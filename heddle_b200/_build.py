@@ -1,5 +1,5 @@
-"""Build the C-ABI shared library ``libheddle_b200.so`` in-tree with nvcc for sm_100a, and ``_native.so``, the host path of the
-tensor-level calls (csrc/ops_native.cpp), with g++ against PyTorch's headers.
+"""Build the C-ABI shared library ``libheddle_b200.so`` in-tree with nvcc for sm_100a, and ``_native-*.so``, the host path
+of the tensor-level calls (csrc/ops_native.cpp), with g++ against PyTorch's headers.
 
 nvcc cross-compiles without a GPU, so this runs on a CPU-only host as well.
 ``python -m heddle_b200._build`` rebuilds; ``build(force=False)`` rebuilds only
@@ -21,7 +21,6 @@ CSRC = PKG_DIR / "csrc"
 OBJ_DIR = CSRC / "build"
 LIB_PATH = PKG_DIR / "libheddle_b200.so"
 NATIVE_SRC = CSRC / "ops_native.cpp"
-NATIVE_PATH = PKG_DIR / "_native.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -46,6 +45,14 @@ def _older(target: Path, deps: list[Path]) -> bool:
     return not target.exists() or any(d.stat().st_mtime > target.stat().st_mtime for d in deps)
 
 
+def native_path() -> Path:
+    """Where the native module for the running PyTorch and Python is: it is compiled against the headers of both, so that one built for
+    others is neither fresh nor loaded."""
+    import torch
+
+    return PKG_DIR / f"_native-{torch.__version__}{sysconfig.get_config_var('EXT_SUFFIX')}"
+
+
 def _header() -> Path:
     return PKG_DIR.parent / "include" / "heddle_b200.h"
 
@@ -55,7 +62,7 @@ def _stale() -> bool:
 
 
 def _native_stale() -> bool:
-    return _older(NATIVE_PATH, [NATIVE_SRC, _header()])
+    return _older(native_path(), [NATIVE_SRC, _header()])
 
 
 def _compile_one(src: Path) -> tuple[Path, str]:
@@ -68,7 +75,7 @@ def _compile_one(src: Path) -> tuple[Path, str]:
 
 
 def _compile_native() -> None:
-    """``_native.so``: PyTorch's libraries are the ones that ``import torch`` has loaded."""
+    """PyTorch's libraries are the ones that ``import torch`` has loaded."""
     import torch
 
     torch_dir = Path(torch.__file__).resolve().parent
@@ -76,7 +83,7 @@ def _compile_native() -> None:
     cuda_include = Path(_nvcc()).resolve().parent.parent / "include"
     includes = [torch_dir / "include", torch_dir / "include/torch/csrc/api/include", cuda_include, sysconfig.get_paths()["include"]]
     cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-           *[f for d in includes for f in ("-isystem", str(d))], str(NATIVE_SRC), "-o", str(NATIVE_PATH),
+           *[f for d in includes for f in ("-isystem", str(d))], str(NATIVE_SRC), "-o", str(native_path()),
            f"-L{torch_dir / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
     proc = subprocess.run(cmd, capture_output=True, text=True)
     if proc.returncode != 0:
@@ -85,8 +92,8 @@ def _compile_native() -> None:
 
 def _build_native() -> None:
     """Without it (no g++, no headers of Python or PyTorch) the tensor-level calls do in Python what it does, at more host time."""
-    NATIVE_PATH.unlink(missing_ok=True)  # one built from other sources may not stay behind
     try:
+        native_path().unlink(missing_ok=True)  # one built from other sources may not stay behind
         _compile_native()
     except Exception as e:
         warnings.warn(f"heddle_b200._native was not built, its host path stays in Python: {e}", RuntimeWarning, stacklevel=2)

@@ -6,9 +6,14 @@ There is deliberately no fallback: if the library is missing or a call fails, a
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
+import sys
 import warnings
 from pathlib import Path
+
+from . import _build
 
 _PKG_DIR = Path(__file__).resolve().parent
 LIB_PATH = _PKG_DIR / "libheddle_b200.so"
@@ -154,14 +159,28 @@ _lib = None
 native = None  # heddle_b200._native, bound to the library, once load() has run
 
 
+def _import_native():
+    """heddle_b200._native as built for the running PyTorch and Python; ImportError where there is none."""
+    import torch  # noqa: F401  (its libraries are those the module needs)
+
+    name = f"{__package__}._native"
+    if name not in sys.modules:
+        path = _build.native_path()
+        spec = importlib.util.spec_from_file_location(name, path, loader=importlib.machinery.ExtensionFileLoader(name, str(path)))
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        sys.modules[name] = module
+    if sys.modules[name] is None:
+        raise ImportError(f"import of {name} halted; None in sys.modules")
+    return sys.modules[name]
+
+
 def _load_native(lib: C.CDLL) -> None:
     """The host path of the tensor-level calls (csrc/ops_native.cpp), calling into ``lib``.  It saves host time only: without it
     ops.py does the same in Python."""
     global native
     try:
-        import torch  # noqa: F401  (its libraries are those the module needs)
-
-        from . import _native
+        _native = _import_native()
     except ImportError as e:
         warnings.warn(f"heddle_b200._native cannot be loaded, calls take the host path in Python: {e} "
                       "(`python -m heddle_b200._build` builds it)", RuntimeWarning, stacklevel=3)

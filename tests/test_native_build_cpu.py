@@ -30,7 +30,7 @@ def test_build_goes_on_without_a_compiler(monkeypatch, tmp_path):
 
     left = tmp_path / "native.so"
     left.write_text("built from other sources")
-    monkeypatch.setattr(_build, "NATIVE_PATH", left)
+    monkeypatch.setattr(_build, "native_path", lambda: left)
 
     def no_compiler():
         raise FileNotFoundError("g++")
@@ -39,3 +39,27 @@ def test_build_goes_on_without_a_compiler(monkeypatch, tmp_path):
     with pytest.warns(RuntimeWarning, match="stays in Python"):
         _build._build_native()
     assert not left.exists() and _build._native_stale()
+
+
+def test_module_of_another_pytorch_is_neither_fresh_nor_loaded(built_lib, monkeypatch):
+    import torch
+
+    from heddle_b200 import _build
+
+    assert not _build._native_stale()
+    monkeypatch.setattr(torch, "__version__", "2.99.0")
+    assert _build._native_stale()
+    err = _python("import torch; torch.__version__ = '2.99.0'\n"
+                  "from heddle_b200 import _lib\n"
+                  "assert _lib.load().hb_version() == 100 and _lib.native is None")
+    assert "host path" in err
+
+
+def test_module_of_another_python_is_neither_fresh_nor_loaded(built_lib, monkeypatch):
+    import sysconfig
+
+    from heddle_b200 import _build
+
+    here = _build.native_path()
+    monkeypatch.setitem(sysconfig.get_config_vars(), "EXT_SUFFIX", ".cpython-399-x86_64-linux-gnu.so")
+    assert _build.native_path() != here and _build._native_stale()
