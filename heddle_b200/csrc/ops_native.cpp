@@ -589,29 +589,36 @@ PyObject* rowwise_program(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (x0 == nullptr || x0->dim() < 1 || dtype16(*x0) < 0) return general();
   const int64_t cols = x0->size(-1), rows = x0->numel() / cols;
   if (!fits_int(cols)) return general();
+  c10::SmallVector<at::Tensor, 8> keep;  // a list may lose its tensors to another thread while the lock is released
   for (Py_ssize_t i = 0; i < n_in; ++i) {
     const at::Tensor* t = plain(in[i], dev);
     if (t == nullptr || t->sizes() != x0->sizes() || t->scalar_type() != x0->scalar_type()) return general();
     a.ld_in[i] = row_stride(*t, cols, rows);
     if (a.ld_in[i] < 0) return general();
     a.inputs[i] = t->data_ptr();
+    keep.push_back(*t);
   }
   for (Py_ssize_t i = 0; i < n_vec; ++i) {
     const at::Tensor* t = plain(vec[i], dev);
     if (t == nullptr || t->scalar_type() != x0->scalar_type() || !t->is_contiguous() || t->numel() != cols) return general();
     a.rowvec[i] = t->data_ptr();
+    keep.push_back(*t);
   }
   for (Py_ssize_t i = 0; i < n_sca; ++i) {
     const at::Tensor* t = plain(sca[i], dev);
     if (t == nullptr || !contiguous_fp32(*t, rows)) return general();
     a.rowscalar[i] = static_cast<float*>(t->data_ptr());
+    keep.push_back(*t);
   }
   for (Py_ssize_t i = 0; i < n_inst; ++i) {
     PyObject** f;
     Py_ssize_t count;
     int64_t index;
     double imm;
-    if (!items(inst[i], f, count) || count != 4 || !integer(f[2], index) || !fits_int(index) || !number(f[3], imm)) return general();
+    // numbers proper: another object's __float__ may change the lists that are being read
+    if (!items(inst[i], f, count) || count != 4 || !integer(f[2], index) || !fits_int(index) || !(PyFloat_Check(f[3]) || PyLong_CheckExact(f[3])) ||
+        !number(f[3], imm))
+      return general();
     const int64_t op = named(g_ew_ops, f[0]), src = f[1] == Py_None ? 0 : named(g_ew_srcs, f[1]);  // EW_SRCS["none"] is 0
     if (op < 0 || src < 0) return general();
     a.program[i].op = static_cast<int32_t>(op);

@@ -220,3 +220,23 @@ def test_tensors_state(built_lib):
     assert state((t, u)) != a
     with torch.inference_mode():
         assert isinstance(state((torch.zeros(3),)), bytes)
+
+
+def test_rowwise_reads_no_list_that_an_operand_may_change(built_lib):
+    """An immediate's __float__ is other people's code: it is left to the general path, which holds what it reads."""
+    from heddle_b200 import _lib, ops
+
+    x = R(8, 64)
+    program = [("load", "input", 0, 0.0), ("mul", "imm", 0, 0.5), ("store_out", None, 0, 0.0)]
+    ref = ops.rowwise_program(program, [x])
+
+    class Half:
+        asked = 0
+
+        def __float__(self):
+            Half.asked += 1
+            return 0.5
+
+    odd = [program[0], ("mul", "imm", 0, Half()), program[2]]
+    assert _lib.native.rowwise_program(odd, [x], (), (), 1, _lib.ROWWISE_AUTO) is NotImplemented and Half.asked == 0
+    assert torch.equal(ops.rowwise_program(odd, [x]), ref)
