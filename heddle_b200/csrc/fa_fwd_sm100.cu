@@ -50,16 +50,22 @@ static int launch_fa(const FaParams& p, int grid, int smem_optin, cudaStream_t s
                               : launch_fa_form<T, D, false>(p, grid, smem_optin, stream);
 }
 
-template <typename T, int D, int NS>
-static int launch_fa_stages(const FaParams& p, int grid, int smem_optin, cudaStream_t stream) {
+template <typename T, int D, int NS, bool Long>
+static int launch_fa_stages_form(const FaParams& p, int grid, int smem_optin, cudaStream_t stream) {
   using Smem = FaSmem<T, D, NS>;
   if ((int)sizeof(Smem) > smem_optin) return set_error(HB_ERR_UNSUPPORTED, "hb_debug_fa_fwd_stages: not enough shared memory");
-  auto kernel = fa_fwd_kernel<T, D, NS, false>;
+  auto kernel = fa_fwd_kernel<T, D, NS, Long>;
   // set on every call: this is a diagnostic path, not worth a per-device table
   HB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
   HB_CUDA_CHECK(launch_dependent_if(launch_early(tile_order_steps(p.order, p.causal != 0, p.nkv)), kernel, grid, kFaThreads,
                                     sizeof(Smem), stream, 0, p));
   return HB_OK;
+}
+// The form that hb_fa_fwd takes; at its own depth the other one.
+template <typename T, int D, int NS>
+static int launch_fa_stages(const FaParams& p, int grid, int smem_optin, cudaStream_t stream) {
+  return (p.nkv >= kFaLongFrom) != (NS == FaConfig<T, D>::kStages) ? launch_fa_stages_form<T, D, NS, true>(p, grid, smem_optin, stream)
+                                                        : launch_fa_stages_form<T, D, NS, false>(p, grid, smem_optin, stream);
 }
 
 static int dispatch_fa(const hb_fa_args* a, const FaParams& p, int grid, int smem_optin) {

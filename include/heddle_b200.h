@@ -479,7 +479,8 @@ int hb_debug_umma(int mode, const void* a, const void* b, float* out, int32_t kn
 /*
  * hb_fa_fwd with the K/V ring of the kernel built `stages` deep (2, 3 or 5; bf16, head_dim 128).
  * The depth only changes when tiles are loaded, so O and LSE must be bit-identical to hb_fa_fwd's
- * (which uses 5): a mismatch means a race in the barrier protocol.  The reference plans the same
+ * (which uses 5): a mismatch means a race in the barrier protocol.  With 2 and 3 the kernel has the form that hb_fa_fwd takes for the
+ * call (one for few, one for many key tiles), with 5 the other form, whose results are the same too.  The reference plans the same
  * stand-in for a race detector ("bitwise comparison between a 1-stage and an N-stage pipeline
  * build"); it has no counterpart there.
  */

@@ -119,8 +119,10 @@ def test_config4_every_head(ops):
 
 
 @pytest.mark.parametrize("B,Hq,Hkv,Sq,Skv,causal", [(2, 8, 8, 4096, 4096, True), (1, 8, 2, 1000, 3000, True),
-                                                    (2, 4, 4, 2048, 2048, False)])
+                                                    (2, 4, 4, 2048, 2048, False), (3, 8, 2, 700, 1407, True),
+                                                    (3, 8, 2, 700, 1409, False)])
 def test_results_do_not_depend_on_the_pipeline_depth(ops, B, Hq, Hkv, Sq, Skv, causal):
+    """Depths 2 and 3 of the form that the call takes (another one from twelve key tiles, 1409 keys, on), and at depth 5 the other form."""
     q, k, v = (t.cuda() for t in O.make_qkv(B, Hq, Hkv, Sq, Skv, 128, seed=Sq + Skv, dtype=torch.bfloat16))
     out, lse = ops.fa_fwd(q, k, v, causal=causal, return_lse=True)
     for stages in (2, 3, 5):
