@@ -67,13 +67,42 @@ def test_fp8_rejects_other_head_dims(ops):
         ops.fa_fwd(x, x, x)
 
 
-@pytest.mark.parametrize("Skv", [1, 63, 64, 65, 128, 192, 193])
-def test_fp8_halves_of_a_key_tile(ops, Skv):
-    """P reaches the MMA in two halves of 64 keys: tiles that end in, at and behind either half, against the same oracle and bounds."""
-    (qq, kq, vq), scales, (qd, kd, vd) = _quantised(2, 2, 1, 300, Skv, 128, seed=Skv)
-    out = ops.fa_fwd(qq.cuda(), kq.cuda(), vq.cuda(), causal=False, scales=scales)
+@pytest.mark.parametrize("tiles", [0, 11])
+@pytest.mark.parametrize("last", [1, 63, 64, 65, 128, 192, 193])
+@pytest.mark.parametrize("Sq,causal", [(300, False), (300, True), (130, False)])
+def test_fp8_halves_of_a_key_tile(ops, Sq, causal, last, tiles):
+    """From twelve key tiles on P reaches the MMA in two halves of 64 keys: tiles that end in, at and behind either half, without and with a
+    mask (whose last steps the two row tiles of a block take apart), a second row tile of a few rows, against the same oracle and bounds.
+    Below, in one piece."""
+    Skv = tiles * 128 + last
+    if causal and Skv < Sq:
+        Sq = Skv
+    (qq, kq, vq), scales, (qd, kd, vd) = _quantised(2, 2, 1, Sq, Skv, 128, seed=Skv)
+    out, lse = ops.fa_fwd(qq.cuda(), kq.cuda(), vq.cuda(), causal=causal, return_lse=True, scales=scales)
     torch.cuda.synchronize()
     assert ops.status_word() == 0
-    ref, _ = O.attention_eager(qd, kd, vd, causal=False)
-    # one key: O = V, exact but for the rounding to bf16; else P in e4m3, 2^-4 relative per weight
-    assert (out.float().cpu() - ref).abs().max().item() <= (6e-2 if Skv > 1 else 2.0**-8 * vd.abs().max().item())
+    ref, ref_lse = O.attention_eager(qd, kd, vd, causal=causal)
+    err = (out.float().cpu() - ref).abs()
+    if not causal:  # one key: O = V, exact but for the rounding to bf16; else P in e4m3, 2^-4 relative per weight
+        assert err.max().item() <= (6e-2 if Skv > 1 else 2.0**-8 * vd.abs().max().item())
+    # Row by row, since rows under a mask see few keys and nothing averages out: 2^-4 of every weight (e4m3 has three bits behind the
+    # point), below its normal range half of 2^-9 / 32 each (weights are stored times 32, the largest is at least 1, and so is
+    # their sum), and the rounding of O to bf16
+    g = qd.shape[1] // kd.shape[1]
+    kk, vv = kd.repeat_interleave(g, 1), vd.repeat_interleave(g, 1).abs()
+    s = qd @ kk.transpose(-1, -2) / 128**0.5
+    seen = torch.ones(Sq, Skv, dtype=torch.bool).tril(Skv - Sq) if causal else torch.ones(Sq, Skv, dtype=torch.bool)
+    weights = torch.softmax(s.masked_fill(~seen, float("-inf")), -1)
+    bound = 2.0**-4 * (weights @ vv) + 2.0**-15 * (seen.float() @ vv) + 2.0**-8 * ref.abs() + 1e-6
+    assert bool((err <= bound).all()), (err / bound).max().item()
+    assert (lse.cpu() - ref_lse).abs().max().item() <= 1e-3
+
+
+def test_fp8_square_mask_of_several_blocks(ops):
+    (qq, kq, vq), scales, (qd, kd, vd) = _quantised(1, 3, 1, 1601, 1601, 128, seed=1601)
+    out, lse = ops.fa_fwd(qq.cuda(), kq.cuda(), vq.cuda(), causal=True, return_lse=True, scales=scales)
+    torch.cuda.synchronize()
+    assert ops.status_word() == 0
+    ref, ref_lse = O.attention_eager(qd, kd, vd, causal=True)
+    assert (out.float().cpu() - ref).abs().max().item() <= 6e-2
+    assert (lse.cpu() - ref_lse).abs().max().item() <= 1e-3

@@ -346,11 +346,11 @@ def test_full_size_projection_by_size_independent_properties(ops):
     assert torch.equal(twice, out * 2)
 
 
-@pytest.mark.parametrize("M,N,K", [(129, 136, 64), (300, 520, 200), (513, 264, 1000), (1500, 3080, 72), (9000, 512, 136)])
+@pytest.mark.parametrize("M,N,K", [(129, 136, 64), (300, 520, 200), (513, 264, 1000), (1500, 3080, 72), (9000, 512, 136), (9000, 2056, 136)])
 @pytest.mark.parametrize("form", ["dense", "wide rows", "in place"])
 def test_residual(ops, M, N, K, form):
-    """A residual that is read tile by tile beside the products: tails in every dimension, several tiles a CTA, rows of a wider tensor with
-    NaN around them, and the result written over it."""
+    """A residual that is read tile by tile beside the products: tails in every dimension, up to five tiles a CTA (9000 x 2056: 324 tiles of
+    256 x 256 for 74 pairs), rows of a wider tensor with NaN around them, and the result written over it."""
     dt = torch.float16
     a, w = _mk(M, N, K, seed=M + N, dtype=dt)
     g = torch.Generator().manual_seed(K)
@@ -366,9 +366,20 @@ def test_residual(ops, M, N, K, form):
     _close(out, ref, tol=2e-3)  # fp32 sums, rounded once to fp16
 
 
-@pytest.mark.parametrize("schedule", ["single", "pair", "split"])
+@pytest.mark.parametrize("B,M,N,K", [(3, 300, 264, 72), (12, 1300, 1032, 136), (40, 130, 520, 64)])
+def test_residual_of_every_batch(ops, B, M, N, K):
+    """Batches of their own residuals, tails in both dimensions, up to five tiles a CTA."""
+    g = torch.Generator().manual_seed(M)
+    a, b = torch.randn(B, M, K, generator=g).half(), (torch.randn(B, K, N, generator=g) * 0.1).half()
+    res = torch.randn(B, M, N, generator=g).half()
+    out = ops.bmm(a.cuda(), b.cuda(), "relu", residual=res.cuda())
+    torch.cuda.synchronize()
+    assert ops.status_word() == 0
+    _close(out, (a.float() @ b.float()).clamp(min=0) + res.float(), tol=2e-3)  # fp32 sums, rounded once to fp16
+
+
 @pytest.mark.parametrize("batch,stride", [(1, 4), (1, -136 * 264), (3, -300 * 264), (3, 8)])
-def test_residual_batch_strides(ops, schedule, batch, stride):
+def test_residual_batch_strides(ops, batch, stride):
     """r_batch_stride of the C ABI: not looked at with one batch; else any multiple of 8 elements whose rows exist, backward and overlapping
     ones too."""
     from heddle_b200 import _lib
@@ -383,7 +394,7 @@ def test_residual_batch_strides(ops, schedule, batch, stride):
     g = _lib.GemmArgs()
     g.a, g.w, g.out, g.residual = a.data_ptr(), w.data_ptr(), out.data_ptr(), rows.data_ptr() + 2 * first
     g.M, g.N, g.K, g.lda, g.ldw, g.ldo, g.ldr = M, N, K, K, K, N, N
-    g.dtype, g.batch, g.r_batch_stride, g.schedule = _lib.HB_FP16, batch, stride, _lib.GEMM_SCHEDULES[schedule]
+    g.dtype, g.batch, g.r_batch_stride, g.schedule = _lib.HB_FP16, batch, stride, _lib.GEMM_SCHEDULES[ops._gemm_schedule]
     g.stream = torch.cuda.current_stream().cuda_stream
     _lib.check(_lib.load().hb_gemm_epilogue(g))
     assert ops.status_word() == 0
