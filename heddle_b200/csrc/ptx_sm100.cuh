@@ -51,7 +51,9 @@ __device__ __forceinline__ int uniform_warp() { return static_cast<int>(warp_uni
 
 // Programmatic dependent launch (launch_dependent() in host_common.h): the next kernel of the stream may be scheduled from
 // grid_launch_dependents() on, and waits in grid_wait() until every earlier kernel is complete and its writes are visible.
-// No kernel touches global memory (its parameters aside) before grid_wait().  A kernel that holds TMEM calls
+// No kernel touches global memory (its parameters aside) before grid_wait(), but for those that hb_fa_bwd chains (BwdParams::chained): dK/dV
+// loads its inputs and dQ runs without a wait, since the preprocess kernel in front lets them in behind its own wait only, when
+// all that is earlier is complete, and dQ waits at its end, so that whoever waits for dQ has them all.  A kernel that holds TMEM calls
 // grid_launch_dependents() only after its own allocation: a dependent that took the columns first would wait for this grid,
 // and this grid for the columns.  Global memory is read by plain loads: what a kernel waits for is written during its own lifetime, which the
 // read-only path (__ldg, const __restrict__ parameters) does not allow; its loads may be moved in front of the wait.

@@ -327,7 +327,8 @@ int hb_fa_bwd_dkdv_workspace(const hb_fa_bwd_args* args, uint64_t* bytes);
 int hb_fa_bwd_dkdv_ws(const hb_fa_bwd_args* args, void* workspace, uint64_t bytes);
 int hb_fa_bwd_dq(const hb_fa_bwd_args* args);
 /* The whole backward pass: hb_fa_bwd_preprocess, hb_fa_bwd_dkdv_ws and hb_fa_bwd_dq, with the same results; the kernels overlap
- * where they leave SMs free, which separate calls cannot.  The workspace is hb_fa_bwd_dkdv_workspace's. */
+ * where they leave SMs free, which separate calls cannot: dQ is written while dK/dV still reads q, k, v, d_o, lse and delta.  So dq, dk, dv,
+ * delta and the workspace may overlap neither the inputs nor one another.  The workspace is hb_fa_bwd_dkdv_workspace's. */
 int hb_fa_bwd(const hb_fa_bwd_args* args, void* workspace, uint64_t bytes);
 
 /*
