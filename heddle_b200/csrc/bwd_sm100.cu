@@ -180,13 +180,6 @@ __device__ __forceinline__ void bwd_load_tile(void* dst, const CUtensorMap* tm, 
 
 // Four probabilities 2^(s * scale_log2 + nl) of one thread's row; with HB_BWD_POLY part of them on the FMA pipe.
 __device__ __forceinline__ void bwd_exp4(const uint32_t* sv, int e, uint64_t sc2, float4 l4, float* out) {
-#ifdef HB_BWD_KO_EXP  // measurement builds only: no exponentials (wrong results)
-  out[0] = __uint_as_float(sv[0]) + l4.x;
-  out[1] = __uint_as_float(sv[1]) + l4.y;
-  out[2] = __uint_as_float(sv[2]) + l4.z;
-  out[3] = __uint_as_float(sv[3]) + l4.w;
-  return;
-#endif
   const uint64_t x0 = fma_f32x2(pack_f32x2(__uint_as_float(sv[0]), __uint_as_float(sv[1])), sc2, pack_f32x2(l4.x, l4.y));
   const uint64_t x1 = fma_f32x2(pack_f32x2(__uint_as_float(sv[2]), __uint_as_float(sv[3])), sc2, pack_f32x2(l4.z, l4.w));
   float a0, a1, b0, b1;
