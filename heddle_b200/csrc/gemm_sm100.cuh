@@ -76,9 +76,9 @@ struct alignas(64) GemmParams {
   int out_slabs;      // ... and staging slabs per epilogue warpgroup (1, 2 or 4); stages + slabs = 7
 };
 // The pair kernel brings a plain product's residual by TMA, into the staging slabs that its results leave through (out_slabs = 2), while
-// the main loop runs.  Read by its threads, a row each (32 lines a load), it cost 14 us of 36: us without a residual | read by threads |
-// by TMA: 1203 x 4464 x 1552 21.5 | 35.9 | 24.1, 5094 x 864 x 1016 18.2 | 32.7 | 20.8, 16384 x 2048 x 128 - | 84.0 | 35.3, 2000 x 4096 x 4096
-// - | 66.3 | 59.7, 16384 x 4096 x 11008 - | 1175 | 1180 (its ring is five stages deep instead of six).
+// the main loop runs.  Read by its threads, a row each (32 lines a load), it cost 15 us of 37: us without a residual | read by threads |
+// by TMA: 1203 x 4464 x 1552 22.0 | 36.9 | 24.1, 5094 x 864 x 1016 18.4 | 33.3 | 20.6, 16384 x 2048 x 128 15.7 | 88.6 | 35.6, 2000 x 4096 x 4096
+// 55 | 65.7 | 59.2; 16384 x 4096 x 11008 1129 | 1150 | 1167, within what runs differ by (its ring is five stages deep instead of six).
 template <bool Residual>
 struct GemmPairParams : GemmParams {};
 template <>
@@ -109,28 +109,53 @@ __device__ __forceinline__ void gemm_tile_coords(const GemmParams& p, int t, int
   m_t = first_m + r - n_t * static_cast<int>(last ? p.div_last.d : p.div_rows.d);
 }
 
-// x / (1 + e^-v) with one ex2 and one rcp (1 ulp) of a number in [1, 2]: no call, no branch, nothing overflows or is flushed on the
-// way (e^-v for v < -88 would be, and 1 / (1 + e^-v) be 0 where the product is a normal number)
-__device__ __forceinline__ float times_sigmoid(float x, float v) {
-  const float t = __expf(-fabsf(v));
-  return x * fast_rcp(1.0f + t) * (v >= 0.0f ? 1.0f : t);
-}
-
+// Eight accumulators through an activation.  SiLU, sigmoid and the tanh form of GELU (0.5 (1 + tanh u) = sigmoid(2 u), which does not cancel
+// for u << 0) are x / (1 + 2^-a): one ex2 and one rcp each, the rest in pairs, no call, no branch.  The Newton step makes the reciprocal (1 ulp)
+// as good as the IEEE division's.  Far below zero, where 2^-a overflows or the quotient is flushed although the product is a normal
+// number, the result is x 2^a to the last bit.  rms error of the fp32 value in units of 2^-24, IEEE division | rcp alone | this: SiLU over
+// [-4, 0] 1.28 | 1.40 | 1.28, [-1, 1] 0.85 | 0.95 | 0.85, [0, 4] 0.77 | 0.80 | 0.77; tanh GELU, tanhf | this: [-4, 0] 1320 | 3.0, [-1, 1] 0.97 | 0.92,
+// [0, 4] 0.60 | 0.77.
 template <int ACT>
-__device__ __forceinline__ float apply_act(float v) {
-  if constexpr (ACT == kActSilu) return times_sigmoid(v, v);
-  if constexpr (ACT == kActRelu) return fmaxf(v, 0.0f);
-  // 0.5 (1 + tanh u) = sigmoid(2 u), which does not cancel for u << 0
-  if constexpr (ACT == kActGeluTanh) return times_sigmoid(v, 1.5957691216f * (v + 0.044715f * v * v * v));
-  if constexpr (ACT == kActSigmoid) return times_sigmoid(1.0f, v);
-  if constexpr (ACT == kActTanh) return tanhf(v);
-  return v;
+__device__ __forceinline__ void apply_act8(float (&v)[8]) {
+  if constexpr (ACT == kActSilu || ACT == kActGeluTanh || ACT == kActSigmoid) {
+    constexpr float kLog2e = 1.4426950409f, kGelu1 = 2.3022081981f, kGelu3 = 0.1029432396f;  // 2 log2(e) sqrt(2 / pi) (v + 0.044715 v^3)
+    const uint64_t one = pack_f32x2(1.0f, 1.0f), minus = pack_f32x2(-1.0f, -1.0f);
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) {
+      const uint64_t x = pack_f32x2(v[e], v[e + 1]);
+      uint64_t by = pack_f32x2(-kLog2e, -kLog2e);
+      if constexpr (ACT == kActGeluTanh) by = fma_f32x2(mul_f32x2(x, x), pack_f32x2(-kGelu3, -kGelu3), pack_f32x2(-kGelu1, -kGelu1));
+      float t0, t1, n0, n1;
+      unpack_f32x2(mul_f32x2(x, by), t0, t1);  // -a
+      const bool far0 = t0 > 92.0f, far1 = t1 > 92.0f;
+      if (far0) t0 = 32.0f - t0;  // 2^a in two steps: the exponential of less than -126 is flushed
+      if (far1) t1 = 32.0f - t1;
+      const float e0 = fast_exp2(t0), e1 = fast_exp2(t1);
+      const uint64_t n = fma_f32x2(pack_f32x2(e0, e1), minus, minus);  // -(1 + 2^-a)
+      unpack_f32x2(n, n0, n1);
+      const uint64_t r = pack_f32x2(fast_rcp(-n0), fast_rcp(-n1));
+      float y0, y1;
+      unpack_f32x2(fma_f32x2(r, fma_f32x2(n, r, one), r), y0, y1);
+      if (far0) y0 = e0 * 0x1p-32f;
+      if (far1) y1 = e1 * 0x1p-32f;
+      if constexpr (ACT == kActSigmoid) {
+        v[e] = y0;
+        v[e + 1] = y1;
+      } else {
+        unpack_f32x2(mul_f32x2(x, pack_f32x2(y0, y1)), v[e], v[e + 1]);
+      }
+    }
+  } else if constexpr (ACT != kActNone) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = ACT == kActRelu ? fmaxf(v[e], 0.0f) : tanhf(v[e]);
+  }
 }
 
 // f(std::integral_constant<int, ACT>) for the activation `act`.  A product chooses once per slab of 64 columns: a choice per element
 // put all five functions, and their branches, behind each of 128 unrolled elements.
-// us, 408 x 17024 x 3232: SiLU 117 -> 55, GELU 159 -> 56, none 52; 14368 x 14144 x 4480 + GELU 3180 -> 1506; 4000 x 8192 x 640:
-// SiLU 238 -> 56, GELU 324 -> 63, bias and row scale 56 -> 51.  The division went with it: 2722 x 3200 x 2640 + SwiGLU 46.5 -> 44.6.
+// us, that with an IEEE division or tanhf -> this, in turn on one GPU: 408 x 17024 x 3232 SiLU 121 -> 53, GELU 159 -> 54, none 49; 14368 x 14144 x
+// 4480 + GELU 2869 -> 1348, none 1280 to 1400; 4000 x 8192 x 640 SiLU 249 -> 56, GELU 326 -> 58, bias 55.3 -> 49; 2722 x 3200 x 2640 + SwiGLU 43.3 ->
+// 42.3.
 template <typename F>
 __device__ __forceinline__ void with_act(int act, F&& f) {
   if (act == kActNone) return f(std::integral_constant<int, kActNone>{});  // no jump table in the way of most products
@@ -283,31 +308,34 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
         return;
       }
       with_act(p.act, [&](auto act) {
+        float v[8][8];  // scale and bias of all first: 16384 x 2048 x 128 + SiLU 42.6 -> 40.4 us against group by group
 #pragma unroll
         for (int g = 0; g < 8; ++g) {
           const int col = col0 + g * 8;
           const uint32_t* a = g < 4 ? &x[g * 8] : &y[(g - 4) * 8];
-          float v[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(a[e]) * rs;
+          for (int e = 0; e < 8; ++e) v[g][e] = __uint_as_float(a[e]) * rs;
           if (p.bias != nullptr && col < p.N_out) {
             float bb[8];
             load_bias8<T>(p, col, bb);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] += bb[e];
+            for (int e = 0; e < 8; ++e) v[g][e] += bb[e];
           }
+        }
 #pragma unroll
-          for (int e = 0; e < 8; ++e) v[e] = apply_act<decltype(act)::value>(v[e]);
+        for (int g = 0; g < 8; ++g) {
+          apply_act8<decltype(act)::value>(v[g]);
+          const int col = col0 + g * 8;
           uint4* const chunk = reinterpret_cast<uint4*>(stage + row_in_tile * 128 + (g ^ (row_in_tile & 7)) * 16);
           if constexpr (ResInSlabs) {
             float res[8];
             unpack8<T>(*chunk, res);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] += res[e];
+            for (int e = 0; e < 8; ++e) v[g][e] += res[e];
           } else if (row_ok && col < p.N_out) {
-            add_residual8<T>(p, b, row, col, v);
+            add_residual8<T>(p, b, row, col, v[g]);
           }
-          *chunk = pack8<T>(v);
+          *chunk = pack8<T>(v[g]);
         }
       });
     };
@@ -373,8 +401,9 @@ __device__ __forceinline__ void gemm_epilogue_row(const GemmParams& p, uint32_t 
             u[e] += bu[e];
           }
         }
+        apply_act8<kActSilu>(v);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = apply_act<kActSilu>(v[e]) * u[e];
+        for (int e = 0; e < 8; ++e) v[e] *= u[e];
         store8<T>(p, b, row, col + g * 8, v);
       }
     }

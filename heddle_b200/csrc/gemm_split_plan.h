@@ -81,14 +81,17 @@ inline GemmWide gemm_wide(int sm_count, int M, int N, int batch) {
 // Beyond these rounds the persistent kernel has always been the faster one, and nothing is estimated.
 inline bool gemm_split_eligible(const GemmWide& w) { return w.tiles < (w.one_row ? 8ll : 2ll) * w.slots; }
 
-// Both estimates are compared with 300 products drawn over 1 .. 3000 rows, 64 .. 30000 columns, K 64 .. 12000 and batches of 1
-// to 128, both sides measured: half of either side's estimates lie between 0.87 and 1.1 of the measured time, the rest between
-// 0.6 and 1.45 (a persistent kernel with an activation epilogue can take four times its estimate; split-K wins there anyway).
-// On 260 other draws the rule takes split-K where it is the slower one by more than 5 % in six, 9 % at most (4.4 | 4.0 us).
-// us, split-K | the persistent kernel, taken where the first is smaller: 24 x 22016 x 4096 33 | 42; 120 x 4096 x 11008 25 | 67; 120 x 12288 x 4096
-// 30 | 40; 1 x 4096 x 4096 11 | 28; 64 x 50000 x 4096 75 | 83; 256 x 4096 x 4096 17 | 25; 512 x 4096 x 4096 23 | 26; 1000 x 4096 x
-// 4096 31 | 28; 256 x 22016 x 4096 61 | 56; batches of short products run several waves: 122 x (52 x 1056 x 88) 39 | 13; 62 x
-// (21 x 1320 x 248) 26 | 11; 35 x (62 x 1976 x 160) 14.7 | 8.3; 4 x (510 x 152 x 168) 4.2 | 5.8.
+// Both estimates were fitted to products without a residual: half of either side's lie between 0.87 and 1.1 of the measured time, the
+// rest between 0.6 and 1.45.  The 1.76 us a round for what is not plain is one figure for all epilogues.  Medians of 500 products, over
+// what is estimated without it: SiLU 4.2, tanh GELU 7.3, SwiGLU 0.5; a residual takes 1.4 and counts as plain, and the split-K kernel takes
+// 1.18 of its estimate with one.  That matters near the line only: of 260 draws over 1 .. 3000 rows, 64 .. 30000 columns, K 64 .. 12000,
+// with activations and residuals, the rule takes the slower kernel by more than 5 % in one; of 240 more whose estimates lie within 0.6 to 1.6
+// of each other, in 12 (179 x 14800 x 64 SiLU + residual split-K 17.1 | 9.6 us, 463 x 3808 x 512 + residual split-K 11.6 | 8.9, 254 x 11440 x
+// 2560 GELU 22.4 | 28.7 persistent).
+// us, split-K | the persistent kernel, taken where the first is smaller: 24 x 22016 x 4096 33 | 39; 120 x 4096 x 11008 25 | 66; 120 x 12288 x 4096
+// 27 | 42; 1 x 4096 x 4096 10 | 26; 64 x 50000 x 4096 75 | 88; 256 x 4096 x 4096 17 | 24; 512 x 4096 x 4096 23.6 | 24.3; 1000 x 4096 x
+// 4096 36 | 32; 256 x 22016 x 4096 60 | 58; 151 x 928 x 10768 SiLU 14.5 | 56; batches of short products run several waves: 122 x (52 x 1056 x
+// 88) 38 | 12; 62 x (21 x 1320 x 248) 26 | 11; 35 x (62 x 1976 x 160) 15 | 8.3; 4 x (510 x 152 x 168) 3.9 | 5.4.
 inline bool gemm_split_wins(const GemmSplitChoice& split, const GemmWide& w, int k_steps, bool plain, double bytes) {
   const double round = k_steps * (w.one_row ? 424.0 : 316.0) + (w.one_row ? 880.0 : 1280.0) + (plain ? 0.0 : 1760.0);
   const long long rounds = (w.tiles + w.slots - 1) / w.slots;

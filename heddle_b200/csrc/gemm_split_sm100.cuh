@@ -308,16 +308,14 @@ __global__ void __launch_bounds__(kGemmSplitThreads, 1) gemm_split_kernel(const 
       gemm_split_sum8(src, part_bytes, splits, v);
       gemm_split_scale_bias8<T>(p, rs, col, v);
       if constexpr (EPI == kEpiPlain) {
-        with_act(p.act, [&](auto act) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) v[e] = apply_act<decltype(act)::value>(v[e]);
-        });
+        with_act(p.act, [&](auto act) { apply_act8<decltype(act)::value>(v); });
       } else if constexpr (EPI == kEpiSwiglu) {
         float u[8];
         gemm_split_sum8(src + static_cast<uint32_t>(p.tile_cols) * 4u, part_bytes, splits, u);
         gemm_split_scale_bias8<T>(p, rs, p.w_row2_offset + col, u);
+        apply_act8<kActSilu>(v);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = apply_act<kActSilu>(v[e]) * u[e];
+        for (int e = 0; e < 8; ++e) v[e] *= u[e];
       } else {
         float x2[8];
         gemm_split_sum8(src + static_cast<uint32_t>(half) * 4u, part_bytes, splits, x2);

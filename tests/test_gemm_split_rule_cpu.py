@@ -8,16 +8,19 @@ ROOT = Path(__file__).resolve().parent.parent
 # epilogue (0 plain, 1 SwiGLU, 2 RoPE; -1 plain with an activation), batch, M, N, K, [K, N] operand, us split-K, us persistent
 MEASURED = [
     # one product: decode steps and short prompts, where tiles of 256 columns leave most SMs idle
-    (1, 1, 24, 22016, 4096, 0, 33, 42), (0, 1, 120, 4096, 11008, 0, 25, 67), (2, 1, 120, 12288, 4096, 0, 30, 40),
-    (0, 1, 1, 4096, 4096, 0, 11, 28), (0, 1, 64, 50000, 4096, 0, 75, 83), (0, 1, 256, 4096, 4096, 0, 17, 25),
-    (0, 1, 512, 4096, 4096, 0, 23, 26), (0, 1, 1000, 4096, 4096, 0, 31, 28), (1, 1, 256, 22016, 4096, 0, 61, 56),
-    (0, 1, 26, 25104, 1720, 0, 18.7, 28.9), (0, 1, 5, 23568, 840, 0, 10.7, 15.5), (0, 1, 548, 3584, 5624, 0, 34.9, 38.3),
-    (2, 1, 344, 1408, 328, 0, 8.7, 13.9), (-1, 1, 151, 928, 10768, 0, 17.9, 86.0), (1, 1, 1913, 2368, 6072, 0, 99.2, 83.1),
-    (1, 1, 2721, 1600, 4928, 0, 65.1, 54.3), (0, 1, 1581, 2896, 64, 0, 11.0, 5.8), (0, 1, 411, 11200, 208, 0, 13.7, 8.2),
+    (1, 1, 24, 22016, 4096, 0, 32.8, 38.7), (0, 1, 120, 4096, 11008, 0, 25.7, 65.5), (2, 1, 120, 12288, 4096, 0, 26.7, 42.1),
+    (0, 1, 1, 4096, 4096, 0, 9.9, 26.3), (0, 1, 64, 50000, 4096, 0, 75.2, 87.7), (0, 1, 256, 4096, 4096, 0, 16.7, 23.7),
+    (0, 1, 512, 4096, 4096, 0, 23.6, 24.3), (0, 1, 1000, 4096, 4096, 0, 36.1, 31.8), (1, 1, 256, 22016, 4096, 0, 60.1, 57.7),
+    (0, 1, 26, 25104, 1720, 0, 20.5, 26.4), (0, 1, 5, 23568, 840, 0, 11.2, 15.2), (0, 1, 548, 3584, 5624, 0, 37.4, 39.3),
+    (2, 1, 344, 1408, 328, 0, 8.2, 18.4), (-1, 1, 151, 928, 10768, 0, 14.5, 56.0), (1, 1, 1913, 2368, 6072, 0, 87.5, 77.2),
+    (1, 1, 2721, 1600, 4928, 0, 58.9, 52.6), (0, 1, 1581, 2896, 64, 0, 11.2, 5.6), (0, 1, 411, 11200, 208, 0, 14.2, 8.1),
+    # SiLU and tanh GELU with a few hundred rows
+    (-1, 1, 295, 2224, 1792, 0, 10.7, 17.6), (-1, 1, 598, 3088, 3136, 0, 18.7, 24.6), (-1, 1, 1014, 4352, 152, 0, 12.6, 11.2),
+    (-1, 1, 714, 7472, 7616, 0, 103.5, 89.2), (-1, 1, 225, 10336, 800, 0, 12.3, 17.3), (-1, 1, 389, 11920, 1080, 0, 32.6, 27.6),
     # batches of short products: several waves of CTAs, each with its own start
-    (0, 122, 52, 1056, 88, 0, 39.0, 12.9), (0, 62, 21, 1320, 248, 1, 26.3, 11.0), (0, 26, 442, 272, 376, 0, 15.9, 9.0),
-    (0, 35, 62, 1976, 160, 1, 14.7, 8.3), (0, 46, 96, 792, 160, 1, 13.7, 8.2), (0, 49, 180, 264, 120, 0, 10.8, 7.3),
-    (0, 82, 12, 336, 144, 0, 9.0, 6.6), (0, 4, 510, 152, 168, 0, 4.2, 5.8), (0, 2, 663, 112, 64, 0, 3.2, 4.0),
+    (0, 122, 52, 1056, 88, 0, 38.0, 12.4), (0, 62, 21, 1320, 248, 1, 26.3, 11.3), (0, 26, 442, 272, 376, 0, 16.1, 9.0),
+    (0, 35, 62, 1976, 160, 1, 15.0, 8.3), (0, 46, 96, 792, 160, 1, 14.0, 8.0), (0, 49, 180, 264, 120, 0, 10.8, 7.3),
+    (0, 82, 12, 336, 144, 0, 8.6, 6.2), (0, 4, 510, 152, 168, 0, 3.9, 5.4), (0, 2, 663, 112, 64, 0, 3.0, 3.8),
 ]
 
 PROGRAM = r'''
