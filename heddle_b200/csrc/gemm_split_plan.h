@@ -83,11 +83,11 @@ inline bool gemm_split_eligible(const GemmWide& w) { return w.tiles < (w.one_row
 
 // Both estimates were fitted to products without a residual: half of either side's lie between 0.87 and 1.1 of the measured time, the
 // rest between 0.6 and 1.45.  The 1.76 us a round for what is not plain is one figure for all epilogues.  Medians of 500 products, over
-// what is estimated without it: SiLU 4.2, tanh GELU 7.3, SwiGLU 0.5; a residual takes 1.4 and counts as plain, and the split-K kernel takes
-// 1.18 of its estimate with one.  That matters near the line only: of 260 draws over 1 .. 3000 rows, 64 .. 30000 columns, K 64 .. 12000,
+// what is estimated without it: SiLU 3.5, tanh GELU 4.9, SwiGLU 0.2; a residual takes 1.4 and counts as plain, and the split-K kernel takes
+// 1.2 of its estimate with one.  That matters near the line only: of 260 draws over 1 .. 3000 rows, 64 .. 30000 columns, K 64 .. 12000,
 // with activations and residuals, the rule takes the slower kernel by more than 5 % in one; of 240 more whose estimates lie within 0.6 to 1.6
-// of each other, in 12 (179 x 14800 x 64 SiLU + residual split-K 17.1 | 9.6 us, 463 x 3808 x 512 + residual split-K 11.6 | 8.9, 254 x 11440 x
-// 2560 GELU 22.4 | 28.7 persistent).
+// of each other, in 12 (179 x 14800 x 64 SiLU + residual split-K 16.3 | 9.0 us, 463 x 3808 x 512 + residual split-K 11.5 | 9.0, 273 x 7856 x 1984
+// GELU 17.7 | 20.4 persistent).
 // us, split-K | the persistent kernel, taken where the first is smaller: 24 x 22016 x 4096 33 | 39; 120 x 4096 x 11008 25 | 66; 120 x 12288 x 4096
 // 27 | 42; 1 x 4096 x 4096 10 | 26; 64 x 50000 x 4096 75 | 88; 256 x 4096 x 4096 17 | 24; 512 x 4096 x 4096 23.6 | 24.3; 1000 x 4096 x
 // 4096 36 | 32; 256 x 22016 x 4096 60 | 58; 151 x 928 x 10768 SiLU 14.5 | 56; batches of short products run several waves: 122 x (52 x 1056 x
