@@ -22,7 +22,7 @@ def ops(built_lib):
 
 class Chain:
     """Every kind of launch in one chain: statistic, row softmax, compiled rowwise programs (both forms), split-K and persistent
-    GEMMs, attention on split keys (with its merge), the general kernel, H2O score (a memset in front), the backward kernels (with
+    GEMMs, attention on split keys (with its merge), the general kernel, H2O score, the backward kernels (with
     the merge of grouped heads).  ``x``, ``y`` and ``a`` are written again while the call before may still read them."""
 
     def __init__(self, ops, seed):
@@ -144,8 +144,7 @@ def test_two_chains_on_two_streams(ops):
 
 
 def test_the_h2o_score_is_cleared_behind_its_last_reader(ops):
-    """hb_h2o_score clears the score and adds to it: with the same storage in every call, the memset and the kernel of one call must
-    stay between the reader of the call before and its own reader."""
+    """With the same storage in every call, the kernel of one call must stay between the reader of the call before and its own reader."""
     g = torch.Generator().manual_seed(7)
     qs, ks = ([torch.randn(1, 4, 300, 64, generator=g).to(torch.float16).cuda() for _ in range(4)] for _ in range(2))
     lse = [ops.fa_fwd(q, k, k, causal=True, return_lse=True)[1] for q, k in zip(qs, ks)]
