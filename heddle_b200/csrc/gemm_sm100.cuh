@@ -78,7 +78,7 @@ struct alignas(64) GemmParams {
 // The pair kernel brings a plain product's residual by TMA, into the staging slabs that its results leave through (out_slabs = 2), while
 // the main loop runs.  Read by its threads, a row each (32 lines a load), it cost 15 us of 37: us without a residual | read by threads |
 // by TMA: 1203 x 4464 x 1552 22.0 | 36.9 | 24.1, 5094 x 864 x 1016 18.4 | 33.3 | 20.6, 16384 x 2048 x 128 15.7 | 88.6 | 35.6, 2000 x 4096 x 4096
-// 55 | 65.7 | 59.2; 16384 x 4096 x 11008 1129 | 1150 | 1167, within what runs differ by (its ring is five stages deep instead of six).
+// 55 | 65.7 | 59.2, 16384 x 4096 x 11008 1119 | 1150 | 1144 (its ring is five stages deep instead of six).
 template <bool Residual>
 struct GemmPairParams : GemmParams {};
 template <>
