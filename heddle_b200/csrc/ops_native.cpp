@@ -20,6 +20,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <limits>
@@ -412,7 +413,8 @@ PyObject* gemm_epilogue(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const at::Tensor *cos = plain(PyTuple_GET_ITEM(args[6], 0), dev), *sin = plain(PyTuple_GET_ITEM(args[6], 1), dev);
     int64_t head_dim, rope_cols;
     if (cos == nullptr || sin == nullptr || cos->dim() < 1 || !integer(PyTuple_GET_ITEM(args[6], 2), head_dim) ||
-        !integer(PyTuple_GET_ITEM(args[6], 3), rope_cols) || !fits_int(head_dim) || !fits_int(rope_cols) || !cos->is_contiguous() || !sin->is_contiguous())
+        !integer(PyTuple_GET_ITEM(args[6], 3), rope_cols) || !fits_int(head_dim) || !fits_int(rope_cols) || !cos->is_contiguous() || !sin->is_contiguous() ||
+        std::min(cos->numel(), sin->numel()) < cos->size(0) * (head_dim / 2))
       return general();
     if (cos->scalar_type() == a->scalar_type() && sin->scalar_type() == a->scalar_type() && aligned16(*cos) && aligned16(*sin)) {
       g.dtype |= HB_GEMM_ROPE_TABLES_16;  // read as they are

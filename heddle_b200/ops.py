@@ -352,7 +352,7 @@ def gemm_epilogue(a: torch.Tensor, w: torch.Tensor, epilogue: str = "none", *,
         out_ptr, ldo = result.data_ptr(), n_out
     else:
         out2 = out.reshape(-1, n_out)
-        if out2.data_ptr() != out.data_ptr() or out2.stride(-1) != 1:
+        if out2.data_ptr() != out.data_ptr() or out2.stride(-1) != 1 or out2.shape[0] < M:
             raise ValueError("out must be viewable as a row-major [M, N_out] matrix")
         result, out_ptr, ldo = out, out2.data_ptr(), out2.stride(0)
     device = a.device
@@ -379,12 +379,16 @@ def gemm_epilogue(a: torch.Tensor, w: torch.Tensor, epilogue: str = "none", *,
             if r2.dtype != a.dtype or r2.stride(-1) != 1:
                 r2 = r2.to(a.dtype).contiguous()
             g.ldr = r2.stride(0)
+        if r2.numel() < M * n_out:
+            raise ValueError("residual must have one row per row of a")
         keep.append(r2)
         g.residual = r2.data_ptr()
     if epilogue == "rope":
         if rope is None:
             raise ValueError("epilogue 'rope' needs rope=(cos, sin, head_dim, rope_cols)")
         cos, sin, hd, rope_cols = rope
+        if min(cos.numel(), sin.numel()) < cos.shape[0] * (int(hd) // 2):
+            raise ValueError("the rope tables must have head_dim / 2 columns")
         if cos.dtype is a.dtype and sin.dtype is a.dtype and cos.is_contiguous() and sin.is_contiguous() \
                 and (cos.data_ptr() | sin.data_ptr()) % 16 == 0:
             g.dtype |= _lib.HB_GEMM_ROPE_TABLES_16  # read as they are: no conversion in front of every call
@@ -504,6 +508,8 @@ def rms_rowstat(x: torch.Tensor, residual: Optional[torch.Tensor] = None, eps: f
     r2 = None
     if residual is not None:
         r2 = residual.reshape(-1, N)
+        if r2.shape[0] < M:
+            raise ValueError("residual must have one row per row of x")
         if r2.stride() != x2.stride() or r2.dtype != x.dtype:
             r2 = r2.to(x.dtype).contiguous()
             x2 = x2.contiguous()
@@ -533,6 +539,8 @@ def prepare_weight(weights: "Sequence[torch.Tensor]", gamma: Optional[torch.Tens
     ws = [w if w.stride(1) == 1 else w.contiguous() for w in ws]
     if gamma is not None:
         gamma = gamma.to(dt).contiguous()
+        if gamma.numel() < K:
+            raise ValueError("prepare_weight: gamma must have K entries")
     out = torch.empty((sum(w.shape[0] for w in ws), K), dtype=dt, device=ws[0].device)
     a = _lib.PrepareArgs()
     for i, w in enumerate(ws):
