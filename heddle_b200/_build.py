@@ -62,7 +62,10 @@ def _stale() -> bool:
 
 
 def _native_stale() -> bool:
-    return _older(native_path(), [NATIVE_SRC, _header()])
+    try:
+        return _older(native_path(), [NATIVE_SRC, _header()])
+    except ImportError:  # no PyTorch: _build_native() says so, and the library is built all the same
+        return True
 
 
 def _compile_one(src: Path) -> tuple[Path, str]:

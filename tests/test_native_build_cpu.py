@@ -63,3 +63,14 @@ def test_module_of_another_python_is_neither_fresh_nor_loaded(built_lib, monkeyp
     here = _build.native_path()
     monkeypatch.setitem(sysconfig.get_config_vars(), "EXT_SUFFIX", ".cpython-399-x86_64-linux-gnu.so")
     assert _build.native_path() != here and _build._native_stale()
+
+
+def test_library_is_built_without_pytorch(built_lib, monkeypatch):
+    from heddle_b200 import _build
+
+    def no_torch():
+        raise ImportError("No module named 'torch'")
+
+    monkeypatch.setattr(_build, "native_path", no_torch)
+    with pytest.warns(RuntimeWarning, match="stays in Python"):
+        assert _build.build() == _build.LIB_PATH
